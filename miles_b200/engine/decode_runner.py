@@ -17,8 +17,11 @@ agreement of expert-parallel ranks and the skew between their hosts are then pai
 """
 from __future__ import annotations
 
+import gc
+import threading
 import time
 import zlib
+from contextlib import contextmanager
 
 import numpy as np
 import torch
@@ -26,6 +29,27 @@ import torch
 from ..models.qwen3 import ForwardMeta, RaggedBatch
 
 BUCKETS = [1, 2, 4, 8, 16, 24, 32, 48, 64, 96, 128, 192, 256, 384, 512, 768, 1024]
+
+
+_captures, _captures_lock = [0, False], threading.Lock()       # captures under way, whether the collector ran before the first of them
+
+
+@contextmanager
+def _collector_paused():
+    """No cyclic garbage collection while a graph is captured: the graphs of a dropped engine (runner and engine refer to each
+    other) would be destroyed in the middle of it, which CUDA refuses and which spoils the capture."""
+    with _captures_lock:
+        if _captures[0] == 0:
+            _captures[1] = gc.isenabled()
+            gc.disable()
+        _captures[0] += 1
+    try:
+        yield
+    finally:
+        with _captures_lock:
+            _captures[0] -= 1
+            if _captures[0] == 0 and _captures[1]:
+                gc.enable()
 
 
 class DecodeRunner:
@@ -369,7 +393,7 @@ class DecodeRunner:
         n0 = ops._k().launch_count()
         self._capturing_feed = len(key) > 2
         try:
-            with torch.cuda.graph(g, pool=self.pool):
+            with _collector_paused(), torch.cuda.graph(g, pool=self.pool):
                 self._forward(B, record)
         finally:
             self._capturing_feed = False

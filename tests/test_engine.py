@@ -501,3 +501,23 @@ def test_multi_rank_engine_server_matches_one_engine(tmp_path, mode, port):
         assert o["output_ids"] == w["output_ids"], (i, o["output_ids"], w["output_ids"])
         a, b = ([x[0] for x in r["meta_info"]["output_token_logprobs"]] for r in (o, w))
         assert max(abs(x - y) for x, y in zip(a, b)) < 1e-4
+
+
+def test_collector_is_paused_while_any_capture_runs():
+    import gc
+
+    from miles_b200.engine.decode_runner import _collector_paused
+
+    assert gc.isenabled()
+    with _collector_paused():
+        with _collector_paused():
+            assert not gc.isenabled()
+        assert not gc.isenabled()              # the outer capture is still under way
+    assert gc.isenabled()
+    gc.disable()
+    try:
+        with _collector_paused():
+            pass
+        assert not gc.isenabled()              # left as it was found
+    finally:
+        gc.enable()

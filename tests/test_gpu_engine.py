@@ -293,3 +293,31 @@ def test_precapture_fills_every_bucket_and_generation_is_unchanged(engine):
     after = engine.generate(prompts, [dict(sp)] * 3)
     assert [o["output_ids"] for o in after] == [o["output_ids"] for o in before]
     assert engine._free_blocks() == engine.allocator.num_blocks
+
+
+def test_capture_beside_a_dropped_engine():
+    """The graphs of an engine that was dropped (it and its runner refer to each other) wait for the cyclic collector; a collection in the
+    middle of another engine's capture must not happen, however eager the collector is."""
+    import gc
+
+    from miles_b200.engine.engine import Engine
+    from miles_b200.models.config import ModelConfig
+
+    cfg = ModelConfig(name="capture", vocab_size=512, hidden_size=256, num_layers=2, num_heads=4, num_kv_heads=2, head_dim=64, ffn_hidden_size=512)
+    kw = dict(device="cuda", dtype=torch.bfloat16, max_running_requests=4, max_context_len=128, num_blocks=16, seed=0)
+    new = {"temperature": 0.0, "max_new_tokens": 4}
+    thresholds = gc.get_threshold()
+    gc.collect()
+    gc.disable()
+    first = Engine(cfg, **kw)
+    want = first.generate([[5, 6, 7]], new)[0]["meta_info"]["output_token_logprobs"]
+    assert first.runner.graphs
+    second = Engine(cfg, **kw)
+    del first
+    gc.enable()
+    gc.set_threshold(1, 1, 1)
+    try:
+        got = second.generate([[5, 6, 7]], new)[0]["meta_info"]["output_token_logprobs"]
+    finally:
+        gc.set_threshold(*thresholds)
+    assert second.runner.graphs and got == want
