@@ -14,9 +14,11 @@
 //     selects which expert's weight block B uses (−1 = unused tile).
 //   grouped wgrad: one output [N',K'] per expert, reduction over that expert's row segment.
 // Every mbarrier wait is bounded; on timeout the kernel raises `*error_flag`, drains and frees TMEM, and returns.
-#include "ptx.cuh"
+#include "gemm_epilogue.cuh"
+#include "gemm_pair.cuh"
 #include "launch.h"
 #include "pdl.cuh"
+#include "ptx.cuh"
 
 namespace mb {
 
@@ -318,89 +320,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
         continue;
       }
-      // Coalesced path: the accumulator arrives one row per thread, but whole 128-byte lines are what the memory system
-      // wants.  Each warp turns 128 bytes of output per row at a time (64 bf16 or 32 fp32 columns) through its staging tile
-      // (16-byte units, XOR-swizzled against bank conflicts): written row-per-lane, read back with 8 lanes covering one
-      // row, so every store instruction writes four full lines.  Needs 16-byte aligned rows; otherwise the plain path below.
+      // Coalesced path: needs 16-byte aligned rows; otherwise the plain path below.
       const int esz = p.out_fp32 ? 4 : 2;
-      const int cols_per_round = 128 / esz;
       if ((((p.ldc * esz) | (p.group_stride_c * esz) | static_cast<long long>(reinterpret_cast<uintptr_t>(p.C))) & 15) == 0 &&
           (p.N * esz) % 16 == 0) {
         const int row0 = m_blk * BM + q * 32;
-        uint8_t* stage = smem_stage + q * 4096;
-        uint8_t* c_tile = reinterpret_cast<uint8_t*>(p.C) +
-                          (static_cast<long long>(group) * p.group_stride_c + static_cast<long long>(row0) * p.ldc) * esz;
-#pragma unroll 1
-        for (int c2 = 0; c2 < BN / cols_per_round; ++c2) {
-          const int colr = n_blk * BN + c2 * cols_per_round;
-          if (colr >= p.N) break;                                  // uniform over the warp
-          if (p.out_fp32) {
-            uint32_t r[32];
-            tmem_ld_32x32(t_row + c2 * 32, r);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              float4 o;
-              o.x = (k_blocks == 0) ? 0.f : __uint_as_float(r[4 * i]);
-              o.y = (k_blocks == 0) ? 0.f : __uint_as_float(r[4 * i + 1]);
-              o.z = (k_blocks == 0) ? 0.f : __uint_as_float(r[4 * i + 2]);
-              o.w = (k_blocks == 0) ? 0.f : __uint_as_float(r[4 * i + 3]);
-              *reinterpret_cast<float4*>(stage + lane * 128 + ((i ^ (lane & 7)) << 4)) = o;
-            }
-          } else {
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-              uint32_t r[32];
-              tmem_ld_32x32(t_row + c2 * 64 + half * 32, r);
-              tmem_ld_wait();
-              if (k_blocks == 0) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) r[i] = 0u;
-              }
-              if (p.bias != nullptr) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                  const int col = colr + half * 32 + i;
-                  if (col < p.N) r[i] = __float_as_uint(__uint_as_float(r[i]) + __bfloat162float(p.bias[col]));
-                }
-              }
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                uint4 o;
-                o.x = pack_bf16x2(__uint_as_float(r[8 * i]), __uint_as_float(r[8 * i + 1]));
-                o.y = pack_bf16x2(__uint_as_float(r[8 * i + 2]), __uint_as_float(r[8 * i + 3]));
-                o.z = pack_bf16x2(__uint_as_float(r[8 * i + 4]), __uint_as_float(r[8 * i + 5]));
-                o.w = pack_bf16x2(__uint_as_float(r[8 * i + 6]), __uint_as_float(r[8 * i + 7]));
-                *reinterpret_cast<uint4*>(stage + lane * 128 + (((half * 4 + i) ^ (lane & 7)) << 4)) = o;
-              }
-            }
-          }
-          __syncwarp();
-          const int unit = lane & 7;
-          const int col = colr + unit * (16 / esz);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int rr = k * 4 + (lane >> 3);
-            if (row0 + rr < p.M && col < p.N) {
-              uint8_t* dst = c_tile + (static_cast<long long>(rr) * p.ldc + col) * esz;
-              if (p.out_fp32) {
-                float4 o = *reinterpret_cast<const float4*>(stage + rr * 128 + ((unit ^ (rr & 7)) << 4));
-                if (p.bias != nullptr) {
-                  o.x += __bfloat162float(p.bias[col]); o.y += __bfloat162float(p.bias[col + 1]);
-                  o.z += __bfloat162float(p.bias[col + 2]); o.w += __bfloat162float(p.bias[col + 3]);
-                }
-                if (p.accumulate) {
-                  const float4 old = *reinterpret_cast<const float4*>(dst);
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                }
-                *reinterpret_cast<float4*>(dst) = o;
-              } else {
-                *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((unit ^ (rr & 7)) << 4));
-              }
-            }
-          }
-          __syncwarp();
-        }
+        const TileOut out{reinterpret_cast<uint8_t*>(p.C) + (static_cast<long long>(group) * p.group_stride_c + static_cast<long long>(row0) * p.ldc) * esz,
+                          p.ldc, p.M - row0, p.N, p.out_fp32, p.accumulate, p.bias};
+        store_tile_staged<BN>(out, t_row, smem_stage + q * 4096, n_blk * BN, k_blocks == 0);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tmem_empty[acc]);
@@ -555,23 +482,57 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmPa
   return static_cast<int>(launch_pdl(kern, dim3(grid), dim3(192), L::kTotal, stream, ta, tb, p));
 }
 
+template <int BN, int A_MN, int B_MN, int MODE>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int tiles, cudaStream_t stream) {
+  using L = pair::Layout<BN>;
+  auto kern = pair::gemm_bf16_pair_kernel<BN, A_MN, B_MN, MODE, GemmParams>;
+  static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
+  if (configured != cudaSuccess) return static_cast<int>(configured);
+  const int pairs = num_sms() / 2;
+  return static_cast<int>(launch_pdl(kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(pair::kThreads), L::kTotal, stream, ta, tb, p));
+}
+
+// Which kernel and tile width: 64, 128, 256 for one CTA per tile (128 rows), kPair + 128 or 256 for two (256 rows).
+static constexpr int kPair = 1024;
+
+static int pick_tile(int M, int N, int groups, int forced, const GemmParams& p) {
+  const int esz = p.out_fp32 ? 4 : 2;
+  const bool pair_ok = (((p.ldc * esz) | (p.group_stride_c * esz) | static_cast<long long>(reinterpret_cast<uintptr_t>(p.C))) & 15) == 0 && (N * esz) % 16 == 0;
+  if (forced == 256 || forced == 128 || forced == 64) return forced;
+  if (forced > kPair && pair_ok) return forced;
+  // Least time by waves of tiles × a tile's time per 64-deep step of the reduction.  Measured at 8192³ (ns per step and wave): one CTA
+  // 217, 283, 460 for 64, 128, 256 columns, two 253 and 390 for 128 and 256.  So 256 × 256 wherever the last wave is not nearly empty
+  // (8192³: 825 → 693 µs), and the narrower ones where tiles are few: 1024 × 2560 × 4096 42.6, 40.1, 36.7 | 40.5, 33.0 µs;
+  // 257 × 2560 × 4096 22.5, 24.9, 35.1 | 26.9, 33.1; 257 × 6144 × 2560 24.6, 22.2, 29.5 | 31.7, 26.9.
+  struct Option { int tile, rows, cols, slots, ns; };
+  const int sms = num_sms();
+  const Option options[5] = {{kPair + 256, 2 * BM, 256, sms / 2, 390}, {kPair + 128, 2 * BM, 128, sms / 2, 253}, {256, BM, 256, sms, 460},
+                             {128, BM, 128, sms, 283}, {64, BM, 64, sms, 217}};
+  int best = 64;
+  long long best_ns = 0;
+  for (int i = pair_ok ? 0 : 2; i < 5; ++i) {
+    const Option& o = options[i];
+    const long long tiles = static_cast<long long>((M + o.rows - 1) / o.rows) * ((N + o.cols - 1) / o.cols) * groups;
+    const long long ns = (tiles + o.slots - 1) / o.slots * o.ns;
+    if (best_ns == 0 || ns < best_ns) { best = o.tile; best_ns = ns; }
+  }
+  return best;
+}
+
+// B's tensor-map box has as many rows as one CTA loads of them (K-major; MN-major boxes are 64 × 64 in every kernel)
+static int b_box_rows(int tile) { return tile > kPair ? (tile - kPair) / 2 : tile; }
+
 template <int A_MN, int B_MN, int MODE>
-static int launch_bn(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int tiles, cudaStream_t s) {
-  switch (bn) {
+static int launch_tile(int tile, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int groups, cudaStream_t s) {
+  const int bm = tile > kPair ? 2 * BM : BM, bn = tile > kPair ? tile - kPair : tile;
+  const int tiles = ((p.M + bm - 1) / bm) * ((p.N + bn - 1) / bn) * groups;
+  switch (tile) {
+    case kPair + 256: return launch_pair<256, A_MN, B_MN, MODE>(ta, tb, p, tiles, s);
+    case kPair + 128: return launch_pair<128, A_MN, B_MN, MODE>(ta, tb, p, tiles, s);
     case 256: return launch_one<256, A_MN, B_MN, MODE>(ta, tb, p, tiles, s);
     case 128: return launch_one<128, A_MN, B_MN, MODE>(ta, tb, p, tiles, s);
     default: return launch_one<64, A_MN, B_MN, MODE>(ta, tb, p, tiles, s);
   }
-}
-
-static int pick_bn(int M, int N, int forced) {
-  if (forced == 256 || forced == 128 || forced == 64) return forced;
-  // largest tile width that still gives every SM a tile
-  const int sms = num_sms();
-  const int m_tiles = (M + BM - 1) / BM;
-  if (m_tiles * ((N + 255) / 256) >= sms) return 256;
-  if (m_tiles * ((N + 127) / 128) >= sms) return 128;
-  return 64;
 }
 
 }  // namespace mb
@@ -584,23 +545,22 @@ extern "C" int mb_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
                             long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate, const void* bias,
                             int force_bn, int* error_flag, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
-  const int bn = pick_bn(M, N, force_bn);
-  CUtensorMap ta, tb;
-  int r;
-  r = a_mn ? make_tmap_bf16_2d(&ta, A, K, M, lda, BK, 64) : make_tmap_bf16_2d(&ta, A, M, K, lda, BM, BK);
-  if (r) return 1000 + r;
-  r = b_mn ? make_tmap_bf16_2d(&tb, B, K, N, ldb, BK, 64) : make_tmap_bf16_2d(&tb, B, N, K, ldb, bn, BK);
-  if (r) return 2000 + r;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.out_fp32 = out_fp32; p.accumulate = accumulate;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.error_flag = error_flag;
   p.num_groups = 1;
-  const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
-  if (!a_mn && !b_mn) return launch_bn<0, 0, kDense>(bn, ta, tb, p, tiles, stream);
-  if (!a_mn && b_mn) return launch_bn<0, 1, kDense>(bn, ta, tb, p, tiles, stream);
-  if (a_mn && b_mn) return launch_bn<1, 1, kDense>(bn, ta, tb, p, tiles, stream);
-  return launch_bn<1, 0, kDense>(bn, ta, tb, p, tiles, stream);
+  const int tile = pick_tile(M, N, 1, force_bn, p);
+  CUtensorMap ta, tb;
+  int r;
+  r = a_mn ? make_tmap_bf16_2d(&ta, A, K, M, lda, BK, 64) : make_tmap_bf16_2d(&ta, A, M, K, lda, BM, BK);
+  if (r) return 1000 + r;
+  r = b_mn ? make_tmap_bf16_2d(&tb, B, K, N, ldb, BK, 64) : make_tmap_bf16_2d(&tb, B, N, K, ldb, b_box_rows(tile), BK);
+  if (r) return 2000 + r;
+  if (!a_mn && !b_mn) return launch_tile<0, 0, kDense>(tile, ta, tb, p, 1, stream);
+  if (!a_mn && b_mn) return launch_tile<0, 1, kDense>(tile, ta, tb, p, 1, stream);
+  if (a_mn && b_mn) return launch_tile<1, 1, kDense>(tile, ta, tb, p, 1, stream);
+  return launch_tile<1, 0, kDense>(tile, ta, tb, p, 1, stream);
 }
 
 // Split-K form of C[M,N] = A[M,K]·B[N,K]ᵀ for decode-sized problems (few output tiles, long K): `split_k` CTAs per
@@ -634,22 +594,21 @@ extern "C" int mb_gemm_bf16_grouped(const void* A, const void* B, void* C, int M
                                     const int* tile_expert, int b_mn, int out_fp32, int force_bn, int* error_flag,
                                     cudaStream_t stream) {
   if (M_pad <= 0 || N <= 0) return 0;
-  const int bn = pick_bn(M_pad, N, force_bn);
-  CUtensorMap ta, tb;
-  int r = make_tmap_bf16_2d(&ta, A, M_pad, K, K, BM, BK);
-  if (r) return 1000 + r;
-  r = b_mn ? make_tmap_bf16_2d(&tb, B, static_cast<long long>(num_experts) * K, N, N, BK, 64)
-           : make_tmap_bf16_2d(&tb, B, static_cast<long long>(num_experts) * N, K, K, bn, BK);
-  if (r) return 2000 + r;
   GemmParams p{};
   p.M = M_pad; p.N = N; p.K = K; p.C = C; p.ldc = N; p.out_fp32 = out_fp32;
   p.tile_expert = tile_expert;
   p.b_group_rows = b_mn ? K : N;
   p.error_flag = error_flag;
   p.num_groups = num_experts;
-  const int tiles = (M_pad / BM) * ((N + bn - 1) / bn);
-  if (b_mn) return launch_bn<0, 1, kGroupedFwd>(bn, ta, tb, p, tiles, stream);
-  return launch_bn<0, 0, kGroupedFwd>(bn, ta, tb, p, tiles, stream);
+  const int tile = pick_tile(M_pad, N, 1, force_bn, p);
+  CUtensorMap ta, tb;
+  int r = make_tmap_bf16_2d(&ta, A, M_pad, K, K, BM, BK);
+  if (r) return 1000 + r;
+  r = b_mn ? make_tmap_bf16_2d(&tb, B, static_cast<long long>(num_experts) * K, N, N, BK, 64)
+           : make_tmap_bf16_2d(&tb, B, static_cast<long long>(num_experts) * N, K, K, b_box_rows(tile), BK);
+  if (r) return 2000 + r;
+  if (b_mn) return launch_tile<0, 1, kGroupedFwd>(tile, ta, tb, p, 1, stream);
+  return launch_tile<0, 0, kGroupedFwd>(tile, ta, tb, p, 1, stream);
 }
 
 // Grouped wgrad: dW[e] [N, K] (+)= dY[seg_e, N]ᵀ · X[seg_e, K]; seg_offsets[E+1] are row offsets (multiples of 128).
@@ -657,7 +616,6 @@ extern "C" int mb_gemm_bf16_grouped_wgrad(const void* dY, const void* X, void* d
                                           int num_experts, const int* seg_offsets, int out_fp32, int accumulate,
                                           int force_bn, int* error_flag, cudaStream_t stream) {
   if (N <= 0 || K <= 0 || num_experts <= 0) return 0;
-  const int bn = pick_bn(N * num_experts, K, force_bn);
   CUtensorMap ta, tb;
   int r = make_tmap_bf16_2d(&ta, dY, M_pad, N, N, BK, 64);   // MN-major A: [tokens (k), N (m)]
   if (r) return 1000 + r;
@@ -669,6 +627,5 @@ extern "C" int mb_gemm_bf16_grouped_wgrad(const void* dY, const void* X, void* d
   p.seg_offsets = seg_offsets;
   p.num_groups = num_experts;
   p.error_flag = error_flag;
-  const int tiles = ((N + BM - 1) / BM) * ((K + bn - 1) / bn) * num_experts;
-  return launch_bn<1, 1, kGroupedWgrad>(bn, ta, tb, p, tiles, stream);
+  return launch_tile<1, 1, kGroupedWgrad>(pick_tile(N, K, num_experts, force_bn, p), ta, tb, p, num_experts, stream);
 }
