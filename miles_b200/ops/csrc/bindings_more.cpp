@@ -103,6 +103,21 @@ void paged_decode(const at::Tensor& q, const at::Tensor& kc, const at::Tensor& v
                         scale, num_splits, cur_stream()),
         "mb_paged_decode");
 }
+
+void paged_decode_tiles(const at::Tensor& q, const at::Tensor& kc, const at::Tensor& vc, const at::Tensor& block_table, const at::Tensor& seq_lens,
+                        at::Tensor& out, double scale, const at::Tensor& err) {
+  c10::cuda::CUDAGuard g(q.device());
+  const int64_t B = q.size(0), Hq = q.size(1), D = q.size(2), bs = kc.size(1), Hkv = kc.size(2);
+  const int64_t ctas = 2 * at::cuda::getCurrentDeviceProperties()->multiProcessorCount, rows = 2 * ctas * (Hq / Hkv);
+  // one scratch tensor: partial outputs, partial maxima and sums, the units before each request
+  at::Tensor ws = at::empty({rows * (D + 2) + B + 2}, q.options().dtype(at::kFloat));
+  float* part_o = ws.data_ptr<float>();
+  float* part_ml = part_o + rows * D;
+  check(mb_paged_decode_tiles(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), block_table.data_ptr<int>(), seq_lens.data_ptr<int>(), out.data_ptr(), part_o,
+                              part_ml, reinterpret_cast<int*>(part_ml + rows * 2), B, block_table.size(1), bs, kc.size(0) * bs, Hq, Hkv, D, scale, ctas,
+                              err.data_ptr<int>(), cur_stream()),
+        "mb_paged_decode_tiles");
+}
 #endif  // MB_SERVE_SUBSET
 
 }  // namespace
@@ -127,6 +142,7 @@ void register_more(pybind11::module& m) {
   m.def("flash_bwd", &flash_bwd);
   m.def("flash_bwd_tc", &flash_bwd_tc);
   m.def("paged_decode", &paged_decode);
+  m.def("paged_decode_tiles", &paged_decode_tiles);
   register_fabric(m);
   register_extra(m);
 #endif

@@ -6,6 +6,9 @@
 // K/V tiles of 64 keys are gathered from their cache pages with cp.async into XOR-swizzled shared memory, double
 // buffered; each of the 4 warps owns 16 keys of a tile with its own running (max, sum, O) which are merged through
 // shared memory at the end.  Split partials are combined by `paged_merge_kernel2`.
+//
+// Caches whose pages hold a multiple of 64 tokens (the engine's do) take the form by tiles at the end of this file instead: the same
+// arithmetic, an even share of ALL the 64-key tiles of the batch per CTA, tiles by TMA.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -16,6 +19,11 @@
 #include "debug.cuh"
 #include "mma_sync.cuh"
 #include "pdl.cuh"
+#include "ptx.cuh"
+
+namespace mb {
+int make_tmap_bf16_2d(CUtensorMap* out, const void* base, long long rows, long long cols, long long ld, int box_rows, int box_cols);
+}
 
 namespace mbpd {
 
@@ -234,6 +242,334 @@ __global__ void paged_merge_kernel2(const float* __restrict__ part_o, const floa
 template <int D>
 static size_t smem_bytes() { return static_cast<size_t>(16 * D + 4 * TK * D) * 2 + 64 * sizeof(float) + 4 * 8 * D * sizeof(float); }
 
+// ---- by tiles --------------------------------------------------------------------------------------------------------------------
+//
+// Work is counted in units of (request, KV head, 64-key tile), requests outermost; CTA c takes units [c·per, (c + 1)·per).  A CTA walks
+// through segments (its tiles of one request and KV head): a whole one goes straight to the output, a part goes to one of the CTA's
+// two slots of the partial buffers (0: the segment that holds its first unit, 1: a later one) and `paged_merge_tiles_kernel` adds up the
+// slots of a segment in order.  Which CTAs share a segment follows from the units before each request and `per`, which the last CTA
+// leaves in `plan`; lengths are read on the device, so that one captured launch serves any of them.  No pointer here is __restrict__: these
+// kernels start before the ones in front of them have finished, and a load that the compiler takes for invariant may move up across the
+// dependency wait (read that early, `plan` holds whatever the scratch memory held before).
+//
+// What bounds it: the cache's bytes.  An even split of every request into as many ranges (the form above) lets the longest
+// request of a ragged batch set the time, and two tiles per CTA in flight behind CTA-wide barriers leave the memory idle between them.  Here a
+// producer warp keeps three 32 KB tiles in flight per CTA, two CTAs per SM, and the warps that compute wait for data only.  Attention and merge,
+// the form above → this one (32 query and 4 KV heads of 128): 61 requests of 290 to 4090 tokens 62.4 → 43.6 µs (bytes alone: 28.1), 19 of
+// 300 to 2500 with 8 KV heads 35.5 → 20.5 (12.8), 64 × 4096 102.8 → 93.1 (83.2), 7 of 433 to 3001 14.9 → 13.0; with little to read per
+// CTA the chain length → unit → page → tile shows: 8 × 700 9.7 → 11.4.
+static constexpr int kTileStages = 3, kTileThreads = 160;      // four warps that compute, one that loads
+
+template <int D>
+struct TileSmem {
+  static constexpr int kTile = TK * D * 2;                      // K or V of 64 keys: D / 64 atoms of 64 rows × 128 B
+  static constexpr int o = kTileStages * 2 * kTile;             // [4][8][D] floats
+  static constexpr int ml = o + 4 * 8 * D * 4;                  // [4][8] maxima, [4][8] sums
+  static constexpr int bars = ml + 2 * 32 * 4;
+  static constexpr int total = bars + 64;
+};
+
+// tiles of the request; its units are this times the number of KV heads
+__device__ __forceinline__ int tiles_of(const int* seq_lens, int req) { return (max(seq_lens[req], 0) + TK - 1) / TK; }
+
+template <int D>
+__global__ void __launch_bounds__(kTileThreads, 2)
+paged_decode_tiles_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const bf16* q,
+                          const int* block_table, const int* seq_lens, bf16* out,
+                          float* part_o, float* part_ml, int* plan, int batch, int max_blocks,
+                          int block_size, int cache_rows, int Hq, int Hkv, float scale, int* error_flag) {
+  using S = TileSmem<D>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (mb::smem_u32(smem) & 1023u) {   // swizzled tiles need 1024-byte alignment
+    if (threadIdx.x == 0) atomicExch(error_flag, 61);
+    return;
+  }
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::bars);
+  uint64_t* empty = full + kTileStages;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kTileStages; ++i) { mb::mbar_init(&full[i], 1); mb::mbar_init(&empty[i], 4); }
+    mb::mbar_fence_init();
+    mb::tma_prefetch_desc(&tm_k);
+    mb::tma_prefetch_desc(&tm_v);
+  }
+  __syncthreads();
+  mb::pdl_trigger();
+  mb::pdl_wait();
+  const int group = Hq / Hkv;
+  const int mine = lane < batch ? tiles_of(seq_lens, lane) * Hkv : 0;       // units of requests 0..31: most batches need no second look
+  auto units_of = [&](int r0) { return r0 == 0 ? mine : (r0 + lane < batch ? tiles_of(seq_lens, r0 + lane) * Hkv : 0); };
+  auto sum_to = [&](int n) {                                                // inclusive sum over the lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, n, o);
+      if (lane >= o) n += v;
+    }
+    return n;
+  };
+  int units = mine;
+  for (int r0 = 32; r0 < batch; r0 += 32) units += units_of(r0);
+  units = __reduce_add_sync(0xffffffffu, units);
+  const int per = (units + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  const int begin = static_cast<int>(blockIdx.x) * per, end = min(units, begin + per);
+  if (blockIdx.x == gridDim.x - 1 && warp == 0) {                           // the last CTA has the fewest units, often none
+    int before = 0;
+    for (int r0 = 0; r0 < batch; r0 += 32) {
+      const int n = units_of(r0), sum = sum_to(n);
+      if (r0 + lane < batch) plan[r0 + lane] = before + sum - n;
+      before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) { plan[batch] = before; plan[batch + 1] = per; }
+  }
+  if (begin >= end) return;
+  // where the first unit is
+  int req = 0, at = begin;
+  for (int r0 = 0, before = 0;; r0 += 32) {
+    const int n = units_of(r0), sum = sum_to(n);
+    const uint32_t beyond = __ballot_sync(0xffffffffu, before + sum > begin);
+    if (beyond) {
+      const int l = __ffs(beyond) - 1;
+      req = r0 + l;
+      at = begin - before - __shfl_sync(0xffffffffu, sum - n, l);
+      break;
+    }
+    before += __shfl_sync(0xffffffffu, sum, 31);
+  }
+  int tiles = tiles_of(seq_lens, req);
+  int hk = at / tiles, tile = at % tiles;
+  int stage = 0;
+  uint32_t phase = 0;
+  bool ok = true;
+
+  for (int u = begin; u < end;) {                           // after a failed wait a warp goes on without tiles: it still meets the barriers below
+    const int n = min(tiles - tile, end - u);               // this segment's tiles
+    if (warp == 4) {
+      // ------------------------------ TMA producer ------------------------------
+      const int* bt = block_table + static_cast<long long>(req) * max_blocks;
+      for (int i0 = 0; i0 < n && ok; i0 += 32) {
+        int row = 0;                                        // lane i: first cache row of tile i0 + i
+        if (i0 + lane < n) {
+          const int key = (tile + i0 + lane) * TK;
+          const long long blk = bt[key / block_size];
+          row = mb::dbg::in_bounds(mb::dbg::kKvBlocks, blk, 301) ? static_cast<int>(blk) * block_size + key % block_size : cache_rows;   // past the end: zeros
+        }
+        for (int i = 0; i < min(32, n - i0) && ok; ++i) {
+          const int r = __shfl_sync(0xffffffffu, row, i);
+          ok = __all_sync(0xffffffffu, mb::mbar_wait(&empty[stage], phase ^ 1));
+          if (ok && lane == 0) {
+            mb::mbar_expect_tx(&full[stage], 2 * S::kTile);
+            uint8_t* dst = smem + stage * 2 * S::kTile;
+#pragma unroll
+            for (int a = 0; a < D / 64; ++a) {
+              mb::tma_load_2d(dst + a * (TK * 128), &tm_k, &full[stage], hk * D + a * 64, r);
+              mb::tma_load_2d(dst + S::kTile + a * (TK * 128), &tm_v, &full[stage], hk * D + a * 64, r);
+            }
+          }
+          if (++stage == kTileStages) { stage = 0; phase ^= 1; }
+        }
+      }
+      if (!ok && lane == 0) atomicExch(error_flag, 62);
+    } else {
+      // ------------------------------ scores, softmax, values: 16 keys of each tile per warp ------------------------------
+      const int L = seq_lens[req];
+      uint32_t qa[D / 16][2];                               // A operand: rows 0..7 are the group's heads, 8..15 zero
+      {
+        const int g = lane >> 2;
+        const bf16* qr = q + (static_cast<long long>(req) * Hq + hk * group + g) * D + (lane & 3) * 2;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+          qa[ks][0] = g < group ? *reinterpret_cast<const uint32_t*>(qr + ks * 16) : 0u;
+          qa[ks][1] = g < group ? *reinterpret_cast<const uint32_t*>(qr + ks * 16 + 8) : 0u;
+        }
+      }
+      float o_acc[D / 8][4];
+#pragma unroll
+      for (int i = 0; i < D / 8; ++i) o_acc[i][0] = o_acc[i][1] = o_acc[i][2] = o_acc[i][3] = 0.f;
+      float m_i = -INFINITY, l_i = 0.f;                     // row lane / 4
+      const float sl2 = scale * kLog2e;
+      for (int i = 0; i < n && ok; ++i) {
+        ok = __all_sync(0xffffffffu, mb::mbar_wait(&full[stage], phase));
+        if (!ok) break;
+        uint8_t* sK = smem + stage * 2 * S::kTile;
+        uint8_t* sV = sK + S::kTile;
+        const int key0 = (tile + i) * TK + warp * 16;
+        auto unit16 = [](uint8_t* base, int row, int chunk) {   // 16-byte unit `chunk` of a row, atoms of 64 columns, 128-byte swizzle
+          return base + (chunk >> 3) * (TK * 128) + row * 128 + (((chunk & 7) ^ (row & 7)) << 4);
+        };
+        if (key0 < L) {
+          if (key0 + 16 > L) {                              // rows behind the sequence: weight 0, but whatever the page holds may be no number
+            for (int v = lane; v < 16 * (D / 8); v += 32) {
+              const int row = v / (D / 8);
+              if (key0 + row >= L) *reinterpret_cast<uint4*>(unit16(sV, warp * 16 + row, v % (D / 8))) = make_uint4(0, 0, 0, 0);
+            }
+            mb::fence_proxy_async();                        // … before the next tile is copied over it
+            __syncwarp();
+          }
+          float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+          for (int ks = 0; ks < D / 16; ++ks) {
+            uint32_t b[4];
+            ldsm_x4(s_addr(unit16(sK, warp * 16 + (lane & 7) + ((lane >> 4) << 3), ks * 2 + ((lane >> 3) & 1))), b[0], b[1], b[2], b[3]);
+            const uint32_t a[4] = {qa[ks][0], 0u, qa[ks][1], 0u};
+            mma16816(s[0], a, b[0], b[1]);
+            mma16816(s[1], a, b[2], b[3]);
+          }
+          float mx = m_i;
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              if (key0 + nt * 8 + (lane & 3) * 2 + e >= L) s[nt][e] = -INFINITY;
+              mx = fmaxf(mx, s[nt][e]);
+            }
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+          const float msc = (mx == -INFINITY) ? 0.f : mx * sl2;
+          const float alpha = (m_i == -INFINITY) ? 0.f : exp2f(m_i * sl2 - msc);
+          m_i = mx;
+          float rs = 0.f;
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              s[nt][e] = exp2f(s[nt][e] * sl2 - msc);
+              rs += s[nt][e];
+            }
+          l_i = l_i * alpha + rs;
+#pragma unroll
+          for (int c = 0; c < D / 8; ++c) { o_acc[c][0] *= alpha; o_acc[c][1] *= alpha; }
+          const uint32_t pa[4] = {pack2(s[0][0], s[0][1]), 0u, pack2(s[1][0], s[1][1]), 0u};
+#pragma unroll
+          for (int nc = 0; nc < D / 16; ++nc) {
+            uint32_t b[4];
+            ldsm_x4_t(s_addr(unit16(sV, warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), nc * 2 + (lane >> 4))), b[0], b[1], b[2], b[3]);
+            mma16816(o_acc[2 * nc], pa, b[0], b[1]);
+            mma16816(o_acc[2 * nc + 1], pa, b[2], b[3]);
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mb::mbar_arrive(&empty[stage]);
+        if (++stage == kTileStages) { stage = 0; phase ^= 1; }
+      }
+      // merge the four warps
+      if (!ok && lane == 0) atomicExch(error_flag, 63);
+      float* sO = reinterpret_cast<float*>(smem + S::o);
+      float* sM = reinterpret_cast<float*>(smem + S::ml);
+      float* sL = sM + 32;
+      l_i += __shfl_xor_sync(0xffffffffu, l_i, 1);
+      l_i += __shfl_xor_sync(0xffffffffu, l_i, 2);
+      const int r = lane >> 2;
+      if ((lane & 3) == 0) { sM[warp * 8 + r] = m_i; sL[warp * 8 + r] = l_i; }
+#pragma unroll
+      for (int c = 0; c < D / 8; ++c)
+        *reinterpret_cast<float2*>(&sO[(warp * 8 + r) * D + c * 8 + (lane & 3) * 2]) = make_float2(o_acc[c][0], o_acc[c][1]);
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      const bool whole = tile == 0 && n == tiles;
+      const long long slot = 2 * static_cast<long long>(blockIdx.x) + (u == begin ? 0 : 1);
+      for (int v = threadIdx.x; v < group * (D / 4); v += 128) {
+        const int g = v / (D / 4), d = v % (D / 4) * 4;
+        float mm = -INFINITY, ll = 0.f;
+        float4 oo = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) mm = fmaxf(mm, sM[w * 8 + g]);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const float mw = sM[w * 8 + g];
+          const float a = (mw == -INFINITY) ? 0.f : exp2f((mw - mm) * sl2);
+          const float4 x = *reinterpret_cast<const float4*>(&sO[(w * 8 + g) * D + d]);
+          ll += sL[w * 8 + g] * a;
+          oo.x += x.x * a; oo.y += x.y * a; oo.z += x.z * a; oo.w += x.w * a;
+        }
+        if (whole) {
+          const float inv = ll > 0.f ? 1.f / ll : 0.f;
+          *reinterpret_cast<uint2*>(out + (static_cast<long long>(req) * Hq + hk * group + g) * D + d) =
+              make_uint2(pack2(oo.x * inv, oo.y * inv), pack2(oo.z * inv, oo.w * inv));
+        } else {
+          __stcg(reinterpret_cast<float4*>(part_o + (slot * group + g) * D + d), oo);
+          if (d == 0) __stcg(reinterpret_cast<float2*>(part_ml + (slot * group + g) * 2), make_float2((mm == -INFINITY) ? -INFINITY : mm * sl2, ll));
+        }
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");      // sO is free again
+    }
+    u += n;
+    tile += n;
+    if (tile == tiles && u < end) {
+      tile = 0;
+      if (++hk == Hkv) {
+        hk = 0;
+        do { tiles = tiles_of(seq_lens, ++req); } while (tiles == 0);       // u < end: some request behind has units
+      }
+    }
+  }
+}
+
+// grid (Hq, batch), 128 threads: the slots of one head's segment.  A segment that one CTA did alone is already in place; a request
+// without keys gets zeros.
+template <int D>
+__global__ void __launch_bounds__(128) paged_merge_tiles_kernel(const float* part_o, const float* part_ml,
+                                                               const int* plan, bf16* out, int batch, int Hq, int Hkv) {
+  __shared__ float4 s_o[4][D / 4];
+  __shared__ float s_l[4];
+  mb::pdl_trigger();
+  mb::pdl_wait();
+  const int h = blockIdx.x, req = blockIdx.y, group = Hq / Hkv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per = __ldcg(plan + batch + 1), u_req = __ldcg(plan + req), tiles = (__ldcg(plan + req + 1) - u_req) / Hkv;
+  bf16* o = out + (static_cast<long long>(req) * Hq + h) * D;
+  if (tiles == 0) {
+    if (threadIdx.x < D / 4) *reinterpret_cast<uint2*>(o + threadIdx.x * 4) = make_uint2(0u, 0u);
+    return;
+  }
+  const int u0 = u_req + h / group * tiles, c0 = u0 / per, c1 = (u0 + tiles - 1) / per;
+  if (c0 == c1) return;
+  const int first = u0 == c0 * per ? 0 : 1;                 // the first CTA's slot; the others start with this segment
+  auto at = [&](int c) { return (2ll * c + (c == c0 ? first : 0)) * group + h % group; };
+  float mm = -INFINITY;
+  for (int c = c0 + lane; c <= c1; c += 32) mm = fmaxf(mm, __ldcg(part_ml + at(c) * 2));
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, i));
+  float ll = 0.f;
+  float4 oo = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int c = c0 + warp; c <= c1; c += 4) {
+    const float2 ml = __ldcg(reinterpret_cast<const float2*>(part_ml + at(c) * 2));
+    const float a = (ml.x == -INFINITY) ? 0.f : exp2f(ml.x - mm);
+    ll += ml.y * a;
+    if (lane < D / 4) {
+      const float4 x = __ldcg(reinterpret_cast<const float4*>(part_o + at(c) * D) + lane);
+      oo.x += x.x * a; oo.y += x.y * a; oo.z += x.z * a; oo.w += x.w * a;
+    }
+  }
+  if (lane < D / 4) s_o[warp][lane] = oo;
+  if (lane == 0) s_l[warp] = ll;
+  __syncthreads();
+  if (threadIdx.x < D / 4) {
+    const float4 a = s_o[0][lane], b = s_o[1][lane], c = s_o[2][lane], d = s_o[3][lane];
+    const float l = (s_l[0] + s_l[1]) + (s_l[2] + s_l[3]), inv = l > 0.f ? 1.f / l : 0.f;
+    *reinterpret_cast<uint2*>(o + lane * 4) = make_uint2(pack2((a.x + b.x + c.x + d.x) * inv, (a.y + b.y + c.y + d.y) * inv),
+                                                         pack2((a.z + b.z + c.z + d.z) * inv, (a.w + b.w + c.w + d.w) * inv));
+  }
+}
+
+template <int D>
+static int launch_tiles(const bf16* q, const void* kc, const void* vc, const int* block_table, const int* seq_lens, bf16* out, float* part_o,
+                        float* part_ml, int* plan, int batch, int max_blocks, int block_size, int cache_rows, int Hq, int Hkv, float scale,
+                        int ctas, int* error_flag, cudaStream_t s) {
+  CUtensorMap tk, tv;
+  int rc = mb::make_tmap_bf16_2d(&tk, kc, cache_rows, static_cast<long long>(Hkv) * D, static_cast<long long>(Hkv) * D, TK, 64);
+  if (rc) return 1000 + rc;
+  rc = mb::make_tmap_bf16_2d(&tv, vc, cache_rows, static_cast<long long>(Hkv) * D, static_cast<long long>(Hkv) * D, TK, 64);
+  if (rc) return 2000 + rc;
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(paged_decode_tiles_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, TileSmem<D>::total);
+  if (configured != cudaSuccess) return static_cast<int>(configured);
+  cudaError_t e = mb::launch_pdl(paged_decode_tiles_kernel<D>, dim3(ctas), dim3(kTileThreads), TileSmem<D>::total, s, tk, tv, q, block_table,
+                                 seq_lens, out, part_o, part_ml, plan, batch, max_blocks, block_size, cache_rows, Hq, Hkv, scale, error_flag);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  e = mb::launch_pdl(paged_merge_tiles_kernel<D>, dim3(Hq, batch), dim3(128), 0, s, static_cast<const float*>(part_o), static_cast<const float*>(part_ml),
+                     static_cast<const int*>(plan), out, batch, Hq, Hkv);
+  return static_cast<int>(e);
+}
+
 }  // namespace mbpd
 
 using namespace mbpd;
@@ -309,4 +645,23 @@ extern "C" int mb_paged_decode(const void* q, const void* kc, const void* vc, co
     return -1;
   }
   return static_cast<int>(cudaGetLastError());
+}
+
+// The form by tiles: block_size a multiple of 64.  cache_rows: pages × block_size.  `ctas` CTAs share the work; part_o: 2 · ctas · Hq/Hkv · D
+// floats, part_ml: 2 · ctas · Hq/Hkv · 2 floats, plan: batch + 2 ints (all scratch, written before they are read).
+extern "C" int mb_paged_decode_tiles(const void* q, const void* kc, const void* vc, const int* block_table, const int* seq_lens, void* out,
+                                     float* part_o, float* part_ml, int* plan, int batch, int max_blocks, int block_size, int cache_rows, int Hq,
+                                     int Hkv, int D, float scale, int ctas, int* error_flag, cudaStream_t s) {
+  if (batch == 0) return 0;
+  const int group = Hq / Hkv;
+  if (group > 8 || group * Hkv != Hq || block_size % TK != 0 || batch > 65535) return -2;
+  auto Q = reinterpret_cast<const bf16*>(q);
+  bf16* O = reinterpret_cast<bf16*>(out);
+  if (D == 128)
+    return launch_tiles<128>(Q, kc, vc, block_table, seq_lens, O, part_o, part_ml, plan, batch, max_blocks, block_size, cache_rows, Hq, Hkv, scale, ctas,
+                             error_flag, s);
+  if (D == 64)
+    return launch_tiles<64>(Q, kc, vc, block_table, seq_lens, O, part_o, part_ml, plan, batch, max_blocks, block_size, cache_rows, Hq, Hkv, scale, ctas,
+                            error_flag, s);
+  return -1;
 }

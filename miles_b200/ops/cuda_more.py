@@ -103,11 +103,15 @@ def paged_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens=None, max
         return ref.paged_attention(q, k_cache, v_cache, block_table, seq_lens)
     q = _c(q)
     out = torch.empty_like(q)
+    publish_limit(LIMIT_KV_BLOCKS, k_cache.shape[0])
+    if k_cache.shape[1] % 64 == 0 and k_cache.is_contiguous() and v_cache.is_contiguous() and block_table.is_contiguous():
+        # whole 64-key tiles inside a page: an even share of all tiles per CTA
+        C.paged_decode_tiles(q, k_cache, v_cache, block_table, seq_lens, out, 1.0 / math.sqrt(D), C.error_flag(q))
+        return out
     # enough (request, kv head, split) CTAs for two waves of the 148 SMs, never more splits than that needs
     splits = max(1, min(_DECODE_SPLITS, -(-296 // (B * k_cache.shape[2]))))
     part_o = torch.empty(B * Hq * splits * D, dtype=torch.float32, device=q.device)
     part_ml = torch.empty(B * Hq * splits * 2, dtype=torch.float32, device=q.device)
-    publish_limit(LIMIT_KV_BLOCKS, k_cache.shape[0])
     C.paged_decode(q, k_cache, v_cache, block_table, seq_lens, out, part_o, part_ml, 1.0 / math.sqrt(D), splits)
     return out
 

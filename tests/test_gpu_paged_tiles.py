@@ -1,0 +1,57 @@
+"""Paged decode attention with an even share of all key tiles per CTA, against 64-bit softmax."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(lens, hq, hkv, d, page):
+    g = torch.Generator(device="cuda").manual_seed(9)
+    pages = [max(1, -(-n // page)) for n in lens]
+    total = sum(pages) + 2
+    k, v = (torch.randn(total, page, hkv, d, device="cuda", generator=g).bfloat16() for _ in range(2))
+    order = torch.randperm(total, generator=g, device="cuda").to(torch.int32)
+    table = torch.zeros(len(lens), max(pages) + 1, dtype=torch.int32, device="cuda")
+    at = 0
+    for b, n in enumerate(pages):
+        table[b, :n] = order[at:at + n]
+        at += n
+        if lens[b] % page:                        # what a page holds behind its sequence's end may be no number
+            k[table[b, n - 1], lens[b] % page:] = math.nan
+            v[table[b, n - 1], lens[b] % page:] = math.nan
+    q = torch.randn(len(lens), hq, d, device="cuda", generator=g).bfloat16()
+    return q, k, v, table, torch.tensor(lens, dtype=torch.int32, device="cuda")
+
+
+def _softmax64(q, k, v, table, lens):
+    out = torch.zeros(q.shape, dtype=torch.float64, device=q.device)
+    group = q.shape[1] // k.shape[2]
+    for b, n in enumerate(lens.tolist()):
+        if n:
+            pages = table[b, :-(-n // k.shape[1])].long()
+            kk, vv = (x[pages].flatten(0, 1)[:n].double().transpose(0, 1).repeat_interleave(group, 0) for x in (k, v))
+            p = torch.softmax(q[b].double()[:, None] @ kk.transpose(1, 2) / math.sqrt(q.shape[2]), -1)
+            out[b] = (p @ vv)[:, 0]
+    return out
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(32, 4, 128), (16, 8, 128), (4, 4, 128), (8, 2, 64)])
+@pytest.mark.parametrize("lens,page", [([1], 64), ([1, 63, 64, 65, 700, 0, 128], 64), ([0, 0, 5, 0], 64), ([6000, 1, 1, 3], 64), ([300] * 61, 128),
+                                       ([7] * 300, 64), (list(range(1, 700, 9)), 64), ([0, 0], 64)])
+def test_paged_decode_tiles(hq, hkv, d, lens, page):
+    from miles_b200.ops import cuda as K
+
+    args = _inputs(lens, hq, hkv, d, page)
+    ref = _softmax64(*args)
+    out = K.paged_attention(*args)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):                 # two in a row, the second one's kernels start while the first one's still run
+        K.paged_attention(*args)
+        again = K.paged_attention(*args)
+    graph.replay()
+    assert torch.isfinite(out).all() and torch.equal(out, again)
+    # weights and outputs are rounded to bf16 once each: 2^-9 relative and independent
+    assert (out.double() - ref).norm().item() <= 2 ** -8 * ref.norm().item()
+    assert K.check_error_flag(out) == 0
