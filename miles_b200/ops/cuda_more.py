@@ -63,6 +63,9 @@ def attention_varlen(q, k, v, cu_seqlens, max_seqlen=0, causal=True):
 
 
 _DECODE_SPLITS = int(os.environ.get("MILES_DECODE_SPLITS", "8"))   # KV splits per (request, kv head) in paged decode
+# whoever asks for a number of splits gets the form that has them: a request's sums are then cut in the same places whatever else is in the
+# batch (one split, for rollouts that have to agree with the trainer)
+_DECODE_BY_TILES = "MILES_DECODE_SPLITS" not in os.environ
 
 
 def extend_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens, extend=None):
@@ -104,7 +107,7 @@ def paged_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens=None, max
     q = _c(q)
     out = torch.empty_like(q)
     publish_limit(LIMIT_KV_BLOCKS, k_cache.shape[0])
-    if k_cache.shape[1] % 64 == 0 and k_cache.is_contiguous() and v_cache.is_contiguous() and block_table.is_contiguous():
+    if _DECODE_BY_TILES and k_cache.shape[1] % 64 == 0 and k_cache.is_contiguous() and v_cache.is_contiguous() and block_table.is_contiguous():
         # whole 64-key tiles inside a page: an even share of all tiles per CTA
         C.paged_decode_tiles(q, k_cache, v_cache, block_table, seq_lens, out, 1.0 / math.sqrt(D), C.error_flag(q))
         return out

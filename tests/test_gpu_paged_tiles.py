@@ -55,3 +55,25 @@ def test_paged_decode_tiles(hq, hkv, d, lens, page):
     # weights and outputs are rounded to bf16 once each: 2^-9 relative and independent
     assert (out.double() - ref).norm().item() <= 2 ** -8 * ref.norm().item()
     assert K.check_error_flag(out) == 0
+
+
+def test_asked_for_splits_do_not_depend_on_the_batch():
+    """MILES_DECODE_SPLITS pins where a request's sums are cut."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = """
+import sys
+sys.path.insert(0, %r)
+import torch
+from tests.test_gpu_paged_tiles import _inputs
+from miles_b200.ops import cuda as K
+q, k, v, table, lens = _inputs([700, 64, 3001, 1], 32, 4, 128, 64)
+out = K.paged_attention(q, k, v, table, lens)
+for b in range(4):
+    assert torch.equal(out[b], K.paged_attention(q[b:b + 1], k, v, table[b:b + 1], lens[b:b + 1])[0]), b
+""" % root
+    for splits in ("1", "4"):
+        subprocess.run([sys.executable, "-c", code], check=True, cwd=root, env={**os.environ, "MILES_DECODE_SPLITS": splits})
