@@ -118,6 +118,32 @@ void paged_decode_tiles(const at::Tensor& q, const at::Tensor& kc, const at::Ten
                               err.data_ptr<int>(), cur_stream()),
         "mb_paged_decode_tiles");
 }
+
+const float* fptr_or_null(const c10::optional<at::Tensor>& t) { return t.has_value() && t->defined() ? t->data_ptr<float>() : nullptr; }
+
+// log p(target), entropy and log-sum-exp of softmax(hidden · Wᵀ / temperature) without the logits in memory
+void head_logprob(const at::Tensor& hidden, const at::Tensor& W, const at::Tensor& targets, double inv_temp, at::Tensor& logp, at::Tensor& ent,
+                  at::Tensor& lse, const at::Tensor& err) {
+  c10::cuda::CUDAGuard g(hidden.device());
+  TORCH_CHECK(hidden.is_contiguous() && W.is_contiguous() && targets.is_contiguous(), "head_logprob: contiguous operands");
+  const int64_t R = hidden.size(0), V = W.size(0), parts = (V + 127) / 128;
+  at::Tensor ws = at::empty({parts, R, 4}, hidden.options().dtype(at::kFloat)), tz = at::zeros({R}, hidden.options().dtype(at::kFloat));
+  check(mb_head_stats(hidden.data_ptr(), W.data_ptr(), reinterpret_cast<const long long*>(targets.data_ptr<int64_t>()), ws.data_ptr<float>(), tz.data_ptr<float>(), R, V,
+                      hidden.size(1), inv_temp, err.data_ptr<int>(), cur_stream()),
+        "mb_head_stats");
+  check(mb_head_finish(ws.data_ptr<float>(), tz.data_ptr<float>(), parts, R, logp.data_ptr<float>(), ent.data_ptr<float>(), lse.data_ptr<float>(), cur_stream()),
+        "mb_head_finish");
+}
+
+void head_grad(const at::Tensor& hidden, const at::Tensor& W, const at::Tensor& targets, const at::Tensor& lse, const c10::optional<at::Tensor>& ent,
+               const c10::optional<at::Tensor>& g_lp, const c10::optional<at::Tensor>& g_ent, at::Tensor& out, double inv_temp, const at::Tensor& err) {
+  c10::cuda::CUDAGuard g(hidden.device());
+  TORCH_CHECK(hidden.is_contiguous() && W.is_contiguous() && targets.is_contiguous() && out.is_contiguous(), "head_grad: contiguous operands");
+  check(mb_head_grad(hidden.data_ptr(), W.data_ptr(), reinterpret_cast<const long long*>(targets.data_ptr<int64_t>()), lse.data_ptr<float>(), fptr_or_null(ent),
+                     fptr_or_null(g_lp), fptr_or_null(g_ent), out.data_ptr(), out.size(1), hidden.size(0), W.size(0), hidden.size(1), inv_temp,
+                     err.data_ptr<int>(), cur_stream()),
+        "mb_head_grad");
+}
 #endif  // MB_SERVE_SUBSET
 
 }  // namespace
@@ -141,6 +167,8 @@ void register_more(pybind11::module& m) {
   m.def("flash_fwd_tc_ctas_per_sm", []() { return mb_flash_fwd_tc_ctas_per_sm(); });
   m.def("flash_bwd", &flash_bwd);
   m.def("flash_bwd_tc", &flash_bwd_tc);
+  m.def("head_logprob", &head_logprob);
+  m.def("head_grad", &head_grad);
   m.def("paged_decode", &paged_decode);
   m.def("paged_decode_tiles", &paged_decode_tiles);
   register_fabric(m);

@@ -28,27 +28,6 @@ static constexpr int UMMA_K = 16;
 
 enum GemmMode { kDense = 0, kGroupedFwd = 1, kGroupedWgrad = 2 };
 
-struct GemmParams {
-  int M, N, K;
-  void* C;
-  long long ldc;           // elements
-  long long group_stride_c;  // elements between per-group outputs (grouped wgrad)
-  int out_fp32;
-  int accumulate;
-  const __nv_bfloat16* bias;
-  const int* tile_expert;  // grouped fwd: [m_tiles]
-  const int* seg_offsets;  // grouped wgrad: [groups+1], multiples of BK
-  int num_groups;
-  int b_group_rows;        // grouped fwd: rows of B per expert (N for K-major B, K for MN-major B)
-  int* error_flag;
-  // split-K (dense, few output tiles): `split_k` CTAs share one output tile, each writing the partial sums of its K slice
-  // to its own fp32 plane of `ws` [split_k, M, N]; the last to arrive (counter per tile and 32-row quadrant) adds the
-  // planes in slice order, writes C and resets the counter
-  int split_k;
-  float* ws;
-  int* counters;
-};
-
 template <int BN>
 struct SmemLayout {
   static constexpr int kABytes = BM * BK * 2;
@@ -457,16 +436,6 @@ int make_tmap_bf16_3d(CUtensorMap* out, const void* base, long long outer, long 
   return encode_bf16(out, base, 3, dims, strides, box);
 }
 
-static int g_num_sms = 0;
-static int num_sms() {
-  if (g_num_sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return g_num_sms;
-}
-
 template <int BN, int A_MN, int B_MN, int MODE>
 static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int total_tiles, cudaStream_t stream) {
   using L = SmemLayout<BN>;
@@ -480,16 +449,6 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmPa
   int grid = total_tiles < num_sms() ? total_tiles : num_sms();
   if (grid <= 0) return 0;
   return static_cast<int>(launch_pdl(kern, dim3(grid), dim3(192), L::kTotal, stream, ta, tb, p));
-}
-
-template <int BN, int A_MN, int B_MN, int MODE>
-static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int tiles, cudaStream_t stream) {
-  using L = pair::Layout<BN>;
-  auto kern = pair::gemm_bf16_pair_kernel<BN, A_MN, B_MN, MODE, GemmParams>;
-  static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
-  if (configured != cudaSuccess) return static_cast<int>(configured);
-  const int pairs = num_sms() / 2;
-  return static_cast<int>(launch_pdl(kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(pair::kThreads), L::kTotal, stream, ta, tb, p));
 }
 
 // Which kernel and tile width: 64, 128, 256 for one CTA per tile (128 rows), kPair + 128 or 256 for two (256 rows).
@@ -527,8 +486,8 @@ static int launch_tile(int tile, const CUtensorMap& ta, const CUtensorMap& tb, c
   const int bm = tile > kPair ? 2 * BM : BM, bn = tile > kPair ? tile - kPair : tile;
   const int tiles = ((p.M + bm - 1) / bm) * ((p.N + bn - 1) / bn) * groups;
   switch (tile) {
-    case kPair + 256: return launch_pair<256, A_MN, B_MN, MODE>(ta, tb, p, tiles, s);
-    case kPair + 128: return launch_pair<128, A_MN, B_MN, MODE>(ta, tb, p, tiles, s);
+    case kPair + 256: return pair::launch_pair<256, A_MN, B_MN, MODE>(ta, tb, p, pair::StoreTile{}, tiles, s);
+    case kPair + 128: return pair::launch_pair<128, A_MN, B_MN, MODE>(ta, tb, p, pair::StoreTile{}, tiles, s);
     case 256: return launch_one<256, A_MN, B_MN, MODE>(ta, tb, p, tiles, s);
     case 128: return launch_one<128, A_MN, B_MN, MODE>(ta, tb, p, tiles, s);
     default: return launch_one<64, A_MN, B_MN, MODE>(ta, tb, p, tiles, s);

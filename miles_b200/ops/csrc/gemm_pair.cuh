@@ -25,6 +25,37 @@
 
 namespace mb {
 
+struct GemmParams {
+  int M, N, K;
+  void* C;
+  long long ldc;           // elements
+  long long group_stride_c;  // elements between per-group outputs (grouped wgrad)
+  int out_fp32;
+  int accumulate;
+  const __nv_bfloat16* bias;
+  const int* tile_expert;  // grouped fwd: [m_tiles]
+  const int* seg_offsets;  // grouped wgrad: [groups+1], multiples of BK
+  int num_groups;
+  int b_group_rows;        // grouped fwd: rows of B per expert (N for K-major B, K for MN-major B)
+  int* error_flag;
+  // split-K (dense, few output tiles): `split_k` CTAs share one output tile, each writing the partial sums of its K slice
+  // to its own fp32 plane of `ws` [split_k, M, N]; the last to arrive (counter per tile and 32-row quadrant) adds the
+  // planes in slice order, writes C and resets the counter
+  int split_k;
+  float* ws;
+  int* counters;
+};
+
+static inline int num_sms() {
+  static int g_num_sms = 0;
+  if (g_num_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return g_num_sms;
+}
+
 namespace pair {
 
 static constexpr int kBM = 128, kBK = 64, kUmmaK = 16;      // rows per CTA
@@ -51,10 +82,20 @@ __device__ __forceinline__ void tile_of(int t, int m_tiles, int n_tiles, int& m,
   n = r / rows;
 }
 
+// What a warp does with its 32 rows × COLS columns of the accumulator: stores them, or what head.cu makes of them.
+struct StoreTile {
+  template <int COLS>
+  __device__ __forceinline__ void tile(const GemmParams& p, int group, int row0, uint32_t t_row, uint8_t* stage, int col0, bool empty) const {
+    const TileOut out{reinterpret_cast<uint8_t*>(p.C) + (static_cast<long long>(group) * p.group_stride_c + static_cast<long long>(row0) * p.ldc) * (p.out_fp32 ? 4 : 2),
+                      p.ldc, p.M - row0, p.N, p.out_fp32, p.accumulate, p.bias};
+    store_tile_staged<COLS>(out, t_row, stage, col0, empty);
+  }
+};
+
 // A_MN, B_MN, MODE: as gemm_bf16_kernel.
-template <int BN, int A_MN, int B_MN, int MODE, class P>
+template <int BN, int A_MN, int B_MN, int MODE, class Epi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, P p) {
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p, Epi epi) {
   using L = Layout<BN>;
   constexpr bool kFwd = MODE == 1, kWgrad = MODE == 2;
   constexpr uint32_t kTmemCols = 2 * BN;
@@ -202,7 +243,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     // ------------------------------ epilogue (warps 2..9) ------------------------------
     const int q = warp & 3;  // TMEM lane quadrant this warp may access
     const int col_in_tile = (warp - 2) / 4 * (BN / 2);
-    const int esz = p.out_fp32 ? 4 : 2;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
@@ -216,13 +256,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         if (!pass_of(m, pass, expert, mine)) continue;
         if (__any_sync(0xffffffffu, !mbar_wait_cluster(&tmem_full[acc], acc_phase) || *abort_flag)) { ok = false; break; }
         tc_fence_after();
-        if (mine) {
-          const int row0 = (2 * m + rank) * kBM + q * 32;
-          const TileOut out{reinterpret_cast<uint8_t*>(p.C) + (static_cast<long long>(group) * p.group_stride_c + static_cast<long long>(row0) * p.ldc) * esz,
-                            p.ldc, p.M - row0, p.N, p.out_fp32, p.accumulate, p.bias};
-          store_tile_staged<BN / 2>(out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + col_in_tile, smem_stage + (warp - 2) * 4096,
-                                    n * BN + col_in_tile, k_blocks == 0);
-        }
+        if (mine)
+          epi.template tile<BN / 2>(p, group, (2 * m + rank) * kBM + q * 32, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + col_in_tile,
+                                    smem_stage + (warp - 2) * 4096, n * BN + col_in_tile, k_blocks == 0);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(smem_of_rank(&tmem_empty[acc], 0));
@@ -240,6 +276,16 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, kTmemCols);
   }
+}
+
+template <int BN, int A_MN, int B_MN, int MODE, class Epi>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, const Epi& epi, int tiles, cudaStream_t stream) {
+  using L = Layout<BN>;
+  auto kern = gemm_bf16_pair_kernel<BN, A_MN, B_MN, MODE, Epi>;
+  static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
+  if (configured != cudaSuccess) return static_cast<int>(configured);
+  const int pairs = num_sms() / 2;
+  return static_cast<int>(launch_pdl(kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kThreads), L::kTotal, stream, ta, tb, p, epi));
 }
 
 }  // namespace pair

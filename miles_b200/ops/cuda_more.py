@@ -368,6 +368,11 @@ def _vocab_chunks(V):
     return [(v0, min(V, v0 + _VOCAB_CHUNK)) for v0 in range(0, V, _VOCAB_CHUNK)]
 
 
+def _head_in_place(rows: int, hidden, w) -> bool:
+    """Statistics and gradients in the product's epilogue (head.cu): more rows than the decode-sized kernels take, TMA-readable operands."""
+    return rows > 64 and hidden.shape[1] % 8 == 0 and w.is_contiguous() and w.dtype == BF16
+
+
 class _LogProbEntropy(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, w, targets, temperature, with_entropy, vocab_offset):
@@ -381,6 +386,9 @@ class _LogProbEntropy(torch.autograd.Function):
         lse = torch.empty(R, dtype=torch.float32, device=hidden.device)
         for r0 in range(0, R, _ROW_CHUNK):
             r1 = min(R, r0 + _ROW_CHUNK)
+            if _head_in_place(r1 - r0, hidden, w):
+                C.head_logprob(hidden[r0:r1], w, tg[r0:r1], inv_t, logp[r0:r1], ent[r0:r1], lse[r0:r1], C.error_flag(hidden))
+                continue
             stats = torch.empty(r1 - r0, 4, dtype=torch.float32, device=hidden.device)
             for ci, (v0, v1) in enumerate(_vocab_chunks(V)):
                 logits = gemm_nt(hidden[r0:r1], w[v0:v1], out_dtype=torch.float32)
@@ -404,11 +412,17 @@ class _LogProbEntropy(torch.autograd.Function):
             dwc = None
             for r0 in range(0, R, _ROW_CHUNK):
                 r1 = min(R, r0 + _ROW_CHUNK)
-                logits = gemm_nt(hidden[r0:r1], w[v0:v1], out_dtype=torch.float32)
                 dl = torch.empty(r1 - r0, v1 - v0, dtype=BF16, device=hidden.device)
-                C.logit_grad(logits, tg[r0:r1], lse[r0:r1], ent[r0:r1] if g_ent is not None else None,
-                             g_lp[r0:r1] if g_lp is not None else None, g_ent[r0:r1] if g_ent is not None else None, dl, v0,
-                             ctx.inv_t)
+                in_place = _head_in_place(r1 - r0, hidden, w) and (v1 - v0) % 8 == 0
+                if in_place:
+                    C.head_grad(hidden[r0:r1], w[v0:v1], tg[r0:r1] - v0, lse[r0:r1], ent[r0:r1] if g_ent is not None else None,
+                                g_lp[r0:r1] if g_lp is not None else None, g_ent[r0:r1] if g_ent is not None else None, dl, ctx.inv_t,
+                                C.error_flag(hidden))
+                else:
+                    logits = gemm_nt(hidden[r0:r1], w[v0:v1], out_dtype=torch.float32)
+                    C.logit_grad(logits, tg[r0:r1], lse[r0:r1], ent[r0:r1] if g_ent is not None else None,
+                                 g_lp[r0:r1] if g_lp is not None else None, g_ent[r0:r1] if g_ent is not None else None, dl, v0,
+                                 ctx.inv_t)
                 # dH[r0:r1] += dl · W_c   (fp32 accumulate in place)
                 Mr, Kc, Nh = r1 - r0, v1 - v0, H
                 C.gemm(dl, w[v0:v1], dh[r0:r1], Mr, Nh, Kc, Kc, Nh, H, False, True, True, None, 0)
