@@ -245,23 +245,23 @@ __global__ void __launch_bounds__(ATT_THREADS) flash_fwd_kernel(const bf16* __re
 // backward pre-pass: delta[h, t] = Σ_d dO[t,h,d]·O[t,h,d]
 // ---------------------------------------------------------------------------------------------
 template <int D>
-__global__ void attn_delta_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, float* __restrict__ delta, int T, int Hq) {
-  const long long wid = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (wid >= static_cast<long long>(T) * Hq) return;
-  const long long t = wid / Hq;
-  const int h = static_cast<int>(wid % Hq);
-  const bf16* a = o + (t * Hq + h) * D;
-  const bf16* g = dout + (t * Hq + h) * D;
+__global__ void __launch_bounds__(256) attn_delta_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, float* __restrict__ delta, int T, int Hq) {
+  // D / 8 lanes per (token, head) row with one 16-byte piece of each tensor: bound by the two reads (4-byte loads left it at a third of
+  // the bandwidth: 88 µs for 12 075 × 32 rows, floor 31)
+  constexpr int kLanes = D / 8;
+  const long long row = (blockIdx.x * 256ll + threadIdx.x) / kLanes;
+  const int lane = threadIdx.x % kLanes;
   float s = 0.f;
-  for (int i = lane * 2; i < D; i += 64) {
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(a + i));
-    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(g + i));
-    s += x.x * y.x + x.y * y.y;
+  if (row < static_cast<long long>(T) * Hq) {
+    const uint4 a = *reinterpret_cast<const uint4*>(o + row * D + lane * 8), g = *reinterpret_cast<const uint4*>(dout + row * D + lane * 8);
+    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      s += __uint_as_float(aw[i] << 16) * __uint_as_float(gw[i] << 16) + __uint_as_float(aw[i] & 0xffff0000u) * __uint_as_float(gw[i] & 0xffff0000u);
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) delta[static_cast<long long>(h) * T + t] = s;
+  for (int off = kLanes / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  if (lane == 0 && row < static_cast<long long>(T) * Hq) delta[row % Hq * T + row / Hq] = s;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -691,8 +691,7 @@ extern "C" int mb_flash_fwd(const void* q, const void* k, const void* v, void* o
 // delta[h, t] = Σ_d dO[t, h, d] · O[t, h, d] (the backward's pre-pass, shared by both backward implementations)
 extern "C" int mb_attn_delta(const void* o, const void* dout, float* delta, int total_tokens, int Hq, int D, cudaStream_t s) {
   if (total_tokens == 0) return 0;
-  const long long warps = static_cast<long long>(total_tokens) * Hq;
-  const unsigned blocks = static_cast<unsigned>((warps + 7) / 8);
+  const unsigned blocks = static_cast<unsigned>((static_cast<long long>(total_tokens) * Hq * (D / 8) + 255) / 256);
   if (D == 128) attn_delta_kernel<128><<<blocks, 256, 0, s>>>(reinterpret_cast<const bf16*>(o), reinterpret_cast<const bf16*>(dout), delta, total_tokens, Hq);
   else if (D == 64) attn_delta_kernel<64><<<blocks, 256, 0, s>>>(reinterpret_cast<const bf16*>(o), reinterpret_cast<const bf16*>(dout), delta, total_tokens, Hq);
   else return -1;

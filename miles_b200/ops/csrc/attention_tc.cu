@@ -18,10 +18,10 @@
 // (1086) and 0.53 ms (883), and 0.57 ms (1143) at one sequence of 8190 and one of 3601 with 8 KV heads.  Short sequences pay for the
 // half-masked diagonal blocks and the first block's latency: 450 TFLOP/s at 32 × 512.
 //
-// Schedule.  Items are ordered by query tile, last (longest) first, and dealt to the CTAs forth and back (0..G-1, G-1..0, ...), which
-// keeps the sums of unlike items level without atomics; every warp walks the same list (`Items`), 32 sequences per step.
+// Schedule: attention_items.cuh.
 // Q, K, V are read with 2-D tensor maps over [tokens, heads·128]; rows of a tile that belong to the next sequence are masked as keys and
 // never stored as queries.  All barrier waits are bounded (error flag + early exit).
+#include "attention_items.cuh"
 #include "launch.h"
 #include "pdl.cuh"
 #include "ptx.cuh"
@@ -47,10 +47,9 @@ struct Params {
   const int* cu_seqlens_k;     // null: keys are the queries' own sequences.  Else sequence b has keys [cu_k[b], cu_k[b+1]) and, under
                                // the causal mask, query i sees keys ≤ i + (Lk − Lq): the queries are the LAST Lq positions of the keys
                                // (a prompt continued after a cached prefix, a later chunk of a long prompt)
-  int Hq, Hkv, total_tokens, batch;
+  int Hq, Hkv, total_tokens;
   int pair_heads;              // the two tiles of an item: heads 2i, 2i + 1 (1) or query tiles 2i, 2i + 1 (0)
-  int per_seq;                 // items per (sequence, level): Hq / 2 or Hq
-  int levels;                  // query levels of the longest sequence (128 or 256 queries each)
+  ItemList list;               // levels of 128 or 256 queries, Hq / 2 or Hq items per sequence and level
   float scale;
   int causal;
   int* error_flag;
@@ -61,43 +60,6 @@ struct Smem {
   static constexpr int kv = q + 2 * kTileBytes;
   static constexpr int bars = kv + kSlots * kTileBytes;
   static constexpr int total = bars + 256;   // the dynamic segment is declared 1024-byte aligned; checked at run time
-};
-
-// The items of this CTA, in order.  All lanes of a warp call `next` together.
-struct Items {
-  int level, chunk, base, target, round;
-  uint32_t mask;               // sequences chunk·32 + i that have queries at this level
-  __device__ __forceinline__ void scan(const Params& p) {
-    const int b = chunk * 32 + static_cast<int>(lane_id());
-    int len = 0;
-    if (b < p.batch) len = p.cu_seqlens[b + 1] - p.cu_seqlens[b];
-    mask = __ballot_sync(0xffffffffu, len > level * (p.pair_heads ? BQ : 2 * BQ));
-  }
-  __device__ __forceinline__ void init(const Params& p) {
-    level = p.levels - 1;
-    chunk = base = round = 0;
-    scan(p);
-  }
-  __device__ __forceinline__ bool next(const Params& p, int& b, int& sub) {
-    const int g = static_cast<int>(gridDim.x), i = static_cast<int>(blockIdx.x);
-    target = round * g + ((round & 1) ? g - 1 - i : i);
-    ++round;
-    for (;;) {
-      const int n = __popc(mask) * p.per_seq;
-      if (target < base + n) {
-        const int at = target - base;
-        b = chunk * 32 + static_cast<int>(__fns(mask, 0, at / p.per_seq + 1));
-        sub = at % p.per_seq;
-        return true;
-      }
-      base += n;
-      if (++chunk * 32 >= p.batch) {
-        chunk = 0;
-        if (--level < 0) return false;
-      }
-      scan(p);
-    }
-  }
 };
 
 // One item: where its two tiles are and how many key blocks each of them takes.
@@ -187,7 +149,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   pdl_wait();
 
   Items items;
-  items.init(p);
+  items.init(p.list);
   int b, sub;
   if (warp >= 8) {
     reg_dealloc<88>();
@@ -195,7 +157,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       // ------------------------------ TMA producer ------------------------------
       const bool leader = elect_one();
       uint32_t c = 0, qc[2] = {0, 0};                      // ring slots filled, Q tiles loaded
-      while (!__any_sync(0xffffffffu, *abort_flag) && items.next(p, b, sub)) {
+      while (!__any_sync(0xffffffffu, *abort_flag) && items.next(p.list, b, sub)) {
         const Item it(p, items.level, b, sub);
         if (leader) {
           bool ok = true;
@@ -235,7 +197,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       constexpr uint32_t idesc_o = make_idesc_bf16(BQ, D, 0, 1);     // O = P (tensor memory) · V (MN-major, N = head dim)
       const uint32_t kv_addr = smem_u32(smem + Smem::kv);
       uint32_t c = 0, qc[2] = {0, 0}, pc[2] = {0, 0};      // ring slots consumed, Q tiles, blocks of P
-      while (!__any_sync(0xffffffffu, *abort_flag) && items.next(p, b, sub)) {
+      while (!__any_sync(0xffffffffu, *abort_flag) && items.next(p.list, b, sub)) {
         const Item it(p, items.level, b, sub);
         const int n = max(it.n[0], it.n[1]);
         if (leader) {
@@ -304,7 +266,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const float sl2 = p.scale * kLog2e;
     uint32_t sc = 0, oc = 0;                  // blocks of S, items
     bool ok = true;
-    while (items.next(p, b, sub)) {
+    while (items.next(p.list, b, sub)) {
       const Item it(p, items.level, b, sub);
       const int n = t ? it.n[1] : it.n[0], q0 = t ? it.q0[1] : it.q0[0], h = t ? it.h[1] : it.h[0], qpos = q0 + row;
       if (n == 0) continue;
@@ -451,19 +413,17 @@ extern "C" int mb_flash_fwd_tc(const void* q, const void* k, const void* v, void
   p.Hq = Hq;
   p.Hkv = Hkv;
   p.total_tokens = total_tokens;
-  p.batch = batch;
   p.scale = scale;
   p.causal = causal;
   p.error_flag = error_flag;
   // two heads with the same keys have equal ranges; two neighbouring tiles of one head do not, but serve any number of heads
   p.pair_heads = (Hq / Hkv) % 2 == 0;
-  p.per_seq = p.pair_heads ? Hq / 2 : Hq;
   const int rows = p.pair_heads ? fa::BQ : 2 * fa::BQ;
-  p.levels = (max_seqlen + rows - 1) / rows;
+  p.list = ItemList{cu_seqlens, batch, p.pair_heads ? Hq / 2 : Hq, (max_seqlen + rows - 1) / rows, rows};
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long most = static_cast<long long>(p.levels) * batch * p.per_seq;
+  const long long most = static_cast<long long>(p.list.levels) * batch * p.list.per_seq;
   const int grid = static_cast<int>(most < sms ? most : sms);
   return static_cast<int>(launch_pdl(fa::flash_fwd_tc_kernel, dim3(grid), dim3(fa::kThreads), fa::Smem::total, s, tq, tk, tv, p));
 }

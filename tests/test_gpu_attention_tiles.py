@@ -53,3 +53,25 @@ def test_flash_forward_tiles(heads, lens, key_lens, causal):
     assert ((o.double() - ref).norm() / ref.norm()).item() < 2 ** -8
     assert (lse.double() - ref_lse).abs().max().item() < 1e-4
     assert K.check_error_flag(q) == 0
+
+
+@pytest.mark.parametrize("heads", [(8, 1), (4, 4), (6, 2)])
+@pytest.mark.parametrize("lens,causal", [([1], True), ([127, 128, 129], True), ([255, 257, 0, 64, 700], True), ([300, 1, 129], False), ([64] * 40 + [260], True)])
+def test_flash_backward_tiles(heads, lens, causal):
+    from miles_b200.ops import cuda_more as M
+    from miles_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(6)
+    hq, hkv = heads
+    cu = _offsets(lens)
+    q, k, v, do = (torch.randn(cu[-1], n, 128, device="cuda", generator=g).bfloat16() for n in (hq, hkv, hkv, hq))
+    leaves = [t.clone().requires_grad_() for t in (q, k, v)]
+    o = M._FlashAttn.apply(*leaves, torch.tensor(cu, dtype=torch.int32, device="cuda"), max(lens), causal)
+    o.backward(do)
+    exact = [t.double().requires_grad_() for t in (q, k, v)]
+    _softmax64(*exact, cu, cu, causal)[0].backward(do.double())
+    for a, b in zip(leaves, exact):
+        # P and dS are rounded to bf16 before their products and the gradients after them, Δ comes from a rounded output: 2^-9 each
+        assert (a.grad.double() - b.grad).norm().item() <= 2 ** -6.5 * b.grad.norm().item() + 1e-3 * (b.numel() ** 0.5 if max(lens) == 1 else 0.0)
+        assert torch.isfinite(a.grad).all()
+    assert K.check_error_flag(q) == 0
