@@ -53,6 +53,16 @@ void gemm_splitk(const at::Tensor& A, const at::Tensor& B, at::Tensor& C, int64_
         "mb_gemm_bf16_splitk");
 }
 
+// tokens ≤ 64, weight rows on the 128-row MMA side, `split` CTAs of a cluster per 128 of them (gemm_rows.cu)
+void gemm_rows(const at::Tensor& X, const at::Tensor& W, at::Tensor& C, int64_t tokens, int64_t N, int64_t K, int64_t ldc,
+               const c10::optional<at::Tensor>& bias, int64_t split, bool static_w) {
+  c10::cuda::CUDAGuard g(X.device());
+  int* ef = error_flag_for(X.device()).data_ptr<int>();
+  check(mb_gemm_rows(X.data_ptr(), W.data_ptr(), C.data_ptr(), tokens, N, K, K, K, ldc, C.scalar_type() == at::kFloat, cptr(bias), split, static_w, ef,
+                     cur_stream()),
+        "mb_gemm_rows");
+}
+
 // C[tokens, N] = X[tokens, K] · W[N, K]ᵀ with the weight rows on the 128-row MMA side (decode-sized token counts)
 void gemm_small(const at::Tensor& X, const at::Tensor& W, at::Tensor& C, int64_t tokens, int64_t N, int64_t K, int64_t ldc,
                 const c10::optional<at::Tensor>& bias, int64_t bt, int64_t split_k, const c10::optional<at::Tensor>& ws,
@@ -240,6 +250,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("count_launches", [](int64_t n) { mb_count_launch(static_cast<int>(n)); });
   m.def("gemm", &gemm);
   m.def("gemm_splitk", &gemm_splitk);
+  m.def("gemm_rows", &gemm_rows);
   m.def("gemm_grouped", &gemm_grouped);
   m.def("gemm_small", &gemm_small);
   m.def("gemv", &gemv);

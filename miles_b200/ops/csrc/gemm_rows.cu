@@ -1,0 +1,245 @@
+// Projections of 9 to 64 tokens:  C[tokens, N] = X[tokens, K] · W[N, K]ᵀ  with every SM streaming weights.
+//
+// As in gemm_small.cu the weight rows are the 128-row side of the MMA and the tokens its N side (16, 32 or 64).  A projection of a model
+// has 16 to 160 such tiles, so the reduction is cut as well: a CLUSTER of 1, 2, 4 or 8 CTAs shares one tile, each CTA streams its slice of
+// K, and the partial accumulators meet in distributed shared memory.  CTA r of a cluster owns tokens [r · BT/S, (r + 1) · BT/S): every CTA
+// stores its partial sums of those tokens into r's buffer, and after one cluster barrier r adds them in slice order and writes them out.
+//   warp 0      TMA producer.  Weights that no kernel of the stream writes (`static_w`) are requested before the dependency wait: the
+//               first stages arrive while the kernel in front is still running
+//   warp 1      TMEM + tcgen05.mma issue
+//   warps 2..5  accumulator → owners' buffers → output
+//
+// What bounds it: the weight bytes, and with 5 to 100 MB of them per call the time until all SMs have loads in flight.  Two CTAs fit an SM
+// (72 to 90 KB in flight each), so up to 296 tiles × slices run at once and 152 tiles do not become two waves; where all of them fit with an
+// SM each, the ring is as deep as the SM allows.  The earlier forms were
+// 128-row token tiles (3/4 padding) with 64 columns per CTA, whose sums over K met in global memory behind atomic counters for ≤ 32 tokens.
+// Measured, weights from memory, 9 / 19 / 61 tokens against the 128-row tiles: 5120 × 2048 15.4 / 14.9 / 8.8 → 6.2 / 6.3 / 8.4 µs,
+// 2048 × 4096 17.0 / 13.0 / 13.1 → 6.2 / 6.8 / 8.2, 2560 × 9728 26.6 / 26.7 / 26.7 → 11.1 / 11.7 / 13.9 (7.7 at the memory's speed).
+#include "launch.h"
+#include "pdl.cuh"
+#include "ptx.cuh"
+
+namespace mb {
+
+int make_tmap_bf16_2d(CUtensorMap* out, const void* base, long long rows, long long cols, long long ld, int box_rows, int box_cols);
+
+namespace rows {
+
+static constexpr int BMW = 128;     // weight rows (output features) per tile
+static constexpr int BK = 64;
+static constexpr int kMaxSplit = 8;
+static constexpr int kSms = 148, kWideClusters = 12;
+
+struct Params {
+  int tokens, N, K;
+  void* C;
+  long long ldc;
+  int out_fp32;
+  const __nv_bfloat16* bias;
+  int static_w;
+  int stages;
+  int* error_flag;
+};
+
+template <int BT>
+struct Layout {
+  static constexpr int kShallow = BT == 64 ? 3 : BT == 32 ? 4 : 5, kDeep = BT == 64 ? 8 : BT == 32 ? 10 : 12;   // stages: two CTAs per SM, one
+  static constexpr int kABytes = BMW * BK * 2;         // weights: 16 KB
+  static constexpr int kBBytes = BT * BK * 2;          // tokens: 2 / 4 / 8 KB
+  static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kSumBytes = BT * BMW * 4;       // [slice][own tokens][feature] floats
+  static constexpr int total(int stages) { return stages * kStageBytes + kSumBytes + 256 + 1024; }
+};
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void st_cluster(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+
+template <int BT, int split>
+__global__ void __launch_bounds__(192, 2)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, Params p) {
+  using L = Layout<BT>;
+  constexpr uint32_t kTmemCols = BT < 32 ? 32 : BT;
+  const int stages = p.stages;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem_a = smem;
+  uint8_t* smem_b = smem + stages * L::kABytes;
+  float* sums = reinterpret_cast<float*>(smem + stages * L::kStageBytes);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + stages * L::kStageBytes + L::kSumBytes);
+  uint64_t* empty_bar = full_bar + stages;
+  uint64_t* tmem_full = empty_bar + stages;
+  uint32_t* tmem_base_ptr = reinterpret_cast<uint32_t*>(tmem_full + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slice = static_cast<int>(blockIdx.x) % split, n_blk = static_cast<int>(blockIdx.x) / split;   // the cluster is one tile's slices
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    mbar_init(tmem_full, 1);
+    mbar_fence_init();
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_x);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_base_ptr, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_base_ptr;
+  if (split > 1) cluster_arrive();                 // "my buffer exists": waited for before the first remote store
+  pdl_trigger();
+
+  const int total_kb = (p.K + BK - 1) / BK, per = (total_kb + split - 1) / split;
+  const int kb0 = slice * per, kbs = max(0, min(per, total_kb - kb0));
+
+  if (warp == 0) {
+    if (elect_one()) {
+      auto load_w = [&](int kb, int stage) {
+        mbar_expect_tx(&full_bar[stage], L::kStageBytes);
+        tma_load_2d(smem_a + stage * L::kABytes, &tmap_w, &full_bar[stage], (kb0 + kb) * BK, n_blk * BMW);
+      };
+      auto load_x = [&](int kb, int stage) { tma_load_2d(smem_b + stage * L::kBBytes, &tmap_x, &full_bar[stage], (kb0 + kb) * BK, 0); };
+      const int early = min(kbs, stages);
+      if (p.static_w)
+        for (int kb = 0; kb < early; ++kb) load_w(kb, kb);
+      pdl_wait();
+      for (int kb = 0; kb < early; ++kb) {
+        if (!p.static_w) load_w(kb, kb);
+        load_x(kb, kb);
+      }
+      for (int kb = early; kb < kbs; ++kb) {
+        const int stage = kb % stages;
+        if (!mbar_wait(&empty_bar[stage], (kb / stages - 1) & 1)) { atomicExch(p.error_flag, 45); break; }
+        load_w(kb, stage);
+        load_x(kb, stage);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_idesc_bf16(BMW, BT, 0, 0);
+      for (int kb = 0; kb < kbs; ++kb) {
+        const int stage = kb % stages;
+        if (!mbar_wait(&full_bar[stage], (kb / stages) & 1)) { atomicExch(p.error_flag, 46); break; }
+        tc_fence_after();
+        const uint32_t a_addr = smem_u32(smem_a + stage * L::kABytes);
+        const uint32_t b_addr = smem_u32(smem_b + stage * L::kBBytes);
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          umma_bf16(tmem_base, make_smem_desc_sw128(a_addr + k * 32, 16, 1024), make_smem_desc_sw128(b_addr + k * 32, 16, 1024), idesc, (kb | k) != 0);
+        umma_commit(&empty_bar[stage]);
+      }
+      umma_commit(tmem_full);
+    }
+    __syncwarp();
+  }
+  const int q = warp & 3;
+  const int n = n_blk * BMW + q * 32 + lane;         // output feature of this thread (warps 2..5)
+  float v[BT];
+  if (warp >= 2) {
+    pdl_wait();                                      // C and the bias: after the kernels in front
+    if (!mbar_wait(tmem_full, 0)) atomicExch(p.error_flag, 47);
+    __syncwarp();
+    tc_fence_after();
+#pragma unroll
+    for (int c = 0; c < BT / 16; ++c) {
+      uint32_t r[16];
+      tmem_ld_32x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + c * 16, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[c * 16 + i] = kbs > 0 ? __uint_as_float(r[i]) : 0.f;
+    }
+    tc_fence_before();
+  }
+  const int tokens = n < p.N ? p.tokens : 0;         // a feature past the last one stores nothing
+  const float bias = warp >= 2 && tokens > 0 && p.bias != nullptr ? __bfloat162float(p.bias[n]) : 0.f;
+  auto put = [&](int tok, float x) {                 // lanes hold consecutive features: one 64- or 128-byte store per token and warp
+    if (p.bias != nullptr) x += bias;
+    if (p.out_fp32) reinterpret_cast<float*>(p.C)[tok * p.ldc + n] = x;
+    else reinterpret_cast<__nv_bfloat16*>(p.C)[tok * p.ldc + n] = __float2bfloat16(x);
+  };
+  if (split == 1) {
+    if (warp >= 2) {
+#pragma unroll
+      for (int i = 0; i < BT; ++i)
+        if (i < tokens) put(i, v[i]);
+    }
+  } else {
+    constexpr int own = BT / split;
+    cluster_wait();
+    if (warp >= 2) {
+#pragma unroll
+      for (int o = 0; o < split; ++o) {
+        const uint32_t to = smem_of_rank(sums + slice * own * BMW + q * 32 + lane, o);
+#pragma unroll
+        for (int i = 0; i < own; ++i)
+          if (o * own + i < tokens) st_cluster(to + i * BMW * 4, v[o * own + i]);
+      }
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();                                  // every slice's sums are in their owners' buffers; nothing remote is touched after this
+    if (warp >= 2) {
+#pragma unroll 4
+      for (int i = 0; i < min(own, tokens - slice * own); ++i) {
+        float x = 0.f;
+#pragma unroll
+        for (int s = 0; s < split; ++s) x += sums[(s * own + i) * BMW + q * 32 + lane];
+        put(slice * own + i, x);
+      }
+    }
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+template <int BT, int split>
+static int launch_as(const CUtensorMap& tw, const CUtensorMap& tx, Params p, cudaStream_t s) {
+  using L = Layout<BT>;
+  static const cudaError_t configured = cudaFuncSetAttribute(gemm_rows_kernel<BT, split>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total(L::kDeep));
+  if (configured != cudaSuccess) return static_cast<int>(configured);
+  const int tiles = (p.N + BMW - 1) / BMW;
+  // a CTA with an SM to itself has twice the bytes in flight: the ring is deep where all clusters fit that way.  Eight neighbouring SMs are
+  // found 12 times at least; 16 such clusters took two waves (2048 × 4096, 9 tokens: 9.0 µs, 6.2 for 16 clusters of four)
+  p.stages = tiles <= (split == kMaxSplit ? kWideClusters : kSms / split) ? L::kDeep : L::kShallow;
+  return static_cast<int>(launch_pdl_cluster(gemm_rows_kernel<BT, split>, dim3(tiles * split), dim3(192), split, L::total(p.stages), s, tw, tx, p));
+}
+
+template <int BT>
+static int launch(const CUtensorMap& tw, const CUtensorMap& tx, const Params& p, int split, cudaStream_t s) {
+  switch (split) {
+    case 1: return launch_as<BT, 1>(tw, tx, p, s);
+    case 2: return launch_as<BT, 2>(tw, tx, p, s);
+    case 4: return launch_as<BT, 4>(tw, tx, p, s);
+    default: return launch_as<BT, 8>(tw, tx, p, s);
+  }
+}
+
+}  // namespace rows
+}  // namespace mb
+
+// C[tokens, N] (bf16 or fp32) = X[tokens, K] · W[N, K]ᵀ (+ bias), tokens ≤ 64.  split: 1, 2, 4 or 8 slices of K.  static_w: no kernel that may
+// still run on the stream writes W.
+extern "C" int mb_gemm_rows(const void* X, const void* W, void* C, int tokens, int N, int K, long long ldx, long long ldw, long long ldc, int out_fp32,
+                            const void* bias, int split, int static_w, int* error_flag, cudaStream_t s) {
+  using namespace mb;
+  if (tokens <= 0 || N <= 0) return 0;
+  if (tokens > 64 || (split != 1 && split != 2 && split != 4 && split != rows::kMaxSplit)) return -2;
+  const int bt = tokens <= 16 ? 16 : tokens <= 32 ? 32 : 64;
+  CUtensorMap tw, tx;
+  int r = make_tmap_bf16_2d(&tw, W, N, K, ldw, rows::BMW, rows::BK);
+  if (r) return 1000 + r;
+  r = make_tmap_bf16_2d(&tx, X, tokens, K, ldx, bt, rows::BK);
+  if (r) return 2000 + r;
+  const rows::Params p{tokens, N, K, C, ldc, out_fp32, reinterpret_cast<const __nv_bfloat16*>(bias), static_w, 0, error_flag};
+  switch (bt) {
+    case 16: return rows::launch<16>(tw, tx, p, split, s);
+    case 32: return rows::launch<32>(tw, tx, p, split, s);
+    default: return rows::launch<64>(tw, tx, p, split, s);
+  }
+}

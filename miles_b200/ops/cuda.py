@@ -74,13 +74,19 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *
         out = torch.empty(M, N, dtype=out_dtype or BF16, device=a.device)
     if M and N:
         plain = not accumulate and not force_bn
-        if plain and M <= GEMV_M and _gemv_k_ok(M, K) and N <= GEMV_MAX_N:
+        split = _row_split(M, N, K) if plain and M <= SMALL_M else 0
+        # the matrix-vector kernel takes its rows eight at a time: from nine on a cluster per weight tile is faster (9 rows, N × K: 5120 × 2048
+        # 8.3 → 6.2 µs, 2560 × 4096 11.7 → 6.0, 19456 × 2560 37.3 → 19.6, 6144 × 1024 4.6 → 4.5)
+        if plain and M <= (8 if split else GEMV_M) and M <= GEMV_M and _gemv_k_ok(M, K) and N <= GEMV_MAX_N:
             C.gemv(a, None, None, 0.0, b, bias, out, None, None, bool(b.is_leaf and b.requires_grad))
             return out
-        # measured: the operand-swapped kernel wins where its tiles fill the GPU without split-K (wide outputs such as the
-        # LM head); with split-K its reduction costs more than the padding rows of the general kernel
-        if plain and M <= SMALL_M and K >= 256 and (SMALL_SPLIT or _small_split(M, N, K, small_bt(M)) == 1):
-            return _gemm_small(a, b, out, bias, M, N, K)
+        if plain and M <= SMALL_M:
+            if split:
+                C.gemm_rows(a, b, out, M, N, K, out.stride(0), bias, split, bool(b.is_leaf and b.requires_grad))
+                return out
+            if K >= 256 and not (M > 32 and N <= 296 * 128):
+                C.gemm_small(a, b, out, M, N, K, out.stride(0), bias, small_bt(M), 1, None, None)
+                return out
         split = _pick_split_k(M, N, K) if not force_bn and SPLIT_K else 1
         if split > 1:
             ws, counters = _splitk_workspace(a.device)
@@ -90,8 +96,8 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *
     return out
 
 
-# Decode-sized GEMMs (a handful of 128×64 output tiles over a long K) leave most SMs idle; split-K gives every tile
-# several CTAs, each streaming a slice of the weights.  Workspace: fp32 [split, M, N] planes + arrival counters (zero
+# What is left of decode-sized GEMMs (accumulating ones) has a handful of 128×64 output tiles over a long K and leaves most SMs idle; split-K
+# gives every tile several CTAs, each streaming a slice of the weights.  Workspace: fp32 [split, M, N] planes + arrival counters (zero
 # between calls; the kernel restores that), one per device, so such GEMMs must not overlap on two streams of one device.
 SPLIT_K = os.environ.get("MILES_SPLIT_K", "1") != "0"
 _SPLITK_MAX_M, _SPLITK_MAX_TILES = int(os.environ.get("MILES_SPLIT_K_MAX_M", "32")), 74   # measured: wins below ~32 rows
@@ -150,39 +156,25 @@ def gemv_ok(x, w) -> bool:
 
 
 # Decode-sized token counts: the weight rows go on the 128-row side of the MMA and the tokens on the N side in tiles of
-# 16/32/64 (gemm_small.cu), so no pipeline byte is spent on padding rows; split-K fills the SMs.  0 turns the path off.
+# 16/32/64, so no pipeline byte is spent on padding rows.  0 turns the path off.
 SMALL_M = int(os.environ.get("MILES_SMALL_M", "64"))
-SMALL_SPLIT = os.environ.get("MILES_SMALL_SPLIT", "0") == "1"     # also use it where it needs split-K
-_SMALL_WS_FLOATS, _SMALL_MAX_TILES = 4 << 20, 4096
-_small_ws: dict = {}
 
 
 def small_bt(rows: int) -> int:
     return 16 if rows <= 16 else 32 if rows <= 32 else 64
 
 
-def _small_split(M: int, N: int, K: int, bt: int) -> int:
-    out_tiles = ((N + 127) // 128) * ((M + bt - 1) // bt)
-    kblocks = (K + 63) // 64
-    split = max(1, min(round(148 / out_tiles), kblocks // 2, 32))
-    if split > 1 and (out_tiles > _SMALL_MAX_TILES or split * M * N > _SMALL_WS_FLOATS):
-        return 1
-    per = -(-kblocks // split)
-    return -(-kblocks // per)          # every slice gets at least one K block
-
-
-def _gemm_small(a, b, out, bias, M, N, K):
-    bt = small_bt(M)
-    split = _small_split(M, N, K, bt)
-    ws = counters = None
-    if split > 1:
-        key = a.device.index if a.device.index is not None else torch.cuda.current_device()
-        if key not in _small_ws:
-            _small_ws[key] = (torch.empty(_SMALL_WS_FLOATS, dtype=torch.float32, device=a.device),
-                              torch.zeros(4 * _SMALL_MAX_TILES, dtype=torch.int32, device=a.device))
-        ws, counters = _small_ws[key]
-    C.gemm_small(a, b, out, M, N, K, out.stride(0), bias, bt, split, ws, counters)
-    return out
+def _row_split(M: int, N: int, K: int) -> int:
+    """CTAs that share one 128-row weight tile (gemm_rows.cu): as many as fit the GPU at once, two per SM, with at least two 64-deep steps
+    each; one where sums over K may not be cut (MILES_SPLIT_K=0).  Eight only where twelve clusters of them, an SM per CTA, or all of
+    them in pairs per SM are enough (13 to 18 tiles: four; 16 tiles, K 4096, 61 tokens: 8.2 µs against 12.1).  0: more tiles than that:
+    the persistent kernels walk through them (gemm_small.cu; from 33 tokens also where no reduction is cut and the 128-row tiles of
+    gemm.cu are as fast: 152 tiles, K 2560: 32 tokens 21.9 against 24.1 µs, 48 tokens 25.2 against 24.3)."""
+    tiles, steps = (N + 127) // 128, (K + 63) // 64
+    if tiles > 148 and M > 32:
+        return 0
+    return next((s for s in ((8, 4, 2, 1) if SPLIT_K else (1,))
+                 if tiles * s <= 296 and (steps >= 2 * s or s == 1) and not (s == 8 and 12 < tiles <= 18)), 0)
 
 
 def gemm_nn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *, out_dtype=None, force_bn: int = 0):
