@@ -217,13 +217,7 @@ class MoEFFN(nn.Module):
         if meta.replay_topk is not None:
             # R3: recorded indices replace top-k, weights come from the current scores so the gate
             # still receives gradient (reference: miles/utils/replay_base.py:87-144).
-            probs = torch.softmax(logits, dim=-1)
-            idx = self.ps.sp_slice(meta.replay_topk)[:, self.moe_index, :]
-            bad = (idx < 0).all(dim=-1)
-            if bad.any():
-                _, fresh, _ = ops.router_topk(logits, k, norm)
-                idx = torch.where(bad[:, None], fresh, idx)
-            w = ops.gather_router_weights(probs, idx, norm)
+            w, idx, _ = ops.router_replay(logits, self.ps.sp_slice(meta.replay_topk)[:, self.moe_index, :], norm)
         else:
             w, idx, _ = ops.router_topk(logits, k, norm)
         if meta.record_topk is not None:

@@ -131,6 +131,14 @@ def router_topk(logits, k, normalize=True):
     return ref.router_topk(logits, k, normalize)
 
 
+def router_replay(logits, idx, normalize=True):
+    """`router_topk` with recorded choices [T, k] in the place of the largest: (weights from the current scores, choices, probabilities).
+    Rows without a record (all negative) are chosen afresh."""
+    if logits.is_cuda:
+        return _k().router_replay(logits, idx, normalize)
+    return ref.router_replay(logits, idx, normalize)
+
+
 def gather_router_weights(probs, idx, normalize=True):
     return ref.gather_router_weights(probs, idx, normalize)
 

@@ -31,10 +31,13 @@ __device__ __forceinline__ float wmax(float v) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// `replay`: recorded choices, rows `replay_row` apart.  They replace the top-k and their weights come from these logits; a row without any
+// (all negative) is chosen afresh.  In one launch where softmax, gather, sum and division were kernels of their own behind a host
+// synchronisation that asked whether any row was without: 12 launches and a round trip per layer.
 template <int EPL>  // experts per lane = E / 32
 __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restrict__ logits, float* __restrict__ probs,
                                                           float* __restrict__ topk_w, int* __restrict__ topk_idx, long long T, int E,
-                                                          int K, int normalize) {
+                                                          int K, int normalize, const int* __restrict__ replay, long long replay_row) {
   pdl_trigger();
   pdl_wait();
   const long long t = (blockIdx.x * 256ll + threadIdx.x) >> 5;
@@ -64,7 +67,19 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
   }
   float wsel = 0.f, mine_w = 0.f;
   int mine_i = 0;
-  for (int j = 0; j < K; ++j) {
+  const int recorded = replay != nullptr && lane < K ? replay[t * replay_row + lane] : -1;
+  const bool replayed = __any_sync(0xffffffffu, recorded >= 0);
+  for (int j = 0; replayed && j < K; ++j) {
+    const int e = __shfl_sync(0xffffffffu, recorded, j);
+    float p = 0.f;
+#pragma unroll
+    for (int i = 0; i < EPL; ++i) p = (e >> 5) == i ? v[i] : p;
+    p = __shfl_sync(0xffffffffu, p, e & 31);
+    if (e < 0 || e >= E) p = 0.f;
+    wsel += p;
+    if (lane == j) { mine_w = p; mine_i = e; }
+  }
+  for (int j = 0; !replayed && j < K; ++j) {
     float bv = -1.f;
     int bi = 0x7fffffff;
 #pragma unroll
@@ -416,16 +431,16 @@ using namespace mb;
 MB_DEFINE_BOUNDS_API(mb_moe_bounds)
 
 extern "C" int mb_router_topk(const float* logits, float* probs, float* topk_w, int* topk_idx, long long T, int E, int K,
-                              int normalize, cudaStream_t s) {
+                              int normalize, const int* replay, long long replay_row, cudaStream_t s) {
   if (T == 0) return 0;
   if (E > 256 || K > 32) return -1;
   const unsigned blocks = static_cast<unsigned>((T + 7) / 8);
   const int epl = (E + 31) / 32;
   cudaError_t e;
-  if (epl <= 1) e = launch_pdl(router_topk_kernel<1>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize);
-  else if (epl <= 2) e = launch_pdl(router_topk_kernel<2>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize);
-  else if (epl <= 4) e = launch_pdl(router_topk_kernel<4>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize);
-  else e = launch_pdl(router_topk_kernel<8>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize);
+  if (epl <= 1) e = launch_pdl(router_topk_kernel<1>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row);
+  else if (epl <= 2) e = launch_pdl(router_topk_kernel<2>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row);
+  else if (epl <= 4) e = launch_pdl(router_topk_kernel<4>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row);
+  else e = launch_pdl(router_topk_kernel<8>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row);
   return static_cast<int>(e);
 }
 

@@ -125,8 +125,8 @@ def paged_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens=None, max
 
 class _RouterTopK(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, logits, k, normalize):
-        w, idx, probs = C.router_topk(_c(logits.float()), k, normalize, True)
+    def forward(ctx, logits, k, normalize, replay):
+        w, idx, probs = C.router_topk(_c(logits.float()), k, normalize, True, replay)
         ctx.save_for_backward(probs, idx, w)
         ctx.normalize = normalize
         ctx.mark_non_differentiable(idx)
@@ -148,13 +148,20 @@ class _RouterTopK(torch.autograd.Function):
             gp = gp + gprobs
         # softmax backward
         gl = probs * (gp - (gp * probs).sum(-1, keepdim=True))
-        return gl, None, None
+        return gl, None, None, None
 
 
 def router_topk(logits, k, normalize=True):
     if logits.shape[-1] > 256:
         return ref.router_topk(logits, k, normalize)
-    return _RouterTopK.apply(logits, int(k), bool(normalize))
+    return _RouterTopK.apply(logits, int(k), bool(normalize), None)
+
+
+def router_replay(logits, idx, normalize=True):
+    if logits.shape[-1] > 256 or idx.shape[1] > 32:
+        return ref.router_replay(logits, idx, normalize)
+    idx = idx.to(torch.int32)
+    return _RouterTopK.apply(logits, idx.shape[1], bool(normalize), idx if idx.stride(1) == 1 else idx.contiguous())
 
 
 # ---------------------------------------------------------------------------------------------

@@ -67,6 +67,17 @@ def router_topk(logits: torch.Tensor, k: int, normalize: bool = True):
     return w, idx.to(torch.int32), probs
 
 
+def router_replay(logits: torch.Tensor, idx: torch.Tensor, normalize: bool = True):
+    """Routing replay: recorded choices replace the top-k (rows that are all negative are chosen afresh), weights come from the current
+    scores.  Returns (weights fp32 [T,k], indices [T,k], probs fp32 [T,E])."""
+    probs = torch.softmax(logits.float(), dim=-1)
+    bad = (idx < 0).all(dim=-1)
+    if bad.any():
+        _, fresh, _ = router_topk(logits, idx.shape[1], normalize)
+        idx = torch.where(bad[:, None], fresh, idx)
+    return gather_router_weights(probs, idx, normalize), idx, probs
+
+
 def gather_router_weights(probs: torch.Tensor, idx: torch.Tensor, normalize: bool = True) -> torch.Tensor:
     """Routing replay: weights re-gathered from *current* probabilities at recorded indices."""
     w = probs.gather(1, idx.long())
