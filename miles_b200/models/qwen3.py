@@ -178,10 +178,13 @@ class DenseFFN(nn.Module):
 
     def forward(self, x, meta: ForwardMeta, layer: int):
         lora = getattr(self, "lora", None)
-        h13 = self.ps.column_linear(x, self.w13)
-        if lora is not None and "w13" in lora:
-            h13 = h13 + lora["w13"](x, meta)
-        h = ops.swiglu(h13)
+        if lora is None and self.ps.tp_size == 1:
+            h = ops.linear_swiglu(x, self.w13)
+        else:
+            h13 = self.ps.column_linear(x, self.w13)
+            if lora is not None and "w13" in lora:
+                h13 = h13 + lora["w13"](x, meta)
+            h = ops.swiglu(h13)
         if lora is None and self.ps.defer_allreduce(h):
             return self.ps.row_linear_partial(h, self.w2)             # reduced inside the next add + RMSNorm kernel
         out = self.ps.row_linear(h, self.w2)

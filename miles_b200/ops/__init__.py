@@ -99,6 +99,13 @@ def swiglu(gate_up):
     return ref.swiglu(gate_up)
 
 
+def linear_swiglu(x, w):
+    """swiglu(x · wᵀ), w [2F, H] with the gate rows first."""
+    if x.is_cuda:
+        return _k().linear_swiglu(x, w)
+    return swiglu(linear(x, w))
+
+
 def qk_norm_rope(q, k, q_w, k_w, positions, theta, eps=1e-6):
     """Per-head RMSNorm of q and k (when weights given) followed by NeoX rotary embedding."""
     if q.is_cuda:

@@ -105,6 +105,22 @@ void gemm_small_grouped(const at::Tensor& X, const at::Tensor& W, at::Tensor& C,
         "mb_gemm_small_grouped");
 }
 
+// silu(gate) · up in the product's epilogue: act [M, F] from A [M, K] and B [2F, K] (grouped: [E, 2F, K] and the tile table).  False: sizes
+// that are better served by the two kernels; nothing was done
+bool gemm_glu(const at::Tensor& A, const at::Tensor& B, at::Tensor& act, const c10::optional<at::Tensor>& tile_expert) {
+  c10::cuda::CUDAGuard g(A.device());
+  TORCH_CHECK(A.is_contiguous() && B.is_contiguous() && act.is_contiguous() && A.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16,
+              "gemm_glu: contiguous bf16 operands");
+  const bool grouped = tile_expert.has_value() && tile_expert->defined();
+  const int64_t F = act.size(1), E = grouped ? B.size(0) : 1;
+  TORCH_CHECK(B.size(-2) == 2 * F && B.size(-1) == A.size(1) && A.size(1) % 8 == 0, "gemm_glu: shapes");
+  const int rc = mb_gemm_bf16_glu(A.data_ptr(), B.data_ptr(), act.data_ptr(), A.size(0), F, A.size(1), E, grouped ? tile_expert->data_ptr<int>() : nullptr,
+                                  error_flag_for(A.device()).data_ptr<int>(), cur_stream());
+  if (rc == 1) return false;
+  check(rc, "mb_gemm_bf16_glu");
+  return true;
+}
+
 void gemm_grouped(const at::Tensor& A, const at::Tensor& B, at::Tensor& C, int64_t M_pad, int64_t N, int64_t K, int64_t E,
                   const at::Tensor& tile_expert, bool b_mn, int64_t force_bn) {
   c10::cuda::CUDAGuard g(A.device());
@@ -252,6 +268,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_splitk", &gemm_splitk);
   m.def("gemm_rows", &gemm_rows);
   m.def("gemm_grouped", &gemm_grouped);
+  m.def("gemm_glu", &gemm_glu);
   m.def("gemm_small", &gemm_small);
   m.def("gemv", &gemv);
   m.def("moe_gemv", &moe_gemv, py::arg("x"), py::arg("w13"), py::arg("w2"), py::arg("topk_idx"), py::arg("topk_w"), py::arg("act"), py::arg("out"),

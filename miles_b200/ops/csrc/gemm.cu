@@ -570,6 +570,28 @@ extern "C" int mb_gemm_bf16_grouped(const void* A, const void* B, void* C, int M
   return launch_tile<0, 0, kGroupedFwd>(tile, ta, tb, p, 1, stream);
 }
 
+// act [M, F] = silu(A·Gᵀ) · (A·Uᵀ) (bf16) with [G; U] = B [2F, K], or per expert of expert-sorted rows (tile_expert as above, else null; B [E·2F, K]).
+// 1: not this way (tiles too few for pairs of SMs, or rows of act not 16-byte aligned); nothing was launched.
+extern "C" int mb_gemm_bf16_glu(const void* A, const void* B, void* act, int M, int F, int K, int num_experts, const int* tile_expert, int* error_flag,
+                                cudaStream_t stream) {
+  if (M <= 0 || F <= 0) return 0;
+  GemmParams p{};
+  p.M = M; p.N = 2 * F; p.K = K; p.C = act; p.ldc = F; p.glu_rows = F;
+  p.tile_expert = tile_expert;
+  p.b_group_rows = 2 * F;
+  p.error_flag = error_flag;
+  p.num_groups = num_experts;
+  if (F % 8 != 0 || pick_tile(M, 2 * F, 1, 0, p) != kPair + 256) return 1;
+  CUtensorMap ta, tb;
+  int r = make_tmap_bf16_2d(&ta, A, M, K, K, BM, BK);
+  if (r) return 1000 + r;
+  r = make_tmap_bf16_2d(&tb, B, 2ll * F * num_experts, K, K, 128, BK);
+  if (r) return 2000 + r;
+  const int tiles = ((M + 255) / 256) * ((2 * F + 255) / 256);
+  return tile_expert != nullptr ? pair::launch_pair<256, 0, 0, kGroupedFwd>(ta, tb, p, pair::GluTile{}, tiles, stream)
+                                : pair::launch_pair<256, 0, 0, kDense>(ta, tb, p, pair::GluTile{}, tiles, stream);
+}
+
 // Grouped wgrad: dW[e] [N, K] (+)= dY[seg_e, N]ᵀ · X[seg_e, K]; seg_offsets[E+1] are row offsets (multiples of 128).
 extern "C" int mb_gemm_bf16_grouped_wgrad(const void* dY, const void* X, void* dW, int M_pad, int N, int K,
                                           int num_experts, const int* seg_offsets, int out_fp32, int accumulate,

@@ -37,6 +37,7 @@ struct GemmParams {
   const int* seg_offsets;  // grouped wgrad: [groups+1], multiples of BK
   int num_groups;
   int b_group_rows;        // grouped fwd: rows of B per expert (N for K-major B, K for MN-major B)
+  int glu_rows;            // > 0: B is [gate; up] of this many rows each, see GluTile
   int* error_flag;
   // split-K (dense, few output tiles): `split_k` CTAs share one output tile, each writing the partial sums of its K slice
   // to its own fp32 plane of `ws` [split_k, M, N]; the last to arrive (counter per tile and 32-row quadrant) adds the
@@ -82,13 +83,53 @@ __device__ __forceinline__ void tile_of(int t, int m_tiles, int n_tiles, int& m,
   n = r / rows;
 }
 
-// What a warp does with its 32 rows × COLS columns of the accumulator: stores them, or what head.cu makes of them.
+// What a warp does with its 32 rows of a BN-column accumulator (columns from t_acc on; two warps per lane quadrant, `half` 0 and 1): stores
+// them, makes gate · up of them, or what head.cu makes of them.
 struct StoreTile {
-  template <int COLS>
-  __device__ __forceinline__ void tile(const GemmParams& p, int group, int row0, uint32_t t_row, uint8_t* stage, int col0, bool empty) const {
+  template <int BN>
+  __device__ __forceinline__ void tile(const GemmParams& p, int group, int row0, uint32_t t_acc, uint8_t* stage, int n, int half, bool empty) const {
     const TileOut out{reinterpret_cast<uint8_t*>(p.C) + (static_cast<long long>(group) * p.group_stride_c + static_cast<long long>(row0) * p.ldc) * (p.out_fp32 ? 4 : 2),
                       p.ldc, p.M - row0, p.N, p.out_fp32, p.accumulate, p.bias};
-    store_tile_staged<COLS>(out, t_row, stage, col0, empty);
+    store_tile_staged<BN / 2>(out, t_acc + half * (BN / 2), stage, n * BN + half * (BN / 2), empty);
+  }
+};
+
+// silu(gate) · up of 128 gate and 128 up columns (p.glu_rows > 0: the first CTA loads gate rows, the second up rows) → 128 bf16 columns.
+// Without autograd nobody needs the pre-activations: they are neither written nor read back.  Both are rounded to bf16 first, which makes
+// the result the same bits as the two kernels' (a rollout and its trainer have to agree).
+struct GluTile {
+  template <int BN>
+  __device__ __forceinline__ void tile(const GemmParams& p, int, int row0, uint32_t t_acc, uint8_t* stage, int n, int half, bool) const {
+    static_assert(BN == 256, "64 output columns per warp");
+    const int lane = static_cast<int>(lane_id()), col0 = n * 128 + half * 64, F = p.glu_rows;
+    if (col0 >= F) return;                                    // uniform
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      uint32_t g[32], u[32];
+      tmem_ld_32x32(t_acc + half * 64 + c * 32, g);
+      tmem_ld_32x32(t_acc + 128 + half * 64 + c * 32, u);
+      tmem_ld_wait();
+      uint32_t o[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const uint32_t gp = pack_bf16x2(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1])), up = pack_bf16x2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1]));
+        const float g0 = __uint_as_float(gp << 16), g1 = __uint_as_float(gp & 0xffff0000u);
+        o[i] = pack_bf16x2(g0 / (1.f + __expf(-g0)) * __uint_as_float(up << 16), g1 / (1.f + __expf(-g1)) * __uint_as_float(up & 0xffff0000u));
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint4*>(stage + lane * 128 + (((c * 4 + i) ^ (lane & 7)) << 4)) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+    }
+    __syncwarp();
+    const int unit = lane & 7, col = col0 + unit * 8;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int rr = k * 4 + (lane >> 3);
+      if (row0 + rr < p.M && col < F)
+        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row0 + rr) * p.ldc + col) =
+            *reinterpret_cast<const uint4*>(stage + rr * 128 + ((unit ^ (rr & 7)) << 4));
+    }
+    __syncwarp();
   }
 };
 
@@ -169,7 +210,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         bool mine;
         tile_of(kWgrad ? t % per_group : t, m_tiles, n_tiles, m, n);
         k_range(group, k0, k_blocks);
-        const int a_row = (2 * m + rank) * kBM, b_row = n * BN + rank * (BN / 2);
+        const int a_row = (2 * m + rank) * kBM, b_row = p.glu_rows > 0 ? n * (BN / 2) + rank * p.glu_rows : n * BN + rank * (BN / 2);
         for (int pass = 0; pass < 2 && ok; ++pass) {
           if (!pass_of(m, pass, expert, mine)) continue;
           const int b_off = kFwd ? expert * p.b_group_rows : 0;
@@ -242,7 +283,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   } else {
     // ------------------------------ epilogue (warps 2..9) ------------------------------
     const int q = warp & 3;  // TMEM lane quadrant this warp may access
-    const int col_in_tile = (warp - 2) / 4 * (BN / 2);
+    const int half = (warp - 2) / 4;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
@@ -257,8 +298,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         if (__any_sync(0xffffffffu, !mbar_wait_cluster(&tmem_full[acc], acc_phase) || *abort_flag)) { ok = false; break; }
         tc_fence_after();
         if (mine)
-          epi.template tile<BN / 2>(p, group, (2 * m + rank) * kBM + q * 32, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + col_in_tile,
-                                    smem_stage + (warp - 2) * 4096, n * BN + col_in_tile, k_blocks == 0);
+          epi.template tile<BN>(p, group, (2 * m + rank) * kBM + q * 32, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN,
+                                smem_stage + (warp - 2) * 4096, n, half, k_blocks == 0);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(smem_of_rank(&tmem_empty[acc], 0));

@@ -29,9 +29,12 @@ struct Stats {
   float* target_z;                       // [M], written where the target is in range
   float inv_temp;
 
-  template <int COLS>
-  __device__ __forceinline__ void tile(const GemmParams& p, int, int row0, uint32_t t_row, uint8_t*, int col0, bool) const {
+  template <int BN>
+  __device__ __forceinline__ void tile(const GemmParams& p, int, int row0, uint32_t t_acc, uint8_t*, int n, int half, bool) const {
+    constexpr int COLS = BN / 2;
     static_assert(COLS == kPart, "one part per warp");
+    const uint32_t t_row = t_acc + half * COLS;
+    const int col0 = n * BN + half * COLS;
     if (col0 >= p.N) return;                                  // uniform
     const int row = row0 + static_cast<int>(lane_id());
     const long long target = row < p.M ? targets[row] - col0 : -1;
@@ -95,8 +98,11 @@ struct Grad {
   float inv_temp;
 
   //   d z_j = g_lp·(1[j = target] − p_j) − g_ent·p_j·(z_j − (lse − H)),  d logit = d z · inv_temp,  p_j = exp(z_j − lse)
-  template <int COLS>
-  __device__ __forceinline__ void tile(const GemmParams& p, int, int row0, uint32_t t_row, uint8_t* stage, int col0, bool) const {
+  template <int BN>
+  __device__ __forceinline__ void tile(const GemmParams& p, int, int row0, uint32_t t_acc, uint8_t* stage, int n, int half, bool) const {
+    constexpr int COLS = BN / 2;
+    const uint32_t t_row = t_acc + half * COLS;
+    const int col0 = n * BN + half * COLS;
     const int lane = static_cast<int>(lane_id()), row = row0 + lane;
     const bool in = row < p.M;
     const float l = in ? lse[row] : 0.f, glp = in && g_lp != nullptr ? g_lp[row] : 0.f, ge = in && g_ent != nullptr ? g_ent[row] : 0.f;

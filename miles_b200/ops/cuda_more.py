@@ -204,6 +204,28 @@ def few_token_experts(x, w13, T: int, k: int, ungated: bool = False) -> bool:
             and 65536 + max(8 * (2 * x.shape[1] + 64), T * k * (2 * F + 64)) <= 200 * 1024)
 
 
+def _glu_in_place() -> bool:
+    """The activation may be formed in the bf16 product's epilogue: no block-scaled projection stands in its place, and nothing that
+    the autograd functions would refuse (forward-mode tangents, function transforms) is under way."""
+    from . import cuda as _cuda
+
+    return (not _cuda.MXFP8_LINEAR and not _cuda._MXFP8_WEIGHTS and torch.autograd.forward_ad._current_level < 0
+            and not torch._C._are_functorch_transforms_active())
+
+
+def linear_swiglu(x, w):
+    """swiglu(x · wᵀ) with w [gate; up]; without autograd in one kernel where sizes allow."""
+    from . import cuda as _cuda
+
+    if (torch.is_grad_enabled() or x.numel() < 512 * x.shape[-1] or x.dtype != BF16 or w.dtype != BF16 or not w.is_contiguous()
+            or x.shape[-1] % 8 or not _glu_in_place()):                 # below 512 rows the tiles of 256 are half empty
+        return _cuda.swiglu(_cuda.linear(x, w))
+    act = torch.empty(*x.shape[:-1], w.shape[0] // 2, dtype=BF16, device=x.device)
+    if act.numel() and C.gemm_glu(_c(x).view(-1, x.shape[-1]), w, act.view(-1, act.shape[-1]), None):
+        return act
+    return _cuda.swiglu(_cuda.linear(x, w))
+
+
 def sort_by_expert(x, idx, E: int, bt: int, expert_offset: int = 0):
     """Rows of `x` per (token, choice), sorted by expert, every expert's segment padded to `bt` rows: (rows, segment offsets, expert of
     each row tile, row of each (token, choice))."""
@@ -216,12 +238,19 @@ def sort_by_expert(x, idx, E: int, bt: int, expert_offset: int = 0):
     return x_perm, seg, tile, dst_row
 
 
-def experts_forward(x_perm, w13, w2, seg, tile, bt: int = 128, glu=None):
+def experts_forward(x_perm, w13, w2, seg, tile, bt: int = 128, glu=None, keep: bool = True):
     """Grouped expert FFN on expert-sorted rows whose segments are padded to `bt`. Returns (h1 pre-activation, y_perm).  `glu`: (limit,
-    alpha, shift) of a clamped activation instead of SwiGLU, or "relu2" for experts without a gate (inference)."""
+    alpha, shift) of a clamped activation instead of SwiGLU, or "relu2" for experts without a gate (inference).  `keep`: h1 is wanted (a
+    backward follows); else it may be None."""
     max_rows, H = x_perm.shape
     E, F2, _ = w13.shape
     F = w2.shape[2]
+    if not keep and glu is None and bt == 128 and _glu_in_place():
+        act = torch.empty(max_rows, F, dtype=x_perm.dtype, device=x_perm.device)
+        if C.gemm_glu(x_perm, w13, act, tile):
+            y_perm = torch.empty(max_rows, H, dtype=x_perm.dtype, device=x_perm.device)
+            C.gemm_grouped(act, w2, y_perm, max_rows, H, F, E, tile, False, 0)
+            return None, y_perm
     h1 = torch.empty(max_rows, F2, dtype=x_perm.dtype, device=x_perm.device)
     act = h1 if glu == "relu2" else torch.empty(max_rows, F, dtype=x_perm.dtype, device=x_perm.device)      # squared in place
     y_perm = torch.empty(max_rows, H, dtype=x_perm.dtype, device=x_perm.device)
@@ -296,7 +325,7 @@ class _MoEFFN(torch.autograd.Function):
     """y[t] = Σ_j w[t,j] · W2[e]·swiglu(W13[e]·x[t]) with e = idx[t,j] − expert_offset ∈ [0, E_local) (others skipped)."""
 
     @staticmethod
-    def forward(ctx, x, w13, w2, topk_w, topk_idx, expert_offset):
+    def forward(ctx, x, w13, w2, topk_w, topk_idx, expert_offset, keep):
         T, H = x.shape
         E, F2, _ = w13.shape
         F = F2 // 2
@@ -309,7 +338,7 @@ class _MoEFFN(torch.autograd.Function):
         x_perm = torch.empty(max_rows, H, dtype=x.dtype, device=x.device)
         publish_limit(LIMIT_MOE_PAIRS, x.shape[0] * k)
         C.moe_gather(x, x_perm, row_src, seg, k)
-        h1, y_perm = experts_forward(x_perm, w13, w2, seg, tile)        # bf16 grouped GEMMs, or block-scaled under the MXFP8 recipe
+        h1, y_perm = experts_forward(x_perm, w13, w2, seg, tile, keep=keep)        # bf16 grouped GEMMs, or block-scaled under the MXFP8 recipe
         out = torch.empty(T, H, dtype=x.dtype, device=x.device)
         C.moe_combine(y_perm, wf, dst_row, out, k)
         ctx.save_for_backward(x, w13, w2, wf, seg, tile, row_src, dst_row, h1, y_perm)
@@ -346,7 +375,7 @@ class _MoEFFN(torch.autograd.Function):
         C.gemm_grouped(dh1, w13, dx_perm, max_rows, H, F2, E, tile, True, 0)
         dx = torch.empty_like(x)
         C.moe_combine(dx_perm, None, dst_row, dx, k)
-        return dx, dw13, dw2, dw_flat.view(T, k), None, None
+        return dx, dw13, dw2, dw_flat.view(T, k), None, None, None
 
 
 def moe_ffn(x, w13, w2, topk_w, topk_idx, expert_offset: int = 0):
@@ -361,7 +390,7 @@ def moe_ffn(x, w13, w2, topk_w, topk_idx, expert_offset: int = 0):
     bt = small_moe_bt(topk_idx.numel(), w13.shape[0], w13, w2)
     if bt != 128 and x.shape[0]:
         return _moe_ffn_small(x, w13, w2, topk_w, topk_idx, int(expert_offset), bt)
-    return _MoEFFN.apply(x, w13, w2, topk_w, topk_idx, int(expert_offset))
+    return _MoEFFN.apply(x, w13, w2, topk_w, topk_idx, int(expert_offset), torch.is_grad_enabled())
 
 
 # ---------------------------------------------------------------------------------------------

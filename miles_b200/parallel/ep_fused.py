@@ -80,7 +80,7 @@ def _decode_path(C, fab, b, x, w13, w2, wf, idx32, sent_row, cap, T, H, k, e_loc
     C.moe_recv_align(b.recv_meta, b.counter, cap, e_local, seg, tile, row_src, bt, b.flag_ptrs, me, ep, CH_EP, fab.epochs, fab.err)
     x_perm = torch.empty(max_rows, H, dtype=x.dtype, device=dev)
     C.moe_gather(b.recv_x.view(b.cap, H), x_perm, row_src, seg, 1)
-    _, y_perm = experts_forward(x_perm, w13, w2, seg, tile, bt)
+    _, y_perm = experts_forward(x_perm, w13, w2, seg, tile, bt, keep=False)
     C.moe_return_signal(y_perm, row_src, b.recv_meta, seg, b.ret_ptrs, ep, b.flag_ptrs, me, CH_EP2, fab.epochs, b.tickets[1:2])
     out = torch.empty(T, H, dtype=x.dtype, device=dev)
     C.moe_combine_wait(b.ret.view(b.max_pairs, H), wf, sent_row, out, k, b.flag_ptrs, me, ep, CH_EP2, fab.epochs, fab.err)
