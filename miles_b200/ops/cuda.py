@@ -56,6 +56,29 @@ def _c(x: torch.Tensor) -> torch.Tensor:
     return x if x.is_contiguous() else x.contiguous()
 
 
+class _NoTape:
+    """The context of a forward pass that nothing will differentiate."""
+
+    def save_for_backward(self, *tensors):
+        pass
+
+    def mark_non_differentiable(self, *tensors):
+        pass
+
+
+def transformed() -> bool:
+    """A forward-mode level or a function transform is active: what an autograd function refuses or handles is left to it."""
+    return torch.autograd.forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+
+
+def _apply(fn, *args):
+    """`fn.apply`; without gradients the forward pass alone (building a node that is dropped again takes as long as a launch: 4 of the
+    20 µs of host time per kernel of a short prefill)."""
+    if torch.is_grad_enabled() or transformed():
+        return fn.apply(*args)
+    return fn.forward(_NoTape(), *args)
+
+
 # ---------------------------------------------------------------------------------------------
 # GEMM
 # ---------------------------------------------------------------------------------------------
@@ -311,8 +334,8 @@ def linear(x, w, bias=None):
             return y if bias is None else y + bias
     # per-call weight quantisation only pays for itself on training-sized batches: decode-sized calls stay on the bf16 kernels
     if MXFP8_LINEAR and w.dim() == 2 and w.shape[1] % 128 == 0 and w.shape[0] >= 128 and x.numel() // x.shape[-1] >= MXFP8_MIN_ROWS:
-        return _LinearMXFP8.apply(x, w, bias)
-    return _Linear.apply(x, w, bias)
+        return _apply(_LinearMXFP8, x, w, bias)
+    return _apply(_Linear, x, w, bias)
 
 
 class _LinearFP32(torch.autograd.Function):
@@ -338,7 +361,7 @@ class _LinearFP32(torch.autograd.Function):
 def linear_fp32(x, w):
     if x.dtype != BF16:
         return torch.nn.functional.linear(x, w.to(x.dtype)).float()
-    return _LinearFP32.apply(x, w)
+    return _apply(_LinearFP32, x, w)
 
 
 def linear_dgrad(gy, w):
@@ -393,13 +416,13 @@ class _AddRMSNorm(torch.autograd.Function):
 def rmsnorm(x, w, eps=1e-6):
     if x.dtype != BF16:
         return ref.rmsnorm(x, w, eps)
-    return _RMSNorm.apply(x, w, eps)
+    return _apply(_RMSNorm, x, w, eps)
 
 
 def add_rmsnorm(x, residual, w, eps=1e-6):
     if x.dtype != BF16:
         return ref.add_rmsnorm(x, residual, w, eps)
-    return _AddRMSNorm.apply(x, residual, w, eps)
+    return _apply(_AddRMSNorm, x, residual, w, eps)
 
 
 class _SwiGLU(torch.autograd.Function):
@@ -422,7 +445,7 @@ class _SwiGLU(torch.autograd.Function):
 def swiglu(gate_up):
     if gate_up.dtype != BF16:
         return ref.swiglu(gate_up)
-    return _SwiGLU.apply(gate_up)
+    return _apply(_SwiGLU, gate_up)
 
 
 class _QKNormRope(torch.autograd.Function):
@@ -457,7 +480,7 @@ def qk_norm_rope(q, k, q_w, k_w, positions, theta, eps=1e-6):
         if q_w is not None:
             q, k = ref.rmsnorm(q, q_w, eps), ref.rmsnorm(k, k_w, eps)
         return ref.rope(q, positions, theta), ref.rope(k, positions, theta)
-    return _QKNormRope.apply(q, k, q_w, k_w, positions, float(theta), float(eps))
+    return _apply(_QKNormRope, q, k, q_w, k_w, positions, float(theta), float(eps))
 
 
 def qk_norm_rope_cache(q, k, v, q_w, k_w, positions, theta, eps, k_cache, v_cache, slot_mapping):
@@ -496,7 +519,7 @@ class _Rope(torch.autograd.Function):
 def rope(x, positions, theta, inverse=False):
     if x.dtype != BF16 or x.dim() != 3 or x.shape[-1] not in (64, 128) or x.stride(2) != 1 or x.stride(1) != x.shape[2]:
         return ref.rope(x, positions, theta, inverse)
-    return _Rope.apply(x, positions.to(torch.int32), theta, inverse)
+    return _apply(_Rope, x, positions.to(torch.int32), theta, inverse)
 
 
 def kv_cache_write(k, v, k_cache, v_cache, slot_mapping):

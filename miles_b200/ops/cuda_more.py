@@ -7,7 +7,7 @@ import os
 import torch
 
 from . import reference as ref
-from .cuda import BF16, LIMIT_KV_BLOCKS, LIMIT_MOE_PAIRS, C, _c, gemm_nn, gemm_nt, gemm_tn, publish_limit
+from .cuda import BF16, LIMIT_KV_BLOCKS, LIMIT_MOE_PAIRS, C, _apply, _c, gemm_nn, gemm_nt, gemm_tn, publish_limit, transformed
 
 # ---------------------------------------------------------------------------------------------
 # attention
@@ -59,7 +59,7 @@ class _FlashAttn(torch.autograd.Function):
 def attention_varlen(q, k, v, cu_seqlens, max_seqlen=0, causal=True):
     if q.dtype != BF16 or q.shape[-1] not in (64, 128):
         return ref.attention_varlen(q, k, v, cu_seqlens, causal)
-    return _FlashAttn.apply(q, k, v, cu_seqlens.to(torch.int32), int(max_seqlen), bool(causal))
+    return _apply(_FlashAttn, q, k, v, cu_seqlens.to(torch.int32), int(max_seqlen), bool(causal))
 
 
 _DECODE_SPLITS = int(os.environ.get("MILES_DECODE_SPLITS", "8"))   # KV splits per (request, kv head) in paged decode
@@ -154,14 +154,14 @@ class _RouterTopK(torch.autograd.Function):
 def router_topk(logits, k, normalize=True):
     if logits.shape[-1] > 256:
         return ref.router_topk(logits, k, normalize)
-    return _RouterTopK.apply(logits, int(k), bool(normalize), None)
+    return _apply(_RouterTopK, logits, int(k), bool(normalize), None)
 
 
 def router_replay(logits, idx, normalize=True):
     if logits.shape[-1] > 256 or idx.shape[1] > 32:
         return ref.router_replay(logits, idx, normalize)
     idx = idx.to(torch.int32)
-    return _RouterTopK.apply(logits, idx.shape[1], bool(normalize), idx if idx.stride(1) == 1 else idx.contiguous())
+    return _apply(_RouterTopK, logits, idx.shape[1], bool(normalize), idx if idx.stride(1) == 1 else idx.contiguous())
 
 
 # ---------------------------------------------------------------------------------------------
@@ -209,8 +209,7 @@ def _glu_in_place() -> bool:
     the autograd functions would refuse (forward-mode tangents, function transforms) is under way."""
     from . import cuda as _cuda
 
-    return (not _cuda.MXFP8_LINEAR and not _cuda._MXFP8_WEIGHTS and torch.autograd.forward_ad._current_level < 0
-            and not torch._C._are_functorch_transforms_active())
+    return not _cuda.MXFP8_LINEAR and not _cuda._MXFP8_WEIGHTS and not transformed()
 
 
 def linear_swiglu(x, w):
@@ -390,7 +389,7 @@ def moe_ffn(x, w13, w2, topk_w, topk_idx, expert_offset: int = 0):
     bt = small_moe_bt(topk_idx.numel(), w13.shape[0], w13, w2)
     if bt != 128 and x.shape[0]:
         return _moe_ffn_small(x, w13, w2, topk_w, topk_idx, int(expert_offset), bt)
-    return _MoEFFN.apply(x, w13, w2, topk_w, topk_idx, int(expert_offset), torch.is_grad_enabled())
+    return _apply(_MoEFFN, x, w13, w2, topk_w, topk_idx, int(expert_offset), torch.is_grad_enabled())
 
 
 # ---------------------------------------------------------------------------------------------
@@ -477,7 +476,7 @@ def logprob_entropy(hidden, w, targets, temperature=1.0, with_entropy=False, voc
     if hidden.dtype != BF16:
         lp, ent = ref.logprob_entropy(hidden, w, targets, temperature, with_entropy=with_entropy)
         return lp, ent
-    logp, ent, lse = _LogProbEntropy.apply(hidden, w, targets, float(temperature), bool(with_entropy), int(vocab_offset))
+    logp, ent, lse = _apply(_LogProbEntropy, hidden, w, targets, float(temperature), bool(with_entropy), int(vocab_offset))
     if return_lse:
         return logp, ent, lse
     return logp, (ent if with_entropy else None)
