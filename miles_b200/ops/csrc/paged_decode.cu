@@ -246,7 +246,7 @@ static size_t smem_bytes() { return static_cast<size_t>(16 * D + 4 * TK * D) * 2
 //
 // Work is counted in units of (request, KV head, 64-key tile), requests outermost; CTA c takes units [c·per, (c + 1)·per).  A CTA walks
 // through segments (its tiles of one request and KV head): a whole one goes straight to the output, a part goes to one of the CTA's
-// two slots of the partial buffers (0: the segment that holds its first unit, 1: a later one) and `paged_merge_tiles_kernel` adds up the
+// two slots of the partial buffers (0: the segment that holds its first unit, 1: a later one) and a second kernel adds up the
 // slots of a segment in order.  Which CTAs share a segment follows from the units before each request and `per`, which the last CTA
 // leaves in `plan`; lengths are read on the device, so that one captured launch serves any of them.  No pointer here is __restrict__: these
 // kernels start before the ones in front of them have finished, and a load that the compiler takes for invariant may move up across the
@@ -255,8 +255,8 @@ static size_t smem_bytes() { return static_cast<size_t>(16 * D + 4 * TK * D) * 2
 // What bounds it: the cache's bytes.  An even split of every request into as many ranges (the form above) lets the longest
 // request of a ragged batch set the time, and two tiles per CTA in flight behind CTA-wide barriers leave the memory idle between them.  Here a
 // producer warp keeps three 32 KB tiles in flight per CTA, two CTAs per SM, and the warps that compute wait for data only.  Attention and merge,
-// the form above → this one (32 query and 4 KV heads of 128): 61 requests of 290 to 4090 tokens 62.4 → 43.6 µs (bytes alone: 28.1), 19 of
-// 300 to 2500 with 8 KV heads 35.5 → 20.5 (12.8), 64 × 4096 102.8 → 93.1 (83.2), 7 of 433 to 3001 14.9 → 13.0; with little to read per
+// the form above → this one (32 query and 4 KV heads of 128): 61 requests of 290 to 4090 tokens 62.3 → 40.2 µs (bytes alone: 28.1), 19 of
+// 300 to 2500 with 8 KV heads 35.2 → 19.7 (12.8), 64 × 4096 102.7 → 88.8 (83.2), 7 of 433 to 3001 14.9 → 12.7; with little to read per
 // CTA the chain length → unit → page → tile shows: 8 × 700 9.7 → 11.4.
 static constexpr int kTileStages = 3, kTileThreads = 160;      // four warps that compute, one that loads
 
@@ -550,6 +550,86 @@ __global__ void __launch_bounds__(128) paged_merge_tiles_kernel(const float* par
   }
 }
 
+// The same with a warp per head, eight heads per CTA, for batches whose segments have few parts each (`launch_tiles`).  What bounds it is the
+// chain plan → parts → sum: the parts' maxima and the first four parts are requested together, and nothing waits for another warp.
+template <int D>
+__global__ void __launch_bounds__(256) paged_merge_heads_kernel(const float* part_o, const float* part_ml, const int* plan, bf16* out, int batch, int Hq,
+                                                               int Hkv) {
+  constexpr int VPL = D / 32;                               // output columns per lane
+  struct alignas(4 * VPL) Piece { float v[VPL]; };
+  mb::pdl_trigger();
+  mb::pdl_wait();
+  const int row = static_cast<int>(blockIdx.x) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= batch * Hq) return;
+  const int req = row / Hq, h = row % Hq, group = Hq / Hkv;
+  const int per = __ldcg(plan + batch + 1), u_req = __ldcg(plan + req), tiles = (__ldcg(plan + req + 1) - u_req) / Hkv;
+  bf16* o = out + static_cast<long long>(row) * D + lane * VPL;
+  auto store = [&](const float (&x)[VPL], float f) {
+#pragma unroll
+    for (int i = 0; i < VPL; i += 2) *reinterpret_cast<uint32_t*>(o + i) = pack2(x[i] * f, x[i + 1] * f);
+  };
+  float oo[VPL];
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) oo[i] = 0.f;
+  if (tiles == 0) {
+    store(oo, 0.f);
+    return;
+  }
+  const int u0 = u_req + h / group * tiles, c0 = u0 / per, c1 = (u0 + tiles - 1) / per;
+  if (c0 == c1) return;
+  const int first = u0 == c0 * per ? 0 : 1;
+  auto at = [&](int c) { return (2ll * c + (c == c0 ? first : 0)) * group + h % group; };
+  auto part = [&](int c) {
+    Piece x;
+    const float* p = part_o + at(c) * D + lane * VPL;
+    if (VPL == 4) {
+      const float4 y = __ldcg(reinterpret_cast<const float4*>(p));
+      x.v[0] = y.x; x.v[1] = y.y; x.v[VPL - 2] = y.z; x.v[VPL - 1] = y.w;
+    } else {
+      const float2 y = __ldcg(reinterpret_cast<const float2*>(p));
+      x.v[0] = y.x; x.v[1] = y.y;
+    }
+    return x;
+  };
+  float mm = -INFINITY, ll = 0.f;
+  for (int b = c0; b <= c1; b += 32) {                      // 32 parts at a time: lane i holds the maximum and the sum of part b + i
+    const int n = min(32, c1 - b + 1);
+    float2 ml = make_float2(-INFINITY, 0.f);
+    if (lane < n) ml = __ldcg(reinterpret_cast<const float2*>(part_ml + at(b + lane) * 2));
+    Piece x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i < n) x[i] = part(b + i);
+    float m = fmaxf(mm, ml.x);
+#pragma unroll
+    for (int i = 16; i > 0; i >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, i));
+    const float a = ml.x == -INFINITY ? 0.f : exp2f(ml.x - m), old = mm == -INFINITY ? 0.f : exp2f(mm - m);
+    float l = ml.y * a;
+#pragma unroll
+    for (int i = 16; i > 0; i >>= 1) l += __shfl_xor_sync(0xffffffffu, l, i);
+    ll = ll * old + l;
+    mm = m;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) oo[k] *= old;
+    for (int i0 = 0; i0 < n; i0 += 4) {
+      if (i0 > 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (i0 + i < n) x[i] = part(b + i0 + i);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float w = __shfl_sync(0xffffffffu, a, (i0 + i) & 31);
+        if (i0 + i < n) {
+#pragma unroll
+          for (int k = 0; k < VPL; ++k) oo[k] += x[i].v[k] * w;
+        }
+      }
+    }
+  }
+  store(oo, ll > 0.f ? 1.f / ll : 0.f);
+}
+
 template <int D>
 static int launch_tiles(const bf16* q, const void* kc, const void* vc, const int* block_table, const int* seq_lens, bf16* out, float* part_o,
                         float* part_ml, int* plan, int batch, int max_blocks, int block_size, int cache_rows, int Hq, int Hkv, float scale,
@@ -565,8 +645,14 @@ static int launch_tiles(const bf16* q, const void* kc, const void* vc, const int
   cudaError_t e = mb::launch_pdl(paged_decode_tiles_kernel<D>, dim3(ctas), dim3(kTileThreads), TileSmem<D>::total, s, tk, tv, q, block_table,
                                  seq_lens, out, part_o, part_ml, plan, batch, max_blocks, block_size, cache_rows, Hq, Hkv, scale, error_flag);
   if (e != cudaSuccess) return static_cast<int>(e);
-  e = mb::launch_pdl(paged_merge_tiles_kernel<D>, dim3(Hq, batch), dim3(128), 0, s, static_cast<const float*>(part_o), static_cast<const float*>(part_ml),
-                     static_cast<const int*>(plan), out, batch, Hq, Hkv);
+  // a segment is shared by ctas / (batch · Hkv) CTAs on average: up to 4 a warp adds them up (61 requests, 4 KV heads: 43.3 → 40.2 µs with the
+  // attention), beyond that four warps do (7 requests, 11 on average: 12.7 µs, 14.7 with one warp)
+  if (ctas <= 4 * batch * Hkv)
+    e = mb::launch_pdl(paged_merge_heads_kernel<D>, dim3((batch * Hq + 7) / 8), dim3(256), 0, s, static_cast<const float*>(part_o),
+                       static_cast<const float*>(part_ml), static_cast<const int*>(plan), out, batch, Hq, Hkv);
+  else
+    e = mb::launch_pdl(paged_merge_tiles_kernel<D>, dim3(Hq, batch), dim3(128), 0, s, static_cast<const float*>(part_o), static_cast<const float*>(part_ml),
+                       static_cast<const int*>(plan), out, batch, Hq, Hkv);
   return static_cast<int>(e);
 }
 

@@ -39,7 +39,7 @@ def _softmax64(q, k, v, table, lens):
 
 @pytest.mark.parametrize("hq,hkv,d", [(32, 4, 128), (16, 8, 128), (4, 4, 128), (8, 2, 64)])
 @pytest.mark.parametrize("lens,page", [([1], 64), ([1, 63, 64, 65, 700, 0, 128], 64), ([0, 0, 5, 0], 64), ([6000, 1, 1, 3], 64), ([300] * 61, 128),
-                                       ([7] * 300, 64), (list(range(1, 700, 9)), 64), ([0, 0], 64)])
+                                       ([7] * 300, 64), (list(range(1, 700, 9)), 64), ([9000] + [1] * 40, 64), ([0, 0], 64)])
 def test_paged_decode_tiles(hq, hkv, d, lens, page):
     from miles_b200.ops import cuda as K
 
