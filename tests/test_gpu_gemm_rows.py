@@ -37,3 +37,17 @@ def test_split_fits_the_gpu():
                 s, tiles = K._row_split(M, N, Kd), -(-N // 128)
                 assert (s == 0) == (tiles > (296 if M <= 32 else 148))
                 assert s == 0 or (tiles * s <= 296 and (s == 1 or -(-Kd // 64) >= 2 * s))
+
+
+@pytest.mark.parametrize("M", [8, 9, 16, 17])
+def test_from_matrix_vector_to_clusters(M):
+    from miles_b200 import ops
+    from miles_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = torch.randn(M, 1024, device="cuda", generator=g).bfloat16(), torch.randn(640, 1024, device="cuda", generator=g).bfloat16()
+    with torch.no_grad():
+        assert ops.few_token_decode(x, w) == (M <= 8)
+        y = K.linear(x, w)
+    want = x.double() @ w.double().t()
+    assert ((y.double() - want).norm() / want.norm()).item() < 2 ** -8.5          # one rounding to bf16
