@@ -76,7 +76,7 @@ def few_token_decode(x, w) -> bool:
     """True when the matrix-vector decode kernels apply to `x · wᵀ`: CUDA bf16, no autograd, a handful of rows.  They take rows eight at a
     time: from nine on, norms by themselves and a cluster of CTAs per weight tile are faster (decode steps of 8 layers, 9 / 16 rows: hidden
     2048 with 16 experts 875 / 929 → 770 / 800 µs, hidden 2560 1180 / 1289 → 659 / 698, hidden 1024 361 / 424 → 350 / 405)."""
-    return x.is_cuda and x.numel() <= 8 * x.shape[-1] and _k().gemv_ok(x, w)
+    return x.is_cuda and x.numel() <= 8 * x.shape[-1] and w.numel() <= _k().GEMV_MAX_WEIGHTS and _k().gemv_ok(x, w)
 
 
 def add_rmsnorm_linear(x, residual, norm_w, eps, w, bias=None, want_normed=False, out_fp32=False):

@@ -100,7 +100,8 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *
         split = _row_split(M, N, K) if plain and M <= SMALL_M else 0
         # the matrix-vector kernel takes its rows eight at a time: from nine on a cluster per weight tile is faster (9 rows, N × K: 5120 × 2048
         # 8.3 → 6.2 µs, 2560 × 4096 11.7 → 6.0, 19456 × 2560 37.3 → 19.6, 6144 × 1024 4.6 → 4.5)
-        if plain and M <= (8 if split else GEMV_M) and M <= GEMV_M and _gemv_k_ok(M, K) and N <= GEMV_MAX_N:
+        few = GEMV_M if not split else min(8, GEMV_M) if N * K <= GEMV_MAX_WEIGHTS else 0
+        if plain and M <= few and _gemv_k_ok(M, K) and N <= GEMV_MAX_N:
             C.gemv(a, None, None, 0.0, b, bias, out, None, None, bool(b.is_leaf and b.requires_grad))
             return out
         if plain and M <= SMALL_M:
@@ -149,6 +150,10 @@ def _splitk_workspace(device):
 # Up to 16 rows are supported; 0 turns the path off.
 GEMV_M = min(16, int(os.environ.get("MILES_GEMV_M", "16")))
 GEMV_MAX_N = int(os.environ.get("MILES_GEMV_MAX_N", "32768"))
+# Larger weights (24 MB) stream faster through gemm_rows.cu's rings whatever the rows: decode steps of 8 layers, 1 / 4 / 8 rows: hidden 2560
+# (31 to 100 MB per projection) 776 / 816 / 908 → 621 / 633 / 666 µs (all projections there 612 / 630 / 658); hidden 2048 with 16 experts (17 and 21 MB) 565 / 675 / 750 against
+# 555 / 683 / 727, hidden 1024 (up to 12 MB) 300 / 325 / 362 against 299 / 322 / 345.
+GEMV_MAX_WEIGHTS = 12 << 20
 
 
 def _gemv_k_ok(rows: int, K: int) -> bool:
