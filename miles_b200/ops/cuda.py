@@ -150,9 +150,9 @@ def _splitk_workspace(device):
 # Up to 16 rows are supported; 0 turns the path off.
 GEMV_M = min(16, int(os.environ.get("MILES_GEMV_M", "16")))
 GEMV_MAX_N = int(os.environ.get("MILES_GEMV_MAX_N", "32768"))
-# Larger weights (24 MB) stream faster through gemm_rows.cu's rings whatever the rows: decode steps of 8 layers, 1 / 4 / 8 rows: hidden 2560
-# (31 to 100 MB per projection) 776 / 816 / 908 → 621 / 633 / 666 µs (all projections there 612 / 630 / 658); hidden 2048 with 16 experts (17 and 21 MB) 565 / 675 / 750 against
-# 555 / 683 / 727, hidden 1024 (up to 12 MB) 300 / 325 / 362 against 299 / 322 / 345.
+# Larger weights (24 MB) stream faster through gemm_rows.cu's rings whatever the rows.  Decode steps of 8 layers, 1 / 4 / 8 rows: hidden 2560
+# (21 to 100 MB per projection) 776 / 816 / 908 → 621 / 633 / 666 µs, everything there 612 / 630 / 658; hidden 2048 with 16 experts (17 and
+# 21 MB) 565 / 675 / 750 against 555 / 683 / 727, hidden 1024 (up to 12 MB) 300 / 325 / 362 against 299 / 322 / 345.
 GEMV_MAX_WEIGHTS = 12 << 20
 
 
