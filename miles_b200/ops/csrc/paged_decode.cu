@@ -7,8 +7,8 @@
 // buffered; each of the 4 warps owns 16 keys of a tile with its own running (max, sum, O) which are merged through
 // shared memory at the end.  Split partials are combined by `paged_merge_kernel2`.
 //
-// Caches whose pages hold a multiple of 64 tokens (the engine's do) take the form by tiles at the end of this file instead: the same
-// arithmetic, an even share of ALL the 64-key tiles of the batch per CTA, tiles by TMA.
+// More than 32 (request, KV head) segments in caches whose pages hold a multiple of 64 tokens (the engine's do) take the form by tiles at the
+// end of this file instead: the same arithmetic, an even share of ALL the 64-key tiles of the batch per CTA, tiles by TMA.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -256,8 +256,8 @@ static size_t smem_bytes() { return static_cast<size_t>(16 * D + 4 * TK * D) * 2
 // request of a ragged batch set the time, and two tiles per CTA in flight behind CTA-wide barriers leave the memory idle between them.  Here a
 // producer warp keeps three 32 KB tiles in flight per CTA, two CTAs per SM, and the warps that compute wait for data only.  Attention and merge,
 // the form above → this one (32 query and 4 KV heads of 128): 61 requests of 290 to 4090 tokens 62.3 → 40.2 µs (bytes alone: 28.1), 19 of
-// 300 to 2500 with 8 KV heads 35.2 → 19.7 (12.8), 64 × 4096 102.7 → 88.8 (83.2), 7 of 433 to 3001 14.9 → 12.7; with little to read per
-// CTA the chain length → unit → page → tile shows: 8 × 700 9.7 → 11.4.
+// 300 to 2500 with 8 KV heads 35.2 → 19.7 (12.8), 64 × 4096 102.7 → 88.8 (83.2).  With little to read per CTA the chain length → unit →
+// page → tile shows: 8 × 700 10.1 → 12.5.  `paged_attention` has the rule and both sides of it.
 static constexpr int kTileStages = 3, kTileThreads = 160;      // four warps that compute, one that loads
 
 template <int D>

@@ -66,6 +66,12 @@ _DECODE_SPLITS = int(os.environ.get("MILES_DECODE_SPLITS", "8"))   # KV splits p
 # whoever asks for a number of splits gets the form that has them: a request's sums are then cut in the same places whatever else is in the
 # batch (one split, for rollouts that have to agree with the trainer)
 _DECODE_BY_TILES = "MILES_DECODE_SPLITS" not in os.environ
+# Up to so many (request, KV head) segments the form that splits each of them runs as one wave, eight CTAs per segment on 148 SMs × 2, and an
+# even share of all tiles has nothing to even out, but a longer chain from length to page.  µs per layer, split / tiles, cache from memory:
+# 8 requests × 4 KV heads of 300, 700, 1500, 3000 keys 8.8 / 10.2, 10.1 / 12.5, 11.9 / 13.7, 16.0 / 18.4; 4 × 8 7.9 / 9.1, 9.1 / 11.1,
+# 10.8 / 11.8, 15.0 / 16.3; 7 × 4 of 430 to 3000 14.8 / 14.2; 1 × 4 8.4 / 7.6 (700), 13.2 / 12.8 (3000).  Beyond it the split form needs a
+# second wave or longer splits: 10 × 4 10.6 / 10.2, 12.5 / 13.1, 18.0 / 14.8, 26.1 / 19.9, of 430 to 3000 17.9 / 15.2; 6 × 8 26.7 / 21.0 (3000).
+_DECODE_TILES_FROM = 33
 
 
 def extend_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens, extend=None):
@@ -107,7 +113,8 @@ def paged_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens=None, max
     q = _c(q)
     out = torch.empty_like(q)
     publish_limit(LIMIT_KV_BLOCKS, k_cache.shape[0])
-    if _DECODE_BY_TILES and k_cache.shape[1] % 64 == 0 and k_cache.is_contiguous() and v_cache.is_contiguous() and block_table.is_contiguous():
+    if (_DECODE_BY_TILES and B * k_cache.shape[2] >= _DECODE_TILES_FROM and k_cache.shape[1] % 64 == 0 and k_cache.is_contiguous()
+            and v_cache.is_contiguous() and block_table.is_contiguous()):
         # whole 64-key tiles inside a page: an even share of all tiles per CTA
         C.paged_decode_tiles(q, k_cache, v_cache, block_table, seq_lens, out, 1.0 / math.sqrt(D), C.error_flag(q))
         return out

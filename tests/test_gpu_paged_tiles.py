@@ -40,9 +40,13 @@ def _softmax64(q, k, v, table, lens):
 @pytest.mark.parametrize("hq,hkv,d", [(32, 4, 128), (16, 8, 128), (4, 4, 128), (8, 2, 64)])
 @pytest.mark.parametrize("lens,page", [([1], 64), ([1, 63, 64, 65, 700, 0, 128], 64), ([0, 0, 5, 0], 64), ([6000, 1, 1, 3], 64), ([300] * 61, 128),
                                        ([7] * 300, 64), (list(range(1, 700, 9)), 64), ([9000] + [1] * 40, 64), ([0, 0], 64)])
-def test_paged_decode_tiles(hq, hkv, d, lens, page):
+@pytest.mark.parametrize("tiles_from", [0, None])           # every batch by tiles; as many segments as the rule asks for
+def test_paged_decode_tiles(monkeypatch, hq, hkv, d, lens, page, tiles_from):
     from miles_b200.ops import cuda as K
+    from miles_b200.ops import cuda_more
 
+    if tiles_from is not None:
+        monkeypatch.setattr(cuda_more, "_DECODE_TILES_FROM", tiles_from)
     args = _inputs(lens, hq, hkv, d, page)
     ref = _softmax64(*args)
     out = K.paged_attention(*args)
@@ -55,6 +59,21 @@ def test_paged_decode_tiles(hq, hkv, d, lens, page):
     # weights and outputs are rounded to bf16 once each: 2^-9 relative and independent
     assert (out.double() - ref).norm().item() <= 2 ** -8 * ref.norm().item()
     assert K.check_error_flag(out) == 0
+
+
+@pytest.mark.parametrize("rows,hq,hkv", [(1, 32, 4), (8, 32, 4), (9, 32, 4), (4, 16, 8), (5, 16, 8), (32, 8, 1)])
+def test_few_segments_are_split_as_they_always_were(rows, hq, hkv):
+    """Up to 32 (request, KV head) segments the split form runs as one wave: it is the faster one, and its sums keep their order."""
+    from miles_b200.ops import cuda as K
+
+    q, k, v, table, lens = _inputs([1801 - 31 * b for b in range(rows)], hq, hkv, 128, 64)
+    splits = max(1, min(8, -(-296 // (rows * hkv))))
+    part = lambda n: torch.empty(rows * hq * splits * n, dtype=torch.float32, device="cuda")
+    want, tiles = torch.empty_like(q), torch.empty_like(q)
+    K.C.paged_decode(q, k, v, table, lens, want, part(128), part(2), 1 / math.sqrt(128), splits)
+    K.C.paged_decode_tiles(q, k, v, table, lens, tiles, 1 / math.sqrt(128), K.C.error_flag(q))
+    assert not torch.equal(want, tiles)
+    assert torch.equal(K.paged_attention(q, k, v, table, lens), want if rows * hkv <= 32 else tiles)
 
 
 def test_asked_for_splits_do_not_depend_on_the_batch():
