@@ -843,24 +843,18 @@ extern "C" int mb_rmsnorm_fwd(const void* x, const void* residual, const void* w
   cudaError_t e;
   const bool add = residual != nullptr;
   const dim3 wgrid(static_cast<unsigned>((T + 7) / 8));
-  // rows of a multiple of 512 up to 4096 elements with 16-byte aligned pointers: one warp per row.  Powers of two from T = 64; the others from
-  // eight rows per SM (2560: 11 791 rows 77 → 70 µs, but 257 rows 3.9 → 6.6)
+  // rows of 1024 / 2048 / 4096 elements with 16-byte aligned pointers: one warp per row (T ≥ 64 so that the grid fills the SMs).  The other
+  // widths stay with a CTA per row: a warp per row adds the squares up in another order, and there a token's norm does not depend on how many
+  // tokens are beside it (11 791 rows of 2560: 77 µs, a warp per row 70)
   const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w) |
                          reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(res_out)) & 15) == 0;
-  if (aligned && H % 512 == 0 && H <= 4096 && T >= (H == 1024 || H == 2048 || H == 4096 ? 64 : 148 * 8)) {
+  if (aligned && T >= 64 && (H == 1024 || H == 2048 || H == 4096)) {
     auto launch = [&](auto kern) {
       return launch_pdl(kern, wgrid, dim3(256), 0, s, X, (cbf)residual, (cbf)w, (bf)y, (bf)res_out, rstd, static_cast<long long>(T), eps);
     };
-    switch (H / 256) {
-      case 2: e = add ? launch(rmsnorm_fwd_warp_kernel<true, 2>) : launch(rmsnorm_fwd_warp_kernel<false, 2>); break;
-      case 4: e = add ? launch(rmsnorm_fwd_warp_kernel<true, 4>) : launch(rmsnorm_fwd_warp_kernel<false, 4>); break;
-      case 6: e = add ? launch(rmsnorm_fwd_warp_kernel<true, 6>) : launch(rmsnorm_fwd_warp_kernel<false, 6>); break;
-      case 8: e = add ? launch(rmsnorm_fwd_warp_kernel<true, 8>) : launch(rmsnorm_fwd_warp_kernel<false, 8>); break;
-      case 10: e = add ? launch(rmsnorm_fwd_warp_kernel<true, 10>) : launch(rmsnorm_fwd_warp_kernel<false, 10>); break;
-      case 12: e = add ? launch(rmsnorm_fwd_warp_kernel<true, 12>) : launch(rmsnorm_fwd_warp_kernel<false, 12>); break;
-      case 14: e = add ? launch(rmsnorm_fwd_warp_kernel<true, 14>) : launch(rmsnorm_fwd_warp_kernel<false, 14>); break;
-      default: e = add ? launch(rmsnorm_fwd_warp_kernel<true, 16>) : launch(rmsnorm_fwd_warp_kernel<false, 16>); break;
-    }
+    if (H == 1024) e = add ? launch(rmsnorm_fwd_warp_kernel<true, 4>) : launch(rmsnorm_fwd_warp_kernel<false, 4>);
+    else if (H == 2048) e = add ? launch(rmsnorm_fwd_warp_kernel<true, 8>) : launch(rmsnorm_fwd_warp_kernel<false, 8>);
+    else e = add ? launch(rmsnorm_fwd_warp_kernel<true, 16>) : launch(rmsnorm_fwd_warp_kernel<false, 16>);
     return static_cast<int>(e);
   }
   if (residual != nullptr)

@@ -1,4 +1,5 @@
-"""Row kernels for many tokens: norms of every width that a warp (or several) takes in registers, rotation of several heads by one warp."""
+"""Row kernels for many tokens: norms whose backward (and, at 1024, 2048 and 4096, whose forward) takes a row in the registers of a warp or
+several, rotation of several heads by one warp."""
 import pytest
 import torch
 
@@ -23,6 +24,22 @@ def test_rmsnorm_widths(T, H):
     torch.autograd.backward([yd, sd], [dy.double(), dr.double()])
     for got, want in ((y, yd), (ins[0].grad, sd.grad), (ins[1].grad, sd.grad), (ins[2].grad, wd.grad)):
         assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4 * want.abs().max()).all()
+
+
+@pytest.mark.parametrize("T", [1183, 1184, 1191])
+@pytest.mark.parametrize("H", [512, 520, 1536, 2560, 3072, 3584])
+def test_a_token_is_normed_alike_in_every_batch(T, H):
+    """Widths with one kernel: the same bits for a token among 16 and among all (trainer and engine batch differently)."""
+    from miles_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, r, w = rand(T, H), rand(T, H), rand(H)
+    with torch.no_grad():
+        y, (ya, total) = K.rmsnorm(x, w, 1e-6), K.add_rmsnorm(x, r, w, 1e-6)
+        few = [(K.rmsnorm(x[i:i + 16], w, 1e-6), *K.add_rmsnorm(x[i:i + 16], r[i:i + 16], w, 1e-6)) for i in range(0, T, 16)]
+        assert all(torch.equal(all_rows, torch.cat(f)) for all_rows, f in zip((y, ya, total), zip(*few)))
+        assert torch.equal(y[-1:], K.rmsnorm(x[-1:], w, 1e-6))
 
 
 @pytest.mark.parametrize("T,Hq,Hk,D,norm", [(1184, 4, 4, 128, True), (601, 32, 4, 128, True), (500, 40, 8, 128, False), (3001, 6, 1, 128, True), (700, 32, 8, 64, True)])
