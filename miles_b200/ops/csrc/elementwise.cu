@@ -412,6 +412,12 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
 // Per-head RMSNorm (optional) + NeoX rotary embedding on q and k, in one pass.  One warp per (token, head).
 // Layout [T, heads, D]; pairs are (i, i + D/2).  D ∈ {64, 128}.
 // ---------------------------------------------------------------------------------------------
+// (x1, x2) turned by the angle of cosine c and sine s.  The contraction is spelled out: left to the compiler, two kernels round the same token in
+// two ways.
+__device__ __forceinline__ float2 rotate_pair(float x1, float x2, float c, float s) {
+  return make_float2(__fmaf_rn(x1, c, -__fmul_rn(x2, s)), __fmaf_rn(x1, s, __fmul_rn(x2, c)));
+}
+
 template <int D>
 __device__ __forceinline__ void norm_rope_row(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst,
                                               const __nv_bfloat16* __restrict__ w, float pos, float log2_theta, float eps,
@@ -442,7 +448,8 @@ __device__ __forceinline__ void norm_rope_row(const __nv_bfloat16* __restrict__ 
     const float inv_freq = exp2f(-log2_theta * (2.f * j) / D);
     float s, c;
     sincosf(pos * inv_freq, &s, &c);
-    const __nv_bfloat16 o1 = __float2bfloat16(x1 * c - x2 * s), o2 = __float2bfloat16(x2 * c + x1 * s);
+    const float2 r = rotate_pair(x1, x2, c, s);
+    const __nv_bfloat16 o1 = __float2bfloat16(r.x), o2 = __float2bfloat16(r.y);
     dst[j] = o1;
     dst[D / 2 + j] = o2;
     if (dst2 != nullptr) {
@@ -505,17 +512,24 @@ __global__ void __launch_bounds__(256) qk_norm_rope_many_kernel(const __nv_bfloa
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const bf *pa = reinterpret_cast<const bf*>(&a[i]), *pb = reinterpret_cast<const bf*>(&b[i]);
-    float x1[4], x2[4], ss = 0.f;
+    float x1[4], x2[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       x1[e] = __bfloat162float(pa[e]);
       x2[e] = __bfloat162float(pb[e]);
-      ss += x1[e] * x1[e] + x2[e] * x2[e];
     }
     if (w != nullptr) {
+      // the order of norm_rope_row's sum, so that a token is normed alike in every batch: its lanes 2l and 2l + 1 hold what is this lane's,
+      // and meet in the last step
+      float ss[2] = {0.f, 0.f};
 #pragma unroll
-      for (int d = 8; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-      const float rstd = rsqrtf(ss / D + eps);
+      for (int e = 0; e < 4; ++e) ss[e >> 1] += x1[e] * x1[e] + x2[e] * x2[e];
+#pragma unroll
+      for (int d = 8; d > 0; d >>= 1) {
+        ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], d);
+        ss[1] += __shfl_xor_sync(0xffffffffu, ss[1], d);
+      }
+      const float rstd = rsqrtf((ss[0] + ss[1]) / D + eps);
       if (rstd_out != nullptr && (lane & 15) == 0) rstd_out[2 * i + half] = rstd;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -527,8 +541,9 @@ __global__ void __launch_bounds__(256) qk_norm_rope_many_kernel(const __nv_bfloa
     bf *p1 = reinterpret_cast<bf*>(&o1), *p2 = reinterpret_cast<bf*>(&o2);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      p1[e] = __float2bfloat16(x1[e] * cs[e] - x2[e] * sn[e]);
-      p2[e] = __float2bfloat16(x2[e] * cs[e] + x1[e] * sn[e]);
+      const float2 r = rotate_pair(x1[e], x2[e], cs[e], sn[e]);
+      p1[e] = __float2bfloat16(r.x);
+      p2[e] = __float2bfloat16(r.y);
     }
     bf* to = dst + (2 * i + half) * D + j;
     *reinterpret_cast<uint2*>(to) = o1;

@@ -42,13 +42,15 @@ def test_a_token_is_normed_alike_in_every_batch(T, H):
         assert torch.equal(y[-1:], K.rmsnorm(x[-1:], w, 1e-6))
 
 
-@pytest.mark.parametrize("T,Hq,Hk,D,norm", [(1184, 4, 4, 128, True), (601, 32, 4, 128, True), (500, 40, 8, 128, False), (3001, 6, 1, 128, True), (700, 32, 8, 64, True)])
-def test_rotation_of_many_tokens(T, Hq, Hk, D, norm):
+@pytest.mark.parametrize("T,Hq,Hk,D,norm,offset", [(1184, 4, 4, 128, True, 0), (601, 32, 4, 128, True, 0), (500, 40, 8, 128, False, 0), (3001, 6, 1, 128, True, 0),
+                                                   (700, 32, 8, 64, True, 0)])
+def test_rotation_of_many_tokens(T, Hq, Hk, D, norm, offset):
     from miles_b200.ops import cuda as K
 
     g = torch.Generator(device="cuda").manual_seed(T)
     rand = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
-    qkv = rand(T, (Hq + 2 * Hk) * D)
+    width = (Hq + 2 * Hk) * D
+    qkv = rand(T * width + offset)[offset:].view(T, width)               # an offset of one or two elements: no 8-byte pieces
     q, k, v = (t.view(T, -1, D) for t in qkv.split([Hq * D, Hk * D, Hk * D], -1))
     qw, kw = (rand(D), rand(D)) if norm else (None, None)
     pos = torch.randint(0, 30000, (T,), device="cuda", generator=g, dtype=torch.int32)
@@ -61,13 +63,20 @@ def test_rotation_of_many_tokens(T, Hq, Hk, D, norm):
         q2, k2 = K.qk_norm_rope(q, k, qw, kw, pos, 1e6, 1e-6)
         kc, vc = cache.clone().unsqueeze(1)
         q3, k3 = K.qk_norm_rope_cache(q, k, v, qw, kw, pos, 1e6, 1e-6, kc, vc, slots)
-    # both forms round the normalised head to bf16 before they rotate it, and the result: 2^-9 of the pair's length each; sums of other order
-    # may flip the first rounding (2^-8)
-    def close(got, want):
-        pair = want.float().view(*want.shape[:-1], 2, D // 2).norm(dim=-2, keepdim=True).expand(*want.shape[:-1], 2, D // 2).reshape(want.shape)
-        return ((got.float() - want.float()).abs() <= 2.0 ** -6.5 * pair).all()
-
-    assert close(q2, q1) and close(k2, k1) and torch.equal(q3, q2) and torch.equal(k3, k2)
+    # a token is rotated alike in every batch: the engine's few rows, its prefill and the trainer's pack
+    assert torch.equal(q2, q1) and torch.equal(k2, k1) and torch.equal(q3, q2) and torch.equal(k3, k2)
+    pair = lambda x: x.double().view(*x.shape[:-1], 2, D // 2)
+    for x, wn, got in ((q, qw, q2), (k, kw, k2)):
+        # against 64 bits: the normalised head and the result are rounded to bf16 once each (2^-9 of the pair's length); an angle of up to 30 000
+        # is a product of fp32 numbers (2^-24 of it) whose second one is an exp2f of a rounded exponent (2^-22), taken in turns by another (2^-24)
+        xd = x.double()
+        if norm:
+            xd = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * wn.double()
+        angle = pos.double()[:, None] * 1e6 ** (-2 * torch.arange(D // 2, device="cuda").double() / D)
+        c, s = angle.cos()[:, None], angle.sin()[:, None]
+        a, b = pair(xd).unbind(-2)
+        want = torch.stack([a * c - b * s, b * c + a * s], -2)
+        assert ((pair(got) - want).norm(dim=-2) <= (2.0 ** -8 + 30000 * (2.0 ** -22 + 2.0 ** -23)) * want.norm(dim=-2) + 1e-6).all()
     want = cache.clone()
     want[0, slots[slots >= 0]], want[1, slots[slots >= 0]] = k3[slots >= 0], v[slots >= 0]
     assert torch.equal(kc[0], want[0]) and torch.equal(vc[0], want[1])
