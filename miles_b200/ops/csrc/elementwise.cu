@@ -596,8 +596,14 @@ __global__ void __launch_bounds__(256) qk_norm_rope_cache_kernel(const __nv_bflo
     constexpr int EPL = D / 32;   // 4 (8 bytes) or 2 (4 bytes) elements per lane
     const __nv_bfloat16* src = v + t * v_tok_stride + hk * D + lane * EPL;
     __nv_bfloat16* dst = vc + (slot * Hk + hk) * D + lane * EPL;
-    if (EPL == 4) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(src);
-    else *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(src);
+    if ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) % (2 * EPL)) {   // rows of a view that starts anywhere
+#pragma unroll
+      for (int e = 0; e < EPL; ++e) dst[e] = src[e];
+    } else if (EPL == 4) {
+      *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(src);
+    } else {
+      *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(src);
+    }
   }
 }
 

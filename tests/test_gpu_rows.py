@@ -43,7 +43,7 @@ def test_a_token_is_normed_alike_in_every_batch(T, H):
 
 
 @pytest.mark.parametrize("T,Hq,Hk,D,norm,offset", [(1184, 4, 4, 128, True, 0), (601, 32, 4, 128, True, 0), (500, 40, 8, 128, False, 0), (3001, 6, 1, 128, True, 0),
-                                                   (700, 32, 8, 64, True, 0)])
+                                                   (700, 32, 8, 64, True, 0), (601, 32, 4, 128, True, 2), (601, 32, 4, 128, False, 1), (77, 4, 4, 64, True, 1)])
 def test_rotation_of_many_tokens(T, Hq, Hk, D, norm, offset):
     from miles_b200.ops import cuda as K
 
