@@ -67,8 +67,10 @@ class _NoTape:
 
 
 def transformed() -> bool:
-    """A forward-mode level or a function transform is active: what an autograd function refuses or handles is left to it."""
-    return torch.autograd.forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+    """A forward-mode level, a function transform or a trace is active: what an autograd function refuses or handles is left to it (a
+    trace records the function as one node; it sees nothing of a kernel that is called without one)."""
+    return (torch.autograd.forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+            or torch._C._is_tracing())
 
 
 def _apply(fn, *args):

@@ -1,4 +1,4 @@
-"""Without gradients the forward passes run outside of autograd: the same results, and forward mode is refused as before."""
+"""Without gradients the forward passes run outside of autograd: the same results, forward mode is refused and traces run the kernels as before."""
 import pytest
 import torch
 
@@ -34,3 +34,27 @@ def test_same_without_gradients(name):
         assert not plain.requires_grad and torch.equal(plain, taped)
         with fwd.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
             f(fwd.make_dual(x, torch.ones_like(x)))
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("name", ["linear", "linear_fp32", "rmsnorm", "add_rmsnorm", "swiglu", "rope", "qk_norm_rope", "attention", "router"])
+def test_trace_without_gradients(name):
+    """A trace made under no_grad computes: it holds the function, not the memory that its kernels wrote while it was made."""
+    f, x = _ops()[name]
+    with torch.no_grad():
+        traced = torch.jit.trace(f, x.clone(), check_trace=False)
+        other = (x.float() * 0.5 + 0.25).to(x.dtype)
+        assert torch.equal(traced(other), f(other))
+
+
+@pytest.mark.filterwarnings("ignore")
+def test_trace_of_gate_and_up():
+    from miles_b200.ops import cuda_more
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, w = rand(9000, 1024), rand(4096, 1024) * 0.03                 # sizes of the fused product
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda x: cuda_more.linear_swiglu(x, w), x, check_trace=False)
+        other = rand(9000, 1024)
+        assert torch.equal(traced(other), cuda_more.linear_swiglu(other, w))
