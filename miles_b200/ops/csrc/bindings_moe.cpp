@@ -21,18 +21,22 @@ inline void check(int rc, const char* what) {
 }
 
 // logits fp32 [T,E] → (weights fp32 [T,K], idx int32 [T,K], probs fp32 [T,E])
-// replay: int32 [T, K] recorded choices (rows may be apart), see moe.cu
-std::vector<at::Tensor> router_topk(const at::Tensor& logits, int64_t K, bool normalize, bool want_probs, const c10::optional<at::Tensor>& replay) {
+// replay: int32 [T, K] recorded choices (rows may be apart), err: the error flag that a choice of no expert raises; see moe.cu
+std::vector<at::Tensor> router_topk(const at::Tensor& logits, int64_t K, bool normalize, bool want_probs, const c10::optional<at::Tensor>& replay,
+                                    const c10::optional<at::Tensor>& err) {
   c10::cuda::CUDAGuard g(logits.device());
   const int64_t T = logits.size(0), E = logits.size(1);
   auto w = at::empty({T, K}, logits.options());
   auto idx = at::empty({T, K}, logits.options().dtype(at::kInt));
   const int* recorded = replay.has_value() && replay->defined() ? replay->data_ptr<int>() : nullptr;
   TORCH_CHECK(recorded == nullptr || (replay->size(0) == T && replay->size(1) == K && (K == 1 || replay->stride(1) == 1)), "router_topk: replay [T, K]");
+  TORCH_CHECK(recorded == nullptr || (replay->device() == logits.device() && err.has_value() && err->device() == logits.device()),
+              "router_topk: recorded choices on ", recorded != nullptr ? replay->device() : logits.device(), ", logits on ", logits.device());
   at::Tensor probs;
   if (want_probs) probs = at::empty({T, E}, logits.options());
   check(mb_router_topk(logits.data_ptr<float>(), want_probs ? probs.data_ptr<float>() : nullptr, w.data_ptr<float>(),
-                       idx.data_ptr<int>(), T, E, K, normalize, recorded, recorded != nullptr ? replay->stride(0) : 0, cur_stream()),
+                       idx.data_ptr<int>(), T, E, K, normalize, recorded, recorded != nullptr ? replay->stride(0) : 0,
+                       recorded != nullptr ? err->data_ptr<int>() : nullptr, cur_stream()),
         "mb_router_topk");
   return {w, idx, probs};
 }
@@ -82,7 +86,8 @@ void moe_combine_bwd(const at::Tensor& dout, const at::Tensor& y_perm, const at:
 }  // namespace
 
 void register_moe(pybind11::module& m) {
-  m.def("router_topk", &router_topk, py::arg("logits"), py::arg("k"), py::arg("normalize"), py::arg("want_probs"), py::arg("replay") = py::none());
+  m.def("router_topk", &router_topk, py::arg("logits"), py::arg("k"), py::arg("normalize"), py::arg("want_probs"), py::arg("replay") = py::none(),
+        py::arg("err") = py::none());
   m.def("moe_align", &moe_align, py::arg("idx"), py::arg("E"), py::arg("expert_offset"), py::arg("max_rows"), py::arg("n_dev"),
         py::arg("pad") = 128);
   m.def("moe_gather", &moe_gather);

@@ -123,7 +123,7 @@ int mb_paged_bounds_read(long long* out4, int clear);
 
 // ---- moe.cu ----
 int mb_router_topk(const float* logits, float* probs, float* topk_w, int* topk_idx, long long T, int E, int K, int normalize, const int* replay, long long replay_row,
-                   cudaStream_t s);
+                   int* error_flag, cudaStream_t s);
 int mb_moe_align(const int* idx, int n, const int* n_ptr, int E, int expert_offset, int* seg_offsets, int* tile_expert, int* row_src,
                  int* dst_row, int max_rows, cudaStream_t s);
 int mb_moe_align_pad(const int* idx, int n, const int* n_ptr, int E, int expert_offset, int* seg_offsets, int* tile_expert,

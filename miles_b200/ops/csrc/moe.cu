@@ -32,12 +32,14 @@ __device__ __forceinline__ float wmax(float v) {
 
 // ---------------------------------------------------------------------------------------------
 // `replay`: recorded choices, rows `replay_row` apart.  They replace the top-k and their weights come from these logits; a row without any
-// (all negative) is chosen afresh.  In one launch where softmax, gather, sum and division were kernels of their own behind a host
+// (all negative) is chosen afresh.  A choice outside [0, E) in another row is no record of this model: it raises the error flag (72), and
+// expert 0 with weight 0 stands in its place, so that nothing behind reads out of range.  In one launch where softmax, gather, sum and division were kernels of their own behind a host
 // synchronisation that asked whether any row was without: 12 launches and a round trip per layer.
 template <int EPL>  // experts per lane = E / 32
 __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restrict__ logits, float* __restrict__ probs,
                                                           float* __restrict__ topk_w, int* __restrict__ topk_idx, long long T, int E,
-                                                          int K, int normalize, const int* __restrict__ replay, long long replay_row) {
+                                                          int K, int normalize, const int* __restrict__ replay, long long replay_row,
+                                                          int* error_flag) {
   pdl_trigger();
   pdl_wait();
   const long long t = (blockIdx.x * 256ll + threadIdx.x) >> 5;
@@ -75,9 +77,11 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
 #pragma unroll
     for (int i = 0; i < EPL; ++i) p = (e >> 5) == i ? v[i] : p;
     p = __shfl_sync(0xffffffffu, p, e & 31);
-    if (e < 0 || e >= E) p = 0.f;
+    const bool valid = e >= 0 && e < E;
+    if (!valid) p = 0.f;
     wsel += p;
-    if (lane == j) { mine_w = p; mine_i = e; }
+    if (lane == j) { mine_w = p; mine_i = valid ? e : 0; }
+    if (!valid && lane == 0) atomicCAS(error_flag, 0, 72);
   }
   for (int j = 0; !replayed && j < K; ++j) {
     float bv = -1.f;
@@ -431,16 +435,16 @@ using namespace mb;
 MB_DEFINE_BOUNDS_API(mb_moe_bounds)
 
 extern "C" int mb_router_topk(const float* logits, float* probs, float* topk_w, int* topk_idx, long long T, int E, int K,
-                              int normalize, const int* replay, long long replay_row, cudaStream_t s) {
+                              int normalize, const int* replay, long long replay_row, int* error_flag, cudaStream_t s) {
   if (T == 0) return 0;
   if (E > 256 || K > 32) return -1;
   const unsigned blocks = static_cast<unsigned>((T + 7) / 8);
   const int epl = (E + 31) / 32;
   cudaError_t e;
-  if (epl <= 1) e = launch_pdl(router_topk_kernel<1>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row);
-  else if (epl <= 2) e = launch_pdl(router_topk_kernel<2>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row);
-  else if (epl <= 4) e = launch_pdl(router_topk_kernel<4>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row);
-  else e = launch_pdl(router_topk_kernel<8>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row);
+  if (epl <= 1) e = launch_pdl(router_topk_kernel<1>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row, error_flag);
+  else if (epl <= 2) e = launch_pdl(router_topk_kernel<2>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row, error_flag);
+  else if (epl <= 4) e = launch_pdl(router_topk_kernel<4>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row, error_flag);
+  else e = launch_pdl(router_topk_kernel<8>, dim3(blocks), dim3(256), 0, s, logits, probs, topk_w, topk_idx, T, E, K, normalize, replay, replay_row, error_flag);
   return static_cast<int>(e);
 }
 

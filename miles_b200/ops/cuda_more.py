@@ -133,7 +133,7 @@ def paged_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens=None, max
 class _RouterTopK(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, k, normalize, replay):
-        w, idx, probs = C.router_topk(_c(logits.float()), k, normalize, True, replay)
+        w, idx, probs = C.router_topk(_c(logits.float()), k, normalize, True, replay, C.error_flag(logits) if replay is not None else None)
         ctx.save_for_backward(probs, idx, w)
         ctx.normalize = normalize
         ctx.mark_non_differentiable(idx)
@@ -165,6 +165,7 @@ def router_topk(logits, k, normalize=True):
 
 
 def router_replay(logits, idx, normalize=True):
+    """A choice outside the experts, in a row that has any, raises the device error flag (72) and counts nothing."""
     if logits.shape[-1] > 256 or idx.shape[1] > 32:
         return ref.router_replay(logits, idx, normalize)
     idx = idx.to(torch.int32)

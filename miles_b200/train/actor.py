@@ -356,9 +356,21 @@ class TrainActor:
 
         batches = self.profiler.iterate("train_log_probs", micro_batches) if hasattr(self, "profiler") else micro_batches
         self._step_runner().forward_only_step(batches, pack, keep, replay=replay)
+        self._refuse_invalid_routing(replay)
         if tag is not None and tag != "actor":
             self.backuper.restore("actor")
         return [out[i] for i in sorted(out)]
+
+    def _refuse_invalid_routing(self, replay: bool):
+        """A record that names an expert the model does not have leaves log-probs of fewer experts behind and the device error flag raised:
+        nothing is done with them."""
+        if not replay or self.device.type != "cuda":
+            return
+        from ..ops import cuda as K
+
+        flag = K.check_error_flag(torch.empty(0, device=self.device))
+        if flag:
+            raise RuntimeError(f"device error flag {flag} after a pass with recorded routing (72: a record names an expert outside the model)")
 
     def _pad_multiple(self) -> int:
         zigzag = 2 if (self.ps.cp_size > 1 and self.ps.cp_comm_type in ("p2p", "a2a+p2p")) else 1     # ring CP: two pieces per rank
@@ -519,6 +531,7 @@ class TrainActor:
         # a custom one): this method only says how a micro-batch is packed and how its loss is computed
         runner = self._step_runner()
         runner.forward_backward_step(mbs, pack, score, want_ent=want_ent, replay=replay)
+        self._refuse_invalid_routing(replay)
         self._finalize_grads()
         if self.dumper is not None:
             with self.dumper.phase("fwd_bwd") as d:
