@@ -249,7 +249,7 @@ class DecoderLayer(nn.Module):
                     else DenseFFN(cfg, ps, dtype, device, gen, tag))
 
     def _forward_few_tokens(self, x, residual, meta: ForwardMeta):
-        """Decode with a handful of rows: each norm is fused into the matrix-vector projection that consumes it."""
+        """Decode with a handful of rows: the 1 / rms of each norm multiplies the sums of the projection that consumes it."""
         attn, mlp = self.attn, self.mlp
         qkv, residual, _ = ops.add_rmsnorm_linear(x, residual, self.ln1, self.eps, attn.wqkv, attn.bqkv)
         h = attn(None, meta, self.layer, qkv=qkv)

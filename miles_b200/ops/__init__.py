@@ -73,14 +73,13 @@ def rmsnorm(x, w, eps=1e-6):
 
 
 def few_token_decode(x, w) -> bool:
-    """True when the matrix-vector decode kernels apply to `x · wᵀ`: CUDA bf16, no autograd, a handful of rows.  They take rows eight at a
-    time: from nine on, norms by themselves and a cluster of CTAs per weight tile are faster (decode steps of 8 layers, 9 / 16 rows: hidden
-    2048 with 16 experts 875 / 929 → 770 / 800 µs, hidden 2560 1180 / 1289 → 659 / 698, hidden 1024 361 / 424 → 350 / 405)."""
-    return x.is_cuda and x.numel() <= 8 * x.shape[-1] and w.numel() <= _k().GEMV_MAX_WEIGHTS and _k().gemv_ok(x, w)
+    """True when the decode forms with the norm's 1 / rms behind the product (`add_rmsnorm_linear`) apply to `x · wᵀ`: CUDA bf16, no autograd,
+    a handful of rows."""
+    return x.is_cuda and _k().gemv_ok(x, w)
 
 
 def add_rmsnorm_linear(x, residual, norm_w, eps, w, bias=None, want_normed=False, out_fp32=False):
-    """rmsnorm(x + residual) · wᵀ in one kernel (only where `few_token_decode` holds).
+    """rmsnorm(x + residual) · wᵀ, rounded no more often than in one kernel (only where `few_token_decode` holds).
     Returns (y, x + residual, normalised activations or None)."""
     y, res, xn = _k().add_rmsnorm_linear(x, residual, norm_w, eps, w, bias, want_normed, out_fp32)
     return y, (x if res is None else res), xn

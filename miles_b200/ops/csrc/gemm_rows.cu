@@ -1,4 +1,10 @@
-// Projections of 9 to 64 tokens:  C[tokens, N] = X[tokens, K] · W[N, K]ᵀ  with every SM streaming weights.
+// Projections of up to 64 tokens:  C[tokens, N] = X[tokens, K] · W[N, K]ᵀ  with every SM streaming weights.  Up to 8 tokens that is for weights
+// of more than 12 Mi elements (smaller ones: gemv.cu), from 9 on for any.
+//
+// Up to 16 tokens with an RMSNorm in front (norm_rows): the staged operand is bf16(h · norm_w), h the sum with the residual as it is stored, and
+// 1 / rms multiplies the fp32 sums in the epilogue.  That is the arithmetic of gemv.cu: one rounding of the operand where the norm weight
+// is not a power of two, none where it is one; bf16(h / rms · norm_w) always has one (outputs in bf16, norm weights of one, hidden 2560: 2.4e-3
+// from 64 bits, 1.7e-3 this way, which is the rounding of the output alone; fp32 router scores lose that rounding altogether).
 //
 // As in gemm_small.cu the weight rows are the 128-row side of the MMA and the tokens its N side (16, 32 or 64).  A projection of a model
 // has 16 to 160 such tiles, so the reduction is cut as well: a CLUSTER of 1, 2, 4 or 8 CTAs shares one tile, each CTA streams its slice of
@@ -36,6 +42,7 @@ struct Params {
   long long ldc;
   int out_fp32;
   const __nv_bfloat16* bias;
+  const float* row_scale;             // [tokens] factors on the sums, or null
   int static_w;
   int stages;
   int* error_flag;
@@ -137,9 +144,12 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   }
   const int q = warp & 3;
   const int n = n_blk * BMW + q * 32 + lane;         // output feature of this thread (warps 2..5)
+  __shared__ float scale[4][BT];                     // a copy per warp, fetched while the products run
   float v[BT];
   if (warp >= 2) {
-    pdl_wait();                                      // C and the bias: after the kernels in front
+    pdl_wait();                                      // C, the bias and the factors: after the kernels in front
+    if (p.row_scale != nullptr)
+      for (int i = lane; i < p.tokens; i += 32) scale[q][i] = p.row_scale[i];
     if (!mbar_wait(tmem_full, 0)) atomicExch(p.error_flag, 47);
     __syncwarp();
     tc_fence_after();
@@ -156,6 +166,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   const int tokens = n < p.N ? p.tokens : 0;         // a feature past the last one stores nothing
   const float bias = warp >= 2 && tokens > 0 && p.bias != nullptr ? __bfloat162float(p.bias[n]) : 0.f;
   auto put = [&](int tok, float x) {                 // lanes hold consecutive features: one 64- or 128-byte store per token and warp
+    if (p.row_scale != nullptr) x *= scale[q][tok];
     if (p.bias != nullptr) x += bias;
     if (p.out_fp32) reinterpret_cast<float*>(p.C)[tok * p.ldc + n] = x;
     else reinterpret_cast<__nv_bfloat16*>(p.C)[tok * p.ldc + n] = __float2bfloat16(x);
@@ -220,13 +231,80 @@ static int launch(const CUtensorMap& tw, const CUtensorMap& tx, const Params& p,
   }
 }
 
+// One row per CTA: h = bf16(x + residual) → sum (if there is a residual), bf16(h · w) → scaled, 1 / rms(h) → rstd and, if wanted, bf16(h / rms · w)
+// → normed.  A handful of rows: the time is one launch and two trips to memory.
+__global__ void __launch_bounds__(256) norm_rows_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual, const __nv_bfloat16* w, float eps, int K,
+                                                        __nv_bfloat16* scaled, float* rstd_out, __nv_bfloat16* sum, __nv_bfloat16* normed) {
+  __shared__ float part[8];
+  pdl_trigger();
+  pdl_wait();
+  const long long row = static_cast<long long>(blockIdx.x) * K;
+  auto two = [](uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); };
+  auto times_w = [&](uint4 h, int at, float f) {
+    const uint4 wv = *reinterpret_cast<const uint4*>(w + at);
+    const uint32_t hs[4] = {h.x, h.y, h.z, h.w}, ws[4] = {wv.x, wv.y, wv.z, wv.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 a = two(hs[i]), b = two(ws[i]);
+      o[i] = pack_bf16x2(a.x * f * b.x, a.y * f * b.y);
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+  };
+  float ss = 0.f;
+  for (int at = threadIdx.x * 8; at < K; at += 2048) {
+    uint4 h = *reinterpret_cast<const uint4*>(x + row + at);
+    uint32_t* hs = &h.x;
+    if (residual != nullptr) {
+      const uint4 r = *reinterpret_cast<const uint4*>(residual + row + at);
+      const uint32_t rs[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 a = two(hs[i]), b = two(rs[i]);
+        hs[i] = pack_bf16x2(a.x + b.x, a.y + b.y);
+      }
+      *reinterpret_cast<uint4*>(sum + row + at) = h;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 a = two(hs[i]);
+      ss += a.x * a.x + a.y * a.y;
+    }
+    *reinterpret_cast<uint4*>(scaled + row + at) = times_w(h, at, 1.f);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) ss += part[i];
+  const float rstd = rsqrtf(ss / K + eps);
+  if (threadIdx.x == 0) rstd_out[blockIdx.x] = rstd;
+  if (normed != nullptr)
+    for (int at = threadIdx.x * 8; at < K; at += 2048)       // this thread's own pieces again
+      *reinterpret_cast<uint4*>(normed + row + at) = times_w(*reinterpret_cast<const uint4*>((residual != nullptr ? sum : x) + row + at), at, rstd);
+}
+
 }  // namespace rows
 }  // namespace mb
 
-// C[tokens, N] (bf16 or fp32) = X[tokens, K] · W[N, K]ᵀ (+ bias), tokens ≤ 64.  split: 1, 2, 4 or 8 slices of K.  static_w: no kernel that may
-// still run on the stream writes W.
+// See norm_rows_kernel; x, residual (or null), sum, scaled, normed (or null) [T, K] bf16, w [K] bf16, all 16-byte aligned, K a multiple of 8.
+extern "C" int mb_norm_rows(const void* x, const void* residual, const void* w, float eps, int T, int K, void* scaled, float* rstd, void* sum, void* normed,
+                            cudaStream_t s) {
+  using namespace mb;
+  typedef const __nv_bfloat16* cbf;
+  typedef __nv_bfloat16* bf;
+  if (T <= 0) return 0;
+  if (K % 8 || (residual != nullptr && sum == nullptr)) return -2;
+  return static_cast<int>(launch_pdl(rows::norm_rows_kernel, dim3(T), dim3(256), 0, s, (cbf)x, (cbf)residual, (cbf)w, eps, K, (bf)scaled, rstd, (bf)sum,
+                                     (bf)normed));
+}
+
+// C[tokens, N] (bf16 or fp32) = X[tokens, K] · W[N, K]ᵀ (· row_scale[token]) (+ bias), tokens ≤ 64.  split: 1, 2, 4 or 8 slices of K.  static_w: no
+// kernel that may still run on the stream writes W.
 extern "C" int mb_gemm_rows(const void* X, const void* W, void* C, int tokens, int N, int K, long long ldx, long long ldw, long long ldc, int out_fp32,
-                            const void* bias, int split, int static_w, int* error_flag, cudaStream_t s) {
+                            const void* bias, const float* row_scale, int split, int static_w, int* error_flag, cudaStream_t s) {
   using namespace mb;
   if (tokens <= 0 || N <= 0) return 0;
   if (tokens > 64 || (split != 1 && split != 2 && split != 4 && split != rows::kMaxSplit)) return -2;
@@ -236,7 +314,7 @@ extern "C" int mb_gemm_rows(const void* X, const void* W, void* C, int tokens, i
   if (r) return 1000 + r;
   r = make_tmap_bf16_2d(&tx, X, tokens, K, ldx, bt, rows::BK);
   if (r) return 2000 + r;
-  const rows::Params p{tokens, N, K, C, ldc, out_fp32, reinterpret_cast<const __nv_bfloat16*>(bias), static_w, 0, error_flag};
+  const rows::Params p{tokens, N, K, C, ldc, out_fp32, reinterpret_cast<const __nv_bfloat16*>(bias), row_scale, static_w, 0, error_flag};
   switch (bt) {
     case 16: return rows::launch<16>(tw, tx, p, split, s);
     case 32: return rows::launch<32>(tw, tx, p, split, s);

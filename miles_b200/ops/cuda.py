@@ -100,10 +100,7 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *
     if M and N:
         plain = not accumulate and not force_bn
         split = _row_split(M, N, K) if plain and M <= SMALL_M else 0
-        # the matrix-vector kernel takes its rows eight at a time: from nine on a cluster per weight tile is faster (9 rows, N × K: 5120 × 2048
-        # 8.3 → 6.2 µs, 2560 × 4096 11.7 → 6.0, 19456 × 2560 37.3 → 19.6, 6144 × 1024 4.6 → 4.5)
-        few = GEMV_M if not split else min(8, GEMV_M) if N * K <= GEMV_MAX_WEIGHTS else 0
-        if plain and M <= few and _gemv_k_ok(M, K) and N <= GEMV_MAX_N:
+        if plain and M <= _gemv_rows(split, N, K) and _gemv_k_ok(M, K) and N <= GEMV_MAX_N:
             C.gemv(a, None, None, 0.0, b, bias, out, None, None, bool(b.is_leaf and b.requires_grad))
             return out
         if plain and M <= SMALL_M:
@@ -148,14 +145,22 @@ def _splitk_workspace(device):
     return _splitk_ws[key]
 
 
-# A handful of tokens (decode with a nearly drained batch): matrix-vector kernels without pipeline set-up (gemv.cu).
-# Up to 16 rows are supported; 0 turns the path off.
+# A handful of tokens (decode with a nearly drained batch): matrix-vector kernels without pipeline set-up (gemv.cu), and the norm in front of a
+# projection inside it.  Up to 16 rows are supported (`_gemv_rows`: which of them gemm_rows.cu takes instead); 0 turns the path off.
 GEMV_M = min(16, int(os.environ.get("MILES_GEMV_M", "16")))
 GEMV_MAX_N = int(os.environ.get("MILES_GEMV_MAX_N", "32768"))
 # Larger weights (24 MB) stream faster through gemm_rows.cu's rings whatever the rows.  Decode steps of 8 layers, 1 / 4 / 8 rows: hidden 2560
-# (21 to 100 MB per projection) 776 / 816 / 908 → 621 / 633 / 666 µs, everything there 612 / 630 / 658; hidden 2048 with 16 experts (17 and
-# 21 MB) 565 / 675 / 750 against 555 / 683 / 727, hidden 1024 (up to 12 MB) 300 / 325 / 362 against 299 / 322 / 345.
+# (21 to 100 MB per projection) 776 / 816 / 908 → 621 / 633 / 666 µs, everything there 612 / 630 / 658.  For smaller ones it is within 2 % either
+# way up to 4 rows (hidden 2048 with 16 experts, 17 and 21 MB: 565 / 675 / 750 against 555 / 683 / 727; hidden 1024, up to 12 MB: 300 / 325 / 362
+# against 299 / 322 / 345), and they keep the order of their sums.
 GEMV_MAX_WEIGHTS = 12 << 20
+
+
+def _gemv_rows(split: int, N: int, K: int) -> int:
+    """Most rows of a projection that the matrix-vector kernel takes where gemm_rows.cu would cut it `split` ways (0: not its size).  It takes
+    them eight at a time: from nine on a cluster per weight tile is faster (9 rows, N × K: 5120 × 2048 8.3 → 6.2 µs, 2560 × 4096 11.7 → 6.0,
+    19456 × 2560 37.3 → 19.6, 6144 × 1024 4.6 → 4.5)."""
+    return GEMV_M if not split else min(8, GEMV_M) if N * K <= GEMV_MAX_WEIGHTS else 0
 
 
 def _gemv_k_ok(rows: int, K: int) -> bool:
@@ -164,8 +169,8 @@ def _gemv_k_ok(rows: int, K: int) -> bool:
 
 
 def add_rmsnorm_linear(x, residual, norm_w, eps, w, bias=None, want_normed: bool = False, out_fp32: bool = False):
-    """Inference only, ≤ GEMV_M rows: y = rmsnorm(x + residual) · wᵀ in one kernel.
-    Returns (y, x + residual or None, normalised activations or None)."""
+    """Inference only, ≤ GEMV_M rows: y = rmsnorm(x + residual) · wᵀ with the sums multiplied by 1 / rms, in one kernel or, where the projection
+    is gemm_rows.cu's, in two.  Returns (y, x + residual or None, normalised activations or None)."""
     K = x.shape[-1]
     x2 = _c(x.reshape(-1, K))
     r2 = _c(residual.reshape(-1, K)) if residual is not None else None
@@ -173,7 +178,14 @@ def add_rmsnorm_linear(x, residual, norm_w, eps, w, bias=None, want_normed: bool
     y = torch.empty(M, N, dtype=torch.float32 if out_fp32 else BF16, device=x.device)
     res_out = torch.empty_like(x2) if r2 is not None else None
     xn = torch.empty_like(x2) if want_normed else None
-    C.gemv(x2, r2, norm_w, float(eps), w, bias, y, res_out, xn, bool(w.is_leaf and w.requires_grad))
+    static_w = bool(w.is_leaf and w.requires_grad)
+    split = _row_split(M, N, K) if M <= SMALL_M else 0
+    if split and M > _gemv_rows(split, N, K):
+        scaled, rstd = torch.empty_like(x2), torch.empty(M, dtype=torch.float32, device=x.device)
+        C.norm_rows(x2, r2, norm_w, float(eps), scaled, rstd, res_out, xn)
+        C.gemm_rows(scaled, w, y, M, N, K, N, bias, split, static_w, rstd)
+    else:
+        C.gemv(x2, r2, norm_w, float(eps), w, bias, y, res_out, xn, static_w)
     shp = x.shape[:-1]
     return (y.view(*shp, N), res_out.view(x.shape) if res_out is not None else None, xn.view(x.shape) if xn is not None else None)
 

@@ -47,7 +47,67 @@ def test_from_matrix_vector_to_clusters(M, N):
     g = torch.Generator(device="cuda").manual_seed(M)
     x, w = torch.randn(M, 1024, device="cuda", generator=g).bfloat16(), torch.randn(N, 1024, device="cuda", generator=g).bfloat16()
     with torch.no_grad():
-        assert ops.few_token_decode(x, w) == (M <= 8 and N <= 12288)
+        assert ops.few_token_decode(x, w) == (M <= 16)
+        assert (M <= K._gemv_rows(K._row_split(M, N, 1024), N, 1024)) == (M <= 8 and N <= 12288)
         y = K.linear(x, w)
     want = x.double() @ w.double().t()
     assert ((y.double() - want).norm() / want.norm()).item() < 2 ** -8.5          # one rounding to bf16
+
+
+@pytest.mark.parametrize("M,N,Kd", [(1, 640, 2048), (8, 640, 2048), (9, 640, 2048), (16, 16, 2048), (16, 5120, 2048), (1, 6144, 2560), (4, 6144, 2560),
+                                    (13, 19456, 2560), (8, 12416, 1024), (9, 200, 4064)])
+@pytest.mark.parametrize("ones", [True, False])
+@pytest.mark.parametrize("with_residual", [True, False])
+def test_few_rows_behind_a_norm(M, N, Kd, ones, with_residual):
+    """Whichever kernel takes the projection: with norm weights of one its operand is the sum itself, not a rounded quotient."""
+    from miles_b200 import ops
+    from miles_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, r, w = rand(M, Kd).bfloat16(), rand(M, Kd).bfloat16() if with_residual else None, (rand(N, Kd) * 0.05).bfloat16()
+    nw = torch.ones(Kd, device="cuda").bfloat16() if ones else (1 + 0.1 * rand(Kd)).bfloat16()
+    bias = rand(N).bfloat16()
+    h = (x.double() + r.double()).bfloat16() if with_residual else x
+    quotient = h.double() * torch.rsqrt(h.double().pow(2).mean(-1, keepdim=True) + 1e-6)
+    want = quotient * nw.double() @ w.double().t() + bias.double()
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
+    with torch.no_grad():
+        assert ops.few_token_decode(x, w)                 # what a decoder layer asks; else it norms first and multiplies then
+        y, total, normed = K.add_rmsnorm_linear(x, r, nw, 1e-6, w, bias, want_normed=True)
+        y32, _, none = K.add_rmsnorm_linear(x, r, nw, 1e-6, w, bias, out_fp32=True)
+    assert none is None and ((total is None) if r is None else torch.equal(total, h))
+    assert rel(normed, quotient * nw.double()) < 2 ** -9                          # one rounding to bf16: 2^-9 of each value at most
+    # fp32: the order of sums of up to 4064 terms; times norm weights, one rounding of the operand on the way (2^-9 of each term, independent)
+    assert rel(y32, want) < (1e-5 if ones else 2 ** -9)
+    assert rel(y, want) < (2 ** -9 if ones else 2 ** -8.5)                        # … and one of the result
+    assert K.check_error_flag(x) == 0
+
+
+def test_weights_ahead_of_the_rows():
+    """Weights that nothing on the stream writes are requested before the kernel in front, which makes the rows, has finished."""
+    from miles_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x, nw = torch.randn(16, 2560, device="cuda", generator=g).bfloat16(), torch.ones(2560, device="cuda").bfloat16()
+    ws = [torch.nn.Parameter((torch.randn(2560, 2560, device="cuda", generator=g) * 0.02).bfloat16()) for _ in range(6)]
+    with torch.no_grad():
+        def chain():
+            y = x
+            for w in ws:                                  # norm and product in turn: each kernel reads what the one in front writes
+                y = K.add_rmsnorm_linear(y, None, nw, 1e-6, w)[0]
+            return y
+        first = chain()
+        stepwise = x
+        for w in ws:
+            torch.cuda.synchronize()
+            stepwise = K.add_rmsnorm_linear(stepwise, None, nw, 1e-6, w)[0]
+            torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = chain()
+        for _ in range(20):
+            captured.zero_()
+            graph.replay()
+            assert torch.equal(captured, stepwise)
+    assert torch.equal(first, stepwise) and K.check_error_flag(x) == 0
