@@ -221,10 +221,10 @@ __global__ void __launch_bounds__(256) moe_dispatch_kernel(const bf16* __restric
 // peer's publish, read and reset the receive counter, counting-sort the received rows by local expert;
 // `moe_return_signal` = return + publish; `moe_combine_wait` = wait + weighted sum.  Four launches where the general path
 // takes eight (dispatch, barrier, expert-id scan, align, …, return, barrier, combine).
-__global__ void __launch_bounds__(256) moe_dispatch_signal_kernel(const bf16* __restrict__ x, const int* __restrict__ topk_idx,
+__global__ void __launch_bounds__(256) moe_dispatch_signal_kernel(const bf16* x, const int* topk_idx,
                                                                   long long n_pairs, int k, int H, int e_local, int rank,
                                                                   PeerPtrs recv_x, PeerPtrs recv_meta, PeerPtrs counters, int capacity,
-                                                                  int* __restrict__ sent_row, int* err, PeerPtrs flags, int world,
+                                                                  int* sent_row, int* err, PeerPtrs flags, int world,
                                                                   int channel, int* epochs, int* ticket) {
   // programmatic dependent launch: the successor may be scheduled at once (it waits for this grid's completion before it
   // reads anything), and nothing a predecessor wrote is read here before the wait
@@ -264,9 +264,9 @@ __global__ void __launch_bounds__(256) moe_dispatch_signal_kernel(const bf16* __
 }
 
 // One block.  Outputs as `moe_align`: seg_offsets[E+1] (segments padded to `pad`), tile_expert[max_rows / pad], row_src[max_rows].
-__global__ void __launch_bounds__(1024) moe_recv_align_kernel(const int4* __restrict__ meta, int* __restrict__ counter, int capacity, int E,
-                                                              int* __restrict__ seg_offsets, int* __restrict__ tile_expert,
-                                                              int* __restrict__ row_src, int max_rows, int pad, PeerPtrs flags, int rank,
+__global__ void __launch_bounds__(1024) moe_recv_align_kernel(const int4* meta, int* counter, int capacity, int E,
+                                                              int* seg_offsets, int* tile_expert,
+                                                              int* row_src, int max_rows, int pad, PeerPtrs flags, int rank,
                                                               int world, int channel, const int* epochs, int* err) {
   extern __shared__ int sh[];   // counts[E], cursor[E], seg[E+1], n
   int* counts = sh;
@@ -322,8 +322,8 @@ __global__ void __launch_bounds__(1024) moe_recv_align_kernel(const int4* __rest
   }
 }
 
-__global__ void __launch_bounds__(256) moe_return_signal_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ row_src,
-                                                                const int4* __restrict__ meta, const int* __restrict__ seg_offsets, int E,
+__global__ void __launch_bounds__(256) moe_return_signal_kernel(const bf16* y_perm, const int* row_src,
+                                                                const int4* meta, const int* seg_offsets, int E,
                                                                 int H, int max_rows, PeerPtrs ret, PeerPtrs flags, int rank, int world,
                                                                 int channel, int* epochs, int* ticket) {
   pdl_trigger();
@@ -345,8 +345,8 @@ __global__ void __launch_bounds__(256) moe_return_signal_kernel(const bf16* __re
 }
 
 // out[t, :] = Σ_j w[t, j] · ret[t·k + j, :] over the pairs that took part (sent_row ≥ 0), after every peer's publish arrived
-__global__ void __launch_bounds__(256) moe_combine_wait_kernel(const bf16* __restrict__ ret, const float* __restrict__ w,
-                                                               const int* __restrict__ sent_row, bf16* __restrict__ out, long long T, int k,
+__global__ void __launch_bounds__(256) moe_combine_wait_kernel(const bf16* ret, const float* w,
+                                                               const int* sent_row, bf16* out, long long T, int k,
                                                                int H, PeerPtrs flags, int rank, int world, int channel, const int* epochs,
                                                                int* err) {
   // the next kernel of the stream (the following layer's fused norm + projection) is released at once: it streams its

@@ -23,8 +23,8 @@ template <typename T> __device__ __forceinline__ float decay_of(float raw, float
 static constexpr float kUnitEps = 1e-6f;
 
 template <typename T, int V, int TAPS>
-__global__ void __launch_bounds__(kConv) delta_conv_kernel(const T* __restrict__ proj, long long ld, MbDelta m, const int* __restrict__ tiles,
-                                                           const int* __restrict__ cu_q, int blocks, T* __restrict__ act) {
+__global__ void __launch_bounds__(kConv) delta_conv_kernel(const T* proj, long long ld, MbDelta m, const int* tiles,
+                                                           const int* cu_q, int blocks, T* act) {
   pdl_trigger();
   pdl_wait();
   const int tile = blockIdx.x / blocks, cb = blockIdx.x % blocks;
@@ -41,8 +41,8 @@ static constexpr int kSlice = 32;   // state columns (of V) per CTA
 
 // grid (column slices, heads, sequences), 128 threads: lane = column, warp w owns the rows d ≡ w (mod 4) of the slice
 template <typename T>
-__global__ void __launch_bounds__(128) delta_seq_kernel(const T* __restrict__ proj, long long ld, const T* __restrict__ act, MbDelta m,
-                                                        const int* __restrict__ cu_q, T* __restrict__ out) {
+__global__ void __launch_bounds__(128) delta_seq_kernel(const T* proj, long long ld, const T* act, MbDelta m,
+                                                        const int* cu_q, T* out) {
   extern __shared__ __align__(16) float sm[];
   const int K = m.K, V = m.V, H = m.H, CH = channels_of(m);
   float* S = sm;                         // [K][kSlice]
@@ -134,8 +134,8 @@ static constexpr int kStepRows = 16, kStepThreads = 512;      // state rows of a
 // grid (heads, rows of the batch), 32·⌈V/16⌉ threads; V % 4 == 0.  A warp owns 16 state columns: lane = (4 columns lane % 4, rows lane / 4 + 8·u), so
 // that both sums over rows are exchanges inside the warp.  THREADS: the most a launch has.
 template <typename T, int U, int THREADS>
-__global__ void __launch_bounds__(THREADS, 512 / THREADS) delta_step_kernel(const T* __restrict__ proj, long long ld, MbDelta m, const T* __restrict__ norm_w,
-                                                                            const T* __restrict__ gate, long long gate_ld, float eps, T* __restrict__ out) {
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) delta_step_kernel(const T* proj, long long ld, MbDelta m, const T* __restrict__ norm_w,
+                                                                            const T* gate, long long gate_ld, float eps, T* out) {
   extern __shared__ __align__(16) float sm[];
   __shared__ float part[kStepThreads / 32];
   pdl_trigger();

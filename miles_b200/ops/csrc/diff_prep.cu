@@ -56,10 +56,10 @@ __device__ __forceinline__ void norm_rows(const T* __restrict__ x, const T* __re
 }
 
 template <typename T, bool VEC, bool GROUPED>
-__global__ void __launch_bounds__(kDiff) diff_prep_kernel(const T* __restrict__ proj, long long ld, const int* __restrict__ positions,
-                                                          const long long* __restrict__ slots, const T* __restrict__ q_norm,
-                                                          const T* __restrict__ k_norm, const T* __restrict__ lvec, float* __restrict__ lam,
-                                                          T* __restrict__ kc, T* __restrict__ vc, T* __restrict__ q, MbDiffPrep L, MbAside a) {
+__global__ void __launch_bounds__(kDiff) diff_prep_kernel(const T* proj, long long ld, const int* positions,
+                                                          const long long* slots, const T* __restrict__ q_norm,
+                                                          const T* __restrict__ k_norm, const T* __restrict__ lvec, float* lam,
+                                                          T* kc, T* vc, T* q, MbDiffPrep L, MbAside a) {
   pdl_trigger();
   pdl_wait();
   constexpr int V = VEC ? 16 / static_cast<int>(sizeof(T)) : 1;
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kDiff) diff_prep_kernel(const T* __restrict__ 
 
 // a warp per (token, head)
 template <typename T>
-__global__ void __launch_bounds__(256) diff_combine_kernel(const float* __restrict__ a, T* __restrict__ out, long long o_row, long long n, int heads,
+__global__ void __launch_bounds__(256) diff_combine_kernel(const float* a, T* out, long long o_row, long long n, int heads,
                                                            int vdim, MbDiff d) {
   pdl_trigger();
   pdl_wait();

@@ -38,8 +38,7 @@ struct alignas(16) bf16x8 {
   __nv_bfloat162 v[4];
 };
 
-__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
-  const bf16x8 t = *reinterpret_cast<const bf16x8*>(p);
+__device__ __forceinline__ void decode8(const bf16x8& t, float (&f)[8]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float2 a = __bfloat1622float2(t.v[i]);
@@ -47,6 +46,7 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
     f[2 * i + 1] = a.y;
   }
 }
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) { decode8(*reinterpret_cast<const bf16x8*>(p), f); }
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   bf16x8 t;
 #pragma unroll
@@ -59,9 +59,9 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 //   ADD: r_new = x + residual (rounded to bf16, written to `res_out`), y = rmsnorm(r_new)·w
 // ---------------------------------------------------------------------------------------------
 template <bool ADD>
-__global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
-                                                          const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                                                          __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int H,
+__global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual,
+                                                          const __nv_bfloat16* __restrict__ w, __nv_bfloat16* y,
+                                                          __nv_bfloat16* res_out, float* rstd_out, int H,
                                                           float eps) {
   __shared__ float sh[32];
   pdl_trigger();
@@ -69,17 +69,26 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
   const long long row = blockIdx.x;
   const __nv_bfloat16* xr = x + row * H;
   constexpr int MAXI = 4;  // rows up to 256·8·4 = 8192 wide stay in registers
-  float vals[MAXI][8];
-  float ss = 0.f;
+  bf16x8 raw[MAXI], res[MAXI];   // all of them requested before the first store: to the compiler the sum may lie over either
   const int nvec = H / 8;
 #pragma unroll
   for (int it = 0; it < MAXI; ++it) {
     const int v = threadIdx.x + it * 256;
     if (v < nvec) {
-      load8(xr + v * 8, vals[it]);
+      raw[it] = *reinterpret_cast<const bf16x8*>(xr + v * 8);
+      if (ADD) res[it] = *reinterpret_cast<const bf16x8*>(residual + row * H + v * 8);
+    }
+  }
+  float vals[MAXI][8];
+  float ss = 0.f;
+#pragma unroll
+  for (int it = 0; it < MAXI; ++it) {
+    const int v = threadIdx.x + it * 256;
+    if (v < nvec) {
+      decode8(raw[it], vals[it]);
       if (ADD) {
         float r[8];
-        load8(residual + row * H + v * 8, r);
+        decode8(res[it], r);
 #pragma unroll
         for (int i = 0; i < 8; ++i) vals[it][i] = __bfloat162float(__float2bfloat16(vals[it][i] + r[i]));
         store8(res_out + row * H + v * 8, vals[it]);
@@ -129,9 +138,9 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
 // loads in flight at once (2·VPL·16 bytes), the row sum needs shuffles only — no shared memory, no CTA barrier — and the
 // post-add values wait in registers as packed bf16.  Eight rows per CTA.
 template <bool ADD, int VPL>
-__global__ void __launch_bounds__(256) rmsnorm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
-                                                               const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                                                               __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out,
+__global__ void __launch_bounds__(256) rmsnorm_fwd_warp_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual,
+                                                               const __nv_bfloat16* __restrict__ w, __nv_bfloat16* y,
+                                                               __nv_bfloat16* res_out, float* rstd_out,
                                                                long long T, float eps) {
   pdl_trigger();
   pdl_wait();
@@ -365,8 +374,8 @@ __global__ void __launch_bounds__(1024) colsum_kernel(const float* __restrict__ 
 // ---------------------------------------------------------------------------------------------
 // SwiGLU: in [T, 2F] (gate | up) → out [T, F]
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
-                                                         long long T, int F, const int* __restrict__ rows_ptr) {
+__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* in, __nv_bfloat16* out,
+                                                         long long T, int F, const int* rows_ptr) {
   pdl_trigger();
   pdl_wait();
   const int nvec = F / 8;
@@ -564,13 +573,13 @@ static bool rope_by_fours(long long T, int Hq, int Hk, int heads, int D, long lo
 // Engine form: the same per-head norm + rotary for q and k, with the rotated k and the raw v also written into the
 // paged KV cache at each token's slot (slot < 0: token not cached).  One warp per (token, q/k/v head).
 template <int D>
-__global__ void __launch_bounds__(256) qk_norm_rope_cache_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                                                                 const __nv_bfloat16* __restrict__ v, long long q_tok_stride,
+__global__ void __launch_bounds__(256) qk_norm_rope_cache_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k,
+                                                                 const __nv_bfloat16* v, long long q_tok_stride,
                                                                  long long k_tok_stride, long long v_tok_stride,
                                                                  const __nv_bfloat16* __restrict__ qw, const __nv_bfloat16* __restrict__ kw,
-                                                                 const int* __restrict__ positions, __nv_bfloat16* __restrict__ qo,
-                                                                 __nv_bfloat16* __restrict__ ko, __nv_bfloat16* __restrict__ kc,
-                                                                 __nv_bfloat16* __restrict__ vc, const long long* __restrict__ slots,
+                                                                 const int* positions, __nv_bfloat16* qo,
+                                                                 __nv_bfloat16* ko, __nv_bfloat16* kc,
+                                                                 __nv_bfloat16* vc, const long long* slots,
                                                                  long long T, int Hq, int Hk, float log2_theta, float eps) {
   pdl_trigger();
   pdl_wait();

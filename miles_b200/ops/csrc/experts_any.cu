@@ -9,8 +9,8 @@ static constexpr int kExp = 256;
 
 // act[pair, f] = clamped_glu(W13[e][f]·x, W13[e][F + f]·x), or with alpha = 0 relu(W13[e][f]·x)² of [E, F, H] experts.  grid (pairs, feature blocks of 8 warps)
 template <typename T>
-__global__ void __launch_bounds__(kExp) experts_up_kernel(const T* __restrict__ x, const T* __restrict__ w13, const int* __restrict__ index,
-                                                          T* __restrict__ act, int k, int E, int H, int F, float limit, float alpha,
+__global__ void __launch_bounds__(kExp) experts_up_kernel(const T* x, const T* __restrict__ w13, const int* index,
+                                                          T* act, int k, int E, int H, int F, float limit, float alpha,
                                                           float shift) {
   extern __shared__ float xs[];
   pdl_trigger();
@@ -38,8 +38,8 @@ __global__ void __launch_bounds__(kExp) experts_up_kernel(const T* __restrict__ 
 
 // out[t, h] = Σ_j weights[t, j] · (W2[e][h]·act[t·k + j])
 template <typename T>
-__global__ void __launch_bounds__(kExp) experts_down_kernel(const T* __restrict__ act, const T* __restrict__ w2, const int* __restrict__ index,
-                                                            const float* __restrict__ weights, T* __restrict__ out, int k, int E, int H, int F) {
+__global__ void __launch_bounds__(kExp) experts_down_kernel(const T* act, const T* __restrict__ w2, const int* index,
+                                                            const float* weights, T* out, int k, int E, int H, int F) {
   pdl_trigger();
   pdl_wait();
   const long long t = blockIdx.x;

@@ -488,8 +488,8 @@ __device__ __forceinline__ int pair_of(unsigned long long mask, int tok, int k) 
 // for all tokens, silu(gate) · up (or its clamped form) stored for the tokens routed to it.  Otherwise 16 rows of a [F, H] expert, relu(·)².  A warp's weight stream runs
 // across its items without a break (the ring keeps filling while the CTA reduces and stores an item).
 template <bool GATED>
-__global__ void __launch_bounds__(kThreads) moe_gemv_up_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w13,
-                                                               const int* __restrict__ topk_idx, bf16* __restrict__ act, int T, int k,
+__global__ void __launch_bounds__(kThreads) moe_gemv_up_kernel(const bf16* x, const bf16* __restrict__ w13,
+                                                               const int* topk_idx, bf16* act, int T, int k,
                                                                int E, int offset, int H, int F, float limit, float alpha, float shift) {
   constexpr int S = kMoeStages, kFeat = GATED ? 8 : 16;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -606,9 +606,9 @@ __global__ void __launch_bounds__(kThreads) moe_gemv_up_kernel(const bf16* __res
 // the 32-wide k chunks of EVERY expert round-robin (equal work per warp whatever the routing), a warp's weight stream runs
 // across the experts without a break.
 // out[t, h] = Σ_experts gate_w(t, e) · (W2[e][h, :] · act[pair(t, e), :])
-__global__ void __launch_bounds__(kThreads) moe_gemv_down_kernel(const bf16* __restrict__ act, const bf16* __restrict__ w2,
-                                                                 const int* __restrict__ topk_idx, const float* __restrict__ topk_w,
-                                                                 bf16* __restrict__ out, int T, int k, int E, int offset, int H, int F) {
+__global__ void __launch_bounds__(kThreads) moe_gemv_down_kernel(const bf16* act, const bf16* __restrict__ w2,
+                                                                 const int* topk_idx, const float* topk_w,
+                                                                 bf16* out, int T, int k, int E, int offset, int H, int F) {
   constexpr int S = kMoeStages;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ float red[kWarps][16][8];

@@ -15,11 +15,11 @@ namespace mx {
 // form; later ones the rotated part and the padding of an absorbed query [H][pitch] (head_linear fills [0, rank)).
 // VEC: rows and head parts start on 16-byte boundaries and are whole 16-byte pieces.
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256) latent_prep_kernel(const T* __restrict__ q_in, long long q_ld, const T* __restrict__ kv_in, long long kv_ld,
-                                                          const int* __restrict__ positions,
-                                                          const long long* __restrict__ slots, const double* __restrict__ freq,
+__global__ void __launch_bounds__(256) latent_prep_kernel(const T* q_in, long long q_ld, const T* kv_in, long long kv_ld,
+                                                          const int* positions,
+                                                          const long long* slots, const double* __restrict__ freq,
                                                           float magnitude, const T* __restrict__ kv_norm, float eps,
-                                                          T* __restrict__ cache, T* __restrict__ q_abs, T* __restrict__ q_full, int t_long,
+                                                          T* cache, T* q_abs, T* q_full, int t_long,
                                                           int q_nope, int q_width, MbLatent L) {
   extern __shared__ float cs[];          // [rot/2] cosines, [rot/2] sines
   __shared__ float sh[8];
@@ -96,9 +96,9 @@ __global__ void __launch_bounds__(256) latent_prep_kernel(const T* __restrict__ 
 
 // y[t, h, n] = Σ_k x[t, h, k] · w[h](n, k); w [H, N, K] when NK, else [H, K, N].  Any sizes; one output per thread.
 template <typename T, bool NK>
-__global__ void __launch_bounds__(128) head_linear_kernel(const T* __restrict__ x, long long x_t, long long x_h, const T* __restrict__ w,
-                                                          T* __restrict__ y, long long y_t, long long y_h, int N, int K,
-                                                          const T* __restrict__ gate, long long gate_ld) {
+__global__ void __launch_bounds__(128) head_linear_kernel(const T* x, long long x_t, long long x_h, const T* __restrict__ w,
+                                                          T* y, long long y_t, long long y_h, int N, int K,
+                                                          const T* gate, long long gate_ld) {
   extern __shared__ float xs[];
   pdl_trigger();
   pdl_wait();

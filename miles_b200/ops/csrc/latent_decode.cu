@@ -40,9 +40,9 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 }
 
 // one warp per packed row: row i of sequence b is position base[b] + (i − cu_k[b])
-__global__ void __launch_bounds__(256) latent_gather_kernel(const bf16* __restrict__ cache, const int* __restrict__ block_table, int max_blocks,
-                                                            int block_size, const int* __restrict__ cu_k, const int* __restrict__ base,
-                                                            bf16* __restrict__ out, int n_seq, int total, int pitch) {
+__global__ void __launch_bounds__(256) latent_gather_kernel(const bf16* cache, const int* block_table, int max_blocks,
+                                                            int block_size, const int* cu_k, const int* base,
+                                                            bf16* out, int n_seq, int total, int pitch) {
   pdl_trigger();
   pdl_wait();
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -61,9 +61,9 @@ __global__ void __launch_bounds__(256) latent_gather_kernel(const bf16* __restri
 
 // grid (N / (32·NW), H, ceil(T / 64)), 128 threads; warp = 8·NW output columns, all token tiles.  NK: w [H, N, K], else [H, K, N].
 template <bool NK, int NW>
-__global__ void __launch_bounds__(128) head_linear_mma_kernel(const bf16* __restrict__ x, long long x_t, long long x_h,
-                                                              const bf16* __restrict__ w, bf16* __restrict__ y, long long y_t, long long y_h,
-                                                              int T, int N, int K, const bf16* __restrict__ gate, long long gate_ld) {
+__global__ void __launch_bounds__(128) head_linear_mma_kernel(const bf16* x, long long x_t, long long x_h,
+                                                              const bf16* __restrict__ w, bf16* y, long long y_t, long long y_h,
+                                                              int T, int N, int K, const bf16* gate, long long gate_ld) {
   constexpr int TN = 32 * NW, S = NW == 2 ? 2 : 3, XP = 72, WP = NK ? 72 : TN + 8, WR = NK ? TN : 64;
   __shared__ __align__(16) bf16 sx[S][64 * XP];
   __shared__ __align__(16) bf16 sw[S][WR * WP];
@@ -166,11 +166,11 @@ struct Dec {
 };
 
 template <int MT>
-__global__ void __launch_bounds__(512) latent_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache,
-                                                            const int* __restrict__ block_table, int max_blocks, int block_size,
-                                                            const int* __restrict__ token_seq, const int* __restrict__ positions,
-                                                            const long long* __restrict__ slots, float* __restrict__ part_o,
-                                                            float* __restrict__ part_ml, float scale, int window, int num_splits,
+__global__ void __launch_bounds__(512) latent_decode_kernel(const bf16* q, const bf16* cache,
+                                                            const int* block_table, int max_blocks, int block_size,
+                                                            const int* token_seq, const int* positions,
+                                                            const long long* slots, float* part_o,
+                                                            float* part_ml, float scale, int window, int num_splits,
                                                             int num_blocks, MbLatent L) {
   using G = Dec<MT>;
   constexpr int TK = G::TK, NG = G::NG, HT = G::HT;
@@ -353,8 +353,8 @@ __global__ void __launch_bounds__(512) latent_decode_kernel(const bf16* __restri
 }
 
 // grid (heads, tokens), 128 threads: combine the splits, add the sink to the denominator, write [rank] bf16
-__global__ void __launch_bounds__(128) latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                           const bf16* __restrict__ sink, bf16* __restrict__ out, int num_splits, MbLatent L) {
+__global__ void __launch_bounds__(128) latent_merge_kernel(const float* part_o, const float* part_ml,
+                                                           const bf16* __restrict__ sink, bf16* out, int num_splits, MbLatent L) {
   pdl_trigger();
   pdl_wait();
   const long long th = static_cast<long long>(blockIdx.y) * L.heads + blockIdx.x;

@@ -298,9 +298,9 @@ __global__ void __launch_bounds__(kThreads, OUT ? 1 : 2) linear_chunk_kernel(Arg
 }
 
 // grid (elements / 1024, heads, sequences): seg_state[i] ← state before segment i (4 elements per thread)
-__global__ void __launch_bounds__(256) linear_scan_kernel(const float* __restrict__ state, const int* __restrict__ slots,
-                                                          const int* __restrict__ positions, const float* __restrict__ decay,
-                                                          const int* __restrict__ segs, const int* __restrict__ seq_segs,
+__global__ void __launch_bounds__(256) linear_scan_kernel(const float* state, const int* slots,
+                                                          const int* positions, const float* decay,
+                                                          const int* segs, const int* seq_segs,
                                                           float* seg_state, int H, int sz) {
   pdl_trigger();
   pdl_wait();

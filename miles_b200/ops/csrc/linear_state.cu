@@ -13,10 +13,10 @@ static constexpr int kCols = 32;    // state columns (of dv) per CTA
 
 // grid (column slices, heads, sequences), 128 threads: lane = column, warp w owns the rows d ≡ w (mod 4) of the slice
 template <typename T>
-__global__ void __launch_bounds__(128) linear_state_seq_kernel(const T* __restrict__ proj, long long ld, const float* __restrict__ decay,
-                                                               float* __restrict__ state, const int* __restrict__ slots,
-                                                               const int* __restrict__ cu_q, const int* __restrict__ positions,
-                                                               T* __restrict__ out, int H, int dk, int dv) {
+__global__ void __launch_bounds__(128) linear_state_seq_kernel(const T* proj, long long ld, const float* decay,
+                                                               float* state, const int* slots,
+                                                               const int* cu_q, const int* positions,
+                                                               T* out, int H, int dk, int dv) {
   extern __shared__ __align__(16) float sm[];
   float* S = sm;                         // [dk][kCols]
   float* sq = S + dk * kCols;            // [kTB][dk]
@@ -80,9 +80,9 @@ __global__ void __launch_bounds__(128) linear_state_seq_kernel(const T* __restri
 
 // grid (128-column slices, heads, rows), 256 threads: lane = 4 columns, warp w owns the rows d ≡ w (mod 8).  dv % 4 == 0.
 template <typename T>
-__global__ void __launch_bounds__(256) linear_state_step_kernel(const T* __restrict__ proj, long long ld, const float* __restrict__ decay,
-                                                                float* __restrict__ state, const int* __restrict__ slots,
-                                                                const int* __restrict__ positions, T* __restrict__ out, int H, int dk,
+__global__ void __launch_bounds__(256) linear_state_step_kernel(const T* proj, long long ld, const float* decay,
+                                                                float* state, const int* slots,
+                                                                const int* positions, T* out, int H, int dk,
                                                                 int dv) {
   extern __shared__ __align__(16) float sm[];
   float* sq = sm;                 // [dk]

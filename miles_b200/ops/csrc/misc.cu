@@ -33,10 +33,10 @@ __device__ __forceinline__ MS ms_merge(MS a, MS b) {
 
 // One CTA per row.  logits fp32 [B, V]; inv_temp[B]; greedy[B] (bool as uint8); seeds[B].
 // token = argmax(logit·inv_temp + Gumbel) (greedy: argmax logit); logprob = logit[token]·inv_temp − lse.
-__global__ void __launch_bounds__(1024) sample_logprob_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
-                                                              const uint8_t* __restrict__ greedy, const long long* __restrict__ seeds,
-                                                              long long step, long long* __restrict__ tokens,
-                                                              float* __restrict__ logprobs, int V) {
+__global__ void __launch_bounds__(1024) sample_logprob_kernel(const float* logits, const float* temperature,
+                                                              const uint8_t* greedy, const long long* seeds,
+                                                              long long step, long long* tokens,
+                                                              float* logprobs, int V) {
   __shared__ float sh_m[32], sh_s[32], sh_best[32];
   __shared__ int sh_idx[32];
   pdl_trigger();
@@ -89,11 +89,11 @@ __global__ void __launch_bounds__(1024) sample_logprob_kernel(const float* __res
 
 // The same for few rows: `parts` CTAs per row each take a slice of the vocabulary and leave (max, Σexp, best score, best
 // index) in `ws`; the last CTA of a row to arrive (counter) merges the slices.  counters[row] is zero on entry and on exit.
-__global__ void __launch_bounds__(256) sample_logprob_split_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
-                                                                   const uint8_t* __restrict__ greedy, const long long* __restrict__ seeds,
-                                                                   long long step, long long* __restrict__ tokens,
-                                                                   float* __restrict__ logprobs, int V, int parts, float4* __restrict__ ws,
-                                                                   int* __restrict__ counters) {
+__global__ void __launch_bounds__(256) sample_logprob_split_kernel(const float* logits, const float* temperature,
+                                                                   const uint8_t* greedy, const long long* seeds,
+                                                                   long long step, long long* tokens,
+                                                                   float* logprobs, int V, int parts, float4* ws,
+                                                                   int* counters) {
   __shared__ float sh_m[8], sh_s[8], sh_best[8];
   __shared__ int sh_idx[8];
   __shared__ int sh_last;
@@ -255,12 +255,12 @@ namespace mb {
 // Hand-over between two decode steps of one host round trip, one thread per row: record the step's outputs, feed the
 // sampled token back, advance position and length of live rows (length 0 = padding row), look the new cache slot up in
 // the block table, advance the random seed.
-__global__ void decode_advance_kernel(const long long* __restrict__ o_tok, const float* __restrict__ o_lp, const int* __restrict__ o_routed,
-                                      long long* __restrict__ h_tok, float* __restrict__ h_lp, int* __restrict__ h_routed,
-                                      int routed_per_row, int* __restrict__ tok, int* __restrict__ pos, int* __restrict__ len,
-                                      const int* __restrict__ block_table, int max_blocks, int block_size,
-                                      long long* __restrict__ slot, long long* __restrict__ seed, int B, int vocab,
-                                      int* __restrict__ error_flag, int* __restrict__ prev) {
+__global__ void decode_advance_kernel(const long long* o_tok, const float* o_lp, const int* o_routed,
+                                      long long* h_tok, float* h_lp, int* h_routed,
+                                      int routed_per_row, int* tok, int* pos, int* len,
+                                      const int* block_table, int max_blocks, int block_size,
+                                      long long* slot, long long* seed, int B, int vocab,
+                                      int* error_flag, int* prev) {
   pdl_trigger();
   pdl_wait();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;

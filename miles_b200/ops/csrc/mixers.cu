@@ -15,10 +15,10 @@ static constexpr int kRow = 256;
 // x[t] = embed[tok] + table[(prev·mul_prev + tok·mul_cur) mod buckets] (the last row of the table for a sequence's first token) + sines and
 // cosines of position · freq (pairs of neighbours share a frequency; angles in double precision, reduced by whole turns)
 template <typename T, int V>
-__global__ void __launch_bounds__(128) bigram_embed_kernel(const int* __restrict__ tok, const int* __restrict__ prev,
+__global__ void __launch_bounds__(128) bigram_embed_kernel(const int* tok, const int* prev,
                                                            const T* __restrict__ embed, const T* __restrict__ table, long long buckets,
-                                                           long long mul_prev, long long mul_cur, const int* __restrict__ positions,
-                                                           const double* __restrict__ freq, float* __restrict__ x, T* __restrict__ xb, int D) {
+                                                           long long mul_prev, long long mul_cur, const int* positions,
+                                                           const double* __restrict__ freq, float* x, T* xb, int D) {
   pdl_trigger();
   pdl_wait();
   const long long t = blockIdx.x;
@@ -54,9 +54,9 @@ __global__ void __launch_bounds__(128) bigram_embed_kernel(const int* __restrict
 
 // x += mult · y / rms(y) · nw · ls (ls null: 1);  xb = x, or x / rms(x) · fw · gain (the next norm, or the model's final one)
 template <typename T, int V>
-__global__ void __launch_bounds__(kRow) output_norm_kernel(float* __restrict__ x, const T* __restrict__ y, const T* __restrict__ nw,
+__global__ void __launch_bounds__(kRow) output_norm_kernel(float* x, const T* y, const T* __restrict__ nw,
                                                            const T* __restrict__ ls, float mult, const T* __restrict__ fw, float gain,
-                                                           T* __restrict__ xb, int D, float eps) {
+                                                           T* xb, int D, float eps) {
   __shared__ float sh[kRow / 32];
   pdl_trigger();
   pdl_wait();
@@ -99,9 +99,9 @@ __global__ void __launch_bounds__(kRow) output_norm_kernel(float* __restrict__ x
 }
 
 template <typename T, int V>
-__global__ void __launch_bounds__(256) clamped_glu_kernel(const T* __restrict__ in, long long ld_in, T* __restrict__ out, long long ld_out,
+__global__ void __launch_bounds__(256) clamped_glu_kernel(const T* in, long long ld_in, T* out, long long ld_out,
                                                           long long n, int F, float limit, float alpha, float shift,
-                                                          const int* __restrict__ rows) {
+                                                          const int* rows) {
   pdl_trigger();
   pdl_wait();
   const int per = F / V;
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) clamped_glu_kernel(const T* __restrict__ 
 }
 
 template <typename T, int V>
-__global__ void __launch_bounds__(256) relu_square_kernel(T* __restrict__ x, long long T_, int n, const int* __restrict__ rows) {
+__global__ void __launch_bounds__(256) relu_square_kernel(T* x, long long T_, int n, const int* rows) {
   pdl_trigger();
   pdl_wait();
   if (rows != nullptr) T_ = min(T_, static_cast<long long>(*rows));
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kRow) sum_norm_kernel(MbSumNorm p) {
 
 // out = x / rms(x) · w for every one of `parts` equal parts of a row (of x: ld elements apart); grid (rows, parts)
 template <typename T, int V>
-__global__ void __launch_bounds__(kRow) part_norm_kernel(const T* __restrict__ xs, long long ld, const T* __restrict__ w, T* __restrict__ out, int n,
+__global__ void __launch_bounds__(kRow) part_norm_kernel(const T* xs, long long ld, const T* __restrict__ w, T* out, int n,
                                                          int parts, float eps) {
   __shared__ float sh[kRow / 32];
   constexpr int kHold = 4;                 // vectors per thread that stay in registers between the two passes
@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(kRow) part_norm_kernel(const T* __restrict__ x
 
 // out = o / rms(o) · w · sigmoid(gate) over all C = heads · vdim channels of a token
 template <typename T, int V>
-__global__ void __launch_bounds__(kRow) gated_norm_kernel(const T* __restrict__ o, const T* __restrict__ w, const T* __restrict__ gate,
-                                                          long long gate_ld, T* __restrict__ out, int C, float eps) {
+__global__ void __launch_bounds__(kRow) gated_norm_kernel(const T* o, const T* __restrict__ w, const T* gate,
+                                                          long long gate_ld, T* out, int C, float eps) {
   __shared__ float sh[kRow / 32];
   pdl_trigger();
   pdl_wait();
@@ -308,8 +308,8 @@ __global__ void __launch_bounds__(kRow) gated_norm_kernel(const T* __restrict__ 
 
 // out = o / rms(o) · w · sigmoid(gate), every head's V channels by themselves: `lanes` (a power of two up to 32) threads a head
 template <typename T, int N>
-__global__ void __launch_bounds__(256) head_gated_norm_kernel(const T* __restrict__ o, const T* __restrict__ w, const T* __restrict__ gate,
-                                                              long long gate_ld, T* __restrict__ out, long long heads, int H, int V, int lanes,
+__global__ void __launch_bounds__(256) head_gated_norm_kernel(const T* o, const T* __restrict__ w, const T* gate,
+                                                              long long gate_ld, T* out, long long heads, int H, int V, int lanes,
                                                               float eps) {
   pdl_trigger();
   pdl_wait();
@@ -354,7 +354,7 @@ template <typename T> __device__ __forceinline__ float exp_rest(float z) {
 }
 
 template <typename T, int V>
-__global__ void __launch_bounds__(256) xielu_kernel(const T* __restrict__ z, const T* __restrict__ act, T* __restrict__ out, long long n) {
+__global__ void __launch_bounds__(256) xielu_kernel(const T* z, const T* act, T* out, long long n) {
   pdl_trigger();
   pdl_wait();
   const float pos = softplus_t<T>(to_f(act[0])), neg = 0.5f + softplus_t<T>(to_f(act[1]));
@@ -368,8 +368,8 @@ __global__ void __launch_bounds__(256) xielu_kernel(const T* __restrict__ z, con
 }
 
 template <typename T, int V>
-__global__ void __launch_bounds__(256) gelu_rows_kernel(const T* __restrict__ z, long long ld, const int* __restrict__ tok, const T* __restrict__ table,
-                                                        long long table_ld, int col, T* __restrict__ out, long long rows, int n) {
+__global__ void __launch_bounds__(256) gelu_rows_kernel(const T* z, long long ld, const int* tok, const T* __restrict__ table,
+                                                        long long table_ld, int col, T* out, long long rows, int n) {
   pdl_trigger();
   pdl_wait();
   const int per = n / V;
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(256) gelu_rows_kernel(const T* __restrict__ z,
 }
 
 template <bool EXACT, int V>
-__global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ x, long long n, float cap) {
+__global__ void __launch_bounds__(256) softcap_kernel(float* x, long long n, float cap) {
   pdl_trigger();
   pdl_wait();
   const float inv = __fdiv_rn(1.f, cap);

@@ -36,9 +36,9 @@ __device__ __forceinline__ float wmax(float v) {
 // expert 0 with weight 0 stands in its place, so that nothing behind reads out of range.  In one launch where softmax, gather, sum and division were kernels of their own behind a host
 // synchronisation that asked whether any row was without: 12 launches and a round trip per layer.
 template <int EPL>  // experts per lane = E / 32
-__global__ void __launch_bounds__(256) router_topk_kernel(const float* __restrict__ logits, float* __restrict__ probs,
-                                                          float* __restrict__ topk_w, int* __restrict__ topk_idx, long long T, int E,
-                                                          int K, int normalize, const int* __restrict__ replay, long long replay_row,
+__global__ void __launch_bounds__(256) router_topk_kernel(const float* logits, float* probs,
+                                                          float* topk_w, int* topk_idx, long long T, int E,
+                                                          int K, int normalize, const int* replay, long long replay_row,
                                                           int* error_flag) {
   pdl_trigger();
   pdl_wait();
@@ -114,9 +114,9 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
 // ---------------------------------------------------------------------------------------------
 // Single-CTA counting sort.  idx[n] holds global expert ids; local expert = id − expert_offset, others skipped.
 // Outputs: seg_offsets[E+1] (segments padded to `pad` rows), tile_expert[max_rows / pad], row_src[max_rows], dst_row[n].
-__global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__ idx, int n, const int* __restrict__ n_ptr, int E,
-                                                         int expert_offset, int* __restrict__ seg_offsets, int* __restrict__ tile_expert,
-                                                         int* __restrict__ row_src, int* __restrict__ dst_row, int max_rows, int pad) {
+__global__ void __launch_bounds__(1024) moe_align_kernel(const int* idx, int n, const int* n_ptr, int E,
+                                                         int expert_offset, int* seg_offsets, int* tile_expert,
+                                                         int* row_src, int* dst_row, int max_rows, int pad) {
   extern __shared__ int sh[];  // counts[E], cursor[E], seg[E+1]
   pdl_trigger();
   pdl_wait();

@@ -10,11 +10,11 @@ namespace mx {
 
 // grid (heads, tokens), 128 threads: each warp takes every fourth key with its own running softmax; RL · 32 ≥ dv.
 template <typename T, typename O, int RL>
-__global__ void __launch_bounds__(128) paged_attend_kernel(const T* __restrict__ q, const T* __restrict__ kc, const T* __restrict__ vc,
-                                                           const int* __restrict__ block_table, int max_blocks, int block_size,
-                                                           const int* __restrict__ token_seq, const int* __restrict__ positions,
-                                                           const long long* __restrict__ slots, const T* __restrict__ sink,
-                                                           O* __restrict__ out, MbAttend A, MbScores x) {
+__global__ void __launch_bounds__(128) paged_attend_kernel(const T* q, const T* kc, const T* vc,
+                                                           const int* block_table, int max_blocks, int block_size,
+                                                           const int* token_seq, const int* positions,
+                                                           const long long* slots, const T* __restrict__ sink,
+                                                           O* out, MbAttend A, MbScores x) {
   extern __shared__ float sm[];
   float* sq = sm;                        // [dk]
   float* so = sq + A.dk;                 // [4][dv]

@@ -36,12 +36,12 @@ template <int D>
 __device__ __forceinline__ int toff(int row, int chunk) { return row * D + ((chunk ^ (row & 7)) << 3); }
 
 template <int D>
-__global__ void __launch_bounds__(128) paged_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kc,
-                                                               const bf16* __restrict__ vc, const int* __restrict__ block_table,
-                                                               const int* __restrict__ seq_lens, float* __restrict__ part_o,
-                                                               float* __restrict__ part_ml, int max_blocks, int block_size, int Hq,
-                                                               int Hkv, int group, float scale, int num_splits, bf16* __restrict__ out,
-                                                               int* __restrict__ counters) {
+__global__ void __launch_bounds__(128) paged_decode_mma_kernel(const bf16* q, const bf16* kc,
+                                                               const bf16* vc, const int* block_table,
+                                                               const int* seq_lens, float* part_o,
+                                                               float* part_ml, int max_blocks, int block_size, int Hq,
+                                                               int Hkv, int group, float scale, int num_splits, bf16* out,
+                                                               int* counters) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   bf16* sQ = reinterpret_cast<bf16*>(smem_raw);   // 16 × D
   bf16* sK = sQ + 16 * D;                         // 2 × TK × D
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(128) paged_decode_mma_kernel(const bf16* __res
 
 // partial maxima are stored pre-multiplied by scale·log2(e)
 template <int D>
-__global__ void paged_merge_kernel2(const float* __restrict__ part_o, const float* __restrict__ part_ml, bf16* __restrict__ out,
+__global__ void paged_merge_kernel2(const float* part_o, const float* part_ml, bf16* out,
                                     int num_splits) {
   mb::pdl_trigger();
   mb::pdl_wait();

@@ -8,6 +8,9 @@
 //   * every kernel launched with `launch_pdl` calls `pdl_wait()` before its first dependent global access;
 //   * `pdl_trigger()` sits at the top of the kernel (the dependent's CTAs then queue behind this grid's own CTAs: a
 //     dependent is only released once ALL CTAs of this grid have been scheduled and reached the trigger);
+//   * of the pointer parameters of such a kernel only weights and constant tables are `__restrict__`: the compiler may take what lies behind one
+//     for memory that nobody else touches, the wait included, and move a load of it up in front of the wait, where the kernel in front has
+//     not written it yet.  Whatever writes weights (an optimizer's step, a weight sync) does not trigger early;
 //   * a kernel with these calls can still be launched with `<<<>>>`: both instructions are no-ops then.
 #pragma once
 #include <cuda_runtime.h>

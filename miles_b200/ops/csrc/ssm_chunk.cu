@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(kThreads, OUT ? 1 : 2) ssm_chunk_kernel(Args a
 }
 
 // grid (elements / 1024, heads, sequences): seg_state[i] ← state before segment i (4 elements per thread)
-__global__ void __launch_bounds__(256) ssm_scan_kernel(MbSsm m, const int* __restrict__ segs, const int* __restrict__ seq_segs, float* seg_state,
-                                                       const float* __restrict__ seg_decay, int sz) {
+__global__ void __launch_bounds__(256) ssm_scan_kernel(MbSsm m, const int* segs, const int* seq_segs, float* seg_state,
+                                                       const float* seg_decay, int sz) {
   mb::pdl_trigger();
   mb::pdl_wait();
   const int h = blockIdx.y, b = blockIdx.z, H = m.H;

@@ -18,9 +18,9 @@ inline __host__ __device__ MbConv conv_of(const MbSsm& m) {
 
 // 1-D grid: n_tiles · (channel blocks + 1), then one CTA per token for the aside.  TAPS 0: any number, one load per tap and token.
 template <typename T, int V, int TAPS, bool GROUPED>
-__global__ void __launch_bounds__(kConv) ssm_conv_kernel(const T* __restrict__ proj, long long ld, MbSsm m, const int* __restrict__ tiles,
-                                                         const int* __restrict__ cu_q, int n_tiles, int blocks, T* __restrict__ xbc,
-                                                         float* __restrict__ dt, float* __restrict__ la, MbAside a) {
+__global__ void __launch_bounds__(kConv) ssm_conv_kernel(const T* proj, long long ld, MbSsm m, const int* tiles,
+                                                         const int* cu_q, int n_tiles, int blocks, T* xbc,
+                                                         float* dt, float* la, MbAside a) {
   pdl_trigger();
   pdl_wait();
   const int inner = m.H * m.V, CH = inner + 2 * m.G * m.N;
@@ -53,8 +53,8 @@ static constexpr int kSlice = 32;   // state columns (of V) per CTA
 
 // grid (column slices, heads, sequences), 128 threads: lane = column, warp w owns the rows d ≡ w (mod 4) of the slice
 template <typename T>
-__global__ void __launch_bounds__(128) ssm_seq_kernel(const T* __restrict__ proj, long long ld, const T* __restrict__ xbc, const float* __restrict__ dt,
-                                                      const float* __restrict__ la, MbSsm m, const int* __restrict__ cu_q, T* __restrict__ out) {
+__global__ void __launch_bounds__(128) ssm_seq_kernel(const T* proj, long long ld, const T* xbc, const float* dt,
+                                                      const float* la, MbSsm m, const int* cu_q, T* out) {
   extern __shared__ __align__(16) float sm[];
   const int N = m.N, V = m.V, H = m.H, inner = H * V, CH = inner + 2 * m.G * N;
   float* S = sm;                         // [N][kSlice]
@@ -127,7 +127,7 @@ static constexpr int kStep = 256;
 // the convolution of B and C, and enough of the state is on its way.  A thread owns four columns of a head in every (256 / (HP · V / 4))-th
 // state row.
 template <typename T, bool GROUPED, int HP>
-__global__ void __launch_bounds__(kStep) ssm_step_kernel(const T* __restrict__ proj, long long ld, MbSsm m, T* __restrict__ out, MbAside a,
+__global__ void __launch_bounds__(kStep) ssm_step_kernel(const T* proj, long long ld, MbSsm m, T* out, MbAside a,
                                                          int aside_vec_ok) {
   extern __shared__ __align__(16) float sm[];
   pdl_trigger();

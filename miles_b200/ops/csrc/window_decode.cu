@@ -40,11 +40,11 @@ struct Smem {
 };
 
 template <int DK, int DV, int R, bool BIAS>
-__global__ void __launch_bounds__(128) window_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kc, const bf16* __restrict__ vc,
-                                                            const int* __restrict__ block_table, int max_blocks, int block_size,
-                                                            const int* __restrict__ token_seq, const int* __restrict__ positions,
-                                                            const long long* __restrict__ slots, const bf16* __restrict__ sink,
-                                                            bf16* __restrict__ out, long long o_row, float scale, MbWindow L, MbDiff D, MbScores X) {
+__global__ void __launch_bounds__(128) window_decode_kernel(const bf16* q, const bf16* kc, const bf16* vc,
+                                                            const int* block_table, int max_blocks, int block_size,
+                                                            const int* token_seq, const int* positions,
+                                                            const long long* slots, const bf16* __restrict__ sink,
+                                                            bf16* out, long long o_row, float scale, MbWindow L, MbDiff D, MbScores X) {
   using S = Smem<DK, DV, R>;
   extern __shared__ __align__(128) uint8_t smem[];
   bf16* sQ = reinterpret_cast<bf16*>(smem + S::q);

@@ -69,10 +69,10 @@ __device__ __forceinline__ void norm_rotate(const T* __restrict__ x, const T* __
 }
 
 template <typename T, bool VEC, bool GROUPED>
-__global__ void __launch_bounds__(kPrep) window_prep_kernel(const T* __restrict__ proj, long long ld, const int* __restrict__ positions,
-                                                            const long long* __restrict__ slots, const double* __restrict__ freq,
+__global__ void __launch_bounds__(kPrep) window_prep_kernel(const T* proj, long long ld, const int* positions,
+                                                            const long long* slots, const double* __restrict__ freq,
                                                             float magnitude, const T* __restrict__ q_norm, const T* __restrict__ k_norm, int v_norm,
-                                                            float eps, T* __restrict__ kc, T* __restrict__ vc, T* __restrict__ q, MbWindow L,
+                                                            float eps, T* kc, T* vc, T* q, MbWindow L,
                                                             MbAside a) {
   extern __shared__ float cs[];          // [rot/2] cosines, [rot/2] sines
   __shared__ float sh[kPrep / 32];
