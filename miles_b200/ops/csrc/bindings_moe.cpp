@@ -43,7 +43,7 @@ std::vector<at::Tensor> router_topk(const at::Tensor& logits, int64_t K, bool no
 
 // idx int32 [n] global expert ids → seg_offsets [E+1], tile_expert [max_rows/pad], row_src [max_rows], dst_row [n]
 std::vector<at::Tensor> moe_align(const at::Tensor& idx, int64_t E, int64_t expert_offset, int64_t max_rows,
-                                  const c10::optional<at::Tensor>& n_dev, int64_t pad) {
+                                  const c10::optional<at::Tensor>& n_dev, int64_t pad, bool ordered) {
   c10::cuda::CUDAGuard g(idx.device());
   const int64_t n = idx.numel();
   const int* n_ptr = n_dev.has_value() && n_dev->defined() ? n_dev->data_ptr<int>() : nullptr;
@@ -54,7 +54,7 @@ std::vector<at::Tensor> moe_align(const at::Tensor& idx, int64_t E, int64_t expe
   auto row_src = at::empty({max_rows}, opt);
   auto dst_row = at::empty({n}, opt);
   check(mb_moe_align_pad(idx.data_ptr<int>(), n, n_ptr, E, expert_offset, seg.data_ptr<int>(), tile.data_ptr<int>(),
-                         row_src.data_ptr<int>(), dst_row.data_ptr<int>(), max_rows, pad, cur_stream()),
+                         row_src.data_ptr<int>(), dst_row.data_ptr<int>(), max_rows, pad, ordered, cur_stream()),
         "mb_moe_align");
   return {seg, tile, row_src, dst_row};
 }
@@ -89,7 +89,7 @@ void register_moe(pybind11::module& m) {
   m.def("router_topk", &router_topk, py::arg("logits"), py::arg("k"), py::arg("normalize"), py::arg("want_probs"), py::arg("replay") = py::none(),
         py::arg("err") = py::none());
   m.def("moe_align", &moe_align, py::arg("idx"), py::arg("E"), py::arg("expert_offset"), py::arg("max_rows"), py::arg("n_dev"),
-        py::arg("pad") = 128);
+        py::arg("pad") = 128, py::arg("ordered") = true);
   m.def("moe_gather", &moe_gather);
   m.def("moe_combine", &moe_combine, pybind11::arg("y_perm"), pybind11::arg("w"), pybind11::arg("dst_row"), pybind11::arg("out"),
         pybind11::arg("k"), pybind11::arg("identity_rows") = false);

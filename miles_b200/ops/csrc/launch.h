@@ -129,7 +129,7 @@ int mb_router_topk(const float* logits, float* probs, float* topk_w, int* topk_i
 int mb_moe_align(const int* idx, int n, const int* n_ptr, int E, int expert_offset, int* seg_offsets, int* tile_expert, int* row_src,
                  int* dst_row, int max_rows, cudaStream_t s);
 int mb_moe_align_pad(const int* idx, int n, const int* n_ptr, int E, int expert_offset, int* seg_offsets, int* tile_expert,
-                     int* row_src, int* dst_row, int max_rows, int pad, cudaStream_t s);
+                     int* row_src, int* dst_row, int max_rows, int pad, int ordered, cudaStream_t s);
 int mb_moe_gather(const void* x, void* x_perm, const int* row_src, const int* seg_offsets, int E, int k, int H, int max_rows,
                   cudaStream_t s);
 int mb_moe_combine(const void* y_perm, const float* w, const int* dst_row, void* out, long long T, int k, int H, int identity_rows,

@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* idx, int n, 
 // counts it into its own histogram (lanes with the same expert are found with match.any: no atomics); after the counts have been added up
 // across warps and, through distributed shared memory, across CTAs, it walks its range again and hands out rows.  Pairs keep their order
 // within an expert, so the result does not depend on timing.  One CTA with shared-memory atomics on 16 counters was bound by their
-// serialisation: 58 064 pairs, 16 experts: 44 → 17.5 µs (488 pairs: 3.7 → 4.5).
+// serialisation: 58 064 pairs, 16 experts: 44 → 17.5 µs (fewer: `mb_moe_align_pad`).
 static constexpr int kMaxSortExperts = 256, kSortWarps = 32;
 
 __global__ void __launch_bounds__(kSortWarps * 32) moe_sort_kernel(const int* idx, int n, const int* n_ptr, int E, int expert_offset, int* seg_offsets,
@@ -450,9 +450,12 @@ extern "C" int mb_router_topk(const float* logits, float* probs, float* topk_w, 
 
 // pad: rows every expert segment is rounded up to (128 for the training GEMMs, 16/32/64 for the decode-sized grouped GEMM)
 extern "C" int mb_moe_align_pad(const int* idx, int n, const int* n_ptr, int E, int expert_offset, int* seg_offsets, int* tile_expert,
-                                int* row_src, int* dst_row, int max_rows, int pad, cudaStream_t s) {
+                                int* row_src, int* dst_row, int max_rows, int pad, int ordered, cudaStream_t s) {
   if (E > 2048 || pad <= 0) return -1;
-  if (E <= kMaxSortExperts) {
+  // Where the order of a segment's rows does not matter (nothing is summed over them), the counters are faster as long as they are few, one
+  // thread adds up the segments, and the pairs are (488 pairs: 8 experts 2.5 against 3.4 µs, 16 3.0 / 3.8, 32 4.0 / 4.3, but 64 6.0 / 5.6;
+  // 16 experts: 2048 pairs 3.9 / 5.4, 4096 4.9 / 7.1, 8192 7.1 / 6.4)
+  if (E <= kMaxSortExperts && (ordered || E > 32 || n > 4096)) {
     // eight CTAs from where one's passes over its range outlast two cluster barriers; the warps' histograms take 128 bytes per expert
     // and a warp is worth its row of the histogram from two passes over 32 pairs
     const int ctas = n > 4096 ? 8 : 1, warps = n > 1024 ? kSortWarps : n > 512 ? 16 : 8;
@@ -469,7 +472,7 @@ extern "C" int mb_moe_align_pad(const int* idx, int n, const int* n_ptr, int E, 
 
 extern "C" int mb_moe_align(const int* idx, int n, const int* n_ptr, int E, int expert_offset, int* seg_offsets, int* tile_expert,
                             int* row_src, int* dst_row, int max_rows, cudaStream_t s) {
-  return mb_moe_align_pad(idx, n, n_ptr, E, expert_offset, seg_offsets, tile_expert, row_src, dst_row, max_rows, kPad, s);
+  return mb_moe_align_pad(idx, n, n_ptr, E, expert_offset, seg_offsets, tile_expert, row_src, dst_row, max_rows, kPad, 1, s);
 }
 
 extern "C" int mb_moe_gather(const void* x, void* x_perm, const int* row_src, const int* seg_offsets, int E, int k, int H,

@@ -238,7 +238,7 @@ def sort_by_expert(x, idx, E: int, bt: int, expert_offset: int = 0):
     each row tile, row of each (token, choice))."""
     T, k = idx.shape
     max_rows = moe_max_rows(T * k, E) if bt == 128 else moe_max_rows_pad(T * k, E, bt)
-    seg, tile, row_src, dst_row = C.moe_align(_c(idx.to(torch.int32)).view(-1), E, expert_offset, max_rows, None, bt)
+    seg, tile, row_src, dst_row = C.moe_align(_c(idx.to(torch.int32)).view(-1), E, expert_offset, max_rows, None, bt, False)
     x_perm = torch.empty(max_rows, x.shape[1], dtype=x.dtype, device=x.device)
     publish_limit(LIMIT_MOE_PAIRS, T * k)
     C.moe_gather(_c(x), x_perm, row_src, seg, k)
@@ -341,7 +341,7 @@ class _MoEFFN(torch.autograd.Function):
         idx32 = _c(topk_idx.to(torch.int32)).view(-1)
         wf = _c(topk_w.float())
         max_rows = moe_max_rows(T * k, E)
-        seg, tile, row_src, dst_row = C.moe_align(idx32, E, expert_offset, max_rows, None)
+        seg, tile, row_src, dst_row = C.moe_align(idx32, E, expert_offset, max_rows, None, 128, keep)     # weight gradients are sums over a segment's rows
         x_perm = torch.empty(max_rows, H, dtype=x.dtype, device=x.device)
         publish_limit(LIMIT_MOE_PAIRS, x.shape[0] * k)
         C.moe_gather(x, x_perm, row_src, seg, k)

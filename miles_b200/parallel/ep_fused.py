@@ -126,7 +126,7 @@ class _FusedMoE(torch.autograd.Function):
         # decode-sized calls (about n_pairs rows arrive when the routing is balanced): pad segments to 16/32/64 rows
         bt = 128 if need_bwd else small_moe_bt(n_pairs, e_local, w13, w2)
         max_rows = moe_max_rows_pad(cap, e_local, bt)
-        seg, tile, row_src, _ = C.moe_align(b.expert_ids[:cap], e_local, 0, max_rows, b.n_recv, bt)
+        seg, tile, row_src, _ = C.moe_align(b.expert_ids[:cap], e_local, 0, max_rows, b.n_recv, bt, need_bwd)
         x_perm = torch.empty(max_rows, H, dtype=x.dtype, device=x.device)
         C.moe_gather(b.recv_x.view(b.cap, H), x_perm, row_src, seg, 1)
         h1, y_perm = experts_forward(x_perm, w13, w2, seg, tile, bt)
