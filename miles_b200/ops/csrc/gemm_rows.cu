@@ -297,6 +297,9 @@ extern "C" int mb_norm_rows(const void* x, const void* residual, const void* w, 
   typedef __nv_bfloat16* bf;
   if (T <= 0) return 0;
   if (K % 8 || (residual != nullptr && sum == nullptr)) return -2;
+  const uintptr_t pointers = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(w) |
+                             reinterpret_cast<uintptr_t>(scaled) | reinterpret_cast<uintptr_t>(sum) | reinterpret_cast<uintptr_t>(normed);
+  if (pointers & 15) return -1;
   return static_cast<int>(launch_pdl(rows::norm_rows_kernel, dim3(T), dim3(256), 0, s, (cbf)x, (cbf)residual, (cbf)w, eps, K, (bf)scaled, rstd, (bf)sum,
                                      (bf)normed));
 }

@@ -84,6 +84,22 @@ def test_few_rows_behind_a_norm(M, N, Kd, ones, with_residual):
     assert K.check_error_flag(x) == 0
 
 
+@pytest.mark.parametrize("which", ["x", "residual", "norm weights"])
+def test_rows_off_a_16_byte_boundary_are_refused(which):
+    """By the host, whichever kernel the projection goes to (the matrix-vector one at 8 rows looks at the rows alone, as it always did)."""
+    from miles_b200.ops import cuda as K
+
+    off = lambda *s: torch.zeros(math.prod(s) + 1, device="cuda", dtype=torch.bfloat16)[1:].view(*s)
+    on = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)
+    make = lambda name: off if name == which else on
+    w = on(640, 2048)
+    for M in (8, 9) if which == "x" else (9,):
+        x, r, nw = make("x")(M, 2048), make("residual")(M, 2048), make("norm weights")(2048)
+        assert (K._row_split(M, 640, 2048) > 0 and M > K._gemv_rows(K._row_split(M, 640, 2048), 640, 2048)) == (M == 9)
+        with torch.no_grad(), pytest.raises(RuntimeError):
+            K.add_rmsnorm_linear(x, r, nw, 1e-6, w)
+
+
 def test_weights_ahead_of_the_rows():
     """Weights that nothing on the stream writes are requested before the kernel in front, which makes the rows, has finished."""
     from miles_b200.ops import cuda as K
