@@ -136,11 +136,12 @@ void head_logprob(const at::Tensor& hidden, const at::Tensor& W, const at::Tenso
 }
 
 void head_grad(const at::Tensor& hidden, const at::Tensor& W, const at::Tensor& targets, const at::Tensor& lse, const c10::optional<at::Tensor>& ent,
-               const c10::optional<at::Tensor>& g_lp, const c10::optional<at::Tensor>& g_ent, at::Tensor& out, double inv_temp, const at::Tensor& err) {
+               const c10::optional<at::Tensor>& g_lp, const c10::optional<at::Tensor>& g_ent, at::Tensor& out, int64_t first, double inv_temp,
+               const at::Tensor& err) {
   c10::cuda::CUDAGuard g(hidden.device());
   TORCH_CHECK(hidden.is_contiguous() && W.is_contiguous() && targets.is_contiguous() && out.is_contiguous(), "head_grad: contiguous operands");
   check(mb_head_grad(hidden.data_ptr(), W.data_ptr(), reinterpret_cast<const long long*>(targets.data_ptr<int64_t>()), lse.data_ptr<float>(), fptr_or_null(ent),
-                     fptr_or_null(g_lp), fptr_or_null(g_ent), out.data_ptr(), out.size(1), hidden.size(0), W.size(0), hidden.size(1), inv_temp,
+                     fptr_or_null(g_lp), fptr_or_null(g_ent), out.data_ptr(), out.size(1), hidden.size(0), W.size(0), first, hidden.size(1), inv_temp,
                      err.data_ptr<int>(), cur_stream()),
         "mb_head_grad");
 }

@@ -91,10 +91,11 @@ struct Stats {
 };
 
 struct Grad {
-  const long long* targets;              // [M], of this range (out of range: none here)
+  const long long* targets;              // [M] (outside this range: none here)
   const float *lse, *ent, *g_lp, *g_ent; // [M]; ent and g_ent null without an entropy gradient, g_lp null without one of log p
   __nv_bfloat16* out;                    // [M, ld]
   long long ld;
+  int first;                             // of the range
   float inv_temp;
 
   //   d z_j = g_lp·(1[j = target] − p_j) − g_ent·p_j·(z_j − (lse − H)),  d logit = d z · inv_temp,  p_j = exp(z_j − lse)
@@ -107,7 +108,7 @@ struct Grad {
     const bool in = row < p.M;
     const float l = in ? lse[row] : 0.f, glp = in && g_lp != nullptr ? g_lp[row] : 0.f, ge = in && g_ent != nullptr ? g_ent[row] : 0.f;
     const float mean = in && g_ent != nullptr ? l - ent[row] : 0.f;
-    const long long target = in ? targets[row] - col0 : -1;
+    const long long target = in ? targets[row] - first - col0 : -1;
     const float2 minus_l = make_float2(-l, -l), l2e = make_float2(kLog2e, kLog2e), zero = make_float2(0.f, 0.f);
 #pragma unroll 1
     for (int c2 = 0; c2 < COLS / 64; ++c2) {
@@ -217,12 +218,13 @@ extern "C" int mb_head_finish(const float* parts, const float* target_z, int n_p
   return static_cast<int>(cudaGetLastError());
 }
 
-// W: rows of the range, Vc of them (a multiple of 8); targets as for the range (target − first row); out [R, ld] bf16, 16-byte aligned rows.
+// W: rows of the range, Vc of them (a multiple of 8) from number `first` of the vocabulary on; out [R, ld] bf16, 16-byte aligned rows.
 extern "C" int mb_head_grad(const void* hidden, const void* W, const long long* targets, const float* lse, const float* ent, const float* g_lp,
-                            const float* g_ent, void* out, long long ld, int R, int Vc, int H, float inv_temp, int* error_flag, cudaStream_t s) {
+                            const float* g_ent, void* out, long long ld, int R, int Vc, int first, int H, float inv_temp, int* error_flag,
+                            cudaStream_t s) {
   if (R <= 0 || Vc <= 0) return 0;
   if (Vc % 8 || ld % 8 || reinterpret_cast<uintptr_t>(out) % 16) return -2;
   GemmParams p{};
   p.M = R; p.N = Vc; p.K = H; p.num_groups = 1; p.error_flag = error_flag;
-  return head::launch(hidden, W, p, head::Grad{targets, lse, ent, g_lp, g_ent, reinterpret_cast<__nv_bfloat16*>(out), ld, inv_temp}, s);
+  return head::launch(hidden, W, p, head::Grad{targets, lse, ent, g_lp, g_ent, reinterpret_cast<__nv_bfloat16*>(out), ld, first, inv_temp}, s);
 }

@@ -28,7 +28,7 @@ int mb_head_stats(const void* hidden, const void* W, const long long* targets, f
                   int* error_flag, cudaStream_t s);
 int mb_head_finish(const float* parts, const float* target_z, int n_parts, long long R, float* logp, float* ent, float* lse, cudaStream_t s);
 int mb_head_grad(const void* hidden, const void* W, const long long* targets, const float* lse, const float* ent, const float* g_lp, const float* g_ent,
-                 void* out, long long ld, int R, int Vc, int H, float inv_temp, int* error_flag, cudaStream_t s);
+                 void* out, long long ld, int R, int Vc, int first, int H, float inv_temp, int* error_flag, cudaStream_t s);
 int mb_gemm_bf16_glu(const void* A, const void* B, void* act, int M, int F, int K, int num_experts, const int* tile_expert, int* error_flag,
                      cudaStream_t s);
 int mb_gemm_bf16_grouped(const void* A, const void* B, void* C, int M_pad, int N, int K, int num_experts,

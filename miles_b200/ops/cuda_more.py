@@ -458,8 +458,8 @@ class _LogProbEntropy(torch.autograd.Function):
                 dl = torch.empty(r1 - r0, v1 - v0, dtype=BF16, device=hidden.device)
                 in_place = _head_in_place(r1 - r0, hidden, w) and (v1 - v0) % 8 == 0
                 if in_place:
-                    C.head_grad(hidden[r0:r1], w[v0:v1], tg[r0:r1] - v0, lse[r0:r1], ent[r0:r1] if g_ent is not None else None,
-                                g_lp[r0:r1] if g_lp is not None else None, g_ent[r0:r1] if g_ent is not None else None, dl, ctx.inv_t,
+                    C.head_grad(hidden[r0:r1], w[v0:v1], tg[r0:r1], lse[r0:r1], ent[r0:r1] if g_ent is not None else None,
+                                g_lp[r0:r1] if g_lp is not None else None, g_ent[r0:r1] if g_ent is not None else None, dl, v0, ctx.inv_t,
                                 C.error_flag(hidden))
                 else:
                     logits = gemm_nt(hidden[r0:r1], w[v0:v1], out_dtype=torch.float32)

@@ -47,3 +47,40 @@ def test_targets_outside_the_shard_and_no_finite_logit():
     h[3] = float("nan")
     lp, ent = K.logprob_entropy(h, w, t, 1.0, True)
     assert torch.isnan(lp[3]) and torch.isnan(ent[3]) and torch.isfinite(lp[4:]).all()
+
+
+@pytest.mark.parametrize("sign", [1, -1])
+def test_infinite_logits(sign):
+    """A logit of −∞ has no weight and its row stays a number, one of +∞ makes its row none; other rows see nothing of either."""
+    from miles_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    h, w = torch.randn(70, 64, device="cuda", generator=g).bfloat16(), torch.randn(304, 64, device="cuda", generator=g).bfloat16()
+    t = torch.randint(8, 304, (70,), device="cuda", generator=g)
+    h[:, 0], w[:, 0] = 0, 0
+    h[3, 0], w[7, 0] = 1e30, sign * 1e30                                  # their product is beyond fp32
+    h = h.requires_grad_()
+    lp, _ = K.logprob_entropy(h, w, t, 1.0, False)
+    z = h.detach().double() @ w.double().t()
+    z[3, 7] = sign * float("inf")
+    want = torch.log_softmax(z, -1).gather(1, t[:, None])[:, 0]
+    assert torch.equal(torch.isnan(lp), torch.isnan(want)) and torch.isnan(lp[3]).item() == (sign > 0)
+    ok = ~torch.isnan(want)
+    assert (lp.double() - want)[ok].abs().max().item() < 5e-5             # as above
+    lp[ok].sum().backward()
+    rows = ok.clone()
+    rows[3] = False                                                       # its gradient is 0 · w with an element of 1e30: left out
+    assert torch.isfinite(h.grad[rows]).all() and K.check_error_flag(h) == 0
+
+
+def test_backward_launches_nothing_beside_its_products():
+    """Several vocabulary chunks: the targets of each are found in the kernel, not by a subtraction in front of it."""
+    from miles_b200.ops import cuda as K
+
+    h = torch.randn(70, 64, device="cuda").bfloat16().requires_grad_()
+    w = torch.randn(40000, 64, device="cuda").bfloat16().requires_grad_()
+    lp, _ = K.logprob_entropy(h, w, torch.arange(70, device="cuda") * 500, 1.0, False)
+    total = lp.sum()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        total.backward()
+    assert not any(e.key in ("aten::sub", "aten::add") for e in prof.key_averages())
