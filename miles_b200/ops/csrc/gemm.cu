@@ -463,6 +463,7 @@ static int pick_tile(int M, int N, int groups, int forced, const GemmParams& p) 
   // 217, 283, 460 for 64, 128, 256 columns, two 253 and 390 for 128 and 256.  So 256 × 256 wherever the last wave is not nearly empty
   // (8192³: 825 → 693 µs), and the narrower ones where tiles are few: 1024 × 2560 × 4096 42.6, 40.1, 36.7 | 40.5, 33.0 µs;
   // 257 × 2560 × 4096 22.5, 24.9, 35.1 | 26.9, 33.1; 257 × 6144 × 2560 24.6, 22.2, 29.5 | 31.7, 26.9.
+  // Left out: the fill of a short reduction, and how many of a grouped call's M rows are in use (a number on the device).
   struct Option { int tile, rows, cols, slots, ns; };
   const int sms = num_sms();
   const Option options[5] = {{kPair + 256, 2 * BM, 256, sms / 2, 390}, {kPair + 128, 2 * BM, 128, sms / 2, 253}, {256, BM, 256, sms, 460},

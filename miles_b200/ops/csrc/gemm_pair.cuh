@@ -63,6 +63,7 @@ static constexpr int kBM = 128, kBK = 64, kUmmaK = 16;      // rows per CTA
 static constexpr int kStages = 6;
 static constexpr int kEpilogueWarps = 8, kThreads = 64 + 32 * kEpilogueWarps;
 static constexpr int kGroupM = 8;                           // row tiles (of 256) per group of the tile order
+// (1 / 8 / 16: 8192³ 743 / 693 / 696 µs, 16384 × 18992 × 2048 885 / 822 / 800, 16384 × 2048 × 4096 169 / 169 / 173: 8 is never far off)
 
 template <int BN>
 struct Layout {

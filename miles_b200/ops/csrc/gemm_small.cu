@@ -3,8 +3,9 @@
 // The general kernel (gemm.cu) puts tokens on the 128-row M side of the MMA: with 1…64 tokens two thirds of every pipeline
 // stage are padding rows and a projection exposes only N/64 CTAs.  Here the WEIGHT rows are the M side (128 output features
 // per tile, every byte loaded is a weight byte that must be read anyway) and the tokens are the N side in tiles of
-// BT ∈ {16, 32, 64}; the accumulator D[feature, token] is written back transposed.  Parallelism comes from split-K
-// (dense: K slices → fp32 planes, last arriver reduces) or from the experts (grouped).
+// BT ∈ {16, 32, 64}; the accumulator D[feature, token] is written back transposed.  Parallelism comes from the tiles (dense: vocabulary heads
+// and other products of more tiles than gemm_rows.cu has CTAs for, which come here uncut), from split-K (dense, for callers that ask for it: K
+// slices → fp32 planes, last arriver reduces) or from the experts (grouped).
 //   dense    tiles = ⌈N/128⌉ × ⌈tokens/BT⌉ × split_k
 //   grouped  X = expert-sorted rows whose segments are padded to BT (`moe_align` with pad = BT), tile_expert[token tile] gives
 //            the expert (−1: unused tile); W = [E·N, K] stacked.  tiles = ⌈N/128⌉ × token tiles

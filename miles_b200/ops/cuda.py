@@ -119,8 +119,9 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *
     return out
 
 
-# What is left of decode-sized GEMMs (accumulating ones) has a handful of 128×64 output tiles over a long K and leaves most SMs idle; split-K
-# gives every tile several CTAs, each streaming a slice of the weights.  Workspace: fp32 [split, M, N] planes + arrival counters (zero
+# Decode-sized GEMMs that the forms for few rows do not take (accumulating ones; all of them where MILES_GEMV_M and MILES_SMALL_M turn those
+# forms off) have a handful of 128×64 output tiles over a long K and leave most SMs idle; split-K gives every tile several CTAs, each
+# streaming a slice of the weights.  Workspace: fp32 [split, M, N] planes + arrival counters (zero
 # between calls; the kernel restores that), one per device, so such GEMMs must not overlap on two streams of one device.
 SPLIT_K = os.environ.get("MILES_SPLIT_K", "1") != "0"
 _SPLITK_MAX_M, _SPLITK_MAX_TILES = int(os.environ.get("MILES_SPLIT_K_MAX_M", "32")), 74   # measured: wins below ~32 rows
@@ -149,10 +150,11 @@ def _splitk_workspace(device):
 # projection inside it.  Up to 16 rows are supported (`_gemv_rows`: which of them gemm_rows.cu takes instead); 0 turns the path off.
 GEMV_M = min(16, int(os.environ.get("MILES_GEMV_M", "16")))
 GEMV_MAX_N = int(os.environ.get("MILES_GEMV_MAX_N", "32768"))
-# Larger weights (24 MB) stream faster through gemm_rows.cu's rings whatever the rows.  Decode steps of 8 layers, 1 / 4 / 8 rows: hidden 2560
-# (21 to 100 MB per projection) 776 / 816 / 908 → 621 / 633 / 666 µs, everything there 612 / 630 / 658.  For smaller ones it is within 2 % either
-# way up to 4 rows (hidden 2048 with 16 experts, 17 and 21 MB: 565 / 675 / 750 against 555 / 683 / 727; hidden 1024, up to 12 MB: 300 / 325 / 362
-# against 299 / 322 / 345), and they keep the order of their sums.
+# Larger weights (24 MB) stream faster through gemm_rows.cu's rings whatever the rows.  Decode steps of 8 layers, 1 / 4 / 8 rows, all weights
+# here / with this line / all of them there: hidden 2560 (21 to 100 MB per projection) 771 / 795 / 908, 612 / 617 / 665, 608 / 616 / 663 µs.  Smaller
+# ones are here for the order of their sums, which a step of few rows has always had, and not for their speed: it is the same to within 3 % up to 4
+# rows and behind by 4 to 6 % at 8 (hidden 2048 with 16 experts, 17 and 21 MB, this line / all there: 565 / 678 / 745 against 567 / 668 / 711;
+# hidden 1024, up to 12 MB: 303 / 314 / 365 against 297 / 305 / 342).
 GEMV_MAX_WEIGHTS = 12 << 20
 
 
@@ -345,7 +347,7 @@ def linear(x, w, bias=None):
         return torch.nn.functional.linear(x, w.to(x.dtype), bias)
     if _MXFP8_WEIGHTS and not torch.is_grad_enabled():
         reg = _MXFP8_WEIGHTS.get(w.data_ptr())
-        # the block-scaled kernel works on 128×128 tiles: decode-sized batches stay on the split-K bf16 path
+        # the block-scaled kernel works on 128×128 tiles: decode-sized batches stay on the bf16 kernels for few rows
         if reg is not None and x.numel() // x.shape[-1] >= MXFP8_MIN_ROWS:
             from . import extra
 

@@ -167,15 +167,21 @@ def test_kv_cache_write():
 @pytest.mark.parametrize("M,N,K", [(1, 2048, 4096), (64, 2048, 4096), (64, 128, 2048), (8, 4096, 2048), (200, 1000, 3072), (130, 152, 1024)])
 @pytest.mark.parametrize("fp32_out", [False, True])
 def test_gemm_split_k(M, N, K, fp32_out, monkeypatch):
-    """Decode-sized GEMMs go through the split-K path; results match, and the arrival counters are left zero."""
+    """With the forms for few rows turned off, and always where a product is added to its output, the reduction is cut over CTAs; results match,
+    and the arrival counters are left zero."""
     K_ = _k()
     monkeypatch.setattr(K_, "_SPLITK_MAX_M", 256)           # the dispatch default only splits very small M
-    assert K_._pick_split_k(M, N, K) > 1
+    monkeypatch.setattr(K_, "GEMV_M", 0)
+    monkeypatch.setattr(K_, "SMALL_M", 0)
+    split = K_._pick_split_k(M, N, K)
+    assert split > 1
     torch.manual_seed(1)
     a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
     b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
     bias = torch.randn(N, device="cuda", dtype=torch.bfloat16)
     want = a.float() @ b.float().t() + bias.float()
+    ws, counters = K_._splitk_workspace(a.device)
+    ws.fill_(float("nan"))
     for _ in range(3):                                       # back to back: each call must find a clean workspace
         out = K_.gemm_nt(a, b, bias=bias, out_dtype=torch.float32 if fp32_out else None)
         torch.cuda.synchronize()
@@ -183,8 +189,14 @@ def test_gemm_split_k(M, N, K, fp32_out, monkeypatch):
         assert _rel(out, want) < (2e-3 if fp32_out else 1e-2), _rel(out, want)
     nob = K_.gemm_nt(a, b, out_dtype=torch.float32 if fp32_out else None)          # vectorised reduction path
     assert _rel(nob, want - bias.float()) < (2e-3 if fp32_out else 1e-2)
-    ws, counters = K_._splitk_workspace(a.device)
+    assert torch.isfinite(ws[:split * M * N]).all()          # every part went through it
     assert int(counters.abs().max()) == 0
+    monkeypatch.undo()
+    monkeypatch.setattr(K_, "_SPLITK_MAX_M", 256)
+    ws.fill_(float("nan"))
+    total = torch.ones(M, N, device="cuda")
+    K_.gemm_nt(a, b, out=total, accumulate=True)
+    assert _rel(total - 1, want - bias.float()) < 2e-3 and torch.isfinite(ws[:split * M * N]).all() and int(counters.abs().max()) == 0
     plain = K_.gemm_nt(a, b, bias=bias, out_dtype=torch.float32, force_bn=64)     # force_bn bypasses split-K
     assert _rel(out.float(), plain) < 1e-2
 
