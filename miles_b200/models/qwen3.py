@@ -212,12 +212,14 @@ class MoEFFN(nn.Module):
             w2[e - lo].copy_(gen(f"{tag}.e{e}.w2", (H, F), cfg.init_std, dtype, device))
         self.w13, self.w2 = nn.Parameter(w13), nn.Parameter(w2)
 
-    def forward(self, x, meta: ForwardMeta, layer: int, logits: torch.Tensor | None = None):
-        # with sequence parallelism each TP rank routes its own token slice (expert-TP is 1)
-        if logits is None:
+    def forward(self, x, meta: ForwardMeta, layer: int, logits: torch.Tensor | None = None, chosen=None):
+        # with sequence parallelism each TP rank routes its own token slice (expert-TP is 1); `chosen`: (weights, choices) made by the caller
+        if logits is None and chosen is None:
             logits = ops.linear_fp32(x, self.router)  # router scores stay fp32 (no bf16 rounding, no cast kernel)
         k, norm = self.cfg.moe_topk, self.cfg.moe_norm_topk_prob
-        if meta.replay_topk is not None:
+        if chosen is not None:
+            w, idx = chosen
+        elif meta.replay_topk is not None:
             # R3: recorded indices replace top-k, weights come from the current scores so the gate
             # still receives gradient (reference: miles/utils/replay_base.py:87-144).
             w, idx, _ = ops.router_replay(logits, self.ps.sp_slice(meta.replay_topk)[:, self.moe_index, :], norm)
@@ -254,11 +256,23 @@ class DecoderLayer(nn.Module):
         qkv, residual, _ = ops.add_rmsnorm_linear(x, residual, self.ln1, self.eps, attn.wqkv, attn.bqkv)
         h = attn(None, meta, self.layer, qkv=qkv)
         if isinstance(mlp, MoEFFN):
+            if self._routes_few_tokens(h, meta):
+                return self._moe_few_tokens(h, residual, meta)
             logits, residual, hn = ops.add_rmsnorm_linear(h, residual, self.ln2, self.eps, mlp.router, want_normed=True,
                                                           out_fp32=True)
             return mlp(hn, meta, self.layer, logits=logits), residual
         h13, residual, _ = ops.add_rmsnorm_linear(h, residual, self.ln2, self.eps, mlp.w13)
         return ops.linear(ops.swiglu(h13), mlp.w2), residual
+
+    def _routes_few_tokens(self, h, meta: ForwardMeta) -> bool:
+        mlp = self.mlp
+        return (isinstance(mlp, MoEFFN) and meta.replay_topk is None and self.attn.ps.tp_size == 1 and getattr(mlp, "lora", None) is None
+                and mlp.cfg.moe_topk <= mlp.router.shape[0] and ops.few_token_router(h, mlp.router))
+
+    def _moe_few_tokens(self, h, residual, meta: ForwardMeta):
+        mlp = self.mlp
+        hn, residual, w, idx = ops.add_rmsnorm_router(h, residual, self.ln2, self.eps, mlp.router, mlp.cfg.moe_topk, mlp.cfg.moe_norm_topk_prob)
+        return mlp(hn, meta, self.layer, chosen=(w, idx)), residual
 
     def forward(self, x, residual, meta: ForwardMeta):
         # `x` is the previous block's output still to be added to `residual`
@@ -267,6 +281,8 @@ class DecoderLayer(nn.Module):
             return self._forward_few_tokens(x, residual, meta)
         h, residual = add_rmsnorm_reducing(self.attn.ps, x, residual, self.ln1, self.eps)
         h = self.attn(h, meta, self.layer)
+        if self._routes_few_tokens(h, meta):
+            return self._moe_few_tokens(h, residual, meta)
         h, residual = add_rmsnorm_reducing(self.attn.ps, h, residual, self.ln2, self.eps)
         h = self.mlp(h, meta, self.layer)
         return h, residual

@@ -139,6 +139,16 @@ def router_topk(logits, k, normalize=True):
     return ref.router_topk(logits, k, normalize)
 
 
+def few_token_router(x, router) -> bool:
+    """True when norm, router logits and top-k of a decode step are one launch (`add_rmsnorm_router`)."""
+    return x.is_cuda and _k().few_token_router(x, router)
+
+
+def add_rmsnorm_router(x, residual, norm_w, eps, router, k, normalize=True):
+    """(rmsnorm(x + residual), x + residual, top-k weights, top-k choices), only where `few_token_router` holds."""
+    return _k().add_rmsnorm_router(x, residual, norm_w, eps, router, k, normalize)
+
+
 def router_replay(logits, idx, normalize=True):
     """`router_topk` with recorded choices [T, k] in the place of the largest: (weights from the current scores, choices, probabilities).
     Rows without a record (all negative) are chosen afresh."""

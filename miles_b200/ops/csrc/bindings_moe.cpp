@@ -41,6 +41,26 @@ std::vector<at::Tensor> router_topk(const at::Tensor& logits, int64_t K, bool no
   return {w, idx, probs};
 }
 
+// rmsnorm(x (+ residual)) and its top-k experts: x [T, H] bf16 → (sum [T, H] or undefined, normed [T, H], weights fp32 [T, K], idx int32 [T, K])
+std::vector<at::Tensor> norm_router(const at::Tensor& x, const c10::optional<at::Tensor>& residual, const at::Tensor& norm_w, double eps, const at::Tensor& W,
+                                    int64_t K, bool normalize, bool static_w) {
+  c10::cuda::CUDAGuard g(x.device());
+  const int64_t T = x.size(0), H = x.size(1), E = W.size(0);
+  const bool add = residual.has_value() && residual->defined();
+  TORCH_CHECK(x.is_contiguous() && W.is_contiguous() && norm_w.is_contiguous() && W.size(1) == H && norm_w.numel() == H &&
+                  (!add || (residual->is_contiguous() && residual->sizes() == x.sizes())),
+              "norm_router: x, residual [T, H], norm_w [H], W [E, H], contiguous");
+  at::Tensor sum;
+  if (add) sum = at::empty_like(x);
+  auto normed = at::empty_like(x);
+  auto w = at::empty({T, K}, x.options().dtype(at::kFloat));
+  auto idx = at::empty({T, K}, x.options().dtype(at::kInt));
+  check(mb_norm_router(x.data_ptr(), add ? residual->data_ptr() : nullptr, norm_w.data_ptr(), W.data_ptr(), eps, T, H, E, K, normalize, static_w,
+                       add ? sum.data_ptr() : nullptr, normed.data_ptr(), w.data_ptr<float>(), idx.data_ptr<int>(), cur_stream()),
+        "mb_norm_router");
+  return {sum, normed, w, idx};
+}
+
 // idx int32 [n] global expert ids → seg_offsets [E+1], tile_expert [max_rows/pad], row_src [max_rows], dst_row [n]
 std::vector<at::Tensor> moe_align(const at::Tensor& idx, int64_t E, int64_t expert_offset, int64_t max_rows,
                                   const c10::optional<at::Tensor>& n_dev, int64_t pad, bool ordered) {
@@ -88,6 +108,7 @@ void moe_combine_bwd(const at::Tensor& dout, const at::Tensor& y_perm, const at:
 void register_moe(pybind11::module& m) {
   m.def("router_topk", &router_topk, py::arg("logits"), py::arg("k"), py::arg("normalize"), py::arg("want_probs"), py::arg("replay") = py::none(),
         py::arg("err") = py::none());
+  m.def("norm_router", &norm_router);
   m.def("moe_align", &moe_align, py::arg("idx"), py::arg("E"), py::arg("expert_offset"), py::arg("max_rows"), py::arg("n_dev"),
         py::arg("pad") = 128, py::arg("ordered") = true);
   m.def("moe_gather", &moe_gather);

@@ -164,6 +164,32 @@ def router_topk(logits, k, normalize=True):
     return _apply(_RouterTopK, logits, int(k), bool(normalize), None)
 
 
+# Most experts of the one-launch form, one per warp of a token's CTA.  µs per call as norm, logits and top-k / in one launch, weights from memory: hidden 2048,
+# 16 experts, 1, 8, 16, 32, 64 rows 5.9 / 4.1, 9.0 / 4.3, 6.8 / 4.3, 7.4 / 4.3, 11.0 / 4.3; hidden 1024 4.7 / 3.6 to 8.9 / 3.8, hidden 4096 8.5 / 5.2 to
+# 16.7 / 5.4.  With several experts per warp their rows come one after another: 64 experts 6.0 to 11.3 / 10.2, 128 experts 6.3 to 12.3 / 18.
+_ROUTER_EXPERTS = 16
+
+
+def few_token_router(x, router) -> bool:
+    """True when `add_rmsnorm_router` applies: CUDA bf16, no autograd, the rows of a decode step, and sums over K that may take another order
+    than a product's of many rows (MILES_SPLIT_K, MILES_SMALL_M)."""
+    from . import cuda as _cuda
+
+    H = x.shape[-1]
+    T = x.numel() // H
+    return (x.dtype == BF16 and router.dtype == BF16 and router.is_contiguous() and 0 < T <= _cuda.SMALL_M and _cuda.SPLIT_K and H <= 4096 and H % 8 == 0
+            and router.shape[0] <= _ROUTER_EXPERTS and not torch.is_grad_enabled() and not transformed()
+            and x.data_ptr() % 16 == 0 and router.data_ptr() % 16 == 0)
+
+
+def add_rmsnorm_router(x, residual, norm_w, eps, router, k, normalize=True):
+    """(rmsnorm(x + residual), x + residual, weights, choices): what add_rmsnorm, linear_fp32 and router_topk give, with logits of unrounded operands."""
+    H = x.shape[-1]
+    res, xn, w, idx = C.norm_router(_c(x).view(-1, H), _c(residual).view(-1, H) if residual is not None else None, norm_w, float(eps), router, int(k),
+                                    bool(normalize), bool(router.is_leaf and router.requires_grad and norm_w.is_leaf and norm_w.requires_grad))
+    return xn.view(x.shape), (res.view(x.shape) if residual is not None else x), w, idx
+
+
 def router_replay(logits, idx, normalize=True):
     """A choice outside the experts, in a row that has any, raises the device error flag (72) and counts nothing."""
     if logits.shape[-1] > 256 or idx.shape[1] > 32:
