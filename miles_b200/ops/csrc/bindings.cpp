@@ -101,7 +101,7 @@ void moe_gemv(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, 
   const int64_t T = x.size(0), H = x.size(1), k = topk_idx.size(1), E = w13.size(0), F = w13.size(1) / (ungated ? 1 : 2);
   mb_count_launch(1);
   check(mb_moe_gemv(x.data_ptr(), w13.data_ptr(), w2.data_ptr(), topk_idx.data_ptr<int>(), topk_w.data_ptr<float>(), act.data_ptr(),
-                    out.data_ptr(), T, k, E, expert_offset, H, F, limit, alpha, shift, ungated, cur_stream()),
+                    out.data_ptr(), T, k, E, expert_offset, H, F, limit, alpha, shift, ungated, error_flag_for(x.device()).data_ptr<int>(), cur_stream()),
         "mb_moe_gemv");
 }
 

@@ -15,14 +15,15 @@
 //     permutation of k.   lane = 4·g + t: A rows g and g+8, k ∈ [32c + 8t, 32c + 8t + 8); B column (token) g, same k.
 //
 //   gemv            y[M, N] = norm?(x (+ residual)) · W[N, K]ᵀ (+ bias)       M ≤ 16; optional fused add + RMSNorm prologue
-//   moe_gemv_up     act[pair, F] = silu(W13[e][:F] x) · (W13[e][F:] x), or the clamped form of mixers.cuh, or relu(W1[e] x)²
+//   moe_gemv_up     act[pair, F] = gate_w · silu(W13[e][:F] x) · (W13[e][F:] x), or the clamped form of mixers.cuh, or relu(W1[e] x)²
 //                   per distinct expert of the step, T ≤ 8 tokens
-//   moe_gemv_down   out[T, H] = Σ_experts gate_w · W2[e] · act                 accumulated over experts in registers
+//   moe_gemv_down   out[T, H] = Σ_experts W2[e] · act                          accumulated over experts in registers
 #include <cuda_bf16.h>
 
 #include "launch.h"
 #include "mixers.cuh"
 #include "pdl.cuh"
+#include "ptx.cuh"
 
 namespace mb {
 namespace gv {
@@ -451,272 +452,287 @@ __global__ void __launch_bounds__(kThreads) gemv_kernel(GemvParams p) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// MoE for ≤ 8 tokens (≤ 64 (token, choice) pairs).  No sort, gather or combine kernels: every warp holds the pair → expert
-// table in two registers per lane and finds "the first pair of each distinct expert" and "the pair of (expert, token)"
-// with ballots.
+// MoE for ≤ 8 tokens (≤ 64 (token, choice) pairs).  No sort, gather or combine kernels.
+//
+// Eight warps multiply, one brings weight rows to shared memory with bulk copies, 16 rows × `piece` columns to a stage, a row per lane; the
+// fragments are read as in gemv_kernel.  What bounds it: the weights' bytes, once the warps that multiply do nothing else.  With every thread copying
+// its own 16-byte pieces (cp.async) the kernels were bound by their own instructions: some 95 per warp and 32 columns, 6 cycles each with 8 to 16
+// warps per SM, and memory at 24 to 49 % of its rate.  A layer of 16 experts, hidden 2048, 768 features, 8 choices: 1 token 12.7 + 11.6 → 11.8 + 7.2 µs
+// (50 and 25 MB), 7 tokens 21.5 + 17.8 → 20.6 + 12.0 (100 and 50 MB).  Copies of 2 KB: an SM starts one every 45 ns, so that 1 KB each takes 17 µs for
+// the 50 MB; 4 KB, or the two contiguous halves of an item (bank conflicts), leave the ring too coarse (+1 to +2 %).
 // ---------------------------------------------------------------------------------------------
 static constexpr int kMaxPairs = 64;
-static constexpr int kMoeStages = 8;
+static constexpr int kProducer = kWarps, kStorer = kWarps + 1, kMoeThreads = kThreads + 64;   // warps: 8 multiply, 1 copies, 1 stores
+static constexpr int kMaxStages = 8;
 
-struct PairIdx { int lo, hi; };   // local expert of pairs `lane` and `lane + 32`; −1: no pair, or an expert of another rank
-
-__device__ __forceinline__ PairIdx load_pairs(const int* __restrict__ topk_idx, int n_pairs, int E, int offset) {
+// The distinct experts of a step, made by one warp: lane l holds pairs l and l + 32.  Expert and pairs of each, in expert order where the experts
+// are no more than the pairs, else in order of first appearance; returns how many.
+__device__ __forceinline__ int distinct_experts(const int* topk_idx, int n_pairs, int E, int offset, int* slot_e, unsigned long long* slot_mask) {
   const int lane = threadIdx.x & 31;
-  PairIdx pi;
-  pi.lo = lane < n_pairs ? topk_idx[lane] - offset : -1;
-  pi.hi = lane + 32 < n_pairs ? topk_idx[lane + 32] - offset : -1;
-  if (pi.lo < 0 || pi.lo >= E) pi.lo = -1;
-  if (pi.hi < 0 || pi.hi >= E) pi.hi = -1;
-  return pi;
+  int lo = lane < n_pairs ? topk_idx[lane] - offset : -1;
+  int hi = lane + 32 < n_pairs ? topk_idx[lane + 32] - offset : -1;
+  if (lo < 0 || lo >= E) lo = -1;                       // no pair, or an expert of another rank
+  if (hi < 0 || hi >= E) hi = -1;
+  unsigned long long m_lo = __match_any_sync(0xffffffffu, lo), m_hi = 0;
+  if (n_pairs > 32) {
+    m_hi = static_cast<unsigned long long>(__match_any_sync(0xffffffffu, hi)) << 32;
+#pragma unroll 8
+    for (int i = 0; i < 32; ++i) {
+      if (__shfl_sync(0xffffffffu, hi, i) == lo) m_lo |= 1ull << (32 + i);
+      if (__shfl_sync(0xffffffffu, lo, i) == hi) m_hi |= 1ull << i;
+    }
+  }
+  const bool first_lo = lo >= 0 && __ffsll(static_cast<long long>(m_lo)) - 1 == lane, first_hi = hi >= 0 && __ffsll(static_cast<long long>(m_hi)) - 1 == lane + 32;
+  const uint32_t b_lo = __ballot_sync(0xffffffffu, first_lo), b_hi = __ballot_sync(0xffffffffu, first_hi);
+  int s_lo = __popc(b_lo & ((1u << lane) - 1)), s_hi = __popc(b_lo) + __popc(b_hi & ((1u << lane) - 1));
+  if (E <= n_pairs) {                                   // E ≤ 64
+    const uint32_t used0 = __reduce_or_sync(0xffffffffu, (lo >= 0 && lo < 32 ? 1u << lo : 0u) | (hi >= 0 && hi < 32 ? 1u << hi : 0u));
+    const uint32_t used1 = __reduce_or_sync(0xffffffffu, (lo >= 32 ? 1u << (lo - 32) : 0u) | (hi >= 32 ? 1u << (hi - 32) : 0u));
+    const unsigned long long used = (static_cast<unsigned long long>(used1) << 32) | used0;
+    s_lo = __popcll(used & ((1ull << (lo & 63)) - 1));
+    s_hi = __popcll(used & ((1ull << (hi & 63)) - 1));
+  }
+  if (first_lo) { slot_e[s_lo] = lo; slot_mask[s_lo] = m_lo; }
+  if (first_hi) { slot_e[s_hi] = hi; slot_mask[s_hi] = m_hi; }
+  return __popc(b_lo) + __popc(b_hi);
 }
-__device__ __forceinline__ int expert_of(const PairIdx& pi, int p) {
-  const int lo = __shfl_sync(0xffffffffu, pi.lo, p & 31), hi = __shfl_sync(0xffffffffu, pi.hi, p & 31);
-  return p < 32 ? lo : hi;
-}
-__device__ __forceinline__ unsigned long long match_mask(const PairIdx& pi, int e) {
-  const unsigned lo = __ballot_sync(0xffffffffu, pi.lo == e), hi = __ballot_sync(0xffffffffu, pi.hi == e);
-  return (static_cast<unsigned long long>(hi) << 32) | lo;
-}
-__device__ __forceinline__ bool is_first(unsigned long long mask, int p) { return (mask & ((1ull << p) - 1ull)) == 0ull; }
+// the pair of token `tok` among an expert's pairs, −1 if it has none
 __device__ __forceinline__ int pair_of(unsigned long long mask, int tok, int k) {
   const unsigned long long sel = k >= 64 ? ~0ull : ((1ull << k) - 1ull);
   const unsigned long long m = (mask >> (tok * k)) & sel;
   return m ? tok * k + __ffsll(static_cast<long long>(m)) - 1 : -1;
 }
 
-// Persistent grid over (distinct expert, block of features).  GATED: 8 features, gate rows f0..f0+7 and up rows F+f0..F+f0+7 of the expert
-// for all tokens, silu(gate) · up (or its clamped form) stored for the tokens routed to it.  Otherwise 16 rows of a [F, H] expert, relu(·)².  A warp's weight stream runs
-// across its items without a break (the ring keeps filling while the CTA reduces and stores an item).
-template <bool GATED>
-__global__ void __launch_bounds__(kThreads) moe_gemv_up_kernel(const bf16* x, const bf16* __restrict__ w13,
-                                                               const int* topk_idx, bf16* act, int T, int k,
-                                                               int E, int offset, int H, int F, float limit, float alpha, float shift) {
-  constexpr int S = kMoeStages, kFeat = GATED ? 8 : 16;
-  extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ float red[kWarps][16][8];
-  __shared__ int slot_e[kMaxPairs];
-  __shared__ unsigned long long slot_mask[kMaxPairs];
-  __shared__ int n_slots_s;
-  pdl_trigger();
-  pdl_wait();
-  const uint32_t ring = smem_addr(smem);
-  uint8_t* xs = smem + S * 2 * kThreads * 16;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int n_pairs = T * k;
-  if (warp == 0) {
-    // the distinct experts of the step, in order of first appearance
-    const PairIdx pi = load_pairs(topk_idx, n_pairs, E, offset);
-    int cnt = 0;
-    if (E <= n_pairs) {
-      // few local experts: one ballot pair per expert instead of a shuffle + ballot round per pair (the other warps wait
-      // for this table; slots are then in expert order, which only changes which CTA takes which item)
-      for (int e = 0; e < E; ++e) {
-        const unsigned long long m = match_mask(pi, e);
-        if (m == 0ull) continue;
-        if (lane == 0) { slot_e[cnt] = e; slot_mask[cnt] = m; }
-        ++cnt;
-      }
-    } else {
-      for (int p = 0; p < n_pairs; ++p) {
-        const int e = expert_of(pi, p);
-        if (e < 0) continue;
-        const unsigned long long m = match_mask(pi, e);
-        if (!is_first(m, p)) continue;
-        if (lane == 0) { slot_e[cnt] = e; slot_mask[cnt] = m; }
-        ++cnt;
-      }
-    }
-    if (lane == 0) n_slots_s = cnt;
+__device__ __forceinline__ void bulk_row(uint32_t dst, const bf16* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_addr(bar))
+               : "memory");
+}
+
+// What both kernels keep in shared memory beside their rows.
+struct MoeShared {
+  float red[2][kWarps][16][8];
+  unsigned long long mask[kMaxPairs];
+  int expert[kMaxPairs];
+  int row[kMaxPairs][8];                 // down: byte offset of a token's activation row for each expert, or of the row of zeros
+  uint64_t full[kMaxStages], empty[kMaxStages], red_full[2], red_empty[2], table, rows;
+  int n_slots;
+};
+
+__device__ __forceinline__ void moe_shared_init(MoeShared& sh, int stages) {
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < stages; ++i) { mbar_init(&sh.full[i], 1); mbar_init(&sh.empty[i], kWarps); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&sh.red_full[i], kWarps); mbar_init(&sh.red_empty[i], 1); }
+    mbar_init(&sh.table, 1);
+    mbar_init(&sh.rows, 1);
+    mbar_fence_init();
   }
-  stage_rows_async(xs, 8, T, H, x, H);
-  cp_commit();
-  cp_wait<0>();
   __syncthreads();
-  const int nfb = F / kFeat;
-  const int n_items = n_slots_s * nfb;
-  const int n_mine = n_items > static_cast<int>(blockIdx.x) ? (n_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-  const int chunks = H / 32;
-  const int cpw = chunks > warp ? (chunks - warp + kWarps - 1) / kWarps : 0;     // chunks of an item taken by this warp
-  const int total = n_mine * cpw;
-  const int stride = staged_stride(H);
-  // the copies are issued in stream order, so the (item, chunk) cursor advances incrementally: no division per copy
-  int i_u = 0, i_item = blockIdx.x;
-  const long long up_off = static_cast<long long>(GATED ? F : 8) * H;
-  const bf16* i_base = nullptr;
-  auto set_item = [&]() {
-    if (i_item < n_items)
-      i_base = w13 + static_cast<long long>(slot_e[i_item / nfb]) * (GATED ? 2 : 1) * F * H + static_cast<long long>((i_item % nfb) * kFeat + g) * H + t * 8;
-  };
-  set_item();
-  auto issue = [&](int q) {
-    if (q < total) {
-      const bf16* pa = i_base + (warp + i_u * kWarps) * 32;
-      cp16(ring_slot(ring, q & (S - 1), 0), pa);
-      cp16(ring_slot(ring, q & (S - 1), 1), pa + up_off);
-      if (++i_u == cpw) { i_u = 0; i_item += gridDim.x; set_item(); }
-    }
-    cp_commit();
-  };
+}
+
+// Sums of one stage: this warp's 32-column chunks of 16 weight rows (`a`: row g, `stride` apart) against the tokens' rows (`x`; null: no such token).
+__device__ __forceinline__ void moe_stage(float (&c)[4], uint32_t a, int stride, uint32_t x, bool has_x, int chunks, int warp) {
+  for (int ch = warp; ch < chunks; ch += kWarps) {
+    const uint4 wa = lds16(a + ch * 64), wb = lds16(a + 8 * stride + ch * 64);
+    const uint4 xv = has_x ? lds16(x + ch * 64) : make_uint4(0, 0, 0, 0);
+    mma_pair(c, wa, wb, xv);
+  }
+}
+__device__ __forceinline__ void moe_put_sums(float (&red)[16][8], const float (&c)[4], int g, int t) {
+  *reinterpret_cast<float2*>(&red[g][2 * t]) = make_float2(c[0], c[1]);
+  *reinterpret_cast<float2*>(&red[g + 8][2 * t]) = make_float2(c[2], c[3]);
+}
+
+struct MoeUp {
+  const bf16 *x, *w13;
+  const int* topk_idx;
+  const float* topk_w;
+  bf16* act;
+  int T, k, E, offset, H, F, piece, stages;
+  float limit, alpha, shift;
+  int* error_flag;
+};
+
+// Persistent grid over the features of the distinct experts, one expert after another: CTA c takes an even share of them, in items of up to 8 (GATED: gate
+// rows f0.. and up rows F+f0.. of the expert for all tokens, silu(gate) · up or its clamped form stored for the tokens routed to it; otherwise 16 rows
+// of a [F, H] expert, relu(·)²), each times the token's weight of the expert.  An item ends where its expert or the share does; rows that it does not have
+// are not loaded, whatever the ring holds in their place goes into sums that nobody reads.  A warp of its own (9) adds up the warps' sums and stores,
+// so that the stream of weights runs across items.
+template <bool GATED>
+__global__ void __launch_bounds__(kMoeThreads) moe_gemv_up_kernel(MoeUp p) {
+  constexpr int kFeat = GATED ? 8 : 16;
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ MoeShared sh;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int F = p.F, H = p.H, row_bytes = staged_stride(p.piece), stage_bytes = 16 * row_bytes, x_stride = staged_stride(H);
+  const uint32_t ring = smem_addr(smem), xs = ring + p.stages * stage_bytes;
+  moe_shared_init(sh, p.stages);
+  pdl_trigger();
+  bool ok = true;
+  if (warp == kProducer) {
+    pdl_wait();
+    if (lane == 0) mbar_expect_tx(&sh.rows, p.T * H * 2);
+    __syncwarp();
+    if (lane < p.T) bulk_row(xs + lane * x_stride, p.x + static_cast<long long>(lane) * H, H * 2, &sh.rows);
+    const int n = distinct_experts(p.topk_idx, p.T * p.k, p.E, p.offset, sh.expert, sh.mask);
+    if (lane == 0) sh.n_slots = n;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh.table);
+  } else {
+    if (warp == kStorer) pdl_wait();
+    ok = __all_sync(0xffffffffu, mbar_wait(&sh.table, 0));
+  }
+  const int features = sh.n_slots * F, share = (features + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  const int begin = min(features, static_cast<int>(blockIdx.x) * share), end = min(features, begin + share);
+  int stage = 0, buf = 0, rows;
+  uint32_t phase = 0, buf_phase = 0;
+  if (warp < kWarps) ok = __all_sync(0xffffffffu, ok && mbar_wait(&sh.rows, 0));
+  for (int f = begin; f < end && ok; f += rows) {
+    const int slot = f / F, f0 = f - slot * F;
+    rows = min(kFeat, min(end - f, F - f0));
+    if (warp == kProducer) {
+      const bool mine = GATED ? lane < 16 && (lane & 7) < rows : lane < rows;
+      const bf16* src = p.w13 + (static_cast<long long>(sh.expert[slot]) * (GATED ? 2 : 1) * F + f0 + (GATED ? (lane & 7) + (lane >= 8 ? F : 0) : lane)) * H;
+      for (int c0 = 0; c0 < H && ok; c0 += p.piece) {
+        const int bytes = min(p.piece, H - c0) * 2;
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.empty[stage], phase ^ 1));
+        if (ok && lane == 0) mbar_expect_tx(&sh.full[stage], rows * (GATED ? 2 : 1) * bytes);
+        __syncwarp();
+        if (ok && mine) bulk_row(ring + stage * stage_bytes + lane * row_bytes, src + c0, bytes, &sh.full[stage]);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+    } else if (warp < kWarps) {
+      const int g = lane >> 2, t = lane & 3;
+      float c[4] = {};
+      for (int c0 = 0; c0 < H && ok; c0 += p.piece) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.full[stage], phase));
+        moe_stage(c, ring + stage * stage_bytes + g * row_bytes + t * 16, row_bytes, xs + g * x_stride + c0 * 2 + t * 16, g < p.T, min(p.piece, H - c0) / 32, warp);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.empty[stage]);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+      ok = ok && __all_sync(0xffffffffu, mbar_wait(&sh.red_empty[buf], buf_phase ^ 1));
+      moe_put_sums(sh.red[buf][warp], c, g, t);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.red_full[buf]);
+      if (++buf == 2) { buf = 0; buf_phase ^= 1; }
+    } else {
+      const unsigned long long mask = sh.mask[slot];
+      ok = __all_sync(0xffffffffu, mbar_wait(&sh.red_full[buf], buf_phase));
 #pragma unroll
-  for (int q = 0; q < S; ++q) issue(q);
-  int q = 0;
-  for (int j = 0; j < n_mine; ++j) {
-    const int item = blockIdx.x + j * gridDim.x;
-    const int s = item / nfb, f0 = (item % nfb) * kFeat;
-    float c[4] = {};
-    for (int u = 0; u < cpw; ++u, ++q) {
-      cp_wait<S - 1>();
-      const int st = q & (S - 1), ch = warp + u * kWarps;
-      const uint4 wa = lds16(ring_slot(ring, st, 0)), wb = lds16(ring_slot(ring, st, 1));
-      const uint4 xv = *reinterpret_cast<const uint4*>(xs + g * stride + ch * 64 + t * 16);
-      mma_pair(c, wa, wb, xv);
-      issue(q + S);
-    }
-    red[warp][g][2 * t] = c[0];
-    red[warp][g][2 * t + 1] = c[1];
-    red[warp][g + 8][2 * t] = c[2];
-    red[warp][g + 8][2 * t + 1] = c[3];
-    __syncthreads();
-    if (threadIdx.x < 8 * kFeat) {
-      const int f = threadIdx.x & (kFeat - 1), tok = threadIdx.x / kFeat;
-      const int pair = tok < T ? pair_of(slot_mask[s], tok, k) : -1;
-      if (pair >= 0) {
+      for (int i = 0; i < 8 * kFeat / 32; ++i) {
+        const int fi = lane & (kFeat - 1), tok = lane / kFeat + i * (32 / kFeat);
+        const int pair = ok && tok < p.T && fi < rows ? pair_of(mask, tok, p.k) : -1;
+        if (pair < 0) continue;
+        const float w = p.topk_w[pair];
         float gate = 0.f, up = 0.f;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-          gate += red[w][f][tok];
-          if (GATED) up += red[w][f + 8][tok];
+        for (int v = 0; v < kWarps; ++v) {
+          gate += sh.red[buf][v][fi][tok];
+          if (GATED) up += sh.red[buf][v][(fi + 8) & 15][tok];
         }
         // the sums are rounded to bf16 first, like the stored pre-activation of the general path
         gate = __bfloat162float(__float2bfloat16(gate));
         up = __bfloat162float(__float2bfloat16(up));
         float a;
         if (!GATED) a = mx::relu_square(gate);
-        else a = alpha != 0.f ? mx::clamped_glu_t<bf16>(gate, up, limit, alpha, shift) : gate / (1.f + __expf(-gate)) * up;
-        act[static_cast<long long>(pair) * F + f0 + f] = __float2bfloat16(a);
+        else a = p.alpha != 0.f ? mx::clamped_glu_t<bf16>(gate, up, p.limit, p.alpha, p.shift) : gate / (1.f + __expf(-gate)) * up;
+        p.act[static_cast<long long>(pair) * F + f0 + fi] = __float2bfloat16(a * w);
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.red_empty[buf]);
+      if (++buf == 2) { buf = 0; buf_phase ^= 1; }
     }
-    __syncthreads();   // `red` is reused by the next item
   }
-  cp_wait<0>();
+  if (!ok && lane == 0) atomicExch(p.error_flag, 48);
 }
 
-// grid (H/16): CTA hb accumulates rows h0..h0+15 of the output over all distinct experts of the step; its 8 warps take
-// the 32-wide k chunks of EVERY expert round-robin (equal work per warp whatever the routing), a warp's weight stream runs
-// across the experts without a break.
-// out[t, h] = Σ_experts gate_w(t, e) · (W2[e][h, :] · act[pair(t, e), :])
-__global__ void __launch_bounds__(kThreads) moe_gemv_down_kernel(const bf16* act, const bf16* __restrict__ w2,
-                                                                 const int* topk_idx, const float* topk_w,
-                                                                 bf16* out, int T, int k, int E, int offset, int H, int F) {
-  constexpr int S = kMoeStages;
+// Row stride of a stage of the down kernel.
+__host__ __device__ inline int down_row_bytes(int F, int piece) { return piece == F ? 2 * F : staged_stride(piece); }
+
+struct MoeDown {
+  const bf16 *act, *w2;
+  const int* topk_idx;
+  bf16* out;
+  int T, k, E, offset, H, F, piece, stages;
+  int* error_flag;
+};
+
+// grid ⌈H / 16⌉: a CTA accumulates 16 rows of the output over all distinct experts of the step; out[t, h] = Σ_experts W2[e][h, :] · act[pair(t, e), :]
+// (activations that carry the weights).  A warp takes every eighth 32-wide chunk of EVERY expert.  The 16 rows of an expert lie one behind the other:
+// where a stage takes whole rows they are one copy, although their fragments then meet two lanes to a bank (7 tokens, 768 features: 12.0 µs, 15.5 with
+// a copy per row).
+__global__ void __launch_bounds__(kMoeThreads) moe_gemv_down_kernel(MoeDown p) {
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ float red[kWarps][16][8];
-  __shared__ int sl_e[kMaxPairs];
-  __shared__ signed char sl_pair[kMaxPairs][8];
-  __shared__ float sl_gw[kMaxPairs][8];
-  __shared__ int n_slots_s;
-  pdl_trigger();
-  pdl_wait();
-  const uint32_t ring = smem_addr(smem);
-  uint8_t* as = smem + S * 2 * kThreads * 16;
+  __shared__ MoeShared sh;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int F = p.F, H = p.H, row_bytes = down_row_bytes(F, p.piece), stage_bytes = 16 * row_bytes, a_stride = staged_stride(F), n_pairs = p.T * p.k;
+  const int h0 = static_cast<int>(blockIdx.x) * 16, rows = min(16, H - h0);
+  const bool whole = p.piece == F;
+  const uint32_t ring = smem_addr(smem), as = ring + p.stages * stage_bytes;
+  moe_shared_init(sh, p.stages);
+  pdl_trigger();
+  bool ok = true;
+  int stage = 0;
+  uint32_t phase = 0;
   const int g = lane >> 2, t = lane & 3;
-  const int h0 = blockIdx.x * 16;
-  const int chunks = F / 32;
-  const int n_pairs = T * k;
-  // all pair rows of the activations → shared memory, in flight while warp 0 builds the expert table (rows of other
-  // ranks' experts are copied too and never read)
-  stage_rows_async(as, n_pairs, n_pairs, F, act, F);
-  cp_commit();
-  if (warp == 0) {
-    // the distinct experts of the step with, per token, the pair routed to them and its gate weight
-    const PairIdx pi = load_pairs(topk_idx, n_pairs, E, offset);
-    int cnt = 0;
-    auto add_slot = [&](int e, unsigned long long mask) {
-      if (lane < 8) {
-        const int pair = lane < T ? pair_of(mask, lane, k) : -1;
-        sl_pair[cnt][lane] = static_cast<signed char>(pair);
-        sl_gw[cnt][lane] = pair >= 0 ? topk_w[pair] : 0.f;
-      }
-      if (lane == 0) sl_e[cnt] = e;
-      ++cnt;
-    };
-    if (E <= n_pairs) {                      // few local experts: a ballot pair per expert (see moe_gemv_up_kernel)
-      for (int e = 0; e < E; ++e) {
-        const unsigned long long mask = match_mask(pi, e);
-        if (mask != 0ull) add_slot(e, mask);
-      }
-    } else {
-      for (int p = 0; p < n_pairs; ++p) {
-        const int e = expert_of(pi, p);
-        if (e < 0) continue;
-        const unsigned long long mask = match_mask(pi, e);
-        if (is_first(mask, p)) add_slot(e, mask);
-      }
-    }
-    if (lane == 0) n_slots_s = cnt;
-  }
-  __syncthreads();
-  const int cnt = n_slots_s;
-  const int cpw = chunks > warp ? (chunks - warp + kWarps - 1) / kWarps : 0;      // chunks of an expert taken by this warp
-  const int total = cnt * cpw;
-  int i_u = 0, i_j = 0;                                         // issue cursor: (expert slot, chunk), advanced in stream order
-  const long long row_off = static_cast<long long>(h0 + g) * F + t * 8;
-  const bf16* i_base = cnt > 0 ? w2 + static_cast<long long>(sl_e[0]) * H * F + row_off : nullptr;
-  auto issue = [&](int q) {
-    if (q < total) {
-      const bf16* pa = i_base + (warp + i_u * kWarps) * 32;
-      cp16(ring_slot(ring, q & (S - 1), 0), pa);
-      cp16(ring_slot(ring, q & (S - 1), 1), pa + 8 * F);
-      if (++i_u == cpw) {
-        i_u = 0;
-        if (++i_j < cnt) i_base = w2 + static_cast<long long>(sl_e[i_j]) * H * F + row_off;
-      }
-    }
-    cp_commit();
-  };
-#pragma unroll
-  for (int q = 0; q < S; ++q) issue(q);
-  cp_wait<S>();          // the activation rows (the oldest group) have landed; the weight ring keeps filling
-  __syncthreads();
-  const int stride = staged_stride(F);
   float c[4] = {};
-  int q = 0;
-  for (int j = 0; j < cnt; ++j) {
-    const int pair = sl_pair[j][g];
-    const uint8_t* arow = as + (pair >= 0 ? pair : 0) * stride + t * 16;
-    float cs[4] = {};
-    for (int u = 0; u < cpw; ++u, ++q) {
-      cp_wait<S - 1>();
-      const int st = q & (S - 1);
-      const uint4 wa = lds16(ring_slot(ring, st, 0)), wb = lds16(ring_slot(ring, st, 1));
-      const uint4 xv = pair >= 0 ? *reinterpret_cast<const uint4*>(arow + (warp + u * kWarps) * 64) : make_uint4(0, 0, 0, 0);
-      mma_pair(cs, wa, wb, xv);
-      issue(q + S);
+  if (warp == kProducer) {
+    pdl_wait();
+    const int n = distinct_experts(p.topk_idx, n_pairs, p.E, p.offset, sh.expert, sh.mask);
+    if (lane == 0) {
+      sh.n_slots = n;
+      mbar_expect_tx(&sh.rows, n_pairs * F * 2);
     }
-    // accumulator columns 2t and 2t+1 are tokens 2t and 2t+1
-    const float gw0 = sl_gw[j][2 * t], gw1 = sl_gw[j][2 * t + 1];
-    c[0] += gw0 * cs[0];
-    c[1] += gw1 * cs[1];
-    c[2] += gw0 * cs[2];
-    c[3] += gw1 * cs[3];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh.table);
+    for (int slot = 0; slot < n && ok; ++slot) {
+      const bf16* src = p.w2 + (static_cast<long long>(sh.expert[slot]) * H + h0 + lane) * F;
+      for (int c0 = 0; c0 < F && ok; c0 += p.piece) {
+        const int bytes = min(p.piece, F - c0) * 2;
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.empty[stage], phase ^ 1));
+        if (ok && lane == 0) mbar_expect_tx(&sh.full[stage], rows * bytes);
+        __syncwarp();
+        if (ok && lane < (whole ? 1 : rows)) bulk_row(ring + stage * stage_bytes + lane * row_bytes, src + c0, whole ? rows * bytes : bytes, &sh.full[stage]);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == kStorer) {
+    pdl_wait();                                          // the rows are the kernel's in front; the choices' table comes meanwhile
+    ok = __all_sync(0xffffffffu, mbar_wait(&sh.table, 0));
+    for (int i = lane; i < n_pairs && ok; i += 32) bulk_row(as + i * a_stride, p.act + static_cast<long long>(i) * F, F * 2, &sh.rows);
+  } else {
+    for (int i = threadIdx.x; i < F / 8; i += kThreads) *reinterpret_cast<uint4*>(smem + p.stages * stage_bytes + n_pairs * a_stride + i * 16) = make_uint4(0, 0, 0, 0);
+    ok = __all_sync(0xffffffffu, mbar_wait(&sh.table, 0));
+    for (int i = threadIdx.x; i < sh.n_slots * 8 && ok; i += kThreads) {
+      const int tok = i & 7, pair = tok < p.T ? pair_of(sh.mask[i >> 3], tok, p.k) : -1;
+      sh.row[i >> 3][tok] = (pair >= 0 ? pair : n_pairs) * a_stride;
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    ok = __all_sync(0xffffffffu, ok && mbar_wait(&sh.rows, 0));
+    const int n = sh.n_slots;
+    for (int slot = 0; slot < n && ok; ++slot) {
+      const uint32_t x = as + sh.row[slot][g] + t * 16;
+      for (int c0 = 0; c0 < F && ok; c0 += p.piece) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.full[stage], phase));
+        moe_stage(c, ring + stage * stage_bytes + g * row_bytes + t * 16, row_bytes, x + c0 * 2, true, min(p.piece, F - c0) / 32, warp);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.empty[stage]);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+    }
+    moe_put_sums(sh.red[0][warp], c, g, t);
   }
-  cp_wait<0>();
-  red[warp][g][2 * t] = c[0];
-  red[warp][g][2 * t + 1] = c[1];
-  red[warp][g + 8][2 * t] = c[2];
-  red[warp][g + 8][2 * t + 1] = c[3];
   __syncthreads();
   if (threadIdx.x < 128) {
     const int row = threadIdx.x & 15, tok = threadIdx.x >> 4;
-    if (tok < T) {
+    if (tok < p.T && row < rows) {
       float s = 0.f;
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) s += red[w][row][tok];
-      out[static_cast<long long>(tok) * H + h0 + row] = __float2bfloat16(s);
+      for (int w = 0; w < kWarps; ++w) s += sh.red[0][w][row][tok];
+      p.out[static_cast<long long>(tok) * H + h0 + row] = __float2bfloat16(s);
     }
   }
+  if (!ok && lane == 0) atomicExch(p.error_flag, 49);
 }
 
 template <typename K>
@@ -837,31 +853,44 @@ extern "C" int mb_gemv_sum_norm(MbGemvSum a, cudaStream_t s) {
   return static_cast<int>(nt == 1 ? launch_gemv<1, kSumNorm>(p, s) : launch_gemv<2, kSumNorm>(p, s));
 }
 
-// MoE FFN for T ≤ 8 tokens (T·k ≤ 64): act [T·k, F] scratch, out [T, H].  alpha ≠ 0: clamped activation, else SwiGLU; ungated:
-// w13 is [E, F, H], the activation relu(·)².  H and F multiples of 32, H a multiple of 16.
+// MoE FFN for ≤ 8 tokens (T·k ≤ 64): act [T·k, F] scratch, out [T, H].  alpha ≠ 0: clamped activation, else SwiGLU; ungated:
+// w13 is [E, F, H], the activation relu(·)².  H and F multiples of 32; x, act and the weights 16-byte aligned.
 extern "C" int mb_moe_gemv(const void* x, const void* w13, const void* w2, const int* topk_idx, const float* topk_w, void* act, void* out,
-                           int T, int k, int E, int expert_offset, int H, int F, float limit, float alpha, float shift, int ungated, cudaStream_t s) {
+                           int T, int k, int E, int expert_offset, int H, int F, float limit, float alpha, float shift, int ungated, int* error_flag,
+                           cudaStream_t s) {
   if (T <= 0) return 0;
   if (T > 8 || T * k > kMaxPairs || H % 32 || F % 32) return -1;
-  const int ring_bytes = kMoeStages * 2 * kThreads * 16;
-  const int up_bytes = ring_bytes + 8 * staged_stride(H);
-  const int down_bytes = ring_bytes + T * k * staged_stride(F);
-  if (up_bytes > kMaxSmem || down_bytes > kMaxSmem) return -2;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = set_smem(moe_gemv_up_kernel<true>, kMaxSmem);
-    if (e == cudaSuccess) e = set_smem(moe_gemv_up_kernel<false>, kMaxSmem);
-    if (e == cudaSuccess) e = set_smem(moe_gemv_down_kernel, kMaxSmem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
-  const int max_items = (T * k < E ? T * k : E) * (F / (ungated ? 16 : 8));
-  const int up_grid = max_items < 2 * 148 ? max_items : 2 * 148;
-  cudaError_t e = launch_pdl(ungated ? moe_gemv_up_kernel<false> : moe_gemv_up_kernel<true>, dim3(up_grid), dim3(kThreads), up_bytes, s, reinterpret_cast<const bf16*>(x),
-                             reinterpret_cast<const bf16*>(w13), topk_idx, reinterpret_cast<bf16*>(act), T, k, E, expert_offset, H, F, limit, alpha,
-                             shift);
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w13) | reinterpret_cast<uintptr_t>(w2) | reinterpret_cast<uintptr_t>(act)) & 15) return -3;
+  constexpr int kMoeSmem = 210 * 1024, kHalfSmem = 100 * 1024;      // beside MoeShared (11 KB) and what an SM keeps: one CTA, two
+  auto piece_of = [](int n) {                                       // columns of a stage: an even cut into at most 1024, in multiples of 64
+    const int pieces = (n + 1023) / 1024;
+    return ((n + pieces - 1) / pieces + 63) / 64 * 64;
+  };
+  const int up_piece = piece_of(H), down_piece = F <= 1024 ? F : piece_of(F);
+  const int up_stage = 16 * staged_stride(up_piece), up_rows = T * staged_stride(H);
+  const int down_stage = 16 * down_row_bytes(F, down_piece), down_rows = (T * k + 1) * staged_stride(F);
+  // two CTAs per SM with two stages each where they fit (7 tokens, hidden 2048: 938 µs for a step of 12 layers, 948 with one CTA and five stages)
+  const bool two = 2 * up_stage + up_rows <= kHalfSmem;
+  const int up_stages = two ? 2 : (kMoeSmem - up_rows) / up_stage < 5 ? (kMoeSmem - up_rows) / up_stage : 5;
+  const int down_stages = (kMoeSmem - down_rows) / down_stage < 6 ? (kMoeSmem - down_rows) / down_stage : 6;
+  if (up_stages < 2 || down_stages < 2) return -2;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int most = (T * k < E ? T * k : E) * F, items = (most + 7) / 8;              // features and items of eight if every choice is another expert
+  const int up_grid = items < (two ? 2 : 1) * sms ? items : (two ? 2 : 1) * sms;
+  static const cudaError_t configured = [] {
+    cudaError_t e = set_smem(moe_gemv_up_kernel<true>, kMoeSmem);
+    if (e == cudaSuccess) e = set_smem(moe_gemv_up_kernel<false>, kMoeSmem);
+    if (e == cudaSuccess) e = set_smem(moe_gemv_down_kernel, kMoeSmem);
+    return e;
+  }();
+  if (configured != cudaSuccess) return static_cast<int>(configured);
+  auto b = [](const void* p) { return reinterpret_cast<const bf16*>(p); };
+  const MoeUp up{b(x), b(w13), topk_idx, topk_w, reinterpret_cast<bf16*>(act), T, k, E, expert_offset, H, F, up_piece, up_stages, limit, alpha, shift, error_flag};
+  cudaError_t e = launch_pdl(ungated ? moe_gemv_up_kernel<false> : moe_gemv_up_kernel<true>, dim3(up_grid), dim3(kMoeThreads), up_stages * up_stage + up_rows, s, up);
   if (e != cudaSuccess) return static_cast<int>(e);
-  e = launch_pdl(moe_gemv_down_kernel, dim3(H / 16), dim3(kThreads), down_bytes, s, reinterpret_cast<const bf16*>(act),
-                 reinterpret_cast<const bf16*>(w2), topk_idx, topk_w, reinterpret_cast<bf16*>(out), T, k, E, expert_offset, H, F);
+  const MoeDown down{b(act), b(w2), topk_idx, reinterpret_cast<bf16*>(out), T, k, E, expert_offset, H, F, down_piece, down_stages, error_flag};
+  e = launch_pdl(moe_gemv_down_kernel, dim3((H + 15) / 16), dim3(kMoeThreads), down_stages * down_stage + down_rows, s, down);
   return static_cast<int>(e);
 }

@@ -42,7 +42,7 @@ int mb_gemm_small_grouped(const void* X, const void* W, void* C, int rows, int N
 int mb_gemv(const void* x, long long ldx, const void* residual, const void* norm_w, float eps, const void* W, const void* bias, void* y, long long ldy,
             int out_fp32, void* res_out, void* xn_out, int M, int N, int K, int static_w, cudaStream_t s);
 int mb_moe_gemv(const void* x, const void* w13, const void* w2, const int* topk_idx, const float* topk_w, void* act, void* out, int T, int k,
-                int E, int expert_offset, int H, int F, float limit, float alpha, float shift, int ungated, cudaStream_t s);
+                int E, int expert_offset, int H, int F, float limit, float alpha, float shift, int ungated, int* error_flag, cudaStream_t s);
 int mb_gemm_bf16_grouped_wgrad(const void* dY, const void* X, void* dW, int M_pad, int N, int K, int num_experts,
                                const int* seg_offsets, int out_fp32, int accumulate, int force_bn, int* error_flag,
                                cudaStream_t stream);

@@ -231,11 +231,11 @@ def moe_max_rows_pad(n_pairs: int, num_experts: int, pad: int) -> int:
 
 def few_token_experts(x, w13, T: int, k: int, ungated: bool = False) -> bool:
     """A handful of tokens: two matrix-vector kernels, no sort / gather / combine (gemv.cu).  Both keep their activations in shared
-    memory next to a 64 KB weight ring.  `ungated`: w13 has no gate rows."""
+    memory next to a weight ring of at least 66 KB.  `ungated`: w13 has no gate rows."""
     F = w13.shape[1] if ungated else w13.shape[1] // 2
     return (x.dtype == BF16 and 0 < T <= MOE_GEMV_T and T * k <= 64 and not torch.is_grad_enabled() and x.shape[1] % 32 == 0
             and F % 32 == 0 and (ungated or w13.shape[1] % 64 == 0)
-            and 65536 + max(8 * (2 * x.shape[1] + 64), T * k * (2 * F + 64)) <= 200 * 1024)
+            and 65536 + max(8 * (2 * x.shape[1] + 64), T * k * (2 * F + 64)) <= 200 * 1024 and 67584 + (T * k + 1) * (2 * F + 64) <= 210 * 1024)
 
 
 def _glu_in_place() -> bool:
