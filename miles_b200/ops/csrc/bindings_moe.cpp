@@ -103,6 +103,17 @@ void moe_combine_bwd(const at::Tensor& dout, const at::Tensor& y_perm, const at:
         "mb_moe_combine_bwd");
 }
 
+// h1 [rows, 2F], act_w [rows, F] (dout · W2 → weighted activation), dh1 [rows, 2F], w and dw fp32 [pairs]
+void moe_glu_bwd(const at::Tensor& h1, at::Tensor& act_w, at::Tensor& dh1, const at::Tensor& w, const at::Tensor& row_src, const at::Tensor& seg, at::Tensor& dw) {
+  c10::cuda::CUDAGuard g(h1.device());
+  TORCH_CHECK(h1.is_contiguous() && act_w.is_contiguous() && dh1.is_contiguous() && w.is_contiguous() && dw.is_contiguous() && h1.sizes() == dh1.sizes() &&
+                  h1.size(0) == act_w.size(0) && h1.size(1) == 2 * act_w.size(1) && w.numel() == dw.numel(),
+              "moe_glu_bwd: h1, dh1 [rows, 2F], act_w [rows, F], w, dw [pairs], contiguous");
+  check(mb_moe_glu_bwd(h1.data_ptr(), act_w.data_ptr(), dh1.data_ptr(), w.data_ptr<float>(), row_src.data_ptr<int>(), seg.data_ptr<int>(), seg.numel() - 1,
+                       dw.data_ptr<float>(), act_w.size(1), act_w.size(0), cur_stream()),
+        "mb_moe_glu_bwd");
+}
+
 }  // namespace
 
 void register_moe(pybind11::module& m) {
@@ -115,4 +126,5 @@ void register_moe(pybind11::module& m) {
   m.def("moe_combine", &moe_combine, pybind11::arg("y_perm"), pybind11::arg("w"), pybind11::arg("dst_row"), pybind11::arg("out"),
         pybind11::arg("k"), pybind11::arg("identity_rows") = false);
   m.def("moe_combine_bwd", &moe_combine_bwd);
+  m.def("moe_glu_bwd", &moe_glu_bwd);
 }

@@ -124,6 +124,8 @@ int mb_paged_bounds_set_limit(int which, long long value);
 int mb_paged_bounds_read(long long* out4, int clear);
 
 // ---- moe.cu ----
+int mb_moe_glu_bwd(const void* h1, void* act_w, void* dh1, const float* w, const int* row_src, const int* seg_offsets, int E, float* dw, int F, int max_rows,
+                   cudaStream_t s);
 int mb_norm_router(const void* x, const void* residual, const void* norm_w, const void* W, float eps, int T, int H, int E, int K, int normalize,
                    int static_w, void* sum, void* normed, float* topk_w, int* topk_idx, cudaStream_t s);
 int mb_router_topk(const float* logits, float* probs, float* topk_w, int* topk_idx, long long T, int E, int K, int normalize, const int* replay, long long replay_row,

@@ -374,40 +374,44 @@ class _MoEFFN(torch.autograd.Function):
         h1, y_perm = experts_forward(x_perm, w13, w2, seg, tile, keep=keep)        # bf16 grouped GEMMs, or block-scaled under the MXFP8 recipe
         out = torch.empty(T, H, dtype=x.dtype, device=x.device)
         C.moe_combine(y_perm, wf, dst_row, out, k)
-        ctx.save_for_backward(x, w13, w2, wf, seg, tile, row_src, dst_row, h1, y_perm)
+        from . import cuda as _cuda
+
+        # the gate weights' gradient ⟨dout, W2 · act⟩ is taken as ⟨dout · W2, act⟩: y is not needed, except where it is not W2 · act (quantised)
+        ctx.save_for_backward(x_perm, w13, w2, wf, seg, tile, row_src, dst_row, h1, y_perm if _cuda.MXFP8_LINEAR else None)
         ctx.k = k
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        x, w13, w2, wf, seg, tile, row_src, dst_row, h1, y_perm = ctx.saved_tensors
+        x_perm, w13, w2, wf, seg, tile, row_src, dst_row, h1, y_perm = ctx.saved_tensors
         k = ctx.k
-        T, H = x.shape
+        T, H = dout.shape
         E, F2, _ = w13.shape
         F = F2 // 2
         max_rows = h1.shape[0]
         dout = _c(dout)
-        dy_perm = torch.empty(max_rows, H, dtype=x.dtype, device=x.device)
-        dw_flat = torch.zeros(T * k, dtype=torch.float32, device=x.device)
-        C.moe_combine_bwd(dout, y_perm, wf.view(-1), row_src, seg, dy_perm, dw_flat, k)
-        # through W2: dact = dy_perm · W2 ; dW2[e] = dy_permᵀ · act
-        act = torch.empty(max_rows, F, dtype=x.dtype, device=x.device)
-        C.swiglu_fwd(h1, act, seg[-1:])
-        dact = torch.empty(max_rows, F, dtype=x.dtype, device=x.device)
-        C.gemm_grouped(dy_perm, w2, dact, max_rows, F, H, E, tile, True, 0)
+        new = lambda *shape: torch.empty(*shape, dtype=h1.dtype, device=h1.device)
+        dw_flat = torch.zeros(T * k, dtype=torch.float32, device=h1.device)
+        dy_perm, act, dh1 = new(max_rows, H), new(max_rows, F), new(max_rows, F2)
+        if y_perm is None:
+            # every row of dout as it is: the weight goes to the activation
+            publish_limit(LIMIT_MOE_PAIRS, T * k)
+            C.moe_gather(dout, dy_perm, row_src, seg, k)
+            C.gemm_grouped(dy_perm, w2, act, max_rows, F, H, E, tile, True, 0)
+            C.moe_glu_bwd(h1, act, dh1, wf.view(-1), row_src, seg, dw_flat)
+        else:
+            C.moe_combine_bwd(dout, y_perm, wf.view(-1), row_src, seg, dy_perm, dw_flat, k)
+            dact = new(max_rows, F)
+            C.swiglu_fwd(h1, act, seg[-1:])
+            C.gemm_grouped(dy_perm, w2, dact, max_rows, F, H, E, tile, True, 0)
+            C.swiglu_bwd(h1, dact, dh1, seg[-1:])
         dw2 = torch.empty_like(w2)
         C.gemm_grouped_wgrad(dy_perm, act, dw2, max_rows, H, F, E, seg, False, 0)
-        dh1 = torch.empty(max_rows, F2, dtype=x.dtype, device=x.device)
-        C.swiglu_bwd(h1, dact, dh1, seg[-1:])
-        x_perm = torch.empty(max_rows, H, dtype=x.dtype, device=x.device)
-        publish_limit(LIMIT_MOE_PAIRS, x.shape[0] * k)
-        C.moe_gather(x, x_perm, row_src, seg, k)
         dw13 = torch.empty_like(w13)
         C.gemm_grouped_wgrad(dh1, x_perm, dw13, max_rows, F2, H, E, seg, False, 0)
-        dx_perm = torch.empty(max_rows, H, dtype=x.dtype, device=x.device)
-        C.gemm_grouped(dh1, w13, dx_perm, max_rows, H, F2, E, tile, True, 0)
-        dx = torch.empty_like(x)
-        C.moe_combine(dx_perm, None, dst_row, dx, k)
+        C.gemm_grouped(dh1, w13, dy_perm, max_rows, H, F2, E, tile, True, 0)              # dy_perm has been read: the input rows' gradient in its place
+        dx = new(T, H)
+        C.moe_combine(dy_perm, None, dst_row, dx, k)
         return dx, dw13, dw2, dw_flat.view(T, k), None, None, None
 
 
