@@ -15,7 +15,7 @@ these tensors along dim 0 (column) or dim 1 (row).
 from __future__ import annotations
 
 import math
-from dataclasses import dataclass, field
+from dataclasses import dataclass, field, replace
 from typing import Callable
 
 import torch
@@ -44,6 +44,7 @@ class ForwardMeta:
     record_topk: "list[torch.Tensor] | None" = None  # filled with int32 [T,k] per MoE layer when not None
     record_width: int = 0                    # k of those records where layers differ in it (narrower layers pad with −1)
     recompute: bool = False                  # activation checkpoint each layer
+    values: bool = True                      # False: a layer run again for its graph alone, the product that ends it is not read
     lora_slots: torch.Tensor | None = None   # int64 [T] adapter slot per token (None → slot 0; -1 → base model only)
     # prefill that continues cached KV (a prefix-cache hit, a later piece of a chunked prompt): packed offsets of the new
     # tokens (cu_q) and of every request's keys (cu_k), flat cache slots of those keys (kv_slots), longest key sequence (max_k)
@@ -179,7 +180,7 @@ class DenseFFN(nn.Module):
     def forward(self, x, meta: ForwardMeta, layer: int):
         lora = getattr(self, "lora", None)
         if lora is None and self.ps.tp_size == 1:
-            h = ops.linear_swiglu(x, self.w13)
+            return ops.swiglu_ffn(x, self.w13, self.w2, meta.values)
         else:
             h13 = self.ps.column_linear(x, self.w13)
             if lora is not None and "w13" in lora:
@@ -227,7 +228,7 @@ class MoEFFN(nn.Module):
             w, idx, _ = ops.router_topk(logits, k, norm)
         if meta.record_topk is not None:
             meta.record_topk.append(idx.detach())
-        return self.ps.moe_ffn(x, self.w13, self.w2, w, idx, self.cfg.num_experts)
+        return self.ps.moe_ffn(x, self.w13, self.w2, w, idx, self.cfg.num_experts, meta.values)
 
 
 def add_rmsnorm_reducing(ps, x, residual, w, eps):
@@ -420,7 +421,50 @@ class VirtualStages(nn.Module):
         return self.chunks[-1].log_probs(hidden, targets, temperature, with_entropy)
 
 
+class _RunAgain(torch.autograd.Function):
+    """One decoder layer of which only the inputs are kept.  The forward pass is the one without gradients (no graph, gate · up formed in the product's
+    epilogue); the backward runs the layer again with them, without the product that ends it, and differentiates that.  `torch.utils.checkpoint` does the
+    same with a hook around every saved tensor and all values made twice: a training step of 4 layers of hidden 1024 over 1580 tokens 7.0 → 4.8 ms (the host), of
+    6 MoE layers over 12 075 tokens 60.8 → 58 to 60."""
+
+    @staticmethod
+    def forward(ctx, layer, meta, params, x, residual, *_params):
+        ctx.layer, ctx.meta, ctx.params = layer, meta, params
+        ctx.set_materialize_grads(False)
+        ctx.save_for_backward(x, residual)
+        return layer(x, residual, meta)
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, *grads):
+        ins = [None if t is None else t.detach().requires_grad_(need) for t, need in zip(ctx.saved_tensors, ctx.needs_input_grad[3:5])]
+        with torch.enable_grad():
+            outs = ctx.layer(*ins, replace(ctx.meta, values=False))
+        wanted = [t for t in ins if t is not None and t.requires_grad] + list(ctx.params)
+        given = [(o, g) for o, g in zip(outs, grads) if g is not None]
+        got = iter(torch.autograd.grad([o for o, _ in given], wanted, [g for _, g in given], allow_unused=True))
+        return (None, None, None, *(next(got) if t is not None and t.requires_grad else None for t in ins), *got)
+
+
+def _runs_again(layer, x, meta) -> bool:
+    """`_RunAgain` applies: a plain decoder layer on one rank, whose forward pass does not depend on whether gradients are recorded, and nobody looks on."""
+    if type(layer) is not DecoderLayer or not x.is_cuda:
+        return False
+    ps, mlp = layer.attn.ps, layer.mlp
+    if ps.tp_size > 1 or ps.ep_size > 1 or ps.cp_size > 1 or meta.record_topk is not None or meta.kv_cache is not None:
+        return False
+    parts = (layer, layer.attn, mlp)
+    if (type(layer.attn) is not Attention or type(mlp) not in (DenseFFN, MoEFFN) or any(getattr(m, "lora", None) is not None for m in parts)
+            or any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in parts)):
+        return False
+    return ops.taped_as_untaped(x, x.shape[0] * mlp.cfg.moe_topk / mlp.cfg.num_experts if isinstance(mlp, MoEFFN) else None)
+
+
 def _checkpoint(layer, x, residual, meta):
+    if _runs_again(layer, x, meta):
+        params = tuple(p for p in layer.parameters() if p.requires_grad)
+        if all(type(p) is nn.Parameter for p in params):
+            return _RunAgain.apply(layer, meta, params, x, residual, *params)
     from torch.utils.checkpoint import checkpoint
 
     if residual is None:

@@ -161,10 +161,23 @@ def gather_router_weights(probs, idx, normalize=True):
     return ref.gather_router_weights(probs, idx, normalize)
 
 
-def moe_ffn(x, w13, w2, topk_w, topk_idx):
+def moe_ffn(x, w13, w2, topk_w, topk_idx, values=True):
+    """`values` False: the result is not read, it only stands in the graph."""
     if x.is_cuda:
-        return _k().moe_ffn(x, w13, w2, topk_w, topk_idx)
+        return _k().moe_ffn(x, w13, w2, topk_w, topk_idx, values=values)
     return ref.moe_ffn(x, w13, w2, topk_w, topk_idx)
+
+
+def swiglu_ffn(x, w13, w2, values=True):
+    """swiglu(x · w13ᵀ) · w2ᵀ; `values` False: the result is not read, it only stands in the graph."""
+    if x.is_cuda:
+        return _k().swiglu_ffn(x, w13, w2, values)
+    return linear(linear_swiglu(x, w13), w2)
+
+
+def taped_as_untaped(x, pairs_per_expert=None) -> bool:
+    """True where a forward pass over these rows takes the same kernels with and without gradients."""
+    return x.is_cuda and _k().taped_as_untaped(x, pairs_per_expert)
 
 
 # ---- attention -------------------------------------------------------------------------------

@@ -180,10 +180,10 @@ void swiglu_fwd(const at::Tensor& in, at::Tensor& out, const c10::optional<at::T
         "mb_swiglu_fwd");
 }
 
-void swiglu_bwd(const at::Tensor& in, const at::Tensor& dout, at::Tensor& din, const c10::optional<at::Tensor>& rows) {
+void swiglu_bwd(const at::Tensor& in, const at::Tensor& dout, at::Tensor& din, const c10::optional<at::Tensor>& rows, const c10::optional<at::Tensor>& act) {
   c10::cuda::CUDAGuard g(in.device());
   const int64_t F = dout.size(-1), T = dout.numel() / std::max<int64_t>(F, 1);
-  check(mb_swiglu_bwd(in.data_ptr(), dout.data_ptr(), din.data_ptr(), T, F,
+  check(mb_swiglu_bwd(in.data_ptr(), dout.data_ptr(), din.data_ptr(), mptr(act), T, F,
                       rows.has_value() && rows->defined() ? rows->data_ptr<int>() : nullptr, cur_stream()),
         "mb_swiglu_bwd");
 }
@@ -290,7 +290,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("swiglu_fwd", &swiglu_fwd);
-  m.def("swiglu_bwd", &swiglu_bwd);
+  m.def("swiglu_bwd", &swiglu_bwd, py::arg("x"), py::arg("dout"), py::arg("dx"), py::arg("rows"), py::arg("act") = py::none());
   m.def("rope", &rope);
   m.def("qk_norm_rope_fwd", &qk_norm_rope_fwd);
   m.def("qk_norm_rope_bwd", &qk_norm_rope_bwd);

@@ -393,8 +393,10 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* in
   }
 }
 
-__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ dout,
-                                                         __nv_bfloat16* __restrict__ din, long long T, int F,
+// act (null, or in dout's place): the activation itself, for the gradient of the weight behind it.  Read once instead of twice: 11 791 rows of 9728:
+// 156 + 252 µs → 320.
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* dout,
+                                                         __nv_bfloat16* __restrict__ din, __nv_bfloat16* act, long long T, int F,
                                                          const int* __restrict__ rows_ptr) {
   const int nvec = F / 8;
   if (rows_ptr != nullptr) T = min(T, static_cast<long long>(*rows_ptr));
@@ -406,6 +408,12 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
     load8(in + t * 2 * F + v * 8, g);
     load8(in + t * 2 * F + F + v * 8, u);
     load8(dout + t * F + v * 8, d);
+    if (act != nullptr) {
+      float a[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) a[k] = g[k] / (1.f + __expf(-g[k])) * u[k];
+      store8(act + t * F + v * 8, a);
+    }
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const float s = 1.f / (1.f + __expf(-g[k]));
@@ -948,12 +956,12 @@ extern "C" int mb_swiglu_fwd(const void* in, void* out, long long T, int F, cons
                                      reinterpret_cast<const __nv_bfloat16*>(in), reinterpret_cast<__nv_bfloat16*>(out), T, F, rows_ptr));
 }
 
-extern "C" int mb_swiglu_bwd(const void* in, const void* dout, void* din, long long T, int F, const int* rows_ptr, cudaStream_t s) {
+extern "C" int mb_swiglu_bwd(const void* in, const void* dout, void* din, void* act, long long T, int F, const int* rows_ptr, cudaStream_t s) {
   if (T == 0) return 0;
   if (F % 8) return -1;
   swiglu_bwd_kernel<<<grid_for(T * (F / 8), 256), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(in),
                                                                 reinterpret_cast<const __nv_bfloat16*>(dout),
-                                                                reinterpret_cast<__nv_bfloat16*>(din), T, F, rows_ptr);
+                                                                reinterpret_cast<__nv_bfloat16*>(din), reinterpret_cast<__nv_bfloat16*>(act), T, F, rows_ptr);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -73,7 +73,7 @@ int mb_rmsnorm_bwd_static(const void* x, const void* w, const void* dy, const vo
 const char* mb_rmsnorm_bwd_static_strerror(int code);
 int mb_colsum(const float* partial, void* out, int R, int C, int out_fp32, cudaStream_t s);
 int mb_swiglu_fwd(const void* in, void* out, long long T, int F, const int* rows_ptr, cudaStream_t s);
-int mb_swiglu_bwd(const void* in, const void* dout, void* din, long long T, int F, const int* rows_ptr, cudaStream_t s);
+int mb_swiglu_bwd(const void* in, const void* dout, void* din, void* act, long long T, int F, const int* rows_ptr, cudaStream_t s);
 int mb_qk_norm_rope_fwd(const void* q, const void* k, long long q_stride, long long k_stride, const void* qw, const void* kw,
                         const int* positions, void* qo, void* ko, float* q_rstd, float* k_rstd, long long T, int Hq, int Hk, int D,
                         float theta, float eps, cudaStream_t s);

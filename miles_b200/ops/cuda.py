@@ -446,6 +446,35 @@ def add_rmsnorm(x, residual, w, eps=1e-6):
     return _apply(_AddRMSNorm, x, residual, w, eps)
 
 
+class _SwiGLUFFN(torch.autograd.Function):
+    """swiglu(x · W13ᵀ) · W2ᵀ that keeps the pre-activation alone: the backward makes the activation again in the kernel that differentiates it.
+    `values` False: nobody reads the result (only a backward follows), W2's product is left out."""
+
+    @staticmethod
+    def forward(ctx, x, w13, w2, values):
+        x2 = x.reshape(-1, x.shape[-1])
+        h13 = gemm_nt(x2, w13)
+        ctx.save_for_backward(x2, w13, w2, h13)
+        ctx.shp = x.shape
+        y = torch.empty(*x.shape[:-1], w2.shape[0], dtype=x.dtype, device=x.device)
+        if values:
+            act = torch.empty(h13.shape[0], w2.shape[1], dtype=x.dtype, device=x.device)
+            C.swiglu_fwd(h13, act, None)
+            gemm_nt(act, w2, out=y.view(-1, w2.shape[0]))
+        return y
+
+    @staticmethod
+    def backward(ctx, gy):
+        x2, w13, w2, h13 = ctx.saved_tensors
+        gy2 = _c(gy.reshape(-1, gy.shape[-1]))
+        act = gemm_nn(gy2, w2)                       # the gradient of the activation; replaced by the activation
+        dh13 = torch.empty_like(h13)
+        C.swiglu_bwd(h13, act, dh13, None, act)
+        need = ctx.needs_input_grad
+        return (gemm_nn(dh13, w13).view(ctx.shp) if need[0] else None, gemm_tn(dh13, x2) if need[1] else None,
+                gemm_tn(gy2, act) if need[2] else None, None)
+
+
 class _SwiGLU(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gate_up):
@@ -467,6 +496,21 @@ def swiglu(gate_up):
     if gate_up.dtype != BF16:
         return ref.swiglu(gate_up)
     return _apply(_SwiGLU, gate_up)
+
+
+def swiglu_ffn(x, w13, w2, values: bool = True):
+    """swiglu(x · w13ᵀ) · w2ᵀ.  `values` False: the result is not read, it only stands in the graph."""
+    if x.dtype != BF16 or w13.dtype != BF16 or w2.dtype != BF16 or MXFP8_LINEAR or not torch.is_grad_enabled():
+        return linear(linear_swiglu(x, w13), w2)                       # noqa: F821  (cuda_more)
+    return _SwiGLUFFN.apply(x, w13, w2, values)
+
+
+def taped_as_untaped(x, pairs_per_expert: float | None = None) -> bool:
+    """A forward pass over these rows takes the same kernels whether a backward follows or not: none of the forms for few rows, no weights that
+    a rollout engine registered quantised, no transform that an autograd function would handle."""
+    rows = x.numel() // x.shape[-1]
+    return (x.is_cuda and x.dtype == BF16 and rows > max(SMALL_M, GEMV_M) and not _MXFP8_WEIGHTS and not transformed()
+            and not torch.is_autocast_enabled("cuda") and (pairs_per_expert is None or pairs_per_expert > max(32.0, SMALL_MOE_AVG)))       # noqa: F821
 
 
 class _QKNormRope(torch.autograd.Function):

@@ -358,7 +358,7 @@ class _MoEFFN(torch.autograd.Function):
     """y[t] = Σ_j w[t,j] · W2[e]·swiglu(W13[e]·x[t]) with e = idx[t,j] − expert_offset ∈ [0, E_local) (others skipped)."""
 
     @staticmethod
-    def forward(ctx, x, w13, w2, topk_w, topk_idx, expert_offset, keep):
+    def forward(ctx, x, w13, w2, topk_w, topk_idx, expert_offset, keep, values):
         T, H = x.shape
         E, F2, _ = w13.shape
         F = F2 // 2
@@ -371,10 +371,15 @@ class _MoEFFN(torch.autograd.Function):
         x_perm = torch.empty(max_rows, H, dtype=x.dtype, device=x.device)
         publish_limit(LIMIT_MOE_PAIRS, x.shape[0] * k)
         C.moe_gather(x, x_perm, row_src, seg, k)
-        h1, y_perm = experts_forward(x_perm, w13, w2, seg, tile, keep=keep)        # bf16 grouped GEMMs, or block-scaled under the MXFP8 recipe
-        out = torch.empty(T, H, dtype=x.dtype, device=x.device)
-        C.moe_combine(y_perm, wf, dst_row, out, k)
         from . import cuda as _cuda
+
+        out = torch.empty(T, H, dtype=x.dtype, device=x.device)
+        if keep and not values and not _cuda.MXFP8_LINEAR:                         # only a backward follows: what it needs
+            h1, y_perm = torch.empty(max_rows, F2, dtype=x.dtype, device=x.device), None
+            C.gemm_grouped(x_perm, w13, h1, max_rows, F2, H, E, tile, False, 0)
+        else:
+            h1, y_perm = experts_forward(x_perm, w13, w2, seg, tile, keep=keep)    # bf16 grouped GEMMs, or block-scaled under the MXFP8 recipe
+            C.moe_combine(y_perm, wf, dst_row, out, k)
 
         # the gate weights' gradient ⟨dout, W2 · act⟩ is taken as ⟨dout · W2, act⟩: y is not needed, except where it is not W2 · act (quantised)
         ctx.save_for_backward(x_perm, w13, w2, wf, seg, tile, row_src, dst_row, h1, y_perm if _cuda.MXFP8_LINEAR else None)
@@ -412,10 +417,11 @@ class _MoEFFN(torch.autograd.Function):
         C.gemm_grouped(dh1, w13, dy_perm, max_rows, H, F2, E, tile, True, 0)              # dy_perm has been read: the input rows' gradient in its place
         dx = new(T, H)
         C.moe_combine(dy_perm, None, dst_row, dx, k)
-        return dx, dw13, dw2, dw_flat.view(T, k), None, None, None
+        return dx, dw13, dw2, dw_flat.view(T, k), None, None, None, None
 
 
-def moe_ffn(x, w13, w2, topk_w, topk_idx, expert_offset: int = 0):
+def moe_ffn(x, w13, w2, topk_w, topk_idx, expert_offset: int = 0, values: bool = True):
+    """`values` False: the result is not read, it only stands in the graph."""
     if x.dtype != BF16:
         return ref.moe_ffn(x, w13, w2, topk_w, topk_idx)
     T, k = topk_idx.shape
@@ -427,7 +433,7 @@ def moe_ffn(x, w13, w2, topk_w, topk_idx, expert_offset: int = 0):
     bt = small_moe_bt(topk_idx.numel(), w13.shape[0], w13, w2)
     if bt != 128 and x.shape[0]:
         return _moe_ffn_small(x, w13, w2, topk_w, topk_idx, int(expert_offset), bt)
-    return _apply(_MoEFFN, x, w13, w2, topk_w, topk_idx, int(expert_offset), torch.is_grad_enabled())
+    return _apply(_MoEFFN, x, w13, w2, topk_w, topk_idx, int(expert_offset), torch.is_grad_enabled(), values)
 
 
 # ---------------------------------------------------------------------------------------------

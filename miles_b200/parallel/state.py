@@ -254,9 +254,9 @@ class ParallelState:
         from . import tp
         return tp.all_gather_last_dim(x, self)
 
-    def moe_ffn(self, x, w13, w2, topk_w, topk_idx, num_experts):
+    def moe_ffn(self, x, w13, w2, topk_w, topk_idx, num_experts, values=True):
         if self.ep_size == 1:
-            return ops.moe_ffn(x, w13, w2, topk_w, topk_idx)
+            return ops.moe_ffn(x, w13, w2, topk_w, topk_idx, values)
         from . import ep
         return ep.expert_parallel_ffn(x, w13, w2, topk_w, topk_idx, num_experts, self)
 
