@@ -105,6 +105,21 @@ void moe_gemv(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, 
         "mb_moe_gemv");
 }
 
+// Experts of 9 to 64 tokens without a sort (moe_rows.cu): x [T, H], w13 [E, 2F, H], w2 [E, H, F], idx int32 and w fp32 [T, k], out [T, H]
+void moe_rows(const at::Tensor& x, const at::Tensor& w13, const at::Tensor& w2, const at::Tensor& idx, const at::Tensor& w, at::Tensor& out, int64_t offset) {
+  c10::cuda::CUDAGuard g(x.device());
+  const int64_t T = x.size(0), H = x.size(1), k = idx.size(1), E = w13.size(0), F = w2.size(2), n = std::min(E, T * k);
+  TORCH_CHECK(x.is_contiguous() && w13.is_contiguous() && w2.is_contiguous() && idx.is_contiguous() && w.is_contiguous() && out.is_contiguous() &&
+                  w13.size(1) == 2 * F && w13.size(2) == H && w2.size(0) == E && w2.size(1) == H && idx.sizes() == w.sizes() && idx.size(0) == T && out.sizes() == x.sizes(),
+              "moe_rows: shapes");
+  auto act = at::empty({T, n * F}, x.options());
+  auto slots = at::empty({1 + n}, x.options().dtype(at::kInt));
+  mb_count_launch(1);
+  check(mb_moe_rows(x.data_ptr(), w13.data_ptr(), w2.data_ptr(), idx.data_ptr<int>(), w.data_ptr<float>(), act.data_ptr(), slots.data_ptr<int>(), out.data_ptr(), T, k, E,
+                    offset, H, F, error_flag_for(x.device()).data_ptr<int>(), cur_stream()),
+        "mb_moe_rows");
+}
+
 void gemm_small_grouped(const at::Tensor& X, const at::Tensor& W, at::Tensor& C, int64_t rows, int64_t N, int64_t K, int64_t E,
                         const at::Tensor& tile_expert, const c10::optional<at::Tensor>& used_rows, int64_t bt) {
   c10::cuda::CUDAGuard g(X.device());
@@ -285,6 +300,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_gemv", &moe_gemv, py::arg("x"), py::arg("w13"), py::arg("w2"), py::arg("topk_idx"), py::arg("topk_w"), py::arg("act"), py::arg("out"),
         py::arg("expert_offset"), py::arg("limit") = 0.0, py::arg("alpha") = 0.0, py::arg("shift") = 1.0, py::arg("ungated") = false);
   m.def("gemm_small_grouped", &gemm_small_grouped);
+  m.def("moe_rows", &moe_rows);
   m.def("gemm_grouped_wgrad", &gemm_grouped_wgrad);
 #ifndef MB_SERVE_SUBSET      // the training and grouped-query kernels of elementwise.cu
   m.def("rmsnorm_fwd", &rmsnorm_fwd);

@@ -34,7 +34,7 @@ namespace rows {
 static constexpr int BMW = 128;     // weight rows (output features) per tile
 static constexpr int BK = 64;
 static constexpr int kMaxSplit = 8;
-static constexpr int kSms = 148, kWideClusters = 12;
+static constexpr int kSms = 148, kWideClusters = 12, kMaxExperts = 256;
 
 struct Params {
   int tokens, N, K;
@@ -46,6 +46,8 @@ struct Params {
   int static_w;
   int stages;
   int* error_flag;
+  const int* slots;                   // experts: how many there are and which, see below
+  int steps_per;                      // experts: 64-deep steps of one expert's share of the reduction
 };
 
 template <int BT>
@@ -62,7 +64,8 @@ __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void st_cluster(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 
-template <int BT, int split>
+// kExperts: the weights are [E, N, K_e] and the reduction runs over the experts of `slots` one after another (X has their columns in that order).
+template <int BT, int split, bool kExperts>
 __global__ void __launch_bounds__(192, 2)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, Params p) {
   using L = Layout<BT>;
@@ -98,14 +101,25 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   if (split > 1) cluster_arrive();                 // "my buffer exists": waited for before the first remote store
   pdl_trigger();
 
-  const int total_kb = (p.K + BK - 1) / BK, per = (total_kb + split - 1) / split;
+  __shared__ int slot_e[kExperts ? kMaxExperts : 1];
+  int total_kb = (p.K + BK - 1) / BK;
+  if (kExperts) {                                  // nothing is known before the kernel in front has written the list
+    pdl_wait();
+    const int n = p.slots[0];
+    for (int i = threadIdx.x; i < n; i += 192) slot_e[i] = p.slots[1 + i];
+    __syncthreads();
+    total_kb = n * p.steps_per;
+  }
+  const int per = (total_kb + split - 1) / split;
   const int kb0 = slice * per, kbs = max(0, min(per, total_kb - kb0));
 
   if (warp == 0) {
     if (elect_one()) {
       auto load_w = [&](int kb, int stage) {
         mbar_expect_tx(&full_bar[stage], L::kStageBytes);
-        tma_load_2d(smem_a + stage * L::kABytes, &tmap_w, &full_bar[stage], (kb0 + kb) * BK, n_blk * BMW);
+        const int at = kb0 + kb;
+        if (kExperts) tma_load_2d(smem_a + stage * L::kABytes, &tmap_w, &full_bar[stage], at % p.steps_per * BK, slot_e[at / p.steps_per] * p.N + n_blk * BMW);
+        else tma_load_2d(smem_a + stage * L::kABytes, &tmap_w, &full_bar[stage], at * BK, n_blk * BMW);
       };
       auto load_x = [&](int kb, int stage) { tma_load_2d(smem_b + stage * L::kBBytes, &tmap_x, &full_bar[stage], (kb0 + kb) * BK, 0); };
       const int early = min(kbs, stages);
@@ -209,25 +223,37 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   }
 }
 
-template <int BT, int split>
+template <int BT, int split, bool kExperts>
 static int launch_as(const CUtensorMap& tw, const CUtensorMap& tx, Params p, cudaStream_t s) {
   using L = Layout<BT>;
-  static const cudaError_t configured = cudaFuncSetAttribute(gemm_rows_kernel<BT, split>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total(L::kDeep));
+  constexpr int kDeep = kExperts && BT == 64 ? L::kDeep - 1 : L::kDeep;        // room for the list of experts
+  auto kern = gemm_rows_kernel<BT, split, kExperts>;
+  static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total(kDeep));
   if (configured != cudaSuccess) return static_cast<int>(configured);
   const int tiles = (p.N + BMW - 1) / BMW;
   // a CTA with an SM to itself has twice the bytes in flight: the ring is deep where all clusters fit that way.  Eight neighbouring SMs are
   // found 12 times at least; 16 such clusters took two waves (2048 × 4096, 9 tokens: 9.0 µs, 6.2 for 16 clusters of four)
-  p.stages = tiles <= (split == kMaxSplit ? kWideClusters : kSms / split) ? L::kDeep : L::kShallow;
-  return static_cast<int>(launch_pdl_cluster(gemm_rows_kernel<BT, split>, dim3(tiles * split), dim3(192), split, L::total(p.stages), s, tw, tx, p));
+  p.stages = tiles <= (split == kMaxSplit ? kWideClusters : kSms / split) ? kDeep : L::kShallow;
+  return static_cast<int>(launch_pdl_cluster(kern, dim3(tiles * split), dim3(192), split, L::total(p.stages), s, tw, tx, p));
 }
 
 template <int BT>
 static int launch(const CUtensorMap& tw, const CUtensorMap& tx, const Params& p, int split, cudaStream_t s) {
   switch (split) {
-    case 1: return launch_as<BT, 1>(tw, tx, p, s);
-    case 2: return launch_as<BT, 2>(tw, tx, p, s);
-    case 4: return launch_as<BT, 4>(tw, tx, p, s);
-    default: return launch_as<BT, 8>(tw, tx, p, s);
+    case 1: return launch_as<BT, 1, false>(tw, tx, p, s);
+    case 2: return launch_as<BT, 2, false>(tw, tx, p, s);
+    case 4: return launch_as<BT, 4, false>(tw, tx, p, s);
+    default: return launch_as<BT, 8, false>(tw, tx, p, s);
+  }
+}
+
+template <int BT>
+static int launch_experts(const CUtensorMap& tw, const CUtensorMap& tx, const Params& p, int split, cudaStream_t s) {
+  switch (split) {
+    case 1: return launch_as<BT, 1, true>(tw, tx, p, s);
+    case 2: return launch_as<BT, 2, true>(tw, tx, p, s);
+    case 4: return launch_as<BT, 4, true>(tw, tx, p, s);
+    default: return launch_as<BT, 8, true>(tw, tx, p, s);
   }
 }
 
@@ -317,10 +343,34 @@ extern "C" int mb_gemm_rows(const void* X, const void* W, void* C, int tokens, i
   if (r) return 1000 + r;
   r = make_tmap_bf16_2d(&tx, X, tokens, K, ldx, bt, rows::BK);
   if (r) return 2000 + r;
-  const rows::Params p{tokens, N, K, C, ldc, out_fp32, reinterpret_cast<const __nv_bfloat16*>(bias), row_scale, static_w, 0, error_flag};
+  const rows::Params p{tokens, N, K, C, ldc, out_fp32, reinterpret_cast<const __nv_bfloat16*>(bias), row_scale, static_w, 0, error_flag, nullptr, 0};
   switch (bt) {
     case 16: return rows::launch<16>(tw, tx, p, split, s);
     case 32: return rows::launch<32>(tw, tx, p, split, s);
     default: return rows::launch<64>(tw, tx, p, split, s);
+  }
+}
+
+// C[tokens, N] bf16 = Σ_i X[tokens, i · F ..] · W[e_i]ᵀ over the slots[0] ≤ n_max experts e_i = slots[1 + i]: X [tokens, n_max · F], W [E, N, F], F a multiple of 64.
+extern "C" int mb_gemm_rows_experts(const void* X, const void* W, void* C, int tokens, int N, int F, int E, int n_max, const int* slots, int* error_flag,
+                                    cudaStream_t s) {
+  using namespace mb;
+  if (tokens <= 0 || N <= 0) return 0;
+  if (tokens > 64 || F % rows::BK || E > rows::kMaxExperts) return -2;
+  const int bt = tokens <= 16 ? 16 : tokens <= 32 ? 32 : 64;
+  CUtensorMap tw, tx;
+  int r = make_tmap_bf16_2d(&tw, W, static_cast<long long>(E) * N, F, F, rows::BMW, rows::BK);
+  if (r) return 1000 + r;
+  r = make_tmap_bf16_2d(&tx, X, tokens, static_cast<long long>(n_max) * F, static_cast<long long>(n_max) * F, bt, rows::BK);
+  if (r) return 2000 + r;
+  const rows::Params p{tokens, N, 0, C, N, 0, nullptr, nullptr, 0, 0, error_flag, slots, F / rows::BK};
+  // two CTAs per SM: their prologue runs beside the kernel in front (16 tiles, 50 MB, 16 / 61 tokens with the norm in front of it: eight slices 14.2 / 17.1 µs,
+  // four with an SM each 18 / 21)
+  const int tiles = (N + rows::BMW - 1) / rows::BMW;
+  const int split = tiles * 8 <= 2 * rows::kSms ? 8 : tiles * 4 <= 2 * rows::kSms ? 4 : tiles * 2 <= 2 * rows::kSms ? 2 : 1;
+  switch (bt) {
+    case 16: return rows::launch_experts<16>(tw, tx, p, split, s);
+    case 32: return rows::launch_experts<32>(tw, tx, p, split, s);
+    default: return rows::launch_experts<64>(tw, tx, p, split, s);
   }
 }

@@ -21,6 +21,10 @@ int mb_gemm_rows(const void* X, const void* W, void* C, int tokens, int N, int K
                  const void* bias, const float* row_scale, int split, int static_w, int* error_flag, cudaStream_t s);
 int mb_norm_rows(const void* x, const void* residual, const void* w, float eps, int T, int K, void* scaled, float* rstd, void* sum, void* normed,
                  cudaStream_t s);
+int mb_gemm_rows_experts(const void* X, const void* W, void* C, int tokens, int N, int F, int E, int n_max, const int* slots, int* error_flag, cudaStream_t s);
+// ---- moe_rows.cu ----
+int mb_moe_rows(const void* x, const void* w13, const void* w2, const int* topk_idx, const float* topk_w, void* act, int* slots, void* out, int T, int k, int E,
+                int offset, int H, int F, int* error_flag, cudaStream_t s);
 int mb_gemm_bf16_splitk(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                         int out_fp32, int accumulate, const void* bias, int split_k, float* ws, int* counters, int* error_flag,
                         cudaStream_t stream);

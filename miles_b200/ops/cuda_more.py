@@ -238,6 +238,18 @@ def few_token_experts(x, w13, T: int, k: int, ungated: bool = False) -> bool:
             and 65536 + max(8 * (2 * x.shape[1] + 64), T * k * (2 * F + 64)) <= 200 * 1024 and 67584 + (T * k + 1) * (2 * F + 64) <= 210 * 1024)
 
 
+def all_token_experts(x, w13, w2, T: int, k: int) -> bool:
+    """A decode step's experts without a sort (moe_rows.cu): every expert with some token multiplies all of them.  Up to 32 tokens always, up to 64 where
+    an expert has more than 8: beyond that the tokens that did not choose it are too much of what each CTA reads.  µs of a layer of hidden 2048 and 768
+    features, 8 choices, sorted / all: 16 experts, 9, 32, 64 tokens 42.2 / 32.6, 43.1 / 36.6, 46.9 / 42.0; 64 experts 88 / 75, 113 / 105, 114 / 118; 128
+    experts 104 / 91, 178 / 174, 204 / 216.  Not where sums over the features have to be a single product's (MILES_SPLIT_K)."""
+    from . import cuda as _cuda
+
+    E = w13.shape[0]
+    return (x.dtype == BF16 and 0 < T <= min(64, _cuda.SMALL_M) and (T <= 32 or T * k > 8 * E) and _cuda.SPLIT_K and SMALL_MOE_AVG > 0 and E <= 256
+            and x.shape[1] % 8 == 0 and w2.shape[2] % 64 == 0 and not torch.is_grad_enabled() and not transformed())
+
+
 def _glu_in_place() -> bool:
     """The activation may be formed in the bf16 product's epilogue: no block-scaled projection stands in its place, and nothing that
     the autograd functions would refuse (forward-mode tangents, function transforms) is under way."""
@@ -429,6 +441,10 @@ def moe_ffn(x, w13, w2, topk_w, topk_idx, expert_offset: int = 0, values: bool =
         act = torch.empty(T * k, w13.shape[1] // 2, dtype=x.dtype, device=x.device)
         out = torch.empty_like(x)
         C.moe_gemv(_c(x), _c(w13), _c(w2), _c(topk_idx.to(torch.int32)), _c(topk_w.float()), act, out, int(expert_offset))
+        return out
+    if all_token_experts(x, w13, w2, T, k):
+        out = torch.empty_like(x)
+        C.moe_rows(_c(x), _c(w13), _c(w2), _c(topk_idx.to(torch.int32)), _c(topk_w.float()), out, int(expert_offset))
         return out
     bt = small_moe_bt(topk_idx.numel(), w13.shape[0], w13, w2)
     if bt != 128 and x.shape[0]:
