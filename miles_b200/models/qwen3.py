@@ -131,13 +131,20 @@ class Attention(nn.Module):
         T = qkv.shape[0]
         q, k, v = qkv.split([self.hq * self.d, self.hkv * self.d, self.hkv * self.d], dim=-1)
         q, k, v = q.view(T, self.hq, self.d), k.view(T, self.hkv, self.d), v.view(T, self.hkv, self.d)
+        o = None
         if meta.kv_cache is not None:
             kc, vc = meta.kv_cache[layer]
-            q, k = ops.qk_norm_rope_cache(q, k, v, self.q_norm, self.k_norm, meta.positions, cfg.rope_theta, cfg.rms_eps,
-                                          kc, vc, meta.slot_mapping)
+            if meta.cu_seqlens is None and meta.q_lens is None:
+                o = ops.decode_attention(q, k, v, self.q_norm, self.k_norm, meta.positions, cfg.rope_theta, cfg.rms_eps, kc, vc, meta.slot_mapping,
+                                         meta.block_table, meta.seq_lens)
+            if o is None:
+                q, k = ops.qk_norm_rope_cache(q, k, v, self.q_norm, self.k_norm, meta.positions, cfg.rope_theta, cfg.rms_eps,
+                                              kc, vc, meta.slot_mapping)
         else:
             q, k = ops.qk_norm_rope(q, k, self.q_norm, self.k_norm, meta.positions, cfg.rope_theta, cfg.rms_eps)
-        if meta.cu_seqlens is not None:
+        if o is not None:
+            pass                                                          # a decode step of few rows: rotation, cache write and attention in one launch
+        elif meta.cu_seqlens is not None:
             # training, or an engine prefill that starts from an empty cache: attend within the new tokens
             if self.ps.cp_size > 1 and not self.ps.is_ulysses_cp:
                 # ring (zigzag pieces, K/V travel round the group) or all-gather context parallelism

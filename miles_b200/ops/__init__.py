@@ -198,6 +198,13 @@ def kv_cache_write(k, v, k_cache, v_cache, slot_mapping):
     vc[slot_mapping.long()] = v.detach().to(vc.dtype)
 
 
+def decode_attention(q, k, v, q_w, k_w, positions, theta, eps, k_cache, v_cache, slot_mapping, block_table, seq_lens):
+    """`qk_norm_rope_cache` and `paged_attention` of a decode step in one launch, or None where that form does not apply."""
+    if not q.is_cuda:
+        return None
+    return _k().decode_attention(q, k, v, q_w, k_w, positions, theta, eps, k_cache, v_cache, slot_mapping, block_table, seq_lens)
+
+
 def paged_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens=None, max_q_len=1, extend=None):
     if q.is_cuda:
         return _k().paged_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens, max_q_len, extend)

@@ -104,6 +104,22 @@ void paged_decode(const at::Tensor& q, const at::Tensor& kc, const at::Tensor& v
         "mb_paged_decode");
 }
 
+// qk_norm_rope_cache and the paged decode attention behind it in one launch (decode_attend.cuh): q, k, v [B, heads, 128], tokens anywhere apart → out [B, Hq, 128]
+void decode_attend(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const c10::optional<at::Tensor>& qw, const c10::optional<at::Tensor>& kw,
+                   const at::Tensor& positions, double theta, double eps, at::Tensor& kc, at::Tensor& vc, const at::Tensor& slots, const at::Tensor& block_table,
+                   const at::Tensor& seq_lens, at::Tensor& out, double scale, int64_t split, at::Tensor& err) {
+  c10::cuda::CUDAGuard g(q.device());
+  TORCH_CHECK(kc.is_contiguous() && vc.is_contiguous() && block_table.is_contiguous() && out.is_contiguous() && positions.is_contiguous() && slots.is_contiguous() &&
+                  seq_lens.is_contiguous(),
+              "decode_attend: contiguous caches and tables");
+  auto opt = [](const c10::optional<at::Tensor>& t) -> const void* { return t.has_value() && t->defined() ? t->data_ptr() : nullptr; };
+  check(mb_decode_attend(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), opt(qw), opt(kw), positions.data_ptr<int>(), theta, eps,
+                         kc.data_ptr(), vc.data_ptr(), reinterpret_cast<const long long*>(slots.data_ptr<int64_t>()), block_table.data_ptr<int>(),
+                         seq_lens.data_ptr<int>(), out.data_ptr(), q.size(0), block_table.size(1), kc.size(1), kc.size(0) * kc.size(1), q.size(1), kc.size(2), q.size(2),
+                         scale, split, err.data_ptr<int>(), cur_stream()),
+        "mb_decode_attend");
+}
+
 void paged_decode_tiles(const at::Tensor& q, const at::Tensor& kc, const at::Tensor& vc, const at::Tensor& block_table, const at::Tensor& seq_lens,
                         at::Tensor& out, double scale, const at::Tensor& err) {
   c10::cuda::CUDAGuard g(q.device());
@@ -172,6 +188,7 @@ void register_more(pybind11::module& m) {
   m.def("head_grad", &head_grad);
   m.def("paged_decode", &paged_decode);
   m.def("paged_decode_tiles", &paged_decode_tiles);
+  m.def("decode_attend", &decode_attend);
   register_fabric(m);
   register_extra(m);
 #endif

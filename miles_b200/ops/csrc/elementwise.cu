@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "rope.cuh"
 #include "launch.h"
 #include "debug.cuh"
 #include "pdl.cuh"
@@ -429,49 +430,21 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
 // Per-head RMSNorm (optional) + NeoX rotary embedding on q and k, in one pass.  One warp per (token, head).
 // Layout [T, heads, D]; pairs are (i, i + D/2).  D ∈ {64, 128}.
 // ---------------------------------------------------------------------------------------------
-// (x1, x2) turned by the angle of cosine c and sine s.  The contraction is spelled out: left to the compiler, two kernels round the same token in
-// two ways.
-__device__ __forceinline__ float2 rotate_pair(float x1, float x2, float c, float s) {
-  return make_float2(__fmaf_rn(x1, c, -__fmul_rn(x2, s)), __fmaf_rn(x1, s, __fmul_rn(x2, c)));
-}
-
 template <int D>
 __device__ __forceinline__ void norm_rope_row(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst,
                                               const __nv_bfloat16* __restrict__ w, float pos, float log2_theta, float eps,
                                               float* rstd_out, int lane, __nv_bfloat16* __restrict__ dst2 = nullptr) {
   constexpr int EPL = D / 64;  // elements per lane in each half
-  float a[EPL], b[EPL];
-  float ss = 0.f;
-#pragma unroll
-  for (int e = 0; e < EPL; ++e) {
-    a[e] = __bfloat162float(src[lane * EPL + e]);
-    b[e] = __bfloat162float(src[D / 2 + lane * EPL + e]);
-    ss += a[e] * a[e] + b[e] * b[e];
-  }
-  float rstd = 1.f;
-  if (w != nullptr) {
-    ss = warp_sum(ss);
-    rstd = rsqrtf(ss / D + eps);
-    if (rstd_out != nullptr && lane == 0) *rstd_out = rstd;
-  }
+  __nv_bfloat16 o1[EPL], o2[EPL];
+  norm_rope_values<D>(src, w, pos, log2_theta, eps, rstd_out, lane, o1, o2);
 #pragma unroll
   for (int e = 0; e < EPL; ++e) {
     const int j = lane * EPL + e;
-    float x1 = a[e], x2 = b[e];
-    if (w != nullptr) {
-      x1 = __bfloat162float(__float2bfloat16(x1 * rstd * __bfloat162float(w[j])));
-      x2 = __bfloat162float(__float2bfloat16(x2 * rstd * __bfloat162float(w[D / 2 + j])));
-    }
-    const float inv_freq = exp2f(-log2_theta * (2.f * j) / D);
-    float s, c;
-    sincosf(pos * inv_freq, &s, &c);
-    const float2 r = rotate_pair(x1, x2, c, s);
-    const __nv_bfloat16 o1 = __float2bfloat16(r.x), o2 = __float2bfloat16(r.y);
-    dst[j] = o1;
-    dst[D / 2 + j] = o2;
+    dst[j] = o1[e];
+    dst[D / 2 + j] = o2[e];
     if (dst2 != nullptr) {
-      dst2[j] = o1;
-      dst2[D / 2 + j] = o2;
+      dst2[j] = o1[e];
+      dst2[D / 2 + j] = o2[e];
     }
   }
 }

@@ -106,6 +106,9 @@ int mb_attn_delta(const void* o, const void* dout, float* delta, int total_token
 int mb_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse, float* delta,
                  void* dq, void* dk, void* dv, const int* cu_seqlens, int batch, int max_seqlen, int total_tokens, long long q_stride,
                  long long k_stride, long long v_stride, int Hq, int Hkv, int D, float scale, int causal, cudaStream_t s);
+int mb_decode_attend(const void* q, const void* k, const void* v, long long q_stride, long long k_stride, long long v_stride, const void* qw, const void* kw,
+                     const int* positions, float theta, float eps, void* kc, void* vc, const long long* slots, const int* block_table, const int* seq_lens, void* out,
+                     int batch, int max_blocks, int block_size, int cache_rows, int Hq, int Hkv, int D, float scale, int split, int* error_flag, cudaStream_t s);
 int mb_paged_decode_tiles(const void* q, const void* kc, const void* vc, const int* block_table, const int* seq_lens, void* out, float* part_o,
                           float* part_ml, int* plan, int batch, int max_blocks, int block_size, int cache_rows, int Hq, int Hkv, int D,
                           float scale, int ctas, int* error_flag, cudaStream_t s);

@@ -20,6 +20,7 @@
 #include "mma_sync.cuh"
 #include "pdl.cuh"
 #include "ptx.cuh"
+#include "rope.cuh"
 
 namespace mb {
 int make_tmap_bf16_2d(CUtensorMap* out, const void* base, long long rows, long long cols, long long ld, int box_rows, int box_cols);
@@ -658,6 +659,8 @@ static int launch_tiles(const bf16* q, const void* kc, const void* vc, const int
 
 }  // namespace mbpd
 
+#include "decode_attend.cuh"
+
 using namespace mbpd;
 
 MB_DEFINE_BOUNDS_API(mb_paged_bounds)
@@ -750,4 +753,28 @@ extern "C" int mb_paged_decode_tiles(const void* q, const void* kc, const void* 
     return launch_tiles<64>(Q, kc, vc, block_table, seq_lens, O, part_o, part_ml, plan, batch, max_blocks, block_size, cache_rows, Hq, Hkv, scale, ctas,
                             error_flag, s);
   return -1;
+}
+
+// See decode_attend.cuh.  q, k, v: the step's projections [batch, heads, 128] bf16, `*_stride` elements between tokens; qw, kw: norm weights or null; slots[b]: where the
+// new key and value go (< 0: nowhere); pages of a multiple of 16 tokens; cache_rows: pages × block_size.  split: CTAs per (request, KV head), 1 to 16.
+extern "C" int mb_decode_attend(const void* q, const void* k, const void* v, long long q_stride, long long k_stride, long long v_stride, const void* qw,
+                                const void* kw, const int* positions, float theta, float eps, void* kc, void* vc, const long long* slots, const int* block_table,
+                                const int* seq_lens, void* out, int batch, int max_blocks, int block_size, int cache_rows, int Hq, int Hkv, int D, float scale,
+                                int split, int* error_flag, cudaStream_t s) {
+  if (batch == 0) return 0;
+  if (D != 128 || Hq % Hkv || Hq / Hkv > 8 || block_size % kDaKeys || split < 1 || split > kDaMaxSplit || batch > 65535) return -2;
+  CUtensorMap tk, tv;
+  int rc = mb::make_tmap_bf16_2d(&tk, kc, cache_rows, static_cast<long long>(Hkv) * D, static_cast<long long>(Hkv) * D, kDaKeys, 64);
+  if (rc) return 1000 + rc;
+  rc = mb::make_tmap_bf16_2d(&tv, vc, cache_rows, static_cast<long long>(Hkv) * D, static_cast<long long>(Hkv) * D, kDaKeys, 64);
+  if (rc) return 2000 + rc;
+  static const cudaError_t configured = [] {
+    cudaError_t e = cudaFuncSetAttribute(decode_attend_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, DaSmem<128>::total);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(decode_attend_kernel<128>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  }();
+  if (configured != cudaSuccess) return static_cast<int>(configured);
+  auto b = [](const void* x) { return reinterpret_cast<const bf16*>(x); };
+  const DecodeAttend p{b(q), b(k), b(v), q_stride, k_stride, v_stride, b(qw), b(kw), positions, block_table, seq_lens, slots, reinterpret_cast<bf16*>(kc),
+                       reinterpret_cast<bf16*>(vc), reinterpret_cast<bf16*>(out), max_blocks, block_size, cache_rows, Hq, Hkv, split, log2f(theta), eps, scale, error_flag};
+  return static_cast<int>(mb::launch_pdl_cluster(decode_attend_kernel<128>, dim3(split, Hkv, batch), dim3(kDaWarps * 32), split, DaSmem<128>::total, s, tk, tv, p));
 }

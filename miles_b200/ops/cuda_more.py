@@ -7,7 +7,7 @@ import os
 import torch
 
 from . import reference as ref
-from .cuda import BF16, LIMIT_KV_BLOCKS, LIMIT_MOE_PAIRS, C, _apply, _c, gemm_nn, gemm_nt, gemm_tn, publish_limit, transformed
+from .cuda import BF16, LIMIT_KV_BLOCKS, LIMIT_KV_SLOTS, LIMIT_MOE_PAIRS, C, _apply, _c, gemm_nn, gemm_nt, gemm_tn, publish_limit, transformed
 
 # ---------------------------------------------------------------------------------------------
 # attention
@@ -97,6 +97,39 @@ def extend_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens, extend=
     lse = torch.empty(Hq, T, dtype=torch.float32, device=q.device)
     C.flash_fwd_tc(q, kk, vv, o, lse, extend["cu_q"], max_q, 1.0 / math.sqrt(D), True, C.error_flag(q), extend["cu_k"])
     return o
+
+
+# The one-launch form of a decode step's attention takes up to so many (request, KV head) segments with so many CTAs each: one of the chip's waves, and no more
+# than an SM and a half of each, because the projection behind brings its weights to the SMs' memory meanwhile.  µs of a step of 8 layers, three launches / 6,
+# 7, 8, 12 CTAs per segment: 16 segments of 700 to 3000 keys 606 / 586, 581, 576, 565; 24 of 300 to 900 596 / 585, 587, 582, 635; 28 of 128 to 4096 676 /
+# 649, 648, 634, 657; 32 of 300 to 1500 606 / 594, 596, 615, 649, of 128 to 4096 658 / 635, 635, 621, 659; 4 and 8 segments 8 / 16 CTAs 660 / 645 (12 layers)
+# and 547 / 523.  Beyond, even shares of all tiles: 40 of 128 to 4096 667 / 697 with 8, 687 with 4.
+_ATTEND_SEGMENTS = 32
+
+
+def _attend_split(segments: int) -> int:
+    return 16 if segments <= 8 else 12 if segments <= 18 else 8 if segments <= 28 else 7
+
+
+def decode_attention(q, k, v, q_w, k_w, positions, theta, eps, k_cache, v_cache, slot_mapping, block_table, seq_lens):
+    """A decode step's attention from its projections (one new token per request): norm and rotation of q and k, the cache write of (k, v) and attention over the
+    paged cache, in one launch for few (request, KV head) segments; None where that form does not apply."""
+    B, Hq, D = q.shape
+    Hkv = k.shape[1]
+    segments = B * Hkv
+    if (not _DECODE_BY_TILES or not 0 < segments <= _ATTEND_SEGMENTS or D != 128 or q.dtype != BF16 or k_cache.dtype != BF16 or Hq % Hkv or Hq // Hkv not in (1, 2, 4, 8)
+            or torch.is_grad_enabled() or transformed() or k_cache.shape[1] % 16 or k_cache.shape[2] != Hkv or not k_cache.is_contiguous() or not v_cache.is_contiguous()
+            or (q_w is None) != (k_w is None) or any(t.stride(2) != 1 or t.stride(1) != D for t in (q, k, v)) or k_cache.data_ptr() % 16 or v_cache.data_ptr() % 16
+            or positions.dtype != torch.int32 or slot_mapping.dtype != torch.int64 or block_table.dtype != torch.int32 or seq_lens.dtype != torch.int32
+            or not all(t.is_contiguous() for t in (positions, slot_mapping, block_table, seq_lens)) or positions.numel() != B or slot_mapping.numel() != B):
+        return None
+    publish_limit(LIMIT_KV_SLOTS, k_cache.shape[0] * k_cache.shape[1])
+    publish_limit(LIMIT_KV_BLOCKS, k_cache.shape[0])
+    out = torch.empty(B, Hq, D, dtype=q.dtype, device=q.device)
+    split = _attend_split(segments)
+    C.decode_attend(q, k, v, q_w, k_w, positions, float(theta), float(eps), k_cache, v_cache, slot_mapping, block_table, seq_lens, out, 1.0 / math.sqrt(D), split,
+                    C.error_flag(q))
+    return out
 
 
 def paged_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens=None, max_q_len=1, extend=None):
