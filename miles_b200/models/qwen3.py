@@ -269,8 +269,8 @@ class DecoderLayer(nn.Module):
             logits, residual, hn = ops.add_rmsnorm_linear(h, residual, self.ln2, self.eps, mlp.router, want_normed=True,
                                                           out_fp32=True)
             return mlp(hn, meta, self.layer, logits=logits), residual
-        h13, residual, _ = ops.add_rmsnorm_linear(h, residual, self.ln2, self.eps, mlp.w13)
-        return ops.linear(ops.swiglu(h13), mlp.w2), residual
+        h, residual = ops.add_rmsnorm_swiglu(h, residual, self.ln2, self.eps, mlp.w13)
+        return ops.linear(h, mlp.w2), residual
 
     def _routes_few_tokens(self, h, meta: ForwardMeta) -> bool:
         mlp = self.mlp

@@ -85,6 +85,12 @@ def add_rmsnorm_linear(x, residual, norm_w, eps, w, bias=None, want_normed=False
     return y, (x if res is None else res), xn
 
 
+def add_rmsnorm_swiglu(x, residual, norm_w, eps, w):
+    """(swiglu(rmsnorm(x + residual) · wᵀ), x + residual), only where `few_token_decode` holds."""
+    y, res = _k().add_rmsnorm_swiglu(x, residual, norm_w, eps, w)
+    return y, (x if res is None else res)
+
+
 def add_rmsnorm(x, residual, w, eps=1e-6):
     """(x + residual) → (rmsnorm(sum), sum); residual None means x starts the stream."""
     if residual is None:

@@ -55,11 +55,11 @@ void gemm_splitk(const at::Tensor& A, const at::Tensor& B, at::Tensor& C, int64_
 
 // tokens ≤ 64, weight rows on the 128-row MMA side, `split` CTAs of a cluster per 128 of them (gemm_rows.cu)
 void gemm_rows(const at::Tensor& X, const at::Tensor& W, at::Tensor& C, int64_t tokens, int64_t N, int64_t K, int64_t ldc,
-               const c10::optional<at::Tensor>& bias, int64_t split, bool static_w, const c10::optional<at::Tensor>& row_scale) {
+               const c10::optional<at::Tensor>& bias, int64_t split, bool static_w, const c10::optional<at::Tensor>& row_scale, bool glu) {
   c10::cuda::CUDAGuard g(X.device());
   int* ef = error_flag_for(X.device()).data_ptr<int>();
   check(mb_gemm_rows(X.data_ptr(), W.data_ptr(), C.data_ptr(), tokens, N, K, K, K, ldc, C.scalar_type() == at::kFloat, cptr(bias),
-                     static_cast<const float*>(cptr(row_scale)), split, static_w, ef, cur_stream()),
+                     static_cast<const float*>(cptr(row_scale)), split, static_w, glu, ef, cur_stream()),
         "mb_gemm_rows");
 }
 
@@ -291,7 +291,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm);
   m.def("gemm_splitk", &gemm_splitk);
   m.def("gemm_rows", &gemm_rows, py::arg("x"), py::arg("w"), py::arg("out"), py::arg("tokens"), py::arg("N"), py::arg("K"), py::arg("ldc"), py::arg("bias"),
-        py::arg("split"), py::arg("static_w"), py::arg("row_scale") = py::none());
+        py::arg("split"), py::arg("static_w"), py::arg("row_scale") = py::none(), py::arg("glu") = false);
   m.def("norm_rows", &norm_rows);
   m.def("gemm_grouped", &gemm_grouped);
   m.def("gemm_glu", &gemm_glu);

@@ -19,6 +19,8 @@
 // (72 to 90 KB in flight each), so up to 296 tiles × slices run at once and 152 tiles do not become two waves; where all of them fit with an
 // SM each, the ring is as deep as the SM allows.  The earlier forms were
 // 128-row token tiles (3/4 padding) with 64 columns per CTA, whose sums over K met in global memory behind atomic counters for ≤ 32 tokens.
+// gate · up where the accumulator is read (kGlu) instead of a kernel behind: decode steps of 8 layers, hidden 1024, 12 / 30 / 60 rows 358 / 446 / 506 → 354 / 440 /
+// 500 µs, hidden 2560, 12 layers, 19 rows 1054 → 1036.
 // Measured, weights from memory, 9 / 19 / 61 tokens against the 128-row tiles: 5120 × 2048 15.4 / 14.9 / 8.8 → 6.2 / 6.3 / 8.4 µs,
 // 2048 × 4096 17.0 / 13.0 / 13.1 → 6.2 / 6.8 / 8.2, 2560 × 9728 26.6 / 26.7 / 26.7 → 11.1 / 11.7 / 13.9 (7.7 at the memory's speed).
 #include "launch.h"
@@ -56,8 +58,8 @@ struct Layout {
   static constexpr int kABytes = BMW * BK * 2;         // weights: 16 KB
   static constexpr int kBBytes = BT * BK * 2;          // tokens: 2 / 4 / 8 KB
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kSumBytes = BT * BMW * 4;       // [slice][own tokens][feature] floats
-  static constexpr int total(int stages) { return stages * kStageBytes + kSumBytes + 256 + 1024; }
+  static constexpr int kSumBytes = BT * BMW * 4;       // [slice][own tokens][feature] floats, where the reduction is cut
+  static constexpr int total(int stages, bool cut) { return stages * kStageBytes + (cut ? kSumBytes : 0) + 256 + 1024; }
 };
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
@@ -65,10 +67,15 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 __device__ __forceinline__ void st_cluster(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 
 // kExperts: the weights are [E, N, K_e] and the reduction runs over the experts of `slots` one after another (X has their columns in that order).
-template <int BT, int split, bool kExperts>
+// kGlu: the weights are [gate; up] of N / 2 rows each; a tile has 64 of both, C [tokens, N / 2] = silu(gate) · up, both rounded to bf16 first, which
+// makes the result the same bits as the activation kernel's.
+enum Mode { kPlain = 0, kExpertSum = 1, kGluPair = 2 };
+
+template <int BT, int split, int mode>
 __global__ void __launch_bounds__(192, 2)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, Params p) {
   using L = Layout<BT>;
+  constexpr bool kExperts = mode == kExpertSum, kGlu = mode == kGluPair;
   constexpr uint32_t kTmemCols = BT < 32 ? 32 : BT;
   const int stages = p.stages;
   extern __shared__ uint8_t smem_raw[];
@@ -76,7 +83,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + stages * L::kABytes;
   float* sums = reinterpret_cast<float*>(smem + stages * L::kStageBytes);
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + stages * L::kStageBytes + L::kSumBytes);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + stages * L::kStageBytes + (split > 1 ? L::kSumBytes : 0));
   uint64_t* empty_bar = full_bar + stages;
   uint64_t* tmem_full = empty_bar + stages;
   uint32_t* tmem_base_ptr = reinterpret_cast<uint32_t*>(tmem_full + 1);
@@ -119,7 +126,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         mbar_expect_tx(&full_bar[stage], L::kStageBytes);
         const int at = kb0 + kb;
         if (kExperts) tma_load_2d(smem_a + stage * L::kABytes, &tmap_w, &full_bar[stage], at % p.steps_per * BK, slot_e[at / p.steps_per] * p.N + n_blk * BMW);
-        else tma_load_2d(smem_a + stage * L::kABytes, &tmap_w, &full_bar[stage], at * BK, n_blk * BMW);
+        else if (!kGlu) tma_load_2d(smem_a + stage * L::kABytes, &tmap_w, &full_bar[stage], at * BK, n_blk * BMW);
+        else
+          for (int h = 0; h < 2; ++h)
+            tma_load_2d(smem_a + stage * L::kABytes + h * (L::kABytes / 2), &tmap_w, &full_bar[stage], at * BK, n_blk * (BMW / 2) + h * (p.N / 2));
       };
       auto load_x = [&](int kb, int stage) { tma_load_2d(smem_b + stage * L::kBBytes, &tmap_x, &full_bar[stage], (kb0 + kb) * BK, 0); };
       const int early = min(kbs, stages);
@@ -185,7 +195,28 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     if (p.out_fp32) reinterpret_cast<float*>(p.C)[tok * p.ldc + n] = x;
     else reinterpret_cast<__nv_bfloat16*>(p.C)[tok * p.ldc + n] = __float2bfloat16(x);
   };
-  if (split == 1) {
+  auto put_glu = [&](int tok, float gate, float up) {        // warps on gate rows
+    const float f = p.row_scale != nullptr ? scale[q][tok] : 1.f;
+    gate = __bfloat162float(__float2bfloat16(gate * f));
+    up = __bfloat162float(__float2bfloat16(up * f));
+    reinterpret_cast<__nv_bfloat16*>(p.C)[tok * p.ldc + n_blk * (BMW / 2) + q * 32 + lane] = __float2bfloat16(gate / (1.f + __expf(-gate)) * up);
+  };
+  if (split == 1 && kGlu) {
+    if (warp >= 2) {
+      float* ups = reinterpret_cast<float*>(smem);     // [token][64]: the products are done, nothing reads or writes the ring any more
+      if (q >= 2) {
+#pragma unroll
+        for (int i = 0; i < BT; ++i)
+          if (i < p.tokens) ups[i * 64 + (q - 2) * 32 + lane] = v[i];
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (q < 2) {
+#pragma unroll
+        for (int i = 0; i < BT; ++i)
+          if (i < p.tokens) put_glu(i, v[i], ups[i * 64 + q * 32 + lane]);
+      }
+    }
+  } else if (split == 1) {
     if (warp >= 2) {
 #pragma unroll
       for (int i = 0; i < BT; ++i)
@@ -206,7 +237,18 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     __syncwarp();
     cluster_arrive();
     cluster_wait();                                  // every slice's sums are in their owners' buffers; nothing remote is touched after this
-    if (warp >= 2) {
+    if (warp >= 2 && kGlu) {
+#pragma unroll 4
+      for (int i = 0; q < 2 && i < min(own, p.tokens - slice * own); ++i) {
+        float gate = 0.f, up = 0.f;
+#pragma unroll
+        for (int s = 0; s < split; ++s) {
+          gate += sums[(s * own + i) * BMW + q * 32 + lane];
+          up += sums[(s * own + i) * BMW + 64 + q * 32 + lane];
+        }
+        put_glu(slice * own + i, gate, up);
+      }
+    } else if (warp >= 2) {
 #pragma unroll 4
       for (int i = 0; i < min(own, tokens - slice * own); ++i) {
         float x = 0.f;
@@ -223,37 +265,36 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   }
 }
 
-template <int BT, int split, bool kExperts>
+template <int BT, int split, int mode>
 static int launch_as(const CUtensorMap& tw, const CUtensorMap& tx, Params p, cudaStream_t s) {
   using L = Layout<BT>;
-  constexpr int kDeep = kExperts && BT == 64 ? L::kDeep - 1 : L::kDeep;        // room for the list of experts
-  auto kern = gemm_rows_kernel<BT, split, kExperts>;
-  static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total(kDeep));
+  constexpr int kDeep = mode == kExpertSum && BT == 64 ? L::kDeep - 1 : L::kDeep;        // room for the list of experts
+  auto kern = gemm_rows_kernel<BT, split, mode>;
+  static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total(kDeep, split > 1));
   if (configured != cudaSuccess) return static_cast<int>(configured);
   const int tiles = (p.N + BMW - 1) / BMW;
   // a CTA with an SM to itself has twice the bytes in flight: the ring is deep where all clusters fit that way.  Eight neighbouring SMs are
-  // found 12 times at least; 16 such clusters took two waves (2048 × 4096, 9 tokens: 9.0 µs, 6.2 for 16 clusters of four)
-  p.stages = tiles <= (split == kMaxSplit ? kWideClusters : kSms / split) ? kDeep : L::kShallow;
-  return static_cast<int>(launch_pdl_cluster(kern, dim3(tiles * split), dim3(192), split, L::total(p.stages), s, tw, tx, p));
+  // found 12 times at least.  An uncut reduction has no buffers for sums: room for one stage more beside a second CTA (19456 × 2560, 19 tokens: 20.1 → 19.2 µs)
+  p.stages = tiles <= (split == kMaxSplit ? kWideClusters : kSms / split) ? kDeep : L::kShallow + (split == 1 ? 1 : 0);
+  return static_cast<int>(launch_pdl_cluster(kern, dim3(tiles * split), dim3(192), split, L::total(p.stages, split > 1), s, tw, tx, p));
 }
 
-template <int BT>
+template <int BT, int mode>
 static int launch(const CUtensorMap& tw, const CUtensorMap& tx, const Params& p, int split, cudaStream_t s) {
   switch (split) {
-    case 1: return launch_as<BT, 1, false>(tw, tx, p, s);
-    case 2: return launch_as<BT, 2, false>(tw, tx, p, s);
-    case 4: return launch_as<BT, 4, false>(tw, tx, p, s);
-    default: return launch_as<BT, 8, false>(tw, tx, p, s);
+    case 1: return launch_as<BT, 1, mode>(tw, tx, p, s);
+    case 2: return launch_as<BT, 2, mode>(tw, tx, p, s);
+    case 4: return launch_as<BT, 4, mode>(tw, tx, p, s);
+    default: return launch_as<BT, 8, mode>(tw, tx, p, s);
   }
 }
 
-template <int BT>
-static int launch_experts(const CUtensorMap& tw, const CUtensorMap& tx, const Params& p, int split, cudaStream_t s) {
-  switch (split) {
-    case 1: return launch_as<BT, 1, true>(tw, tx, p, s);
-    case 2: return launch_as<BT, 2, true>(tw, tx, p, s);
-    case 4: return launch_as<BT, 4, true>(tw, tx, p, s);
-    default: return launch_as<BT, 8, true>(tw, tx, p, s);
+template <int mode>
+static int launch_mode(int bt, const CUtensorMap& tw, const CUtensorMap& tx, const Params& p, int split, cudaStream_t s) {
+  switch (bt) {
+    case 16: return launch<16, mode>(tw, tx, p, split, s);
+    case 32: return launch<32, mode>(tw, tx, p, split, s);
+    default: return launch<64, mode>(tw, tx, p, split, s);
   }
 }
 
@@ -331,24 +372,21 @@ extern "C" int mb_norm_rows(const void* x, const void* residual, const void* w, 
 }
 
 // C[tokens, N] (bf16 or fp32) = X[tokens, K] · W[N, K]ᵀ (· row_scale[token]) (+ bias), tokens ≤ 64.  split: 1, 2, 4 or 8 slices of K.  static_w: no
-// kernel that may still run on the stream writes W.
+// kernel that may still run on the stream writes W.  glu: W is [gate; up] of N / 2 rows each (a multiple of 64), C [tokens, N / 2] bf16 = silu(gate) · up, no bias.
 extern "C" int mb_gemm_rows(const void* X, const void* W, void* C, int tokens, int N, int K, long long ldx, long long ldw, long long ldc, int out_fp32,
-                            const void* bias, const float* row_scale, int split, int static_w, int* error_flag, cudaStream_t s) {
+                            const void* bias, const float* row_scale, int split, int static_w, int glu, int* error_flag, cudaStream_t s) {
   using namespace mb;
   if (tokens <= 0 || N <= 0) return 0;
+  if (glu && (N % rows::BMW || out_fp32 || bias != nullptr)) return -3;
   if (tokens > 64 || (split != 1 && split != 2 && split != 4 && split != rows::kMaxSplit)) return -2;
   const int bt = tokens <= 16 ? 16 : tokens <= 32 ? 32 : 64;
   CUtensorMap tw, tx;
-  int r = make_tmap_bf16_2d(&tw, W, N, K, ldw, rows::BMW, rows::BK);
+  int r = make_tmap_bf16_2d(&tw, W, N, K, ldw, glu ? rows::BMW / 2 : rows::BMW, rows::BK);
   if (r) return 1000 + r;
   r = make_tmap_bf16_2d(&tx, X, tokens, K, ldx, bt, rows::BK);
   if (r) return 2000 + r;
   const rows::Params p{tokens, N, K, C, ldc, out_fp32, reinterpret_cast<const __nv_bfloat16*>(bias), row_scale, static_w, 0, error_flag, nullptr, 0};
-  switch (bt) {
-    case 16: return rows::launch<16>(tw, tx, p, split, s);
-    case 32: return rows::launch<32>(tw, tx, p, split, s);
-    default: return rows::launch<64>(tw, tx, p, split, s);
-  }
+  return glu ? rows::launch_mode<rows::kGluPair>(bt, tw, tx, p, split, s) : rows::launch_mode<rows::kPlain>(bt, tw, tx, p, split, s);
 }
 
 // C[tokens, N] bf16 = Σ_i X[tokens, i · F ..] · W[e_i]ᵀ over the slots[0] ≤ n_max experts e_i = slots[1 + i]: X [tokens, n_max · F], W [E, N, F], F a multiple of 64.
@@ -368,9 +406,5 @@ extern "C" int mb_gemm_rows_experts(const void* X, const void* W, void* C, int t
   // four with an SM each 18 / 21)
   const int tiles = (N + rows::BMW - 1) / rows::BMW;
   const int split = tiles * 8 <= 2 * rows::kSms ? 8 : tiles * 4 <= 2 * rows::kSms ? 4 : tiles * 2 <= 2 * rows::kSms ? 2 : 1;
-  switch (bt) {
-    case 16: return rows::launch_experts<16>(tw, tx, p, split, s);
-    case 32: return rows::launch_experts<32>(tw, tx, p, split, s);
-    default: return rows::launch_experts<64>(tw, tx, p, split, s);
-  }
+  return rows::launch_mode<rows::kExpertSum>(bt, tw, tx, p, split, s);
 }

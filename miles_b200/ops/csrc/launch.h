@@ -18,7 +18,7 @@ int mb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lon
                  int a_mn, int b_mn, int out_fp32, int accumulate, const void* bias, int force_bn, int* error_flag,
                  cudaStream_t stream);
 int mb_gemm_rows(const void* X, const void* W, void* C, int tokens, int N, int K, long long ldx, long long ldw, long long ldc, int out_fp32,
-                 const void* bias, const float* row_scale, int split, int static_w, int* error_flag, cudaStream_t s);
+                 const void* bias, const float* row_scale, int split, int static_w, int glu, int* error_flag, cudaStream_t s);
 int mb_norm_rows(const void* x, const void* residual, const void* w, float eps, int T, int K, void* scaled, float* rstd, void* sum, void* normed,
                  cudaStream_t s);
 int mb_gemm_rows_experts(const void* X, const void* W, void* C, int tokens, int N, int F, int E, int n_max, const int* slots, int* error_flag, cudaStream_t s);

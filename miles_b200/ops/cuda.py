@@ -192,6 +192,29 @@ def add_rmsnorm_linear(x, residual, norm_w, eps, w, bias=None, want_normed: bool
     return (y.view(*shp, N), res_out.view(x.shape) if res_out is not None else None, xn.view(x.shape) if xn is not None else None)
 
 
+def _rows_glu(M: int, w, K: int) -> int:
+    """CTAs per tile where gate and up of a decode step are gemm_rows.cu's and the activation is formed there (0: elsewhere)."""
+    split = _row_split(M, w.shape[0], K) if M <= SMALL_M and w.shape[0] % 128 == 0 and K % 8 == 0 else 0
+    return split if M > _gemv_rows(split, w.shape[0], K) else 0
+
+
+def add_rmsnorm_swiglu(x, residual, norm_w, eps, w):
+    """As `add_rmsnorm_linear` with swiglu behind it: (swiglu(rmsnorm(x + residual) · wᵀ), x + residual)."""
+    K = x.shape[-1]
+    M, split = x.numel() // K, _rows_glu(x.numel() // K, w, K)
+    if not split:
+        y, res, _ = add_rmsnorm_linear(x, residual, norm_w, eps, w)
+        return swiglu(y), res
+    x2 = _c(x.reshape(-1, K))
+    r2 = _c(residual.reshape(-1, K)) if residual is not None else None
+    res, scaled = torch.empty_like(x2) if r2 is not None else None, torch.empty_like(x2)
+    rstd = torch.empty(M, dtype=torch.float32, device=x.device)
+    act = torch.empty(M, w.shape[0] // 2, dtype=BF16, device=x.device)
+    C.norm_rows(x2, r2, norm_w, float(eps), scaled, rstd, res, None)
+    C.gemm_rows(scaled, w, act, M, w.shape[0], K, act.shape[1], None, split, bool(w.is_leaf and w.requires_grad), rstd, True)
+    return act.view(*x.shape[:-1], -1), res.view(x.shape) if res is not None else None
+
+
 def gemv_ok(x, w) -> bool:
     """True when `add_rmsnorm_linear` applies: bf16, no autograd, few rows, K a multiple of 32."""
     K = x.shape[-1]
@@ -209,16 +232,15 @@ def small_bt(rows: int) -> int:
 
 
 def _row_split(M: int, N: int, K: int) -> int:
-    """CTAs that share one 128-row weight tile (gemm_rows.cu): as many as fit the GPU at once, two per SM, with at least two 64-deep steps
-    each; one where sums over K may not be cut (MILES_SPLIT_K=0).  Eight only where twelve clusters of them, an SM per CTA, or all of
-    them in pairs per SM are enough (13 to 18 tiles: four; 16 tiles, K 4096, 61 tokens: 8.2 µs against 12.1).  0: more tiles than that:
-    the persistent kernels walk through them (gemm_small.cu; from 33 tokens also where no reduction is cut and the 128-row tiles of
-    gemm.cu are as fast: 152 tiles, K 2560: 32 tokens 21.9 against 24.1 µs, 48 tokens 25.2 against 24.3)."""
+    """CTAs that share one 128-row weight tile (gemm_rows.cu): as many as fit the GPU at once, two per SM, with at least four 64-deep steps
+    each; one where sums over K may not be cut (MILES_SPLIT_K=0).  µs of decode steps of 8 layers: hidden 1024, 12 / 30 / 60 rows with at least two
+    steps 368 / 463 / 524, four 358 / 446 / 506, six 381 / 456 / 510.  16 tiles by eight instead of four: hidden 2048 with 16 experts, 16 / 30 rows 674 /
+    707 → 658 / 695.  0: more tiles than that: the persistent kernels walk through them (gemm_small.cu; from 33 tokens also where no reduction is cut
+    and the 128-row tiles of gemm.cu are as fast: 152 tiles, K 2560: 32 tokens 21.9 against 24.1 µs, 48 tokens 25.2 against 24.3)."""
     tiles, steps = (N + 127) // 128, (K + 63) // 64
     if tiles > 148 and M > 32:
         return 0
-    return next((s for s in ((8, 4, 2, 1) if SPLIT_K else (1,))
-                 if tiles * s <= 296 and (steps >= 2 * s or s == 1) and not (s == 8 and 12 < tiles <= 18)), 0)
+    return next((s for s in ((8, 4, 2, 1) if SPLIT_K else (1,)) if tiles * s <= 296 and (steps >= 4 * s or s == 1)), 0)
 
 
 def gemm_nn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *, out_dtype=None, force_bn: int = 0):

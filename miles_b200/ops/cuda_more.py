@@ -295,6 +295,13 @@ def linear_swiglu(x, w):
     """swiglu(x · wᵀ) with w [gate; up]; without autograd in one kernel where sizes allow."""
     from . import cuda as _cuda
 
+    rows = x.numel() // x.shape[-1]
+    if (0 < rows <= _cuda.SMALL_M and not torch.is_grad_enabled() and x.dtype == BF16 and w.dtype == BF16 and w.is_contiguous() and _glu_in_place()
+            and _cuda._rows_glu(rows, w, x.shape[-1])):
+        act = torch.empty(*x.shape[:-1], w.shape[0] // 2, dtype=BF16, device=x.device)
+        C.gemm_rows(_c(x).view(rows, -1), w, act, rows, w.shape[0], x.shape[-1], act.shape[-1], None, _cuda._rows_glu(rows, w, x.shape[-1]),
+                    bool(w.is_leaf and w.requires_grad), None, True)
+        return act
     if (torch.is_grad_enabled() or x.numel() < 512 * x.shape[-1] or x.dtype != BF16 or w.dtype != BF16 or not w.is_contiguous()
             or x.shape[-1] % 8 or not _glu_in_place()):                 # below 512 rows the tiles of 256 are half empty
         return _cuda.swiglu(_cuda.linear(x, w))

@@ -127,3 +127,40 @@ def test_weights_ahead_of_the_rows():
             graph.replay()
             assert torch.equal(captured, stepwise)
     assert torch.equal(first, stepwise) and K.check_error_flag(x) == 0
+
+
+@pytest.mark.parametrize("T", [1, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("F,K", [(64, 256), (3072, 1024), (320, 328), (9472, 512)])
+@pytest.mark.parametrize("split", [1, 2, 4, 8])
+def test_gate_and_up_in_one_product(T, F, K, split):
+    """silu(gate) · up where the sums are: the bits of the product and the activation apart, with and without factors on the rows."""
+    from miles_b200.ops.cuda import C
+
+    if split > 1 and K // 64 < split:
+        pytest.skip("fewer steps than slices")
+    g = torch.Generator(device="cuda").manual_seed(T + F)
+    x, w = torch.randn(T, K, device="cuda", generator=g).bfloat16(), (torch.randn(2 * F, K, device="cuda", generator=g) / K ** 0.5 * 2).bfloat16()
+    for scale in (None, torch.rand(T, device="cuda", generator=g) + 0.5):
+        h, want, got = (torch.empty(T, n, dtype=torch.bfloat16, device="cuda") for n in (2 * F, F, F))
+        C.gemm_rows(x, w, h, T, 2 * F, K, 2 * F, None, split, False, scale)
+        C.swiglu_fwd(h, want, None)
+        C.gemm_rows(x, w, got, T, 2 * F, K, F, None, split, False, scale, True)
+        assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("T", [1, 8, 12, 16, 19, 32, 50])
+@pytest.mark.parametrize("F,K", [(3072, 1024), (9728, 2560), (72, 512)])
+def test_gate_and_up_behind_a_norm(T, F, K):
+    """Through the functions that models call: what the norm, the projection and the activation give one after another."""
+    from miles_b200.ops import cuda as K_
+
+    g = torch.Generator(device="cuda").manual_seed(T + F)
+    x, r = (torch.randn(T, K, device="cuda", generator=g).bfloat16() for _ in range(2))
+    w, nw = torch.nn.Parameter((torch.randn(2 * F, K, device="cuda", generator=g) / K ** 0.5 * 2).bfloat16()), (1 + 0.1 * torch.randn(K, device="cuda", generator=g)).bfloat16()
+    with torch.no_grad():
+        assert torch.equal(K_.linear_swiglu(x, w), K_.swiglu(K_.linear(x, w)))
+        if K_.gemv_ok(x, w):
+            y, res = K_.add_rmsnorm_swiglu(x, r, nw, 1e-6, w)
+            h13, want_res, _ = K_.add_rmsnorm_linear(x, r, nw, 1e-6, w)
+            assert torch.equal(y, K_.swiglu(h13)) and torch.equal(res, want_res)
+    assert K_.check_error_flag(x) == 0
