@@ -243,7 +243,7 @@ at::Tensor qk_norm_rope_bwd(const at::Tensor& x, const c10::optional<at::Tensor>
   float* pp = nullptr;
   void* dwp = nullptr;
   if (w.has_value() && w->defined()) {
-    dw = at::zeros({D}, w->options());
+    dw = T > 0 ? at::empty({D}, w->options()) : at::zeros({D}, w->options());
     if (T > 0) {
       partial = at::empty({mb_qk_norm_rope_bwd_blocks(T, Hn), D}, x.options().dtype(at::kFloat));
       pp = partial.data_ptr<float>();

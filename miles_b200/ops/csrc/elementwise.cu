@@ -263,7 +263,8 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* _
 // The same with WPR warps per row, for rows of 256·VPL·WPR elements: all loads of a row in flight at once and no CTA barrier per row (the form
 // above waits for two of them: 98 µs at 12 075 × 2048 where the bytes take 31).  VPL is kept at 5 or below: the row, its gradient
 // and the weight gradient's sums have to fit the registers of 12 (VPL 5: 8) warps per SM.  The sums stay in registers until the end, where the
-// CTA's warps add theirs up in shared memory.  11 791 × 2560 with the residual's gradient: 134 → 107 µs (37 at the memory's speed).
+// CTA's warps add theirs up in shared memory.  The residual's gradient is requested with the row: behind the sums it was a second trip to memory per
+// row (12 075 × 2048 69 → 47 µs, 11 791 × 2560 99 → 59; 30 and 37 at the memory's speed).
 template <int VPL, int WPR>
 __global__ void __launch_bounds__(128, VPL <= 4 ? 3 : 2) rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                                   const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ dres,
@@ -284,11 +285,12 @@ __global__ void __launch_bounds__(128, VPL <= 4 ? 3 : 2) rmsnorm_bwd_warp_kernel
     const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * H) + v0;
     const bf16x8* gr = reinterpret_cast<const bf16x8*>(dy + row * H) + v0;
     const bf16x8* wr = reinterpret_cast<const bf16x8*>(w) + v0;
-    bf16x8 xv[VPL], gv[VPL];
+    bf16x8 xv[VPL], gv[VPL], rv[VPL];
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       xv[i] = xr[kStep * i];
       gv[i] = gr[kStep * i];
+      if (dres != nullptr) rv[i] = (reinterpret_cast<const bf16x8*>(dres + row * H) + v0)[kStep * i];
     }
     float dot = 0.f;
 #pragma unroll
@@ -324,14 +326,13 @@ __global__ void __launch_bounds__(128, VPL <= 4 ? 3 : 2) rmsnorm_bwd_warp_kernel
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       const bf16x8 wv = wr[kStep * i];
-      bf16x8 o, rv;
-      if (dres != nullptr) rv = (reinterpret_cast<const bf16x8*>(dres + row * H) + v0)[kStep * i];
+      bf16x8 o;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 a = __bfloat1622float2(xv[i].v[j]), g = __bfloat1622float2(gv[i].v[j]), c = __bfloat1622float2(wv.v[j]);
         float o0 = rstd * (g.x * c.x - a.x * rstd * dot), o1 = rstd * (g.y * c.y - a.y * rstd * dot);
         if (dres != nullptr) {
-          const float2 r = __bfloat1622float2(rv.v[j]);
+          const float2 r = __bfloat1622float2(rv[i].v[j]);
           o0 += r.x;
           o1 += r.y;
         }
@@ -721,6 +722,100 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(const __nv_bfloat
   }
 }
 
+// The same for D = 128 with a norm and heads in fours: sixteen lanes per head with 8-byte pieces of both halves, two heads at a time, all loads of the four
+// heads together, frequencies and weights in registers.  A warp per head with 2-byte loads was bound by instructions: 11 791 tokens × 32 heads
+// 104 → 72 µs (44 at the memory's speed).
+__global__ void __launch_bounds__(256) qk_norm_rope_bwd_many_kernel(const __nv_bfloat16* __restrict__ x, long long x_tok_stride,
+                                                                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
+                                                                    const __nv_bfloat16* __restrict__ dy, const int* __restrict__ positions,
+                                                                    __nv_bfloat16* __restrict__ dx, long long dx_tok_stride,
+                                                                    float* __restrict__ dw_partial, long long T, int Hn, float log2_theta) {
+  constexpr int D = 128;
+  __shared__ float sh_dw[16][D];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, half = lane >> 4, j = (lane & 15) * 4;
+  float freq[4], wa[4], wb[4], dwa[4], dwb[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    freq[e] = exp2f(-log2_theta * (2.f * (j + e)) / D);
+    wa[e] = __bfloat162float(w[j + e]);
+    wb[e] = __bfloat162float(w[D / 2 + j + e]);
+    dwa[e] = dwb[e] = 0.f;
+  }
+  auto four = [](const uint2& v, float (&f)[4]) {
+    f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
+    f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
+  };
+  auto pack4 = [](const float (&f)[4]) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+  };
+  const int quads = Hn / 4;
+  const long long items = T * quads;
+  for (long long it = (blockIdx.x * 256ll + threadIdx.x) >> 5; it < items; it += (static_cast<long long>(gridDim.x) * 256) >> 5) {
+    const long long t = it / quads;
+    const int h0 = static_cast<int>(it % quads) * 4 + half;
+    uint2 gl[2][2], xl[2][2];
+    float rs[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const __nv_bfloat16* gr = dy + (t * Hn + h0 + 2 * i) * D + j;
+      const __nv_bfloat16* xr = x + t * x_tok_stride + (h0 + 2 * i) * D + j;
+      gl[i][0] = *reinterpret_cast<const uint2*>(gr);
+      gl[i][1] = *reinterpret_cast<const uint2*>(gr + D / 2);
+      xl[i][0] = *reinterpret_cast<const uint2*>(xr);
+      xl[i][1] = *reinterpret_cast<const uint2*>(xr + D / 2);
+      rs[i] = rstd_in[t * Hn + h0 + 2 * i];
+    }
+    const float pos = static_cast<float>(positions[t]);
+    float sn[4], cs[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sincosf(pos * freq[e], &sn[e], &cs[e]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float d1[4], d2[4], xa[4], xb[4], o1[4], o2[4], dot = 0.f;
+      four(gl[i][0], d1);
+      four(gl[i][1], d2);
+      four(xl[i][0], xa);
+      four(xl[i][1], xb);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float g1 = d1[e] * cs[e] + d2[e] * sn[e], g2 = d2[e] * cs[e] - d1[e] * sn[e];     // transpose of the rotation
+        xa[e] *= rs[i];
+        xb[e] *= rs[i];
+        d1[e] = g1 * wa[e];
+        d2[e] = g2 * wb[e];
+        dot += d1[e] * xa[e] + d2[e] * xb[e];
+        dwa[e] += g1 * xa[e];
+        dwb[e] += g2 * xb[e];
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+      dot /= D;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        o1[e] = rs[i] * (d1[e] - xa[e] * dot);
+        o2[e] = rs[i] * (d2[e] - xb[e] * dot);
+      }
+      __nv_bfloat16* dr = dx + t * dx_tok_stride + (h0 + 2 * i) * D + j;
+      *reinterpret_cast<uint2*>(dr) = pack4(o1);
+      *reinterpret_cast<uint2*>(dr + D / 2) = pack4(o2);
+    }
+  }
+  if (dw_partial == nullptr) return;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    sh_dw[2 * wib + half][j + e] = dwa[e];
+    sh_dw[2 * wib + half][D / 2 + j + e] = dwb[e];
+  }
+  __syncthreads();
+  if (threadIdx.x < D) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s += sh_dw[i][threadIdx.x];
+    dw_partial[static_cast<long long>(blockIdx.x) * D + threadIdx.x] = s;
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 // Rotary embedding alone (NeoX pairing: element i rotates with element i + D/2), forward or inverse (= its own backward).
 // One warp per (token, head); x [T, H, D] with token stride `tok_stride`, y contiguous.
@@ -1018,7 +1113,10 @@ extern "C" int mb_qk_norm_rope_bwd(const void* x, long long x_stride, const void
   auto W = reinterpret_cast<const __nv_bfloat16*>(w);
   auto DY = reinterpret_cast<const __nv_bfloat16*>(dy);
   auto DX = reinterpret_cast<__nv_bfloat16*>(dx);
-  if (D == 128)
+  if (D == 128 && w != nullptr && Hn % 4 == 0 && ((x_stride | dx_stride) & 3) == 0 &&
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 7) == 0)
+    qk_norm_rope_bwd_many_kernel<<<blocks, 256, 0, s>>>(X, x_stride, W, rstd, DY, positions, DX, dx_stride, dw_partial, T, Hn, l2t);
+  else if (D == 128)
     qk_norm_rope_bwd_kernel<128><<<blocks, 256, 0, s>>>(X, x_stride, W, rstd, DY, positions, DX, dx_stride, dw_partial, T, Hn, l2t);
   else if (D == 64)
     qk_norm_rope_bwd_kernel<64><<<blocks, 256, 0, s>>>(X, x_stride, W, rstd, DY, positions, DX, dx_stride, dw_partial, T, Hn, l2t);

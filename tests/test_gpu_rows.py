@@ -80,3 +80,29 @@ def test_rotation_of_many_tokens(T, Hq, Hk, D, norm, offset):
     want = cache.clone()
     want[0, slots[slots >= 0]], want[1, slots[slots >= 0]] = k3[slots >= 0], v[slots >= 0]
     assert torch.equal(kc[0], want[0]) and torch.equal(vc[0], want[1])
+
+
+@pytest.mark.parametrize("T,heads", [(1, 4), (37, 32), (700, 8)])
+@pytest.mark.parametrize("offset", [0, 2])                 # rows off an 8-byte boundary take a warp per head
+def test_qk_norm_rope_backward_four_heads_at_a_time(T, heads, offset):
+    """Gradients of norm and rotation against 64 bits."""
+    from miles_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(T + heads)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    wide = rand(T, (heads + 2) * 128 + 4).bfloat16()
+    x = wide[:, offset:offset + heads * 128].view(T, heads, 128)
+    w, dy, pos = (1 + 0.2 * rand(128)).bfloat16(), rand(T, heads, 128).bfloat16(), torch.randint(0, 5000, (T,), device="cuda", dtype=torch.int32)
+    x64 = x.double().requires_grad_()
+    w64 = w.double().requires_grad_()
+    rstd = torch.rsqrt(x64.pow(2).mean(-1, keepdim=True) + 1e-6)
+    n = x64 * rstd * w64
+    ang = pos.double()[:, None] * 1e6 ** (-torch.arange(0, 128, 2, device="cuda", dtype=torch.float64) / 128)
+    c, s = ang.cos()[:, None], ang.sin()[:, None]
+    y = torch.cat([n[..., :64] * c - n[..., 64:] * s, n[..., 64:] * c + n[..., :64] * s], -1)
+    y.backward(dy.double())
+    dx = torch.empty(T, heads, 128, dtype=torch.bfloat16, device="cuda")
+    dw = K.C.qk_norm_rope_bwd(x, w, rstd.detach().float().view(-1), dy, pos, dx, 1e6)
+    # one rounding to bf16 each (2^-9), angles of up to 5000 in fp32 (5000 · 2^-24 = 3e-4 of a turn's radius)
+    assert ((dx.double() - x64.grad).norm() / x64.grad.norm()).item() < 3e-3
+    assert ((dw.double() - w64.grad).norm() / w64.grad.norm()).item() < 5e-3
