@@ -220,7 +220,7 @@ class MoEFFN(nn.Module):
             w2[e - lo].copy_(gen(f"{tag}.e{e}.w2", (H, F), cfg.init_std, dtype, device))
         self.w13, self.w2 = nn.Parameter(w13), nn.Parameter(w2)
 
-    def forward(self, x, meta: ForwardMeta, layer: int, logits: torch.Tensor | None = None, chosen=None):
+    def forward(self, x, meta: ForwardMeta, layer: int, logits: torch.Tensor | None = None, chosen=None, rows: bool = False):
         # with sequence parallelism each TP rank routes its own token slice (expert-TP is 1); `chosen`: (weights, choices) made by the caller
         if logits is None and chosen is None:
             logits = ops.linear_fp32(x, self.router)  # router scores stay fp32 (no bf16 rounding, no cast kernel)
@@ -235,7 +235,7 @@ class MoEFFN(nn.Module):
             w, idx, _ = ops.router_topk(logits, k, norm)
         if meta.record_topk is not None:
             meta.record_topk.append(idx.detach())
-        return self.ps.moe_ffn(x, self.w13, self.w2, w, idx, self.cfg.num_experts, meta.values)
+        return self.ps.moe_ffn(x, self.w13, self.w2, w, idx, self.cfg.num_experts, meta.values, rows)
 
 
 def add_rmsnorm_reducing(ps, x, residual, w, eps):
@@ -282,9 +282,9 @@ class DecoderLayer(nn.Module):
         hn, residual, w, idx = ops.add_rmsnorm_router(h, residual, self.ln2, self.eps, mlp.router, mlp.cfg.moe_topk, mlp.cfg.moe_norm_topk_prob)
         return mlp(hn, meta, self.layer, chosen=(w, idx)), residual
 
-    def forward(self, x, residual, meta: ForwardMeta):
-        # `x` is the previous block's output still to be added to `residual`
-        if (self.attn.ps.tp_size == 1 and ops.few_token_decode(x, self.attn.wqkv) and getattr(self.attn, "lora", None) is None
+    def forward(self, x, residual, meta: ForwardMeta, rows: bool = False):
+        # `x` is the previous block's output still to be added to `residual`; `rows`: the caller adds up experts' rows itself (`ops.moe_ffn_rows`)
+        if (self.attn.ps.tp_size == 1 and isinstance(x, torch.Tensor) and ops.few_token_decode(x, self.attn.wqkv) and getattr(self.attn, "lora", None) is None
                 and getattr(self.mlp, "lora", None) is None):
             return self._forward_few_tokens(x, residual, meta)
         h, residual = add_rmsnorm_reducing(self.attn.ps, x, residual, self.ln1, self.eps)
@@ -292,8 +292,9 @@ class DecoderLayer(nn.Module):
         if self._routes_few_tokens(h, meta):
             return self._moe_few_tokens(h, residual, meta)
         h, residual = add_rmsnorm_reducing(self.attn.ps, h, residual, self.ln2, self.eps)
-        h = self.mlp(h, meta, self.layer)
-        return h, residual
+        if rows and type(self.mlp) is MoEFFN:
+            return self.mlp(h, meta, self.layer, rows=True), residual
+        return self.mlp(h, meta, self.layer), residual
 
 
 class Qwen3Model(nn.Module):
@@ -344,8 +345,12 @@ class Qwen3Model(nn.Module):
             x = hidden_in
         residual = None
         for layer in self.layers:
+            if not isinstance(x, torch.Tensor) and not _plain(layer):
+                x = x.value()
             if meta.recompute and torch.is_grad_enabled():
                 x, residual = _checkpoint(layer, x, residual, meta)
+            elif self._hands_on_rows(layer):
+                x, residual = layer(x, residual, meta, rows=True)
             else:
                 x, residual = layer(x, residual, meta)
         if not self.has_head:
@@ -355,6 +360,11 @@ class Qwen3Model(nn.Module):
             return x if residual is None else x + residual
         h, _ = add_rmsnorm_reducing(self.ps, x, residual, self.norm, self.cfg.rms_eps)
         return h
+
+    def _hands_on_rows(self, layer) -> bool:
+        """Without gradients a plain MoE layer may leave the weighted sum of its experts' rows to the add and norm that follow it."""
+        return (self.has_head and not torch.is_grad_enabled() and _plain(layer) and type(layer.mlp) is MoEFFN and self.ps.tp_size == 1
+                and self.ps.ep_size == 1 and getattr(layer.mlp, "lora", None) is None)
 
     def global_name(self, name: str) -> str:
         """Parameter name with the model-wide layer index (a pipeline stage numbers its own layers from 0)."""
@@ -451,6 +461,11 @@ class _RunAgain(torch.autograd.Function):
         given = [(o, g) for o, g in zip(outs, grads) if g is not None]
         got = iter(torch.autograd.grad([o for o, _ in given], wanted, [g for _, g in given], allow_unused=True))
         return (None, None, None, *(next(got) if t is not None and t.requires_grad else None for t in ins), *got)
+
+
+def _plain(layer) -> bool:
+    """A decoder layer of this module that nobody looks on."""
+    return type(layer) is DecoderLayer and not any(m._forward_hooks or m._forward_pre_hooks for m in (layer, layer.attn, layer.mlp))
 
 
 def _runs_again(layer, x, meta) -> bool:

@@ -95,6 +95,8 @@ def add_rmsnorm(x, residual, w, eps=1e-6):
     """(x + residual) → (rmsnorm(sum), sum); residual None means x starts the stream."""
     if residual is None:
         return rmsnorm(x, w, eps), x
+    if not isinstance(x, torch.Tensor):
+        return _k().combine_add_rmsnorm(x, residual, w, eps)      # experts' rows, see moe_ffn_rows
     if x.is_cuda:
         return _k().add_rmsnorm(x, residual, w, eps)
     return ref.add_rmsnorm(x, residual, w, eps)
@@ -171,6 +173,13 @@ def moe_ffn(x, w13, w2, topk_w, topk_idx, values=True):
     """`values` False: the result is not read, it only stands in the graph."""
     if x.is_cuda:
         return _k().moe_ffn(x, w13, w2, topk_w, topk_idx, values=values)
+    return ref.moe_ffn(x, w13, w2, topk_w, topk_idx)
+
+
+def moe_ffn_rows(x, w13, w2, topk_w, topk_idx):
+    """`moe_ffn`, or the rows that its weighted sum would take for `combine_add_rmsnorm` (no gradients, many tokens)."""
+    if x.is_cuda:
+        return _k().moe_ffn_rows(x, w13, w2, topk_w, topk_idx)
     return ref.moe_ffn(x, w13, w2, topk_w, topk_idx)
 
 

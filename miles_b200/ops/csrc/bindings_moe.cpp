@@ -103,6 +103,21 @@ void moe_combine_bwd(const at::Tensor& dout, const at::Tensor& y_perm, const at:
         "mb_moe_combine_bwd");
 }
 
+// (rmsnorm(sum) · norm_w, sum) with sum = Σ_j w[t, j] · y_perm[dst_row[t, j]] + residual
+std::vector<at::Tensor> moe_combine_norm(const at::Tensor& y_perm, const at::Tensor& w, const at::Tensor& dst_row, const at::Tensor& residual,
+                                         const at::Tensor& norm_w, int64_t k, double eps) {
+  c10::cuda::CUDAGuard g(residual.device());
+  const int64_t T = residual.size(0), H = residual.size(1);
+  TORCH_CHECK(y_perm.is_contiguous() && w.is_contiguous() && dst_row.is_contiguous() && residual.is_contiguous() && norm_w.is_contiguous() && y_perm.size(1) == H &&
+                  norm_w.numel() == H && w.numel() == T * k && dst_row.numel() == T * k,
+              "moe_combine_norm: shapes");
+  auto y = at::empty_like(residual), sum = at::empty_like(residual);
+  check(mb_moe_combine_norm(y_perm.data_ptr(), w.data_ptr<float>(), dst_row.data_ptr<int>(), residual.data_ptr(), norm_w.data_ptr(), y.data_ptr(), sum.data_ptr(), T,
+                            k, H, eps, cur_stream()),
+        "mb_moe_combine_norm");
+  return {y, sum};
+}
+
 // h1 [rows, 2F], act_w [rows, F] (dout · W2 → weighted activation), dh1 [rows, 2F], w and dw fp32 [pairs]
 void moe_glu_bwd(const at::Tensor& h1, at::Tensor& act_w, at::Tensor& dh1, const at::Tensor& w, const at::Tensor& row_src, const at::Tensor& seg, at::Tensor& dw) {
   c10::cuda::CUDAGuard g(h1.device());
@@ -127,4 +142,5 @@ void register_moe(pybind11::module& m) {
         pybind11::arg("k"), pybind11::arg("identity_rows") = false);
   m.def("moe_combine_bwd", &moe_combine_bwd);
   m.def("moe_glu_bwd", &moe_glu_bwd);
+  m.def("moe_combine_norm", &moe_combine_norm);
 }

@@ -131,6 +131,8 @@ int mb_paged_bounds_set_limit(int which, long long value);
 int mb_paged_bounds_read(long long* out4, int clear);
 
 // ---- moe.cu ----
+int mb_moe_combine_norm(const void* y_perm, const float* w, const int* dst_row, const void* residual, const void* norm_w, void* y, void* res_out, long long T, int k,
+                        int H, float eps, cudaStream_t s);
 int mb_moe_glu_bwd(const void* h1, void* act_w, void* dh1, const float* w, const int* row_src, const int* seg_offsets, int E, float* dw, int F, int max_rows,
                    cudaStream_t s);
 int mb_norm_router(const void* x, const void* residual, const void* norm_w, const void* W, float eps, int T, int H, int E, int K, int normalize,

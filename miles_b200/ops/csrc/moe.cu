@@ -491,6 +491,84 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const bf16* y_perm, co
   }
 }
 
+// The same with the residual stream's add and the next RMSNorm behind it, a warp per token of 256·VPL columns: the weighted sum never goes to memory.  Sums and
+// roundings are those of the two kernels it stands for (rmsnorm_fwd_warp_kernel).  What bounds it: the rows of y.  7258 tokens × 8 × 2048: 49 + 32 → 61 µs,
+// 17 829: 112 + 70 → 130 (123 at the memory's speed; 135 with 256 threads a block, 143 with the registers of five blocks).
+template <int VPL>
+__global__ void __launch_bounds__(128, VPL <= 8 ? 4 : 2) moe_combine_norm_kernel(const bf16* y_perm, const float* w, const int* dst_row, const bf16* residual,
+                                                               const bf16* __restrict__ norm_w, bf16* y, bf16* res_out, long long T, int k, float eps) {
+  constexpr int H = VPL * 256;
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const long long t = blockIdx.x * 4ll + (threadIdx.x >> 5);
+  if (t >= T) return;
+  const uint4* rr = reinterpret_cast<const uint4*>(residual + t * H);
+  uint4 v[VPL];
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) v[i] = rr[lane + 32 * i];
+  auto add8 = [](float (&acc)[8], const uint4& raw, float f) {
+    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 x = __bfloat1622float2(p[e]);
+      acc[2 * e] += f * x.x;
+      acc[2 * e + 1] += f * x.y;
+    }
+  };
+  const int row0 = lane < k ? dst_row[t * k + lane] : -1;              // the first 32 choices; more are read where they are used
+  const float w0 = lane < k ? w[t * k + lane] : 0.f;
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int j0 = 0; j0 < k; j0 += 8) {
+      uint4 raw[8];
+      float wj[8];
+      bool in[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int j = j0 + u;
+        int row = __shfl_sync(0xffffffffu, row0, j & 31);
+        wj[u] = __shfl_sync(0xffffffffu, w0, j & 31);
+        if (j >= 32 && j < k) { row = dst_row[t * k + j]; wj[u] = w[t * k + j]; }
+        in[u] = j < k && row >= 0;
+        raw[u] = in[u] ? reinterpret_cast<const uint4*>(y_perm + static_cast<long long>(row) * H)[lane + 32 * i] : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (in[u]) add8(acc, raw[u], wj[u]);
+    }
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v[i]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = __bfloat1622float2(__floats2bfloat162_rn(acc[2 * e], acc[2 * e + 1])), b = __bfloat1622float2(h[e]);
+      h[e] = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
+    }
+    reinterpret_cast<uint4*>(res_out + t * H)[lane + 32 * i] = v[i];
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < VPL; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&v[i])[e]);
+      ss += a.x * a.x + a.y * a.y;
+    }
+  ss = wsum(ss);
+  const float rstd = rsqrtf(ss / H + eps);
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    const uint4 wv = reinterpret_cast<const uint4*>(norm_w)[lane + 32 * i];
+    uint4 o;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&v[i])[e]), b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&wv)[e]);
+      reinterpret_cast<__nv_bfloat162*>(&o)[e] = __floats2bfloat162_rn(a.x * rstd * b.x, a.y * rstd * b.y);
+    }
+    reinterpret_cast<uint4*>(y + t * H)[lane + 32 * i] = o;
+  }
+}
+
 // dy_perm[row] = w[flat]·dout[token];  dw[flat] = ⟨dout[token], y_perm[row]⟩   (one warp per permuted row)
 __global__ void __launch_bounds__(256) moe_combine_bwd_kernel(const bf16* dout, const bf16* y_perm, const float* w, const int* row_src,
                                                               const int* seg_offsets, int E, bf16* dy_perm, float* dw, int k, int H, int max_rows) {
@@ -541,7 +619,7 @@ __global__ void __launch_bounds__(256) moe_combine_bwd_kernel(const bf16* dout, 
 // d = the row of dout · W2 (in act_w's place):  dw[flat] = ⟨d, a⟩,  dh1 = gradient of h1 for w · d,  act_w = w · a (what W2's gradient multiplies dout
 // with).  Pad rows give zeros.  What bounds it: six passes of the row's width over memory.  It stands for the activation's recomputation, its
 // backward and the sums ⟨dout, y⟩ over rows of y, which nobody has to keep any more: 96 600 rows of 768, hidden 2048: 90 + 156 + 170 µs → 164
-// and a gather (110).
+// and 110 for the gather of the rows of dout.
 __global__ void __launch_bounds__(256) moe_glu_bwd_kernel(const bf16* h1, bf16* act_w, bf16* dh1, const float* w, const int* row_src, const int* seg_offsets, int E,
                                                           float* dw, int F, int max_rows) {
   constexpr int U = 3;
@@ -691,4 +769,18 @@ extern "C" int mb_moe_glu_bwd(const void* h1, void* act_w, void* dh1, const floa
   moe_glu_bwd_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const bf16*>(h1), reinterpret_cast<bf16*>(act_w), reinterpret_cast<bf16*>(dh1), w, row_src,
                                             seg_offsets, E, dw, F, max_rows);
   return static_cast<int>(cudaGetLastError());
+}
+
+// See moe_combine_norm_kernel: y = rmsnorm(Σ_j w · y_perm rows + residual) · norm_w, res_out the sum; H 1024, 2048 or 4096, all 16-byte aligned.
+extern "C" int mb_moe_combine_norm(const void* y_perm, const float* w, const int* dst_row, const void* residual, const void* norm_w, void* y, void* res_out,
+                                   long long T, int k, int H, float eps, cudaStream_t s) {
+  if (T == 0) return 0;
+  if (H != 1024 && H != 2048 && H != 4096) return -1;
+  if ((reinterpret_cast<uintptr_t>(y_perm) | reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(norm_w) | reinterpret_cast<uintptr_t>(y) |
+       reinterpret_cast<uintptr_t>(res_out)) & 15)
+    return -2;
+  auto kern = H == 1024 ? moe_combine_norm_kernel<4> : H == 2048 ? moe_combine_norm_kernel<8> : moe_combine_norm_kernel<16>;
+  return static_cast<int>(launch_pdl(kern, dim3(static_cast<unsigned>((T + 3) / 4)), dim3(128), 0, s, reinterpret_cast<const bf16*>(y_perm), w, dst_row,
+                                     reinterpret_cast<const bf16*>(residual), reinterpret_cast<const bf16*>(norm_w), reinterpret_cast<bf16*>(y),
+                                     reinterpret_cast<bf16*>(res_out), T, k, eps));
 }

@@ -472,6 +472,47 @@ class _MoEFFN(torch.autograd.Function):
         return dx, dw13, dw2, dw_flat.view(T, k), None, None, None, None
 
 
+class Combine:
+    """The experts' rows of a forward pass without gradients, still to be weighted and added up per token: by the add and norm of the next layer
+    (`combine_add_rmsnorm`) or by `value`."""
+
+    def __init__(self, y_perm, w, dst_row, k, like):
+        self.y_perm, self.w, self.dst_row, self.k, self.like = y_perm, w, dst_row, k, like
+
+    def value(self):
+        out = torch.empty_like(self.like)
+        C.moe_combine(self.y_perm, self.w, self.dst_row, out, self.k)
+        return out
+
+
+def combine_add_rmsnorm(x: Combine, residual, norm_w, eps):
+    """(rmsnorm(x + residual) · norm_w, x + residual)."""
+    H = residual.shape[-1]
+    if norm_w.data_ptr() % 16 or residual.data_ptr() % 16 or not norm_w.is_contiguous():
+        from . import cuda as _cuda
+
+        return _cuda.add_rmsnorm(x.value(), residual, norm_w, eps)
+    y, total = C.moe_combine_norm(x.y_perm, x.w, x.dst_row, _c(residual).view(-1, H), norm_w, x.k, float(eps))
+    return y.view(residual.shape), total.view(residual.shape)
+
+
+def moe_ffn_rows(x, w13, w2, topk_w, topk_idx, expert_offset: int = 0):
+    """`moe_ffn` without its last kernel (`Combine`) where the rows that follow are those of `combine_add_rmsnorm`, else its value."""
+    T, k = topk_idx.shape
+    E = w13.shape[0]
+    if (x.dtype != BF16 or torch.is_grad_enabled() or transformed() or T < 64 or x.dim() != 2 or x.shape[1] not in (1024, 2048, 4096)
+            or few_token_experts(x, w13, T, k) or all_token_experts(x, w13, w2, T, k) or small_moe_bt(T * k, E, w13, w2) != 128):
+        return moe_ffn(x, w13, w2, topk_w, topk_idx, expert_offset)
+    x = _c(x)
+    max_rows = moe_max_rows(T * k, E)
+    seg, tile, row_src, dst_row = C.moe_align(_c(topk_idx.to(torch.int32)).view(-1), E, expert_offset, max_rows, None, 128, False)
+    x_perm = torch.empty(max_rows, x.shape[1], dtype=x.dtype, device=x.device)
+    publish_limit(LIMIT_MOE_PAIRS, T * k)
+    C.moe_gather(x, x_perm, row_src, seg, k)
+    _, y_perm = experts_forward(x_perm, w13, w2, seg, tile, keep=False)
+    return Combine(y_perm, _c(topk_w.float()), dst_row, k, x)
+
+
 def moe_ffn(x, w13, w2, topk_w, topk_idx, expert_offset: int = 0, values: bool = True):
     """`values` False: the result is not read, it only stands in the graph."""
     if x.dtype != BF16:

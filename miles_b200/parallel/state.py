@@ -254,9 +254,10 @@ class ParallelState:
         from . import tp
         return tp.all_gather_last_dim(x, self)
 
-    def moe_ffn(self, x, w13, w2, topk_w, topk_idx, num_experts, values=True):
+    def moe_ffn(self, x, w13, w2, topk_w, topk_idx, num_experts, values=True, rows=False):
+        """`rows`: the experts' rows may come back instead of their weighted sums (`ops.moe_ffn_rows`)."""
         if self.ep_size == 1:
-            return ops.moe_ffn(x, w13, w2, topk_w, topk_idx, values)
+            return ops.moe_ffn_rows(x, w13, w2, topk_w, topk_idx) if rows else ops.moe_ffn(x, w13, w2, topk_w, topk_idx, values)
         from . import ep
         return ep.expert_parallel_ffn(x, w13, w2, topk_w, topk_idx, num_experts, self)
 
