@@ -265,6 +265,17 @@ void kv_cache_write(const at::Tensor& k, const at::Tensor& v, at::Tensor& kc, at
         "mb_kv_cache_write");
 }
 
+// k, v [n, Hkv, D]: rows `slots` (int64) of caches [blocks, block size, Hkv, D], all bf16 and contiguous
+std::tuple<at::Tensor, at::Tensor> kv_gather(const at::Tensor& kc, const at::Tensor& vc, const at::Tensor& slots, at::Tensor& error_flag) {
+  c10::cuda::CUDAGuard g(kc.device());
+  const int64_t n = slots.numel(), row = kc.size(2) * kc.size(3);
+  at::Tensor k = at::empty({n, kc.size(2), kc.size(3)}, kc.options()), v = at::empty_like(k);
+  check(mb_kv_gather(kc.data_ptr(), vc.data_ptr(), reinterpret_cast<const long long*>(slots.data_ptr<int64_t>()), n, kc.size(0) * kc.size(1), row,
+                     k.data_ptr(), v.data_ptr(), error_flag.data_ptr<int>(), cur_stream()),
+        "mb_kv_gather");
+  return {k, v};
+}
+
 void adamw(at::Tensor& master, const at::Tensor& grad, at::Tensor& m, at::Tensor& v, const c10::optional<at::Tensor>& decay_mask,
            const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& param_out, double lr, double b1, double b2,
            double eps, double wd, int64_t step) {
@@ -312,6 +323,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("qk_norm_rope_bwd", &qk_norm_rope_bwd);
   m.def("qk_norm_rope_cache", &qk_norm_rope_cache);
   m.def("kv_cache_write", &kv_cache_write);
+  m.def("kv_gather", &kv_gather);
   m.def("adamw", &adamw);
 #endif
   register_more(m);

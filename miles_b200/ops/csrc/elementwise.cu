@@ -865,6 +865,48 @@ __global__ void __launch_bounds__(256) kv_cache_write_kernel(const __nv_bfloat16
 }
 
 // ---------------------------------------------------------------------------------------------
+// Rows of a paged cache, keys and values of every slot in one launch: cache[slots[t], Hkv·D] → k, v [n, Hkv·D].  A warp has four slots, whose eight pieces
+// of 16 bytes per lane are requested together.  A slot outside the cache sets the error flag and gives zeros.  What bounds it: the cache's rows from
+// memory (the copies stay in L2 for the attention behind it).  18 000 slots of 4 heads × 128: from the rotation's end to the
+// attention's start 19 µs with two index_select launches (8.4 + 8.1), 11 with this one.
+// ---------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) kv_gather_kernel(const __nv_bfloat16* kc, const __nv_bfloat16* vc, const long long* slots, long long n,
+                                                        long long n_slots, int row_elems, __nv_bfloat16* k, __nv_bfloat16* v, int* error_flag) {
+  constexpr int U = 4;
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, nvec = row_elems / 8;
+  const long long t0 = (blockIdx.x * 8ll + (threadIdx.x >> 5)) * U;
+  if (t0 >= n) return;
+  long long at[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    at[u] = t0 + u < n ? slots[t0 + u] : 0;
+    if (at[u] < 0 || at[u] >= n_slots) {
+      if (lane == 0) atomicCAS(error_flag, 0, 73);
+      at[u] = -1;
+    }
+  }
+  for (int c = lane; c < nvec; c += 32) {
+    uint4 kr[U], vr[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      kr[u] = vr[u] = make_uint4(0, 0, 0, 0);
+      if (t0 + u < n && at[u] >= 0) {
+        kr[u] = *reinterpret_cast<const uint4*>(kc + at[u] * row_elems + c * 8);
+        vr[u] = *reinterpret_cast<const uint4*>(vc + at[u] * row_elems + c * 8);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (t0 + u < n) {
+        *reinterpret_cast<uint4*>(k + (t0 + u) * row_elems + c * 8) = kr[u];
+        *reinterpret_cast<uint4*>(v + (t0 + u) * row_elems + c * 8) = vr[u];
+      }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // AdamW on a flat fp32 shard with a per-element decay mask and a device-side gradient scale; writes the
 // updated parameter in bf16 (or fp32) to `param_out`.
 // ---------------------------------------------------------------------------------------------
@@ -1134,6 +1176,17 @@ extern "C" int mb_kv_cache_write(const void* k, const void* v, long long k_strid
       reinterpret_cast<const __nv_bfloat16*>(k), reinterpret_cast<const __nv_bfloat16*>(v), k_stride, v_stride,
       reinterpret_cast<__nv_bfloat16*>(kc), reinterpret_cast<__nv_bfloat16*>(vc), slots, T, row_elems);
   return static_cast<int>(cudaGetLastError());
+}
+
+// See kv_gather_kernel.  kc, vc [n_slots, row_elems] bf16, slots [n]; row_elems a multiple of 8, all 16-byte aligned.
+extern "C" int mb_kv_gather(const void* kc, const void* vc, const long long* slots, long long n, long long n_slots, int row_elems, void* k, void* v,
+                            int* error_flag, cudaStream_t s) {
+  if (n == 0) return 0;
+  if (row_elems % 8) return -1;
+  if ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) return -2;
+  return static_cast<int>(launch_pdl(kv_gather_kernel, dim3(static_cast<unsigned>((n + 31) / 32)), dim3(256), 0, s, reinterpret_cast<const __nv_bfloat16*>(kc),
+                                     reinterpret_cast<const __nv_bfloat16*>(vc), slots, n, n_slots, row_elems, reinterpret_cast<__nv_bfloat16*>(k),
+                                     reinterpret_cast<__nv_bfloat16*>(v), error_flag));
 }
 
 extern "C" int mb_adamw(float* master, const float* grad, float* m, float* v, const float* decay_mask, const float* scale_ptr,

@@ -92,6 +92,8 @@ int mb_qk_norm_rope_bwd(const void* x, long long x_stride, const void* w, const 
                         cudaStream_t s);
 int mb_kv_cache_write(const void* k, const void* v, long long k_stride, long long v_stride, void* kc, void* vc,
                       const long long* slots, long long T, int row_elems, cudaStream_t s);
+int mb_kv_gather(const void* kc, const void* vc, const long long* slots, long long n, long long n_slots, int row_elems, void* k, void* v,
+                 int* error_flag, cudaStream_t s);
 int mb_adamw(float* master, const float* grad, float* m, float* v, const float* decay_mask, const float* scale_ptr, void* param_out,
              int out_bf16, long long n, float lr, float b1, float b2, float eps, float wd, int step, cudaStream_t s);
 

@@ -134,8 +134,8 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* logits, f
 // this one 4.4 to 4.6.
 static constexpr int kRouterWarps = 16, kRouterMaxH = 4096;
 
-__global__ void __launch_bounds__(kRouterWarps * 32) norm_router_kernel(const bf16* x, const bf16* residual, const bf16* __restrict__ norm_w,
-                                                                        const bf16* __restrict__ W, float eps, int H, int E, int K, int normalize, int static_w,
+__global__ void __launch_bounds__(kRouterWarps * 32) norm_router_kernel(const bf16* x, const bf16* residual, const bf16* norm_w,
+                                                                        const bf16* W, float eps, int H, int E, int K, int normalize, int static_w,
                                                                         bf16* sum, bf16* normed, float* topk_w, int* topk_idx) {
   constexpr int kPieces = kRouterMaxH / 256;              // 16-byte pieces of a router row per lane
   __shared__ __align__(16) float hs[kRouterMaxH];         // h · norm_w

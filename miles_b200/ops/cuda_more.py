@@ -87,11 +87,16 @@ def extend_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens, extend=
         cu_q = torch.tensor([0] + list(torch.tensor(ql).cumsum(0).tolist()), dtype=torch.int32, device=q.device)
         cu_k = torch.tensor([0] + list(torch.tensor(sl).cumsum(0).tolist()), dtype=torch.int32, device=q.device)
         extend = {"cu_q": cu_q, "cu_k": cu_k, "kv_slots": torch.tensor(slots, dtype=torch.int64, device=q.device), "max_k": max(sl)}
-    kk = k_cache.view(-1, Hkv, D).index_select(0, extend["kv_slots"])
-    vv = v_cache.view(-1, Hkv, D).index_select(0, extend["kv_slots"])
     max_q = int(q_lens.max().item()) if "max_q" not in extend else extend["max_q"]
     if q.dtype != BF16 or D != 128 or not USE_TC_ATTENTION:
         return ref.paged_attention(q, k_cache, v_cache, block_table, seq_lens, q_lens=q_lens)
+    slots = extend["kv_slots"]
+    if (k_cache.dtype == v_cache.dtype == BF16 and k_cache.shape == v_cache.shape and k_cache.is_contiguous() and v_cache.is_contiguous()
+            and slots.dtype == torch.int64 and slots.is_contiguous() and k_cache.data_ptr() % 16 == v_cache.data_ptr() % 16 == 0):
+        kk, vv = C.kv_gather(k_cache, v_cache, slots, C.error_flag(q))
+    else:
+        kk = k_cache.view(-1, Hkv, D).index_select(0, slots)
+        vv = v_cache.view(-1, Hkv, D).index_select(0, slots)
     q = _c(q)
     o = torch.empty(T, Hq, D, dtype=q.dtype, device=q.device)
     lse = torch.empty(Hq, T, dtype=torch.float32, device=q.device)
