@@ -363,8 +363,8 @@ class Qwen3Model(nn.Module):
 
     def _hands_on_rows(self, layer) -> bool:
         """Without gradients a plain MoE layer may leave the weighted sum of its experts' rows to the add and norm that follow it."""
-        return (self.has_head and not torch.is_grad_enabled() and _plain(layer) and type(layer.mlp) is MoEFFN and self.ps.tp_size == 1
-                and self.ps.ep_size == 1 and getattr(layer.mlp, "lora", None) is None)
+        return (type(layer) is DecoderLayer and type(layer.mlp) is MoEFFN and self.has_head and not torch.is_grad_enabled() and self.ps.tp_size == 1
+                and self.ps.ep_size == 1 and getattr(layer.mlp, "lora", None) is None and _plain(layer))
 
     def global_name(self, name: str) -> str:
         """Parameter name with the model-wide layer index (a pipeline stage numbers its own layers from 0)."""

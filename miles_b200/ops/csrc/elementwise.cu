@@ -35,8 +35,15 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
   return sh[0];
 }
 
+// Copies are one 16-byte access: the members' own copy operators are 4-byte ones, which the compiler does not always join.
 struct alignas(16) bf16x8 {
   __nv_bfloat162 v[4];
+  bf16x8() = default;
+  __device__ __forceinline__ bf16x8(const bf16x8& o) { *this = o; }
+  __device__ __forceinline__ bf16x8& operator=(const bf16x8& o) {
+    *reinterpret_cast<uint4*>(this) = *reinterpret_cast<const uint4*>(&o);
+    return *this;
+  }
 };
 
 __device__ __forceinline__ void decode8(const bf16x8& t, float (&f)[8]) {
@@ -47,7 +54,10 @@ __device__ __forceinline__ void decode8(const bf16x8& t, float (&f)[8]) {
     f[2 * i + 1] = a.y;
   }
 }
-__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) { decode8(*reinterpret_cast<const bf16x8*>(p), f); }
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
+  const bf16x8 t = *reinterpret_cast<const bf16x8*>(p);
+  decode8(t, f);
+}
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   bf16x8 t;
 #pragma unroll
@@ -59,140 +69,75 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 // RMSNorm forward (optionally fused with the residual add).  H must be a multiple of 8.
 //   ADD: r_new = x + residual (rounded to bf16, written to `res_out`), y = rmsnorm(r_new)·w
 // ---------------------------------------------------------------------------------------------
-template <bool ADD>
+// A CTA of ⌈H / (16·N)⌉ threads, whole warps, per row: each has its N 16-byte pieces of either operand in flight at once and keeps the sum as packed bf16; one
+// barrier.  The number of threads goes by the width alone, so a token's norm does not depend on how many tokens are beside it.  What bounds it: memory.  Few
+// pieces per thread and many small CTAs keep loads, sums and stores of different rows going side by side; a warp per row with all of its pieces, or 256 threads
+// with room for 8192 columns and three barriers, went through them in turn.  With the add, µs before → now (at the memory's speed): 7258 rows of 2048
+// 31.3 → 19.8 (18.1), 17 829 rows of 1024 35.0 → 24.6 (22.3), of 2048 67.8 → 44.6 (44.6), of 2560 85.4 → 55.3 (55.7), of 4096 142 → 87 (89); one, three or
+// four pieces: the same or up to 1 µs slower; with 4-byte accesses (bf16x8) 24.2, 29.3, 54.2, 66.7, 104.
+template <bool ADD, int N>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual,
                                                           const __nv_bfloat16* __restrict__ w, __nv_bfloat16* y,
                                                           __nv_bfloat16* res_out, float* rstd_out, int H,
                                                           float eps) {
-  __shared__ float sh[32];
+  __shared__ float sh[8];
   pdl_trigger();
   pdl_wait();
-  const long long row = blockIdx.x;
-  const __nv_bfloat16* xr = x + row * H;
-  constexpr int MAXI = 4;  // rows up to 256·8·4 = 8192 wide stay in registers
-  bf16x8 raw[MAXI], res[MAXI];   // all of them requested before the first store: to the compiler the sum may lie over either
-  const int nvec = H / 8;
+  const long long at = blockIdx.x * static_cast<long long>(H);
+  const int nvec = H / 8, nt = blockDim.x;
+  bf16x8 v[N], r[N];   // all of them requested before the first store: to the compiler the sum may lie over either
 #pragma unroll
-  for (int it = 0; it < MAXI; ++it) {
-    const int v = threadIdx.x + it * 256;
-    if (v < nvec) {
-      raw[it] = *reinterpret_cast<const bf16x8*>(xr + v * 8);
-      if (ADD) res[it] = *reinterpret_cast<const bf16x8*>(residual + row * H + v * 8);
-    }
-  }
-  float vals[MAXI][8];
-  float ss = 0.f;
-#pragma unroll
-  for (int it = 0; it < MAXI; ++it) {
-    const int v = threadIdx.x + it * 256;
-    if (v < nvec) {
-      decode8(raw[it], vals[it]);
-      if (ADD) {
-        float r[8];
-        decode8(res[it], r);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) vals[it][i] = __bfloat162float(__float2bfloat16(vals[it][i] + r[i]));
-        store8(res_out + row * H + v * 8, vals[it]);
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) ss += vals[it][i] * vals[it][i];
-    }
-  }
-  for (int v = threadIdx.x + MAXI * 256; v < nvec; v += 256) {  // very wide rows: second read comes from L2
-    float t[8];
-    load8(xr + v * 8, t);
-    if (ADD) {
-      float r[8];
-      load8(residual + row * H + v * 8, r);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) t[i] = __bfloat162float(__float2bfloat16(t[i] + r[i]));
-      store8(res_out + row * H + v * 8, t);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) ss += t[i] * t[i];
-  }
-  ss = block_sum<256>(ss, sh);
-  const float rstd = rsqrtf(ss / H + eps);
-  if (threadIdx.x == 0 && rstd_out != nullptr) rstd_out[row] = rstd;
-#pragma unroll
-  for (int it = 0; it < MAXI; ++it) {
-    const int v = threadIdx.x + it * 256;
-    if (v < nvec) {
-      float wv[8], o[8];
-      load8(w + v * 8, wv);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = vals[it][i] * rstd * wv[i];
-      store8(y + row * H + v * 8, o);
-    }
-  }
-  for (int v = threadIdx.x + MAXI * 256; v < nvec; v += 256) {
-    float t[8], wv[8], o[8];
-    load8((ADD ? res_out : x) + row * H + v * 8, t);
-    load8(w + v * 8, wv);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = t[i] * rstd * wv[i];
-    store8(y + row * H + v * 8, o);
-  }
-}
-
-// The same op with one WARP per row, for rows of 256·VPL elements (VPL 16-byte vectors per lane): every lane has all of its
-// loads in flight at once (2·VPL·16 bytes), the row sum needs shuffles only — no shared memory, no CTA barrier — and the
-// post-add values wait in registers as packed bf16.  Eight rows per CTA.
-template <bool ADD, int VPL>
-__global__ void __launch_bounds__(256) rmsnorm_fwd_warp_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual,
-                                                               const __nv_bfloat16* __restrict__ w, __nv_bfloat16* y,
-                                                               __nv_bfloat16* res_out, float* rstd_out,
-                                                               long long T, float eps) {
-  pdl_trigger();
-  pdl_wait();
-  constexpr int H = VPL * 256;
-  const int lane = threadIdx.x & 31;
-  const long long row = blockIdx.x * 8ll + (threadIdx.x >> 5);
-  if (row >= T) return;
-  const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * H);
-  bf16x8 v[VPL];
-#pragma unroll
-  for (int i = 0; i < VPL; ++i) v[i] = xr[lane + 32 * i];
-  if (ADD) {
-    const bf16x8* rr = reinterpret_cast<const bf16x8*>(residual + row * H);
-    bf16x8 r[VPL];
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) r[i] = rr[lane + 32 * i];
-    bf16x8* ro = reinterpret_cast<bf16x8*>(res_out + row * H);
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 a = __bfloat1622float2(v[i].v[j]), b = __bfloat1622float2(r[i].v[j]);
-        v[i].v[j] = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
-      }
-      ro[lane + 32 * i] = v[i];
+  for (int i = 0; i < N; ++i) {
+    const int c = threadIdx.x + nt * i;
+    if (c < nvec) {
+      v[i] = *reinterpret_cast<const bf16x8*>(x + at + c * 8);
+      if (ADD) r[i] = *reinterpret_cast<const bf16x8*>(residual + at + c * 8);
     }
   }
   float ss = 0.f;
-#pragma unroll
-  for (int i = 0; i < VPL; ++i)
+  auto take = [&](bf16x8& a, const bf16x8& b, int c) {   // a += b, stored; its squares
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float2 a = __bfloat1622float2(v[i].v[j]);
-      ss += a.x * a.x + a.y * a.y;
+      if (ADD) {
+        const float2 p = __bfloat1622float2(a.v[j]), q = __bfloat1622float2(b.v[j]);
+        a.v[j] = __floats2bfloat162_rn(p.x + q.x, p.y + q.y);
+      }
+      const float2 f = __bfloat1622float2(a.v[j]);
+      ss += f.x * f.x + f.y * f.y;
     }
-  ss = warp_sum(ss);
-  const float rstd = rsqrtf(ss / H + eps);
-  if (lane == 0 && rstd_out != nullptr) rstd_out[row] = rstd;
-  const bf16x8* wr = reinterpret_cast<const bf16x8*>(w);
-  bf16x8* yr = reinterpret_cast<bf16x8*>(y + row * H);
+    if (ADD) *reinterpret_cast<bf16x8*>(res_out + at + c * 8) = a;
+  };
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    const bf16x8 wv = wr[lane + 32 * i];
+  for (int i = 0; i < N; ++i)
+    if (threadIdx.x + nt * i < nvec) take(v[i], r[i], threadIdx.x + nt * i);
+  for (int c = threadIdx.x + N * nt; c < nvec; c += nt) {   // rows beyond 8192 columns: read again from L2
+    bf16x8 a = *reinterpret_cast<const bf16x8*>(x + at + c * 8), b = a;
+    if (ADD) b = *reinterpret_cast<const bf16x8*>(residual + at + c * 8);
+    take(a, b, c);
+  }
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (i < nt / 32) ss += sh[i];
+  const float rstd = rsqrtf(ss / H + eps);
+  if (threadIdx.x == 0 && rstd_out != nullptr) rstd_out[blockIdx.x] = rstd;
+  auto put = [&](const bf16x8& a, int c) {
+    const bf16x8 wv = *reinterpret_cast<const bf16x8*>(w + c * 8);
     bf16x8 o;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float2 a = __bfloat1622float2(v[i].v[j]), b = __bfloat1622float2(wv.v[j]);
-      o.v[j] = __floats2bfloat162_rn(a.x * rstd * b.x, a.y * rstd * b.y);
+      const float2 f = __bfloat1622float2(a.v[j]), g = __bfloat1622float2(wv.v[j]);
+      o.v[j] = __floats2bfloat162_rn(f.x * rstd * g.x, f.y * rstd * g.y);
     }
-    yr[lane + 32 * i] = o;
-  }
+    *reinterpret_cast<bf16x8*>(y + at + c * 8) = o;
+  };
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (threadIdx.x + nt * i < nvec) put(v[i], threadIdx.x + nt * i);
+  for (int c = threadIdx.x + N * nt; c < nvec; c += nt) put(*reinterpret_cast<const bf16x8*>((ADD ? res_out : x) + at + c * 8), c);
 }
 
 // RMSNorm backward.  x is the normalised input (the post-add residual stream), dy the gradient of y,
@@ -988,30 +933,13 @@ extern "C" int mb_rmsnorm_fwd(const void* x, const void* residual, const void* w
   auto X = reinterpret_cast<const __nv_bfloat16*>(x);
   typedef const __nv_bfloat16* cbf;
   typedef __nv_bfloat16* bf;
-  cudaError_t e;
-  const bool add = residual != nullptr;
-  const dim3 wgrid(static_cast<unsigned>((T + 7) / 8));
-  // rows of 1024 / 2048 / 4096 elements with 16-byte aligned pointers: one warp per row (T ≥ 64 so that the grid fills the SMs).  The other
-  // widths stay with a CTA per row: a warp per row adds the squares up in another order, and there a token's norm does not depend on how many
-  // tokens are beside it (11 791 rows of 2560: 77 µs, a warp per row 70)
-  const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w) |
-                         reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(res_out)) & 15) == 0;
-  if (aligned && T >= 64 && (H == 1024 || H == 2048 || H == 4096)) {
-    auto launch = [&](auto kern) {
-      return launch_pdl(kern, wgrid, dim3(256), 0, s, X, (cbf)residual, (cbf)w, (bf)y, (bf)res_out, rstd, static_cast<long long>(T), eps);
-    };
-    if (H == 1024) e = add ? launch(rmsnorm_fwd_warp_kernel<true, 4>) : launch(rmsnorm_fwd_warp_kernel<false, 4>);
-    else if (H == 2048) e = add ? launch(rmsnorm_fwd_warp_kernel<true, 8>) : launch(rmsnorm_fwd_warp_kernel<false, 8>);
-    else e = add ? launch(rmsnorm_fwd_warp_kernel<true, 16>) : launch(rmsnorm_fwd_warp_kernel<false, 16>);
-    return static_cast<int>(e);
-  }
-  if (residual != nullptr)
-    e = launch_pdl(rmsnorm_fwd_kernel<true>, dim3(static_cast<unsigned>(T)), dim3(256), 0, s, X, (cbf)residual, (cbf)w, (bf)y, (bf)res_out,
-                   rstd, H, eps);
-  else
-    e = launch_pdl(rmsnorm_fwd_kernel<false>, dim3(static_cast<unsigned>(T)), dim3(256), 0, s, X, (cbf) nullptr, (cbf)w, (bf)y,
-                   (bf) nullptr, rstd, H, eps);
-  return static_cast<int>(e);
+  // two pieces per thread up to 4096 columns, four up to 8192 (and beyond, where the rest is read twice)
+  const int pieces = H <= 4096 ? 2 : 4, threads = H <= 8192 ? (H / 8 + pieces * 32 - 1) / (pieces * 32) * 32 : 256;
+  auto launch = [&](auto kern) {
+    return static_cast<int>(launch_pdl(kern, dim3(static_cast<unsigned>(T)), dim3(threads), 0, s, X, (cbf)residual, (cbf)w, (bf)y, (bf)res_out, rstd, H, eps));
+  };
+  if (residual != nullptr) return pieces == 2 ? launch(rmsnorm_fwd_kernel<true, 2>) : launch(rmsnorm_fwd_kernel<true, 4>);
+  return pieces == 2 ? launch(rmsnorm_fwd_kernel<false, 2>) : launch(rmsnorm_fwd_kernel<false, 4>);
 }
 
 // dw_partial must hold mb_rmsnorm_bwd_blocks(T) × H floats; dw_out receives the reduced weight gradient.

@@ -491,81 +491,92 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const bf16* y_perm, co
   }
 }
 
-// The same with the residual stream's add and the next RMSNorm behind it, a warp per token of 256·VPL columns: the weighted sum never goes to memory.  Sums and
-// roundings are those of the two kernels it stands for (rmsnorm_fwd_warp_kernel).  What bounds it: the rows of y.  7258 tokens × 8 × 2048: 49 + 32 → 61 µs,
-// 17 829: 112 + 70 → 130 (123 at the memory's speed; 135 with 256 threads a block, 143 with the registers of five blocks).
-template <int VPL>
-__global__ void __launch_bounds__(128, VPL <= 8 ? 4 : 2) moe_combine_norm_kernel(const bf16* y_perm, const float* w, const int* dst_row, const bf16* residual,
-                                                               const bf16* __restrict__ norm_w, bf16* y, bf16* res_out, long long T, int k, float eps) {
-  constexpr int H = VPL * 256;
+// The same with the residual stream's add and the next RMSNorm behind it: the weighted sum never goes to memory.  A CTA per token, whose threads own the
+// columns that rmsnorm_fwd_kernel's own (two pieces each, H ≤ 4096): sums and roundings are those of the two kernels it stands for.  What bounds it: the rows
+// of y.  7258 tokens × 8 × 2048: 49 + 19 → 56 µs, 17 829: 112 + 45 → 129 (123 at the memory's speed; a warp per token 61 and 130).
+__global__ void __launch_bounds__(256) moe_combine_norm_kernel(const bf16* y_perm, const float* w, const int* dst_row, const bf16* residual,
+                                                               const bf16* __restrict__ norm_w, bf16* y, bf16* res_out, int k, int H, float eps) {
+  constexpr int N = 2;
+  __shared__ float sh[8];
   pdl_trigger();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const long long t = blockIdx.x * 4ll + (threadIdx.x >> 5);
-  if (t >= T) return;
-  const uint4* rr = reinterpret_cast<const uint4*>(residual + t * H);
-  uint4 v[VPL];
+  const int lane = threadIdx.x & 31, nvec = H / 8, nt = blockDim.x;
+  const long long t = blockIdx.x;
+  uint4 v[N];
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) v[i] = rr[lane + 32 * i];
-  auto add8 = [](float (&acc)[8], const uint4& raw, float f) {
-    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 x = __bfloat1622float2(p[e]);
-      acc[2 * e] += f * x.x;
-      acc[2 * e + 1] += f * x.y;
-    }
-  };
+  for (int i = 0; i < N; ++i) {
+    const int c = threadIdx.x + nt * i;
+    if (c < nvec) v[i] = reinterpret_cast<const uint4*>(residual + t * H)[c];
+  }
   const int row0 = lane < k ? dst_row[t * k + lane] : -1;              // the first 32 choices; more are read where they are used
   const float w0 = lane < k ? w[t * k + lane] : 0.f;
+  float acc[N][8] = {};
+  for (int j0 = 0; j0 < k; j0 += 8) {
+    uint4 raw[8][N];
+    float wj[8];
+    bool in[8];
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int j0 = 0; j0 < k; j0 += 8) {
-      uint4 raw[8];
-      float wj[8];
-      bool in[8];
+    for (int u = 0; u < 8; ++u) {
+      const int j = j0 + u;
+      int row = __shfl_sync(0xffffffffu, row0, j & 31);
+      wj[u] = __shfl_sync(0xffffffffu, w0, j & 31);
+      if (j >= 32 && j < k) { row = dst_row[t * k + j]; wj[u] = w[t * k + j]; }
+      in[u] = j < k && row >= 0;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int j = j0 + u;
-        int row = __shfl_sync(0xffffffffu, row0, j & 31);
-        wj[u] = __shfl_sync(0xffffffffu, w0, j & 31);
-        if (j >= 32 && j < k) { row = dst_row[t * k + j]; wj[u] = w[t * k + j]; }
-        in[u] = j < k && row >= 0;
-        raw[u] = in[u] ? reinterpret_cast<const uint4*>(y_perm + static_cast<long long>(row) * H)[lane + 32 * i] : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < N; ++i) {
+        const int c = threadIdx.x + nt * i;
+        raw[u][i] = in[u] && c < nvec ? reinterpret_cast<const uint4*>(y_perm + static_cast<long long>(row) * H)[c] : make_uint4(0, 0, 0, 0);
       }
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (in[u]) add8(acc, raw[u], wj[u]);
     }
-    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v[i]);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 a = __bfloat1622float2(__floats2bfloat162_rn(acc[2 * e], acc[2 * e + 1])), b = __bfloat1622float2(h[e]);
-      h[e] = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
-    }
-    reinterpret_cast<uint4*>(res_out + t * H)[lane + 32 * i] = v[i];
+    for (int u = 0; u < 8; ++u)
+      if (in[u])
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&raw[u][i])[e]);
+            acc[i][2 * e] += wj[u] * f.x;
+            acc[i][2 * e + 1] += wj[u] * f.y;
+          }
   }
   float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < VPL; ++i)
+  for (int i = 0; i < N; ++i) {
+    const int c = threadIdx.x + nt * i;
+    if (c < nvec) {
+      __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v[i]);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&v[i])[e]);
-      ss += a.x * a.x + a.y * a.y;
+      for (int e = 0; e < 4; ++e) {
+        const float2 a = __bfloat1622float2(__floats2bfloat162_rn(acc[i][2 * e], acc[i][2 * e + 1])), b = __bfloat1622float2(h[e]);
+        h[e] = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
+        const float2 f = __bfloat1622float2(h[e]);
+        ss += f.x * f.x + f.y * f.y;
+      }
+      reinterpret_cast<uint4*>(res_out + t * H)[c] = v[i];
     }
+  }
   ss = wsum(ss);
+  if (lane == 0) sh[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (i < nt / 32) ss += sh[i];
   const float rstd = rsqrtf(ss / H + eps);
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    const uint4 wv = reinterpret_cast<const uint4*>(norm_w)[lane + 32 * i];
+  for (int i = 0; i < N; ++i) {
+    const int c = threadIdx.x + nt * i;
+    if (c >= nvec) continue;
+    const uint4 wv = reinterpret_cast<const uint4*>(norm_w)[c];
     uint4 o;
+    __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&v[i])[e]), b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&wv)[e]);
-      reinterpret_cast<__nv_bfloat162*>(&o)[e] = __floats2bfloat162_rn(a.x * rstd * b.x, a.y * rstd * b.y);
+      q[e] = __floats2bfloat162_rn(a.x * rstd * b.x, a.y * rstd * b.y);
     }
-    reinterpret_cast<uint4*>(y + t * H)[lane + 32 * i] = o;
+    reinterpret_cast<uint4*>(y + t * H)[c] = o;
   }
 }
 
@@ -771,16 +782,15 @@ extern "C" int mb_moe_glu_bwd(const void* h1, void* act_w, void* dh1, const floa
   return static_cast<int>(cudaGetLastError());
 }
 
-// See moe_combine_norm_kernel: y = rmsnorm(Σ_j w · y_perm rows + residual) · norm_w, res_out the sum; H 1024, 2048 or 4096, all 16-byte aligned.
+// See moe_combine_norm_kernel: y = rmsnorm(Σ_j w · y_perm rows + residual) · norm_w, res_out the sum; H ≤ 4096 and a multiple of 8, all 16-byte aligned.
 extern "C" int mb_moe_combine_norm(const void* y_perm, const float* w, const int* dst_row, const void* residual, const void* norm_w, void* y, void* res_out,
                                    long long T, int k, int H, float eps, cudaStream_t s) {
   if (T == 0) return 0;
-  if (H != 1024 && H != 2048 && H != 4096) return -1;
+  if (H <= 0 || H % 8 || H > 4096) return -1;
   if ((reinterpret_cast<uintptr_t>(y_perm) | reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(norm_w) | reinterpret_cast<uintptr_t>(y) |
        reinterpret_cast<uintptr_t>(res_out)) & 15)
     return -2;
-  auto kern = H == 1024 ? moe_combine_norm_kernel<4> : H == 2048 ? moe_combine_norm_kernel<8> : moe_combine_norm_kernel<16>;
-  return static_cast<int>(launch_pdl(kern, dim3(static_cast<unsigned>((T + 3) / 4)), dim3(128), 0, s, reinterpret_cast<const bf16*>(y_perm), w, dst_row,
-                                     reinterpret_cast<const bf16*>(residual), reinterpret_cast<const bf16*>(norm_w), reinterpret_cast<bf16*>(y),
-                                     reinterpret_cast<bf16*>(res_out), T, k, eps));
+  return static_cast<int>(launch_pdl(moe_combine_norm_kernel, dim3(static_cast<unsigned>(T)), dim3((H / 8 + 63) / 64 * 32), 0, s,
+                                     reinterpret_cast<const bf16*>(y_perm), w, dst_row, reinterpret_cast<const bf16*>(residual),
+                                     reinterpret_cast<const bf16*>(norm_w), reinterpret_cast<bf16*>(y), reinterpret_cast<bf16*>(res_out), k, H, eps));
 }

@@ -505,7 +505,7 @@ def moe_ffn_rows(x, w13, w2, topk_w, topk_idx, expert_offset: int = 0):
     """`moe_ffn` without its last kernel (`Combine`) where the rows that follow are those of `combine_add_rmsnorm`, else its value."""
     T, k = topk_idx.shape
     E = w13.shape[0]
-    if (x.dtype != BF16 or torch.is_grad_enabled() or transformed() or T < 64 or x.dim() != 2 or x.shape[1] not in (1024, 2048, 4096)
+    if (x.dtype != BF16 or torch.is_grad_enabled() or transformed() or T < 64 or x.dim() != 2 or x.shape[1] % 8 or x.shape[1] > 4096
             or few_token_experts(x, w13, T, k) or all_token_experts(x, w13, w2, T, k) or small_moe_bt(T * k, E, w13, w2) != 128):
         return moe_ffn(x, w13, w2, topk_w, topk_idx, expert_offset)
     x = _c(x)

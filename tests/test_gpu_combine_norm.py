@@ -5,7 +5,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("T,E,k,H", [(64, 4, 1, 1024), (129, 16, 8, 2048), (300, 40, 9, 4096), (70, 48, 40, 1024)])
+@pytest.mark.parametrize("T,E,k,H", [(64, 4, 1, 1024), (129, 16, 8, 2048), (300, 40, 9, 4096), (70, 48, 40, 1024), (65, 8, 2, 2560), (64, 8, 3, 520)])
 def test_same_bits(T, E, k, H):
     from miles_b200.ops import cuda as K, cuda_more as M
 

@@ -106,3 +106,27 @@ def test_qk_norm_rope_backward_four_heads_at_a_time(T, heads, offset):
     # one rounding to bf16 each (2^-9), angles of up to 5000 in fp32 (5000 · 2^-24 = 3e-4 of a turn's radius)
     assert ((dx.double() - x64.grad).norm() / x64.grad.norm()).item() < 3e-3
     assert ((dw.double() - w64.grad).norm() / w64.grad.norm()).item() < 5e-3
+
+
+@pytest.mark.parametrize("add", [False, True])
+@pytest.mark.parametrize("H", [8, 264, 512, 520, 1024, 2048, 2560, 4096, 4104, 6152, 8192, 8200, 16392])
+def test_rmsnorm_of_any_width(H, add):
+    """Widths around the edges of its pieces and threads; a row's result does not depend on the rows beside it.  y is rounded to bf16 once behind fp32 sums:
+    half a unit in the last of 8 bits, and the norm's own error (squares and their sum in fp32, rsqrt) far below it."""
+    from miles_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x, r = (torch.randn(70, H, device="cuda", generator=g).bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).bfloat16()
+    x[5, 0], x[6] = float("nan"), 0
+    r[6] = 0
+    with torch.no_grad():
+        run = (lambda s: K.add_rmsnorm(x[s], r[s], w, 1e-6)) if add else (lambda s: (K.rmsnorm(x[s], w, 1e-6), x[s]))
+        y, total = run(slice(0, 70))
+        few, few_total = run(slice(60, 63))
+    h = (x.double() + r.double()).bfloat16() if add else x
+    assert torch.equal(total[[0, 69]], h[[0, 69]])
+    want = h.double() * (h.double().pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt() * w.double()
+    ok = torch.arange(70, device="cuda") != 5
+    assert y[5].isnan().all() and ((y.double() - want)[ok].abs() <= want[ok].abs() * 2.0 ** -8 * 1.01).all()
+    assert torch.equal(few, y[60:63]) and torch.equal(few_total, total[60:63])
