@@ -747,7 +747,7 @@ extern "C" int mb_moe_gather(const void* x, void* x_perm, const int* row_src, co
                              int max_rows, cudaStream_t s) {
   if (max_rows == 0) return 0;
   if (H % 8) return -1;
-  const int blocks = (max_rows + 7) / 8 < 148 * 8 ? (max_rows + 7) / 8 : 148 * 8;
+  const int blocks = (max_rows + 7) / 8;   // a row per warp: 7258 tokens × 8 × 2048 54 → 51 µs, 2163 15.6 → 14.6, 12 075 99 → 96 against 8 CTAs an SM that walk
   return static_cast<int>(launch_pdl(moe_gather_kernel, dim3(blocks), dim3(256), 0, s, reinterpret_cast<const bf16*>(x),
                                      reinterpret_cast<bf16*>(x_perm), row_src, seg_offsets, E, k, H, max_rows));
 }
